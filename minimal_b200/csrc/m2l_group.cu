@@ -664,6 +664,13 @@ __device__ __forceinline__ int tile_at(const int *tg_off, int ntiles, int s) {
 // First segment of CTA c of G when nseg segments are cut into equal ranges.
 __device__ __forceinline__ int range_start(int nseg, int c, int G) { return (int)((long long)nseg * c / G); }
 
+// CTAs that take a range when a grid of G shares nseg segments: all of them,
+// unless that would leave ranges of fewer than SEG_MIN segments, whose fixed
+// cost (start-up, one part of a tile written and added again) outweighs the
+// contraction.
+constexpr int SEG_MIN = 4;
+__device__ __forceinline__ int range_ctas(int nseg, int G) { return max(1, min(G, nseg / SEG_MIN)); }
+
 // MAXP: the plan's pieces per warp (pd.maxp); at GP_MAXP_SMALL the
 // accumulators leave registers for two CTAs per SM.
 template <int MAXP>
@@ -704,9 +711,9 @@ __global__ void __launch_bounds__(GP_WARPS * 32, MAXP == GP_MAXP_SMALL ? 2 : 1)
   // by k_m2l_join, as in k_m2l_tc); else tile blockIdx.x
   int r0, r1, tfirst;
   if (part) {
-    const int nseg = tg_off[ntiles];
-    r0 = range_start(nseg, blockIdx.x, gridDim.x);
-    r1 = range_start(nseg, blockIdx.x + 1, gridDim.x);
+    const int nseg = tg_off[ntiles], G = range_ctas(nseg, gridDim.x), c = min((int)blockIdx.x, G);
+    r0 = range_start(nseg, c, G);  // (CTAs without a range: the empty one at the end)
+    r1 = range_start(nseg, min(c + 1, G), G);
     tfirst = r1 > r0 ? tile_at(tg_off, ntiles, r0) : ntiles;
   } else {
     tfirst = blockIdx.x;
@@ -943,15 +950,17 @@ __device__ __forceinline__ void tc_flush_global(uint32_t acc, int t, double inv,
 
 // PT > 0: the order PT with its plan and stage count as compile-time
 // constants (the run-time arguments are then ignored); PT = 0: any order.
-// Work split of the orders compiled with their plan and a running sum in
-// TMEM ("balanced"): one CTA per SM, each taking an equal contiguous range of
-// the (tile, group) segments -- the tiles hold 182 to 325 segments at 1M
-// uniform bodies, and with two tiles per SM the SM that drew the longest
-// ones set the kernel's time (720 us against 557 us of average SM work).  A
-// CTA stores the tiles that lie wholly in its range; of a tile cut by a
+// Work split of the orders with a running sum in TMEM ("balanced"): one CTA
+// per SM, each taking an equal contiguous range of the (tile, group)
+// segments -- the tiles hold 182 to 325 segments at 1M uniform bodies, and
+// with two tiles per SM the SM that drew the longest ones set the kernel's
+// time (720 us against 557 us of average SM work).  Small trees have fewer
+// tiles than SMs, each a serial chain of a few hundred segments (20,000
+// bodies at P = 6: 5 tiles), so there too the ranges are what fills the GPU.
+// A CTA stores the tiles that lie wholly in its range; of a tile cut by a
 // range boundary it writes its partial sums to `part` (slot 0: its first
 // tile, 1: its last), which k_m2l_join adds in CTA order (deterministic).
-// Otherwise one CTA per tile.
+// Orders whose running sum is L in global memory (P > 12): one CTA per tile.
 template <int PT>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, const int *tg_off, const int *tg_gid,
                                                           const int *tg_src, const unsigned char *ops,
@@ -961,7 +970,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
                                                           const unsigned long long *m16_max, int *err, long wait_ns,
                                                           long stall_ns, int ntiles, double2 *part) {
   constexpr bool FIX = PT > 0;
-  constexpr bool BAL = FIX && TcFixed<PT>::acc.fold != 0;
+  const bool BAL = FIX ? TcFixed<PT>::acc.fold != 0 : part != nullptr;
   const int P = FIX ? PT : P_, KP = FIX ? TcFixed<PT>::KP : KP_, nstage = FIX ? TcFixed<PT>::nstage : nstage_;
   const TcPlan pl = FIX ? TcFixed<PT>::plan : pl_;
   const TcAcc ta = FIX ? TcFixed<PT>::acc : ta_;
@@ -1003,9 +1012,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
   // this CTA's segments [g0, g1) and the first tile they touch
   int g0, g1, tfirst;
   if (BAL) {
-    const int nseg = tg_off[ntiles];
-    g0 = range_start(nseg, blockIdx.x, gridDim.x);
-    g1 = range_start(nseg, blockIdx.x + 1, gridDim.x);
+    const int nseg = tg_off[ntiles], G = range_ctas(nseg, gridDim.x), c = min((int)blockIdx.x, G);
+    g0 = range_start(nseg, c, G);  // (CTAs without a range: the empty one at the end)
+    g1 = range_start(nseg, min(c + 1, G), G);
     tfirst = g1 > g0 ? tile_at(tg_off, ntiles, g0) : 0;
   } else {
     tfirst = blockIdx.x;
@@ -1244,13 +1253,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
 
 // Tiles cut by the balanced ranges of k_m2l_tc / k_gemm64 (tiles of tile_n
 // targets): L of the tile's targets is the sum of the CTAs' parts, added in
-// CTA order.  One CTA per tile; threads run over (target row, coefficient)
-// with the coefficient fastest, so the parts and L are read and written
-// contiguously.
+// CTA order.  A column of CTAs per tile; threads run over (target row,
+// coefficient) with the coefficient fastest, so the parts and L are read and
+// written contiguously.  The work is latency: a tile of a small tree is cut
+// into tens of parts, so its elements are spread over blockIdx.y.
 constexpr int JOIN_T = 256;
-__global__ void __launch_bounds__(JOIN_T) k_m2l_join(const int *tile_tgt, const int *tg_off, int ntiles, int G,
+__global__ void __launch_bounds__(JOIN_T) k_m2l_join(const int *tile_tgt, const int *tg_off, int ntiles, int grid,
                                                      const double2 *part, int NT, int tile_n, double2 *L) {
-  const int t = blockIdx.x, nseg = tg_off[ntiles];
+  const int t = blockIdx.x, nseg = tg_off[ntiles], G = range_ctas(nseg, grid);
   const int a = tg_off[t], b = tg_off[t + 1];
   if (b <= a) return;
   // the CTA whose range holds segment s
@@ -1266,18 +1276,26 @@ __global__ void __launch_bounds__(JOIN_T) k_m2l_join(const int *tile_tgt, const 
   // start inside it; for c0 it is the last (slot 1) unless c0's range
   // starts at the tile
   const int slot0 = range_start(nseg, c0, G) < a ? 1 : 0;
-  for (int e = threadIdx.x; e < tile_n * NT; e += JOIN_T) {
+  const size_t len = (size_t)tile_n * NT;
+  for (int e = blockIdx.y * JOIN_T + threadIdx.x; e < (int)len; e += gridDim.y * JOIN_T) {
     const int row = e / NT, o = e - row * NT, tgt = tile_tgt[t * tile_n + row];
     if (tgt < 0) continue;
-    double2 sum = make_double2(0, 0);
-    for (int c = c0; c <= c1; c++) {
-      const int slot = c == c0 ? slot0 : 0;
-      const double2 v = part[(size_t)(2 * c + slot) * tile_n * NT + e];
+    double2 sum = part[(size_t)(2 * c0 + slot0) * len + e];
+#pragma unroll 4
+    for (int c = c0 + 1; c <= c1; c++) {
+      const double2 v = part[(size_t)(2 * c) * len + e];
       sum.x += v.x;
       sum.y += v.y;
     }
     L[(long)tgt * NT + o] = sum;
   }
+}
+
+// k_m2l_join's grid: about two CTAs per SM in all, at most one per JOIN_T
+// elements of a tile.
+dim3 join_grid(int ntiles, int nsm, int elems) {
+  const int most = (elems + JOIN_T - 1) / JOIN_T;
+  return dim3(ntiles, std::max(1, std::min(most, 2 * nsm / ntiles)));
 }
 
 struct PlanCache {
@@ -1364,14 +1382,15 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
   const long nseg = h.g_nseg;
   int *tg_src = h.g_tg.as<int>(), *tg_gid = tg_src + (size_t)nseg * tile_n, *tg_off = tg_gid + nseg;
   DevCounters *ctr = h.counters.as<DevCounters>();
+  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   if (tcore) {
     FMM_CUDA(cudaMemsetAsync(&ctr->tc_error, 0, sizeof(int), s));
-    // the orders compiled with their plan as constants; those with a running
-    // sum in TMEM take balanced segment ranges, one CTA per SM
+    // orders with a running sum in TMEM (6, 8, 10 and 12, compiled with their
+    // plan, and the others up to 12) take balanced segment ranges, one CTA
+    // per SM
     const bool fixed = P == 6 || P == 8 || P == 10 || P == 12;
-    const bool bal = fixed && tc_acc_fixed(KP16, tp).fold != 0;
-    if (bal && h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
-    const int G = bal ? std::min(ntiles, h.nsm) : ntiles, NT = tri(P);
+    const bool bal = (fixed ? tc_acc_fixed(KP16, tp) : tc_acc_layout(KP16)).fold != 0;
+    const int G = bal ? h.nsm : ntiles, NT = tri(P);
     if (bal) h.g_part.need((size_t)G * 2 * TC_TILE * NT * sizeof(double2));
     double2 *part = bal ? h.g_part.as<double2>() : nullptr;
     auto launch = [&](auto kern) {
@@ -1388,8 +1407,8 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
       default: launch(k_m2l_tc<0>);
     }
     if (bal) {
-      k_m2l_join<<<ntiles, JOIN_T, 0, s>>>(h.g_tile.as<int>(), tg_off, ntiles, G, part, NT, TC_TILE,
-                                          h.L.as<double2>());
+      k_m2l_join<<<join_grid(ntiles, h.nsm, TC_TILE * NT), JOIN_T, 0, s>>>(h.g_tile.as<int>(), tg_off, ntiles, G, part,
+                                                                          NT, TC_TILE, h.L.as<double2>());
       h.launches++;
     }
     h.tc_stall_ns = 0;  // the test hook stalls one launch
@@ -1399,8 +1418,9 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
     // two pipeline stages where they fit in shared memory (P <= 12), else
     // one.  P <= 11: equal segment ranges over as many CTAs as fit on the GPU
     // at once (at 1M uniform bodies 7.82 -> 7.29 ms per evaluation at P = 8,
-    // 9.03 -> 8.47 at P = 10, 9.69 -> 9.35 at P = 11); above, one CTA per
-    // tile (P = 12, two one-stage CTAs per SM: 9.69 against 9.78 ms with the
+    // 9.03 -> 8.47 at P = 10, 9.69 -> 9.35 at P = 11), and at every order
+    // while the tiles alone do not fill the GPU; above, one CTA per tile
+    // (P = 12, two one-stage CTAs per SM: 9.69 against 9.78 ms with the
     // ranges)
     auto kern = gp.maxp == GP_MAXP_SMALL ? k_gemm64<GP_MAXP_SMALL> : k_gemm64<GP_MAXP>;
     int nst = gemm64_smem(gp, 2) <= TC_SMEM_MAX ? 2 : 1;
@@ -1411,15 +1431,15 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
       if (occ1 >= 2 * occ2) nst = 1;
     }
     const size_t smem = gemm64_smem(gp, nst);
-    const bool bal = P <= 11;
+    int occ = 1;
+    FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, GP_WARPS * 32, smem));
+    const int slots = h.nsm * std::max(occ, 1);
+    const bool bal = P <= 11 || ntiles < slots;
     int G = ntiles;
     const int NT = tri(P);
     double2 *part = nullptr;
     if (bal) {
-      int occ = 1;
-      FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, GP_WARPS * 32, smem));
-      if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
-      G = std::max(1, std::min(ntiles, h.nsm * std::max(occ, 1)));
+      G = slots;
       h.g_part.need((size_t)G * 2 * GP_TILE * NT * sizeof(double2));
       part = h.g_part.as<double2>();
     }
@@ -1427,8 +1447,8 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
                                         h.g_mt.as<double>(), h.c_xr.as<double4>(), h.L.as<double2>(), pd, nst, ntiles,
                                         part);
     if (bal) {
-      k_m2l_join<<<ntiles, JOIN_T, 0, s>>>(h.g_tile.as<int>(), tg_off, ntiles, G, part, NT, GP_TILE,
-                                          h.L.as<double2>());
+      k_m2l_join<<<join_grid(ntiles, h.nsm, GP_TILE * NT), JOIN_T, 0, s>>>(h.g_tile.as<int>(), tg_off, ntiles, G, part,
+                                                                          NT, GP_TILE, h.L.as<double2>());
       h.launches++;
     }
   }
