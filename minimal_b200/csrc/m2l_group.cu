@@ -690,17 +690,16 @@ __global__ void __launch_bounds__(GP_WARPS * 32, MAXP == GP_MAXP_SMALL ? 2 : 1)
   const int KPAD = gp_kpad(KP);
   const size_t sstride = (size_t)pd.wsize + (size_t)GP_TILE * KPAD;  // doubles per stage (even: 16-byte rows)
   const int ar = lane >> 2, ak = lane & 3;
-  // group g's operator and its 32 gathered multipoles into stage b, as
-  // asynchronous copies (absent targets: zeros).  The multipoles stay in
-  // rows (target-major, X[col][k]): each source row, KP contiguous doubles,
-  // is copied in 16-byte chunks by 8 threads (thread t: row t / 8, chunks
-  // t % 8, t % 8 + 8, ...), one index load per row.
+  // a group's operator (slot gid) and its 32 gathered multipoles into stage
+  // b, as asynchronous copies (absent targets, s < 0: zeros).  The
+  // multipoles stay in rows (target-major, X[col][k]): each source row, KP
+  // contiguous doubles, is copied in 16-byte chunks by 8 threads (thread t:
+  // row t / 8, chunks t % 8, t % 8 + 8, ...), one index load per row.
   const int xcol = tid >> 3, xpart = tid & 7;
-  auto issue = [&](int g, int b) {
+  auto issue = [&](int s, int gid, int b) {
     double *Wd = smd + (size_t)b * sstride, *Xd = Wd + pd.wsize;
-    const double *Wg = ops + (size_t)tg_gid[g] * pd.wsize;
+    const double *Wg = ops + (size_t)gid * pd.wsize;
     for (int i = tid; i < pd.wsize / 2; i += blockDim.x) tc::cp_async16(Wd + 2 * i, Wg + 2 * i, 16u);
-    const int s = tg_src[(long)g * GP_TILE + xcol];
     const double *src = Mt + (long)(s >= 0 ? s : 0) * KP;
     double *dst = Xd + xcol * KPAD;
     for (int c = xpart; c < KP / 2; c += 8) tc::cp_async16(dst + 2 * c, src + 2 * c, s >= 0 ? 16u : 0u);
@@ -728,26 +727,44 @@ __global__ void __launch_bounds__(GP_WARPS * 32, MAXP == GP_MAXP_SMALL ? 2 : 1)
   for (int p = 0; p < MAXP; p++)
 #pragma unroll
     for (int cb = 0; cb < 4; cb++) acc[p][cb][0] = acc[p][cb][1] = 0;
-  if (nstage == 2) issue(g0, 0);
+  // Two stages, one barrier per group: past the barrier every warp has
+  // finished group g - 1, so the next group's copies go into its stage and
+  // run under the contraction of group g.  Their source row and operator
+  // slot were loaded a group earlier: loaded here, each group began with a
+  // wait of an L2 round trip.  (1M uniform bodies, P = 10, the kernel alone:
+  // 2171 -> 2044 us against two barriers and late index loads; the DMMA
+  // flops it executes take 1400 us at the FP64 peak.)
+  int s_next = tg_src[(long)g0 * GP_TILE + xcol], gid_next = tg_gid[g0];
+  auto prefetch = [&](int g) {
+    if (g < g1) {
+      s_next = tg_src[(long)g * GP_TILE + xcol];
+      gid_next = tg_gid[g];
+    }
+  };
+  if (nstage == 2) {
+    issue(s_next, gid_next, 0);
+    prefetch(g0 + 1);
+  }
   for (int g = g0; g < g1; g++) {
-    // two stages: the next group's copies run while this one is contracted
     const int b = nstage == 2 ? (g - g0) & 1 : 0;
     if (nstage != 2) {
-      issue(g, 0);
-      tc::cp_async_wait_all();
-    } else if (g + 1 < g1) {
-      issue(g + 1, b ^ 1);
-      tc::cp_async_wait_1();
-    } else {
-      tc::cp_async_wait_all();
+      __syncthreads();  // group g - 1 is done with the stage
+      issue(s_next, gid_next, 0);
+      prefetch(g + 1);
     }
+    tc::cp_async_wait_all();
     __syncthreads();
+    if (nstage == 2 && g + 1 < g1) {
+      issue(s_next, gid_next, b ^ 1);
+      prefetch(g + 2);
+    }
     const double *Wsm = smd + (size_t)b * sstride, *Xsm = Wsm + pd.wsize;
 #pragma unroll
     for (int p = 0; p < MAXP; p++) {
       if (pc[p] < 0) continue;
       const int k0 = (pc[p] >> 8) & 4095, k1 = pc[p] >> 20;
       const double *Wb = Wsm + wo[p];
+#pragma unroll 4  // 2044 -> 1911 us (unrolled by 2: 1956, by 7: 1986; pairs of k steps from 16-byte loads: 2004-2061)
       for (int k = k0; k < k1; k += 4) {
         const double a = Wb[(k + ak) * 8 + ar];
         const double *xb = Xsm + ar * KPAD + k + ak;
@@ -755,7 +772,6 @@ __global__ void __launch_bounds__(GP_WARPS * 32, MAXP == GP_MAXP_SMALL ? 2 : 1)
         for (int cb = 0; cb < 4; cb++) dmma(acc[p][cb][0], acc[p][cb][1], a, xb[cb * 8 * KPAD]);
       }
     }
-    __syncthreads();  // stage b is free for group g + 2
   }
   // reduce the pieces into Y[row][col] (rank 0 stores, higher ranks add)
   double *Y = smd;
