@@ -29,6 +29,7 @@
 #include <mutex>
 
 #include "fmm.cuh"
+#include "pair64.cuh"
 
 namespace {
 
@@ -69,17 +70,17 @@ __global__ void __launch_bounds__(DT) k_ds_sum(const double4 *xq, long nt, const
       }
       __syncthreads();
       const int m = (int)min((long)DT, s1 - b);
-      for (int k = 0; k < m; k++) {
-        const double4 s = tile[k];
-        const double dx = T.x - s.x, dy = T.y - s.y, dz = T.z - s.z;
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        const double ir = r2 > 0 ? rsqrt(r2) : 0.0;  // zero distance skipped (3d/kernel.h:135)
-        const double qir = s.w * ir, qir3 = qir * ir * ir;
-        p += qir;
-        ax += dx * qir3;
-        ay += dy * qir3;
-        az += dz * qir3;
+      double tp = 0, fx = 0, fy = 0, fz = 0;
+#pragma unroll 8
+      for (int k = 0; k < m; k++) fmm::pair_normal(T.x, T.y, T.z, tile[k], tp, fx, fy, fz);
+      if (!isfinite(tp)) {  // a target among the sources: the pairs at distance zero count nothing (3d/kernel.h:135)
+        tp = fx = fy = fz = 0;
+        for (int k = 0; k < m; k++) fmm::pair(T.x, T.y, T.z, tile[k], tp, fx, fy, fz);
       }
+      p += tp;
+      ax += fx;
+      ay += fy;
+      az += fz;
     }
   }
   if (i < nt) {

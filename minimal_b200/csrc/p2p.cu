@@ -11,9 +11,11 @@
 // through a 32-body shared-memory tile (coalesced loads, then a broadcast).
 // Pairs at distance zero are skipped as in the reference.  P2P is the first
 // writer of the outputs, so it stores p and F; L2P adds to them later.
+#include <algorithm>
 #include <type_traits>
 
 #include "fmm.cuh"
+#include "pair64.cuh"
 
 namespace fmm {
 
@@ -22,19 +24,6 @@ namespace {
 constexpr int WARPS = 4;
 constexpr int IMG_SHIFT = 26;
 constexpr u32 IDX_MASK = (1u << IMG_SHIFT) - 1;
-
-__device__ __forceinline__ void pair(double xi, double yi, double zi, const double4 s, double &pot, double &ax,
-                                     double &ay, double &az) {
-  const double dx = xi - s.x, dy = yi - s.y, dz = zi - s.z;
-  const double r2 = dx * dx + dy * dy + dz * dz;
-  const double ir = r2 > 0 ? rsqrt(r2) : 0.0;
-  const double qir = s.w * ir;
-  const double qir3 = qir * ir * ir;
-  pot += qir;
-  ax += dx * qir3;
-  ay += dy * qir3;
-  az += dz * qir3;
-}
 
 __global__ void __launch_bounds__(WARPS * 32) k_p2p(const int *leaves, int nleaves, const int *begin,
                                                     const int *count, const int *off, const u32 *ent,
@@ -79,16 +68,18 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2p(const int *leaves, int nleav
   }
 }
 
-// Direct sum: block = 256 targets x one chunk of sources; partial results
-// are added with FP64 atomics.
+// Direct sum: block = 256 targets x one chunk of sources, staged in tiles;
+// partial results are added with FP64 atomics.  A tile is summed with
+// pair_normal; where that is not finite (a target among the sources, once
+// each) the thread sums the tile again with pair.
 constexpr int DT = 256;
-constexpr int DCHUNK = 8192;
+constexpr long DCHUNK_MIN = 1024;  // sources per chunk at least: below, the atomics count
 
-__global__ void __launch_bounds__(DT) k_direct(const double4 *tgt, long nt, const double4 *src, long ns,
+__global__ void __launch_bounds__(DT) k_direct(const double4 *tgt, long nt, const double4 *src, long ns, long chunk,
                                                double4 *out, int prange, double cycle) {
   __shared__ double4 tile[DT];
   const long i = (long)blockIdx.x * DT + threadIdx.x;
-  const long s0 = (long)blockIdx.y * DCHUNK, s1 = min(ns, s0 + DCHUNK);
+  const long s0 = (long)blockIdx.y * chunk, s1 = min(ns, s0 + chunk);
   const double4 T = i < nt ? tgt[i] : make_double4(0, 0, 0, 0);
   double p = 0, ax = 0, ay = 0, az = 0;
   for (long b = s0; b < s1; b += DT) {
@@ -100,7 +91,17 @@ __global__ void __launch_bounds__(DT) k_direct(const double4 *tgt, long nt, cons
       for (int iy = -prange; iy <= prange; iy++)
         for (int iz = -prange; iz <= prange; iz++) {
           const double tx = T.x - ix * cycle, ty = T.y - iy * cycle, tz = T.z - iz * cycle;
-          for (int k = 0; k < m; k++) pair(tx, ty, tz, tile[k], p, ax, ay, az);
+          double tp = 0, fx = 0, fy = 0, fz = 0;
+#pragma unroll 8
+          for (int k = 0; k < m; k++) pair_normal(tx, ty, tz, tile[k], tp, fx, fy, fz);
+          if (!isfinite(tp)) {
+            tp = fx = fy = fz = 0;
+            for (int k = 0; k < m; k++) pair(tx, ty, tz, tile[k], tp, fx, fy, fz);
+          }
+          p += tp;
+          ax += fx;
+          ay += fy;
+          az += fz;
         }
   }
   if (i < nt) {
@@ -157,20 +158,11 @@ __device__ __forceinline__ float rsqrt_or_zero(float r2) {
 // for |q| < 2^32.
 constexpr float NEAR_TINY = 5.421010862427522e-20f;  // 2^-64
 
-// CHECK: pairs at distance zero contribute nothing (3d/kernel.h:131); the
-// unchecked form serves source leaves other than the target's own, where a
-// zero offset can only come from FP32 rounding.
-template <bool CHECK = true>
+// Pairs at distance zero contribute nothing (3d/kernel.h:131).
 __device__ __forceinline__ void pair_f32(float xi, float yi, float zi, const float4 s, float &pot, float &ax,
                                          float &ay, float &az) {
   const float dx = xi - s.x, dy = yi - s.y, dz = zi - s.z;
-  float ir;
-  if constexpr (CHECK) {
-    ir = rsqrt_or_zero(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
-  } else {
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, NEAR_TINY)));
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ir) : "f"(r2));
-  }
+  const float ir = rsqrt_or_zero(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
   const float qir = s.w * ir;
   const float qir3 = qir * ir * ir;
   pot += qir;
@@ -221,7 +213,9 @@ constexpr float NEAR_DUMMY = 1e15f;
 
 // One target (X, Y, Z = the coordinate in both lanes) against a staged
 // source pair (sx, sy from the first slot, sz, sq from the second); the same
-// arithmetic as pair_f32 in each lane.
+// arithmetic as pair_f32 in each lane.  CHECK false serves source leaves
+// other than the target's own, where a zero offset can only come from FP32
+// rounding.
 template <bool CHECK>
 __device__ __forceinline__ void pair_x2(f2x X, f2x Y, f2x Z, f2x sx, f2x sy, f2x sz, f2x sq, f2x &pot, f2x &ax,
                                         f2x &ay, f2x &az) {
@@ -327,12 +321,13 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2p_f32(const int *leaves, int n
 // always holds it: the acceptance test never accepts a cell with itself) go
 // first, in slots [0, tn) of the first chunk, and only they are swept with
 // the zero-distance check; every group takes its share of both parts, so the
-// warps stay converged.  FP64 form: list order, every pair checked.
+// warps stay converged.  FP64 form: likewise the target leaf first, its pairs
+// with the zero-distance check (pair), the others without (pair_normal).
 constexpr int CT = 128;           // threads per CTA
 // bodies staged at once (the source tile): a template parameter, chosen at
 // run time among 1024, 1536 and 2048 (exafmm_b200_set_tile / the
 // autotuner); the defaults, FP32 1536 (7 CTAs per SM, register-bound) and
-// FP64 1024 (5 CTAs per SM), were tuned on B200 at 1M uniform bodies
+// FP64 1024 (4 CTAs per SM), were tuned on B200 at 1M uniform bodies
 template <bool F32>
 constexpr int ct_cap() { return F32 ? 1536 : 1024; }
 constexpr int CT_MAXTGT = 256;    // target-leaf bodies: two per thread
@@ -356,7 +351,7 @@ struct NearBody<true> {
 };
 
 template <bool F32, int CAP>
-__global__ void __launch_bounds__(CT, F32 ? 7 : 5) k_p2p_cta(const int *leaves, const int *begin, const int *count,
+__global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, const int *begin, const int *count,
                                                 const int *off, const u32 *ent, const double4 *xr,
                                                 const typename NearBody<F32>::T *bodies, double4 *out,
                                                 double cycle) {
@@ -402,9 +397,9 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 5) k_p2p_cta(const int *leaves, 
 #pragma unroll
     for (int q = 0; q < 4; q++) sacc[u][q] = eacc[u][q] = 0;
   const int eb = off[c], ee = off[c + 1];
-  // slots [0, pre) of the first chunk: the target leaf itself (FP32), padded
-  // to an even count (the FP32 stage holds sources in pairs)
-  int pre = F32 ? tn + (tn & 1) : 0;
+  // slots [0, pre) of the first chunk: the target leaf itself, padded to an
+  // even count in the FP32 form (whose stage holds sources in pairs)
+  int pre = F32 ? tn + (tn & 1) : tn;
   for (int e0i = eb; e0i < ee;) {
     // lane k: source leaf k of the chunk candidates
     const int cand = min(32, ee - e0i);
@@ -412,17 +407,16 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 5) k_p2p_cta(const int *leaves, 
     // target leaf's, scaled; FP64: absolute positions, shifted by the
     // periodic image `img` (the shift is formed per body from it)
     int n = 0, base = 0, img = 13;
-    bool self = false;  // FP32: the target leaf's own entry (staged first, so here of size 0)
+    bool self = false;  // the target leaf's own entry (staged first, so here of size 0)
     float ox = 0, oy = 0, oz = 0;
     if (lane < cand) {
       const u32 en = ent[e0i + lane];
       const int sc = (int)(en & IDX_MASK);
       img = (int)(en >> IMG_SHIFT);
-      n = count[sc];
+      self = sc == c && img == 13;
+      n = self ? 0 : count[sc];
       base = begin[sc];
       if constexpr (F32) {
-        self = sc == c && img == 13;
-        if (self) n = 0;
         const double sx = (img % 3 - 1) * cycle, sy = ((img / 3) % 3 - 1) * cycle, sz = (img / 9 - 1) * cycle;
         const double4 CB = xr[sc];
         ox = (float)(CA.x - CB.x - sx) * scale;  // exact: scale is a power of two
@@ -463,6 +457,8 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 5) k_p2p_cta(const int *leaves, 
         stage[2 * pp] = make_float4(a.x, b.x, a.y, b.y);
         stage[2 * pp + 1] = make_float4(a.z, b.z, a.w, b.w);
       }
+    } else {
+      for (int j = tid; j < pre; j += CT) stage[j] = bodies[tb + j];
     }
     for (int j0 = pre + wid * 32; j0 < T; j0 += CT * CT_UNROLL) {
       BT v[CT_UNROLL];
@@ -519,47 +515,6 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 5) k_p2p_cta(const int *leaves, 
     }
     __syncthreads();
     if (act) {
-      // FP64: a slot range, CT_BLOCK sources at a time, four per iteration
-      auto sweep = [&](int from, int to, auto check) {
-        constexpr bool CHECK = decltype(check)::value;
-        const BT *sp = stage + from;
-        for (int c0 = from; c0 < to; c0 += CT_BLOCK) {
-          RT p[CT_TPT][4];
-#pragma unroll
-          for (int u = 0; u < CT_TPT; u++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) p[u][q] = 0;
-          const int cend = min(to, c0 + CT_BLOCK);
-          int cs = c0;
-          auto acc = [&](const BT &sv) {
-#pragma unroll
-            for (int u = 0; u < CT_TPT; u++) {
-              if constexpr (F32) pair_f32<CHECK>(A[u].x, A[u].y, A[u].z, sv, p[u][0], p[u][1], p[u][2], p[u][3]);
-              else pair(A[u].x, A[u].y, A[u].z, sv, p[u][0], p[u][1], p[u][2], p[u][3]);
-            }
-          };
-          for (; cs + 4 <= cend; cs += 4) {
-            const BT s0 = sp[0], s1 = sp[1], s2 = sp[2], s3 = sp[3];
-            sp += 4;
-            acc(s0);
-            acc(s1);
-            acc(s2);
-            acc(s3);
-          }
-          for (; cs < cend; cs++) {
-            const BT s0 = sp[0];
-            sp += 1;
-            acc(s0);
-          }
-#pragma unroll
-          for (int u = 0; u < CT_TPT; u++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-              if constexpr (F32) two_sum_acc(sacc[u][q], eacc[u][q], p[u][q]);  // compensated per block
-              else sacc[u][q] += p[u][q];
-            }
-        }
-      };
       if constexpr (F32) {
         // packed FP32x2: one target against a staged source pair per step;
         // the target leaf's own pairs (a few per thread) with the
@@ -609,7 +564,43 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 5) k_p2p_cta(const int *leaves, 
         }
         if (from == to && nps) flush();  // only the target leaf's pairs
       } else {
-        sweep(g * T / G, (g + 1) * T / G, std::true_type{});
+        // FP64: a slot range, CT_BLOCK sources at a time.  CHECK false: the
+        // block is summed with pair_normal, and again with pair where a
+        // potential is not finite (coincident bodies of a periodic image,
+        // coordinates at the ends of the range)
+        auto sweep = [&](int from, int to, auto check) {
+          constexpr bool CHECK = decltype(check)::value;
+          for (int c0 = from; c0 < to; c0 += CT_BLOCK) {
+            const int cend = min(to, c0 + CT_BLOCK);
+            RT p[CT_TPT][4];
+            auto block = [&](auto body) {
+#pragma unroll
+              for (int u = 0; u < CT_TPT; u++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) p[u][q] = 0;
+#pragma unroll 4  // with 4 CTAs per SM 3398 us at 1M bodies (2: 3449; 5 CTAs: 3424-3478, spills; 6 CTAs: 3423)
+              for (int cs = c0; cs < cend; cs++) {
+                const BT sv = stage[cs];
+#pragma unroll
+                for (int u = 0; u < CT_TPT; u++) body(A[u], sv, p[u]);
+              }
+            };
+            auto checked = [&](const BT &t, const BT &sv, RT *r) { pair(t.x, t.y, t.z, sv, r[0], r[1], r[2], r[3]); };
+            auto normal = [&](const BT &t, const BT &sv, RT *r) { pair_normal(t.x, t.y, t.z, sv, r[0], r[1], r[2], r[3]); };
+            if constexpr (CHECK) {
+              block(checked);
+            } else {
+              block(normal);
+              if (!isfinite(p[0][0]) || !isfinite(p[1][0])) block(checked);
+            }
+#pragma unroll
+            for (int u = 0; u < CT_TPT; u++)
+#pragma unroll
+              for (int q = 0; q < 4; q++) sacc[u][q] += p[u][q];
+          }
+        };
+        sweep(g * pre / G, (g + 1) * pre / G, std::true_type{});
+        sweep(pre + g * (T - pre) / G, pre + (g + 1) * (T - pre) / G, std::false_type{});
       }
     }
     e0i += nl;
@@ -713,10 +704,17 @@ void p2p_pass(Handle &h, cudaStream_t s) {
 }
 
 void direct_sum(Handle &h, double4 *targets, double4 *out, long nt) {
-  dim3 grid(grid_for(nt, DT), grid_for(h.n, DCHUNK));
+  // as many source chunks as give whole waves of resident blocks (four, so
+  // that a block is short against the whole), tiles of DT sources each
+  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
+  int occ = 1;
+  FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_direct, DT, 0));
+  const long gx = grid_for(nt, DT), want = std::max<long>(1, 4L * h.nsm * std::max(occ, 1) / gx);
+  const long chunk = std::max<long>(DCHUNK_MIN, (h.n + want - 1) / want);
+  const dim3 grid(gx, (unsigned)std::min<long>(65535, (h.n + chunk - 1) / chunk));
   int prange = 0;  // periodic images: r = sum_{i < images} 3^i (3dp/traverse_eager.h:139-142)
   for (int i = 0, p3 = 1; i < h.prm.images; i++, p3 *= 3) prange += p3;
-  k_direct<<<grid, DT, 0, h.stream>>>(targets, nt, h.src.as<double4>(), h.n, out, prange,
+  k_direct<<<grid, DT, 0, h.stream>>>(targets, nt, h.src.as<double4>(), h.n, chunk, out, prange,
                                       h.prm.images ? h.prm.cycle : 0.0);
   h.launches++;
   FMM_LAUNCH();
