@@ -380,7 +380,7 @@ int exafmm_b200_destroy(exafmm_b200 *H) {
                  &h.m2l_units, &h.stage, &h.g_mt, &h.g_ekey, &h.g_occ, &h.g_cnt, &h.g_keyof, &h.g_ops,
                  &h.g_tk, &h.g_tile, &h.g_seg, &h.g_tg, &h.g_m16, &h.g_slot, &h.g_pairs, &h.shift_ops, &h.shift_terms,
                  &h.op_scratch, &h.g_gmark, &h.per_harm, &h.g_gharm, &h.per_part,
-                 &h.g_part, &h.body_leaf, &h.l2p_f};
+                 &h.g_part, &h.body_leaf, &h.l2p_f, &h.ew_waves, &h.ew_units, &h.ew_amp, &h.ew_part};
   for (Buf *b : bufs) b->release();
   if (h.ev_ok)
     for (int p = 0; p < PH_COUNT + 1; p++)
@@ -705,25 +705,22 @@ int exafmm_b200_direct(exafmm_b200 *H, double *targets, int64_t nt, int where) {
     if (!targets || nt <= 0) throw Error{EXAFMM_ERR_ARG, "need targets"};
     const int len = rec_len(h);
     const size_t bytes = (size_t)nt * len * sizeof(double);
-    Buf rec, xq, pf;
-    rec.need(bytes);
-    xq.need(nt * sizeof(double4));
-    pf.need(nt * sizeof(double4));
-    FMM_CUDA(cudaMemcpyAsync(rec.p, targets, bytes, where == EXAFMM_HOST ? cudaMemcpyHostToDevice
+    // records, then positions and results as double4 (aligned for them)
+    const size_t at = (bytes + 31) / 32 * 32;
+    h.stage.need(at + 2 * nt * sizeof(double4));
+    double *rec = h.stage.as<double>();
+    double4 *xq = (double4 *)((char *)h.stage.p + at), *pf = xq + nt;
+    FMM_CUDA(cudaMemcpyAsync(rec, targets, bytes, where == EXAFMM_HOST ? cudaMemcpyHostToDevice
                                                                         : cudaMemcpyDeviceToDevice, h.stream));
-    k_direct_prep<<<grid_for(nt, 256), 256, 0, h.stream>>>(rec.as<double>(), nt, len, xq.as<double4>(),
-                                                          pf.as<double4>());
+    k_direct_prep<<<grid_for(nt, 256), 256, 0, h.stream>>>(rec, nt, len, xq, pf);
     FMM_LAUNCH();
-    if (is2d(h)) direct_sum_2d(h, xq.as<double4>(), pf.as<double4>(), nt);
-    else direct_sum(h, xq.as<double4>(), pf.as<double4>(), nt);
-    k_direct_back<<<grid_for(nt, 256), 256, 0, h.stream>>>(pf.as<double4>(), nt, len, rec.as<double>());
+    if (is2d(h)) direct_sum_2d(h, xq, pf, nt);
+    else direct_sum(h, xq, pf, nt);
+    k_direct_back<<<grid_for(nt, 256), 256, 0, h.stream>>>(pf, nt, len, rec);
     FMM_LAUNCH();
-    FMM_CUDA(cudaMemcpyAsync(targets, rec.p, bytes, where == EXAFMM_HOST ? cudaMemcpyDeviceToHost
+    FMM_CUDA(cudaMemcpyAsync(targets, rec, bytes, where == EXAFMM_HOST ? cudaMemcpyDeviceToHost
                                                                         : cudaMemcpyDeviceToDevice, h.stream));
     FMM_CUDA(cudaStreamSynchronize(h.stream));
-    rec.release();
-    xq.release();
-    pf.release();
   });
 }
 
@@ -757,7 +754,7 @@ int exafmm_b200_ewald_parts(exafmm_b200 *H, int parts, int ksize, double alpha, 
     if (ksize < 1 || ksize > 64 || !(alpha > 0) || !(sigma > 0) || !(cutoff > 0))
       throw Error{EXAFMM_ERR_ARG, "ewald: ksize in [1, 64] and positive alpha, sigma, cutoff required"};
     if (!(h.prm.cycle > 0)) throw Error{EXAFMM_ERR_STATE, "ewald() needs a periodic handle (cycle > 0)"};
-    Buf rec;
+    Buf &rec = h.stage;
     rec.need(nt * 64);
     FMM_CUDA(cudaMemcpyAsync(rec.p, targets, nt * 64, where == EXAFMM_HOST ? cudaMemcpyHostToDevice
                                                                           : cudaMemcpyDeviceToDevice, h.stream));
@@ -765,7 +762,6 @@ int exafmm_b200_ewald_parts(exafmm_b200 *H, int parts, int ksize, double alpha, 
     FMM_CUDA(cudaMemcpyAsync(targets, rec.p, nt * 64, where == EXAFMM_HOST ? cudaMemcpyDeviceToHost
                                                                           : cudaMemcpyDeviceToDevice, h.stream));
     FMM_CUDA(cudaStreamSynchronize(h.stream));
-    rec.release();
   });
 }
 

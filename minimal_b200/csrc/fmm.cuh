@@ -185,6 +185,9 @@ struct Handle {
   Buf g_part;   // tensor-core M2L: partial local expansions of tiles split between CTAs
   int nsm = 0;  // streaming multiprocessors of the device (0: not read yet)
   int per_P = 0, per_images = 0;
+  // Ewald: wave list and DFT units of ew_ksize, amplitudes, partial sums
+  Buf ew_waves, ew_units, ew_amp, ew_part;
+  int ew_ksize = 0, ew_nw = 0, ew_nunits = 0;
   double per_cycle = 0;
   // tile shapes chosen at run time (exafmm_b200_set_tile; the autotuner)
   int tile_m2l_flush = 0;  // tensor-core M2L groups per FP32 accumulator window (0: default)

@@ -20,6 +20,7 @@
 // the targets (waves with integer k, 0 < |k| <= ksize, in the half space of
 // initWaves), real part with erfc over all sources within the cutoff at the
 // nearest image per axis, self term -2/sqrt(pi) q alpha.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -214,58 +215,152 @@ __global__ void k_dipole_apply(const double4 *src, double4 *out, long n, const d
 // ---- Ewald
 constexpr int EB = 256;
 
-// One block per wave: structure factor sum_b q_b (cos th, sin th), th = k.x
-// scale, scaled by coef exp(-|K|^2 coef2) / |K|^2 (3dp/ewald.h:22-34, :128-141).
-__global__ void k_ewald_dft(const int4 *waves, const double4 *src, long n, double scale, double coef, double coef2,
-                            double2 *amp) {
-  __shared__ double red[2][EB];
-  const int4 k = waves[blockIdx.x];
-  double re = 0, im = 0;
-  for (long i = threadIdx.x; i < n; i += EB) {
-    const double4 b = src[i];
-    const double th = k.x * b.x * scale + k.y * b.y * scale + k.z * b.z * scale;
-    double s, c;
-    sincos(th, &s, &c);
-    re += b.w * c;
-    im += b.w * s;
-  }
-  red[0][threadIdx.x] = re;
-  red[1][threadIdx.x] = im;
-  __syncthreads();
-  for (int s = EB / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      red[0][threadIdx.x] += red[0][threadIdx.x + s];
-      red[1][threadIdx.x] += red[1][threadIdx.x + s];
+// ---- structure factors (3dp/ewald.h:22-34, :128-141): for every wave k of
+// the list, sum_b q_b e^{i th}, th = k.x scale.
+//
+// e^{i th} factorises over the axes, so a body needs one sincos per axis and
+// its powers e^{i l X}, l <= ksize (products of halves: l's powers carry
+// about log2(l) roundings, fewer than the rounding of l X itself), and a
+// wave is a product of three table entries.  A unit is (l, m, n0), l, m >= 0:
+// with a+ = q ex_l ey_m and a- = q ex_l conj(ey_m), the four real sums over
+// the bodies of re/im(a) cos/sin(n Z), n0 <= n < n0 + DFT_N, give the waves
+// (l, m, +-n) and (l, -m, +-n): 2 x 16 FMAs and 8 products per body for up to
+// 16 waves.  A thread keeps one unit's sums in registers; the block's bodies
+// pass through shared tables, DFT_B at a time.  1M bodies, ksize 11 (2,787
+// waves): 8600 us with a sincos per wave and body.
+constexpr int DFT_T = 256, DFT_B = 32, DFT_N = 4;
+
+// One unit; base[s] (s = 0: +m, 1: -m): where the wave (l, +-m, 0) is, or would
+// be, in the list (its neighbours in n are contiguous), NO_WAVE if (l, +-m) is
+// not in it.
+struct DftUnit {
+  int l, m, n0, nmax;
+  int base[2];
+  int half;  // (0, 0): only n > 0, and no negative n
+  int pad;
+};
+
+constexpr int NO_WAVE = -(1 << 30);
+
+inline size_t dft_smem(int ksize) { return ((size_t)DFT_B * 3 * (ksize + 1) + DFT_N) * sizeof(double2); }
+
+__global__ void __launch_bounds__(DFT_T, 2) k_ewald_dft(const DftUnit *units, int nunits, const double4 *src, long n,
+                                                       long chunk, int ksize, double scale, double2 *part, int nw) {
+  extern __shared__ double2 tab[];  // [DFT_B][3][ksize + 1]: q e^{i l X}, e^{i m Y}, e^{i n Z}
+  const int K1 = ksize + 1, row = 3 * K1;
+  const int u = blockIdx.x * DFT_T + threadIdx.x;
+  const bool act = u < nunits;
+  const DftUnit un = units[act ? u : 0];
+  double sp[DFT_N][4], sm[DFT_N][4];  // sums of (ar c, ai s, ar s, ai c) for a+ and a-
+#pragma unroll
+  for (int j = 0; j < DFT_N; j++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) sp[j][q] = sm[j][q] = 0;
+  const long s0 = (long)blockIdx.y * chunk, s1 = min(n, s0 + chunk);
+  for (long b = s0; b < s1; b += DFT_B) {
+    const int m = (int)min((long)DFT_B, s1 - b);
+    __syncthreads();
+    for (int e = threadIdx.x; e < 3 * m; e += DFT_T) {  // thread per (body, axis)
+      const int ax = e / m, k = e - ax * m;
+      const double4 B = src[b + k];
+      double2 *t = tab + k * row + ax * K1;
+      double2 e1;
+      sincos((ax == 0 ? B.x : ax == 1 ? B.y : B.z) * scale, &e1.y, &e1.x);
+      t[0] = make_double2(1, 0);
+      t[1] = e1;
+      for (int l = 2; l <= ksize; l++) t[l] = cmul(t[l >> 1], t[l - (l >> 1)]);
+      if (ax == 0)
+        for (int l = 0; l <= ksize; l++) t[l] = make_double2(B.w * t[l].x, B.w * t[l].y);
     }
     __syncthreads();
+    if (act) {
+      const double2 *px = tab + un.l, *py = tab + K1 + un.m, *pz = tab + 2 * K1 + un.n0;
+#pragma unroll 2
+      for (int k = 0; k < m; k++) {
+        const double2 x = px[k * row], y = py[k * row];
+        const double rr = x.x * y.x, ii = x.y * y.y, ri = x.x * y.y, ir = x.y * y.x;
+        const double2 ap = make_double2(rr - ii, ri + ir), am = make_double2(rr + ii, ir - ri);
+#pragma unroll
+        for (int j = 0; j < DFT_N; j++) {
+          // past nmax the entry belongs to the next axis or body, or (the
+          // last body's) lies in the pad: read, but never stored
+          const double2 z = pz[k * row + j];
+          sp[j][0] += ap.x * z.x;
+          sp[j][1] += ap.y * z.y;
+          sp[j][2] += ap.x * z.y;
+          sp[j][3] += ap.y * z.x;
+          sm[j][0] += am.x * z.x;
+          sm[j][1] += am.y * z.y;
+          sm[j][2] += am.x * z.y;
+          sm[j][3] += am.y * z.x;
+        }
+      }
+    }
   }
-  if (threadIdx.x == 0) {
-    const double kx = k.x * scale, ky = k.y * scale, kz = k.z * scale;
-    const double k2 = kx * kx + ky * ky + kz * kz;
-    const double f = coef * exp(-k2 * coef2) / k2;
-    amp[blockIdx.x] = make_double2(red[0][0] * f, red[1][0] * f);
+  if (!act) return;
+  double2 *out = part + (size_t)blockIdx.y * nw;
+#pragma unroll
+  for (int j = 0; j < DFT_N; j++) {
+    const int nn = un.n0 + j;
+    if (nn > un.nmax || (un.half && nn == 0)) continue;
+#pragma unroll
+    for (int sgn = 0; sgn < 2; sgn++) {
+      if (un.base[sgn] == NO_WAVE) continue;
+      const double(&v)[4] = sgn ? sm[j] : sp[j];
+      out[un.base[sgn] + nn] = make_double2(v[0] - v[1], v[2] + v[3]);
+      if (nn > 0 && !un.half) out[un.base[sgn] - nn] = make_double2(v[0] + v[1], v[3] - v[2]);
+    }
   }
 }
 
+// The chunks' sums added (32 waves per block, 8 threads per wave over the
+// chunks, then in thread order: deterministic) and scaled by
+// coef exp(-|K|^2 coef2) / |K|^2.
+__global__ void __launch_bounds__(256) k_ewald_amp(const int4 *waves, const double2 *part, int nw, int nchunk,
+                                                   double scale, double coef, double coef2, double2 *amp) {
+  __shared__ double2 red[8][32];
+  const int w = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
+  double2 s = make_double2(0, 0);
+  if (w < nw)
+#pragma unroll 4
+    for (int c = g; c < nchunk; c += 8) {
+      const double2 v = part[(size_t)c * nw + w];
+      s.x += v.x;
+      s.y += v.y;
+    }
+  red[g][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (g > 0 || w >= nw) return;
+  for (int q = 1; q < 8; q++) {
+    s.x += red[q][threadIdx.x].x;
+    s.y += red[q][threadIdx.x].y;
+  }
+  const int4 k = waves[w];
+  const double kx = k.x * scale, ky = k.y * scale, kz = k.z * scale;
+  const double k2 = kx * kx + ky * ky + kz * kz;
+  const double f = coef * exp(-k2 * coef2) / k2;
+  amp[w] = make_double2(s.x * f, s.y * f);
+}
+
 // Real-space term of one source at the nearest image per axis, inside the
-// cutoff (3dp/ewald.h:82-102 realP2P).
+// cutoff (3dp/ewald.h:82-102 realP2P): with g = exp(-(alpha r)^2) and
+// erfc(alpha r) = g erfcx(alpha r), one exponential serves both terms.
+__device__ __forceinline__ double nearest_image(double d, double half, double cycle) {
+  return fabs(d) > half ? d - copysign(cycle, d) : d;
+}
+
 __device__ __forceinline__ void ewald_real_pair(double tx, double ty, double tz, const double4 &b, double c2,
-                                                double alpha, double a3, double half, double cycle, double &p,
-                                                double &fx, double &fy, double &fz) {
-  double dx = tx - b.x, dy = ty - b.y, dz = tz - b.z;
-  if (dx < -half) dx += cycle;
-  if (dx > half) dx -= cycle;
-  if (dy < -half) dy += cycle;
-  if (dy > half) dy -= cycle;
-  if (dz < -half) dz += cycle;
-  if (dz > half) dz -= cycle;
+                                                double alpha, double half, double cycle, double &p, double &fx,
+                                                double &fy, double &fz) {
+  const double dx = nearest_image(tx - b.x, half, cycle), dy = nearest_image(ty - b.y, half, cycle),
+               dz = nearest_image(tz - b.z, half, cycle);
   const double R2 = dx * dx + dy * dy + dz * dz;
   if (0 < R2 && R2 < c2) {
-    const double R2s = R2 * alpha * alpha, Rs = sqrt(R2s);
-    const double invRs = 1 / Rs, invR2s = invRs * invRs, invR3s = invR2s * invRs;
-    const double ec = erfc(Rs);
-    const double dtmp = b.w * (M_2_SQRTPI * exp(-R2s) * invR2s + ec * invR3s) * a3;
-    p += b.w * ec * invRs * alpha;
+    const double ir = rsqrt(R2), Rs = alpha * (R2 * ir);
+    const double g = exp(-(R2 * alpha) * alpha);
+    const double pot = b.w * (g * erfcx(Rs)) * ir;
+    const double dtmp = (b.w * (M_2_SQRTPI * alpha) * g + pot) * ir * ir;
+    p += pot;
     fx -= dx * dtmp;
     fy -= dy * dtmp;
     fz -= dz * dtmp;
@@ -285,21 +380,73 @@ __device__ __forceinline__ void ewald_wave_term(double tx, double ty, double tz,
   fz -= dtmp * k.z * scale;
 }
 
-// One block per target (few targets, many sources): the parts selected by
-// `parts` -- real part over all sources (nearest image per axis, 0 < R <
-// cutoff), the inverse DFT over all waves, the self term; p and F accumulate
-// into the target record.
-__global__ void k_ewald_target(const double4 *src, long n, const int4 *waves, const double2 *amp, int nw,
-                               double scale, double alpha, double cutoff, double cycle, int parts, double *rec) {
+// Few targets, many sources.  k_ewald_real: the real part of RT targets over
+// one chunk of the sources; each source is read once for the RT targets
+// (read once per target, 1,000 targets took 33 GB from L2), and as the
+// sources lie in tree order the 32 of a warp are mostly all inside or all
+// outside a target's cutoff, so warps skip the outside ones.  The chunks'
+// sums go to `part`, which k_ewald_finish adds in order to the target record
+// with the inverse DFT over all waves and the self term: a block per target.
+constexpr int RT = 4;
+
+__global__ void __launch_bounds__(EB) k_ewald_real(const double4 *src, long n, long chunk, double alpha,
+                                                   double cutoff, double cycle, const double *rec, long nt,
+                                                   double *part) {
+  __shared__ double red[EB / 32][RT * 4];
+  const long t0 = (long)blockIdx.x * RT;
+  double tx[RT], ty[RT], tz[RT], acc[RT][4];
+#pragma unroll
+  for (int u = 0; u < RT; u++) {
+    const double *r = rec + 8 * min(t0 + u, nt - 1);
+    tx[u] = r[0];
+    ty[u] = r[1];
+    tz[u] = r[2];
+#pragma unroll
+    for (int q = 0; q < 4; q++) acc[u][q] = 0;
+  }
+  const double c2 = cutoff * cutoff, half = cycle / 2;
+  const long s0 = (long)blockIdx.y * chunk, s1 = min(n, s0 + chunk);
+  for (long i = s0 + threadIdx.x; i < s1; i += EB) {
+    const double4 b = src[i];
+#pragma unroll
+    for (int u = 0; u < RT; u++)
+      ewald_real_pair(tx[u], ty[u], tz[u], b, c2, alpha, half, cycle, acc[u][0], acc[u][1], acc[u][2], acc[u][3]);
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int u = 0; u < RT; u++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      double v = acc[u][q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) red[warp][u * 4 + q] = v;
+    }
+  __syncthreads();
+  if (threadIdx.x < RT * 4 && t0 + threadIdx.x / 4 < nt) {
+    double v = 0;
+    for (int w = 0; w < EB / 32; w++) v += red[w][threadIdx.x];
+    part[((size_t)blockIdx.y * nt + t0) * 4 + threadIdx.x] = v;
+  }
+}
+
+__global__ void __launch_bounds__(EB) k_ewald_finish(const int4 *waves, const double2 *amp, int nw, double scale,
+                                                     double alpha, int parts, const double *part, int nchunk, long nt,
+                                                     double *rec) {
   __shared__ double red[4][EB];
   double *r = rec + 8 * (long)blockIdx.x;
   const double tx = r[0], ty = r[1], tz = r[2], tq = r[3];
   double p = 0, fx = 0, fy = 0, fz = 0;
-  const double c2 = cutoff * cutoff, a3 = alpha * alpha * alpha, half = cycle / 2;
-  if (parts & EXAFMM_EWALD_REAL)
-    for (long i = threadIdx.x; i < n; i += EB) ewald_real_pair(tx, ty, tz, src[i], c2, alpha, a3, half, cycle, p, fx, fy, fz);
   if (parts & EXAFMM_EWALD_WAVE)
     for (int w = threadIdx.x; w < nw; w += EB) ewald_wave_term(tx, ty, tz, waves[w], amp[w], scale, p, fx, fy, fz);
+  if (parts & EXAFMM_EWALD_REAL)
+    for (int c = threadIdx.x; c < nchunk; c += EB) {
+      const double *v = part + ((size_t)c * nt + blockIdx.x) * 4;
+      p += v[0];
+      fx += v[1];
+      fy += v[2];
+      fz += v[3];
+    }
   red[0][threadIdx.x] = p;
   red[1][threadIdx.x] = fx;
   red[2][threadIdx.x] = fy;
@@ -333,14 +480,14 @@ __global__ void __launch_bounds__(EB) k_ewald_targets(const double4 *src, long n
     tx = r[0]; ty = r[1]; tz = r[2]; tq = r[3];
   }
   double p = 0, fx = 0, fy = 0, fz = 0;
-  const double c2 = cutoff * cutoff, a3 = alpha * alpha * alpha, half = cycle / 2;
+  const double c2 = cutoff * cutoff, half = cycle / 2;
   if (parts & EXAFMM_EWALD_REAL)
     for (long b = 0; b < n; b += EB) {
       __syncthreads();
       if (b + threadIdx.x < n) tile[threadIdx.x] = src[b + threadIdx.x];
       __syncthreads();
       const int m = (int)min((long)EB, n - b);
-      for (int k = 0; k < m; k++) ewald_real_pair(tx, ty, tz, tile[k], c2, alpha, a3, half, cycle, p, fx, fy, fz);
+      for (int k = 0; k < m; k++) ewald_real_pair(tx, ty, tz, tile[k], c2, alpha, half, cycle, p, fx, fy, fz);
     }
   if (parts & EXAFMM_EWALD_WAVE)
     for (int w0 = 0; w0 < nw; w0 += EB) {
@@ -366,6 +513,7 @@ __global__ void __launch_bounds__(EB) k_ewald_targets(const double4 *src, long n
 
 void periodic_set_attributes() {
   cudaFuncSetAttribute(k_periodic_harm, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_ewald_dft, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
 }
 
 void periodic_pass(Handle &h) {
@@ -409,43 +557,96 @@ void dipole_correction(Handle &h) {
   part.release();
 }
 
-void ewald(Handle &h, int parts, int ksize, double alpha, double sigma, double cutoff, double cycle, double *rec_dev,
-           long nt) {
-  // waves of initWaves (3dp/ewald.h:53-80)
+// The wave list of initWaves (3dp/ewald.h:53-80) and the units of
+// k_ewald_dft for ksize, kept in the handle until another ksize is asked for.
+static void ewald_plan(Handle &h, int ksize) {
+  if (h.ew_ksize == ksize) return;
   std::vector<int4> w;
+  std::vector<DftUnit> units;
   for (int l = 0; l <= ksize; l++) {
+    std::vector<int> zero(2 * ksize + 1, NO_WAVE);  // index of wave (l, m, 0)
     const int mmin = l == 0 ? 0 : -ksize;
     for (int m = mmin; m <= ksize; m++) {
       const int nmin = (l == 0 && m == 0) ? 1 : -ksize;
+      bool first = true;
       for (int n = nmin; n <= ksize; n++)
-        if (l * l + m * m + n * n <= ksize * ksize) w.push_back(make_int4(l, m, n, 0));
+        if (l * l + m * m + n * n <= ksize * ksize) {
+          if (first) zero[m + ksize] = (int)w.size() - n;
+          first = false;
+          w.push_back(make_int4(l, m, n, 0));
+        }
+    }
+    for (int m = 0; m <= ksize; m++) {
+      if (zero[m + ksize] == NO_WAVE) continue;
+      int nmax = 0;
+      while (l * l + m * m + (nmax + 1) * (nmax + 1) <= ksize * ksize) nmax++;
+      for (int n0 = 0; n0 <= nmax; n0 += DFT_N)
+        units.push_back({l, m, n0, nmax, {zero[m + ksize], m > 0 ? zero[ksize - m] : NO_WAVE}, l == 0 && m == 0, 0});
     }
   }
-  const int nw = (int)w.size();
-  Buf wv, amp;
-  wv.need(nw * sizeof(int4));
-  amp.need(nw * sizeof(double2));
-  FMM_CUDA(cudaMemcpyAsync(wv.p, w.data(), nw * sizeof(int4), cudaMemcpyHostToDevice, h.stream));
+  // a warp's units share n0 (its z entries are then one address)
+  std::stable_sort(units.begin(), units.end(), [](const DftUnit &a, const DftUnit &b) { return a.n0 < b.n0; });
+  h.ew_ksize = 0;  // until both tables are in place
+  h.ew_nw = (int)w.size();
+  h.ew_nunits = (int)units.size();
+  h.ew_waves.need(w.size() * sizeof(int4));
+  h.ew_units.need(units.size() * sizeof(DftUnit));
+  FMM_CUDA(cudaMemcpyAsync(h.ew_waves.p, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice, h.stream));
+  FMM_CUDA(cudaMemcpyAsync(h.ew_units.p, units.data(), units.size() * sizeof(DftUnit), cudaMemcpyHostToDevice,
+                           h.stream));
+  FMM_CUDA(cudaStreamSynchronize(h.stream));
+  h.ew_ksize = ksize;
+}
+
+void ewald(Handle &h, int parts, int ksize, double alpha, double sigma, double cutoff, double cycle, double *rec_dev,
+           long nt) {
+  ewald_plan(h, ksize);
+  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
+  const int nw = h.ew_nw;
+  const int4 *waves = h.ew_waves.as<int4>();
+  h.ew_amp.need(nw * sizeof(double2));
+  double2 *amp = h.ew_amp.as<double2>();
   const double scale = 2 * M_PI / cycle;
   const double coef = 2 / sigma / cycle / cycle / cycle, coef2 = 1 / (4 * alpha * alpha);
   if (parts & EXAFMM_EWALD_WAVE) {
-    k_ewald_dft<<<nw, EB, 0, h.stream>>>(wv.as<int4>(), h.src.as<double4>(), h.n, scale, coef, coef2,
-                                         amp.as<double2>());
-    h.launches++;
+    // two resident blocks per SM, each a chunk of the bodies (whole tiles)
+    const int gx = grid_for(h.ew_nunits, DFT_T);
+    const long want = std::max(1, 2 * h.nsm / gx);
+    const long chunk = ((h.n + want - 1) / want + DFT_B - 1) / DFT_B * DFT_B;
+    const int gy = (int)((h.n + chunk - 1) / chunk);
+    h.ew_part.need((size_t)gy * nw * sizeof(double2));
+    k_ewald_dft<<<dim3(gx, gy), DFT_T, dft_smem(ksize), h.stream>>>(h.ew_units.as<DftUnit>(), h.ew_nunits,
+                                                                    h.src.as<double4>(), h.n, chunk, ksize, scale,
+                                                                    h.ew_part.as<double2>(), nw);
+    k_ewald_amp<<<grid_for(nw, 32), 256, 0, h.stream>>>(waves, h.ew_part.as<double2>(), nw, gy, scale, coef, coef2,
+                                                       amp);
+    h.launches += 2;
+    FMM_LAUNCH();
   }
-  const long n = (parts & (EXAFMM_EWALD_REAL | EXAFMM_EWALD_WAVE)) ? h.n : 0;
-  // a block per target while the targets cannot fill the GPU as threads
-  if (nt < 148L * 4 * EB)
-    k_ewald_target<<<(unsigned)nt, EB, 0, h.stream>>>(h.src.as<double4>(), n, wv.as<int4>(), amp.as<double2>(), nw,
-                                                      scale, alpha, cutoff, cycle, parts, rec_dev);
-  else
-    k_ewald_targets<<<grid_for(nt, EB), EB, 0, h.stream>>>(h.src.as<double4>(), n, wv.as<int4>(), amp.as<double2>(),
-                                                           nw, scale, alpha, cutoff, cycle, parts, rec_dev, nt);
+  // while the targets cannot fill the GPU as threads: chunks of the sources
+  // for RT targets each
+  if (nt < 148L * 4 * EB) {
+    int gy = 0;
+    if (parts & EXAFMM_EWALD_REAL) {
+      int occ = 1;
+      FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ewald_real, EB, 0));
+      const long gx = (nt + RT - 1) / RT, want = std::max<long>(1, 4L * h.nsm * std::max(occ, 1) / gx);
+      const long chunk = std::max<long>(4 * EB, ((h.n + want - 1) / want + EB - 1) / EB * EB);
+      gy = (int)((h.n + chunk - 1) / chunk);
+      h.ew_part.need((size_t)gy * nt * 4 * sizeof(double));
+      k_ewald_real<<<dim3((unsigned)gx, gy), EB, 0, h.stream>>>(h.src.as<double4>(), h.n, chunk, alpha, cutoff, cycle,
+                                                               rec_dev, nt, h.ew_part.as<double>());
+      h.launches++;
+    }
+    k_ewald_finish<<<(unsigned)nt, EB, 0, h.stream>>>(waves, amp, nw, scale, alpha, parts, h.ew_part.as<double>(), gy,
+                                                      nt, rec_dev);
+  } else {
+    const long n = (parts & (EXAFMM_EWALD_REAL | EXAFMM_EWALD_WAVE)) ? h.n : 0;
+    k_ewald_targets<<<grid_for(nt, EB), EB, 0, h.stream>>>(h.src.as<double4>(), n, waves, amp, nw, scale, alpha,
+                                                           cutoff, cycle, parts, rec_dev, nt);
+  }
   h.launches++;
   FMM_LAUNCH();
-  FMM_CUDA(cudaStreamSynchronize(h.stream));
-  wv.release();
-  amp.release();
 }
 
 }  // namespace fmm
