@@ -342,13 +342,45 @@ __global__ void __launch_bounds__(256) k_ewald_amp(const int4 *waves, const doub
   amp[w] = make_double2(s.x * f, s.y * f);
 }
 
-// Real-space term of one source at the nearest image per axis, inside the
-// cutoff (3dp/ewald.h:82-102 realP2P): with g = exp(-(alpha r)^2) and
-// erfc(alpha r) = g erfcx(alpha r), one exponential serves both terms.
+// erfcx(x) = exp(x^2) erfc(x) for 0 <= x <= ERFCX_MAX: (x + 3) erfcx(x) as a
+// polynomial in t = (x - 3) / (x + 3) (the variable of Shepherd and
+// Laframboise, Math. Comp. 36, 1981), here the Chebyshev interpolant of
+// degree 18 on the interval's image in t, computed in 60 digits and written
+// in powers of t; relative error below 6e-16 (mean 1.2e-16), the rounding of
+// the evaluation.
+constexpr double ERFCX_MAX = 6.5;
+__constant__ double c_erfcx[19] = {
+    1.0740069070883398, -0.8833944531698829, 0.5902283571041055, -0.31046726190069107,
+    0.11952776128690286, -0.026827234618913183, -0.0012124166089395308, 0.0030340619011204662,
+    -0.000548310106357097, -0.00027677719242548155, 0.00010756610129636827, 3.0399762259269947e-05,
+    -1.749347841768703e-05, -4.786830389538246e-06, 2.789618347258467e-06, 1.1232517707098393e-06,
+    -2.9310736596525035e-07, -2.466455224073059e-07, -4.3340585473038216e-08};
+
+__device__ __forceinline__ double erfcx_near(double x) {
+  const double d = x + 3.0;
+  double r;  // 1 / d: the hardware's estimate and one third-order Newton step
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double e = fma(-d, r, 1.0);
+  r = fma(r, fma(e, e, e), r);
+  const double t = (x - 3.0) * r;
+  double v = c_erfcx[18];
+#pragma unroll
+  for (int k = 17; k >= 0; k--) v = fma(v, t, c_erfcx[k]);
+  return v * r;
+}
+
 __device__ __forceinline__ double nearest_image(double d, double half, double cycle) {
   return fabs(d) > half ? d - copysign(cycle, d) : d;
 }
 
+// Real-space term of one source at the nearest image per axis, inside the
+// cutoff (3dp/ewald.h:82-102 realP2P): with g = exp(-(alpha r)^2) and
+// erfc(alpha r) = g erfcx(alpha r), one exponential serves both terms.
+// 1/r as in pair_normal (pair64.cuh); a distance outside its range makes
+// alpha r infinite or NaN, and that or alpha r > ERFCX_MAX takes CUDA's
+// functions.  (Those alone: 7460 us against 5400 for 1M sources on 1,000
+// targets, of whose pairs about 60% are computed; their roughly 75 FP64
+// instructions take 2900 us at the FP64 peak.)
 __device__ __forceinline__ void ewald_real_pair(double tx, double ty, double tz, const double4 &b, double c2,
                                                 double alpha, double half, double cycle, double &p, double &fx,
                                                 double &fy, double &fz) {
@@ -356,9 +388,20 @@ __device__ __forceinline__ void ewald_real_pair(double tx, double ty, double tz,
                dz = nearest_image(tz - b.z, half, cycle);
   const double R2 = dx * dx + dy * dy + dz * dz;
   if (0 < R2 && R2 < c2) {
-    const double ir = rsqrt(R2), Rs = alpha * (R2 * ir);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(R2));
+    const double e = fma(-(R2 * y), y, 1.0);
+    double ir = fma(y * e, fma(0.375, e, 0.5), y);
+    double Rs = alpha * (R2 * ir), ex;
+    if (Rs <= ERFCX_MAX) {
+      ex = erfcx_near(Rs);
+    } else {
+      ir = rsqrt(R2);
+      Rs = alpha * (R2 * ir);
+      ex = erfcx(Rs);
+    }
     const double g = exp(-(R2 * alpha) * alpha);
-    const double pot = b.w * (g * erfcx(Rs)) * ir;
+    const double pot = b.w * (g * ex) * ir;
     const double dtmp = (b.w * (M_2_SQRTPI * alpha) * g + pot) * ir * ir;
     p += pot;
     fx -= dx * dtmp;
@@ -381,13 +424,15 @@ __device__ __forceinline__ void ewald_wave_term(double tx, double ty, double tz,
 }
 
 // Few targets, many sources.  k_ewald_real: the real part of RT targets over
-// one chunk of the sources; each source is read once for the RT targets
-// (read once per target, 1,000 targets took 33 GB from L2), and as the
-// sources lie in tree order the 32 of a warp are mostly all inside or all
-// outside a target's cutoff, so warps skip the outside ones.  The chunks'
+// one chunk of the sources; each source is read once for the RT targets, and
+// as the sources lie in tree order the 32 of a warp are mostly all inside or
+// all outside a target's cutoff, so warps skip the outside ones.  RT = 2
+// leaves registers for three blocks per SM (4367 us at 1M sources, 1,000
+// targets; RT = 4: 4586-4826); about 16 waves of blocks, as a last wave of
+// few costs more than the chunks' sums (4 waves: 4833).  The chunks'
 // sums go to `part`, which k_ewald_finish adds in order to the target record
 // with the inverse DFT over all waves and the self term: a block per target.
-constexpr int RT = 4;
+constexpr int RT = 2;
 
 __global__ void __launch_bounds__(EB) k_ewald_real(const double4 *src, long n, long chunk, double alpha,
                                                    double cutoff, double cycle, const double *rec, long nt,
@@ -630,7 +675,7 @@ void ewald(Handle &h, int parts, int ksize, double alpha, double sigma, double c
     if (parts & EXAFMM_EWALD_REAL) {
       int occ = 1;
       FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ewald_real, EB, 0));
-      const long gx = (nt + RT - 1) / RT, want = std::max<long>(1, 4L * h.nsm * std::max(occ, 1) / gx);
+      const long gx = (nt + RT - 1) / RT, want = std::max<long>(1, 16L * h.nsm * std::max(occ, 1) / gx);
       const long chunk = std::max<long>(4 * EB, ((h.n + want - 1) / want + EB - 1) / EB * EB);
       gy = (int)((h.n + chunk - 1) / chunk);
       h.ew_part.need((size_t)gy * nt * 4 * sizeof(double));
