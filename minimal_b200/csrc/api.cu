@@ -28,6 +28,11 @@ void p2p_set_attributes();
 void expansions_set_attributes();
 }  // namespace fmm
 
+void fmm::read_counters(Handle &h) {
+  FMM_CUDA(cudaMemcpyAsync(h.hc, h.counters.p, sizeof(DevCounters), cudaMemcpyDeviceToHost, h.stream));
+  FMM_CUDA(cudaStreamSynchronize(h.stream));
+}
+
 using namespace fmm;
 
 struct exafmm_b200 {
@@ -343,6 +348,7 @@ int exafmm_b200_create(const exafmm_params *params, exafmm_b200 **out) {
     for (cudaEvent_t *e : {&h.fork_ev, &h.up_ev, &h.lists_ev, &h.join_ev})
       FMM_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     FMM_CUDA(cudaMallocHost(&h.flags_host, 4 * sizeof(int)));
+    FMM_CUDA(cudaMallocHost(&h.hc, sizeof(DevCounters)));
     h.flags_host[0] = 0;
     h.ev_ok = true;
     for (int p = 0; p < PH_COUNT + 1; p++)
@@ -377,7 +383,7 @@ int exafmm_b200_destroy(exafmm_b200 *H) {
                  &h.c_nchild, &h.c_parent, &h.c_level, &h.c_xr, &h.c_pre, &h.c_ref, &h.c_leaf_of_body,
                  &h.leaves, &h.pre_tmp, &h.ctmp, &h.geom, &h.counters, &h.frontier[0], &h.frontier[1],
                  &h.m2l_raw, &h.m2l_key, &h.p2p_raw, &h.m2l_off, &h.m2l_ent, &h.p2p_off, &h.p2p_ent, &h.fill, &h.M, &h.L,
-                 &h.m2l_units, &h.stage, &h.g_mt, &h.g_ekey, &h.g_occ, &h.g_cnt, &h.g_keyof, &h.g_ops,
+                 &h.m2l_units, &h.stage, &h.g_mt, &h.g_ekey, &h.g_occ, &h.g_cnt, &h.g_newkeys, &h.g_optab, &h.g_ops,
                  &h.g_tk, &h.g_tile, &h.g_seg, &h.g_tg, &h.g_m16, &h.g_slot, &h.g_pairs, &h.shift_ops, &h.shift_terms,
                  &h.op_scratch, &h.g_gmark, &h.per_harm, &h.g_gharm, &h.per_part,
                  &h.g_part, &h.body_leaf, &h.l2p_f, &h.ew_waves, &h.ew_units, &h.ew_amp, &h.ew_part};
@@ -392,7 +398,7 @@ int exafmm_b200_destroy(exafmm_b200 *H) {
   for (cudaEvent_t e : {h.fork_ev, h.up_ev, h.lists_ev, h.join_ev})
     if (e) cudaEventDestroy(e);
   if (h.flags_host) cudaFreeHost(h.flags_host);
-  if (h.keys_host) cudaFreeHost(h.keys_host);
+  if (h.hc) cudaFreeHost(h.hc);
   delete H;
   return EXAFMM_OK;
 }

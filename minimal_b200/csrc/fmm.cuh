@@ -5,7 +5,6 @@
 #include <stdint.h>
 
 #include <string>
-#include <unordered_map>
 #include <vector>
 
 #include "../../include/exafmm_b200.h"
@@ -85,6 +84,7 @@ struct DevCounters {
   // a non-negative double (the FP16 split's power-of-two normalisation)
   unsigned long long m16_max;
   int nghost;  // ghost sources of image entries (mixed form, periodic)
+  int op_new;  // group keys without a cached M2L operator
 };
 
 // Per-phase timing slots (CUDA events on the handle stream).
@@ -134,7 +134,8 @@ struct Handle {
   Buf ctmp;    // cell-count scratch (level sort, index maps)
   Buf geom;    // RootGeom
   Buf counters;  // DevCounters
-  DevCounters hc{};  // host copy
+  DevCounters *hc = nullptr;  // host copy (pinned)
+  double root_R0 = 0;  // radius of the root cell (one system)
 
   // lists (CSR by target, BFS indices)
   Buf frontier[2];
@@ -156,17 +157,18 @@ struct Handle {
   int m2l_units_P = -1;
 
   // grouped M2L (m2l_group.cu)
-  Buf g_mt, g_ekey, g_occ, g_cnt, g_keyof, g_ops, g_tk, g_tile, g_seg, g_tg, g_m16, g_slot, g_pairs;
+  Buf g_mt, g_ekey, g_occ, g_cnt, g_newkeys, g_ops, g_tk, g_tile, g_seg, g_tg, g_m16, g_slot, g_pairs;
   Buf g_gmark;      // ghost slots: marks, their scan, the slot of every ghost
   int g_nghost = 0;  // ghost multipole rows after the cells' in g_m16
-  // operator cache: group key -> slot in g_ops, for order op_P and layout
-  // op_layout (0: FP64 row blocks, 1: tensor-core FP16 images)
-  std::unordered_map<int, int> op_slot;
-  int op_P = -1, op_layout = -1;
+  // operator cache: g_optab[group key] is the operator's slot in g_ops (-1:
+  // not built), op_count slots built for order op_P, layout op_layout (0:
+  // FP64 row blocks, 1: tensor-core FP16 images) and key space op_ks
+  Buf g_optab;
+  int op_P = -1, op_layout = -1, op_count = 0;
+  long op_ks = 0;
   double op_cycle = 0, op_R0 = 0;  // image-key operators: the geometry they were built for
   int op_depth = -1;
-  std::vector<int> op_host_keys, op_host_slots, op_host_new_keys, op_host_new_slots;
-  int *keys_host = nullptr;  // pinned: the group keys read with the counts
+  bool g_grouped = false;  // the group tables belong to the current lists
   int g_ntiles = 0, g_ngroups = 0, g_nseg = 0;
   bool g_used_tc = false;
   // the grouping of the last grouped M2L (tiles, segments, operator slots),
@@ -224,6 +226,13 @@ void upward_pass(Handle &h, cudaStream_t s);
 void downward_pass(Handle &h, cudaStream_t s, cudaEvent_t before_l2p);
 // m2l.cu
 void m2l_pass(Handle &h);
+// m2l_group.cu: group tables from the key and target marks of the lists.
+// m2l_group_launch() queues the kernels; once the counters have been read,
+// m2l_group_commit() builds the operators of the keys not seen before.
+bool m2l_groups_raw(const Handle &h);  // the walk's own marks are what the grouped M2L contracts
+void m2l_group_launch(Handle &h, long max_groups);
+void m2l_group_commit(Handle &h);
+void read_counters(Handle &h);  // DevCounters to h.hc, and waits for them (api.cu)
 // p2p.cu
 void p2p_pass(Handle &h, cudaStream_t s);  // s: h.stream, or h.side once the FP32 sources are made
 void make_srcf(Handle &h);

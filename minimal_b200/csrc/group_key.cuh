@@ -133,9 +133,32 @@ __device__ __forceinline__ int m2l_ghost_key(const double4 &X, const double4 &Y,
 // Marks a key and a target as present.  A few hundred keys (and every
 // target) take millions of entries: store only what this SM has not seen
 // set, so the L1-cached reads keep the stores off a few hot L2 lines.
-__device__ __forceinline__ void m2l_mark_key(int key, int t, int *occ, int *gflag) {
+__device__ __forceinline__ void m2l_mark_key(int key, int t, unsigned char *occ, int *gflag) {
   if (occ[key] == 0) occ[key] = 1;
   if (gflag[t] == 0) gflag[t] = 1;
+}
+
+// Group tables of a key space of ks keys (a multiple of OCC_TILE), one buffer:
+// the marks (a byte per key), then per 32 keys {marks as a mask, groups before
+// them}, then per tile the number of marked keys.
+constexpr long OCC_TILE = 32768;
+static_assert(KEY_SPACE % OCC_TILE == 0 && IKEY_SPACE % OCC_TILE == 0, "whole tiles of group keys");
+struct GroupTables {
+  unsigned char *occ;
+  uint2 *mask;
+  int *sums;
+};
+inline size_t group_table_bytes(long ks) { return (size_t)ks + (size_t)ks / 32 * sizeof(uint2) + ks / OCC_TILE * sizeof(int); }
+inline GroupTables group_tables(void *p, long ks) {
+  unsigned char *b = (unsigned char *)p;
+  uint2 *m = (uint2 *)(b + ks);
+  return GroupTables{b, m, (int *)(m + ks / 32)};
+}
+
+// Group id of a marked key.
+__device__ __forceinline__ int group_id(const uint2 *mask, int key) {
+  const uint2 w = mask[key >> 5];
+  return (int)w.y + __popc(w.x & ((1u << (key & 31)) - 1u));
 }
 
 }  // namespace fmm

@@ -16,6 +16,8 @@
 // source's depth-first pre-order rank (a depth-first walk meets the sources
 // of one target in pre-order, because a target-side split never reorders
 // them).  The result equals getList's per-cell lists entry for entry.
+#include <cstddef>
+
 #include "group_key.cuh"
 
 namespace fmm {
@@ -58,7 +60,7 @@ __global__ void __launch_bounds__(TB) k_walk(CellView cv, const int2 *fin, const
                                             int2 *fout, unsigned long long *nout, unsigned long long *nnext,
                                             u64 fcap, int2 *m2l, unsigned long long *nm2l, u64 mcap, int2 *p2p,
                                             unsigned long long *np2p, u64 pcap, double theta, double cycle,
-                                            int depth, int *overflow, int *m2l_key, int *occ, int *gflag,
+                                            int depth, int *overflow, int *m2l_key, unsigned char *occ, int *gflag,
                                             int *nres) {
   constexpr int NW = TB / 32, CHUNK = TB * WP;
   static_assert(CHUNK < 4096, "per-block M2L and P2P counts are packed in 12-bit fields");
@@ -398,20 +400,21 @@ void build_lists(Handle &h) {
   h.p2p_cap = std::max<size_t>(h.p2p_cap, (size_t)h.nleaves * 90 + 1024);
   const int images = h.prm.images;
   const long ks = key_space(images, h.depth);
-  h.g_occ.need((size_t)ks * sizeof(int) * 2 + 64);  // key occupancy, then its scan
-  h.g_cnt.need((size_t)C * sizeof(int) * 2 + 64);           // targets with grouped entries, then tile slots
-  int *occ = h.g_occ.as<int>(), *gflag = h.g_cnt.as<int>();
+  h.g_occ.need(group_table_bytes(ks));             // key marks and the tables made from them
+  h.g_cnt.need((size_t)C * sizeof(int) * 2 + 64);  // targets with grouped entries, then tile slots
+  unsigned char *occ = group_tables(h.g_occ.p, ks).occ;
+  int *gflag = h.g_cnt.as<int>();
+  h.g_grouped = false;
   for (int attempt = 0;; attempt++) {
     h.frontier[0].need(h.frontier_cap * sizeof(int2));
     h.frontier[1].need(h.frontier_cap * sizeof(int2));
     h.m2l_raw.need(h.m2l_cap * sizeof(int2));
     h.p2p_raw.need(h.p2p_cap * sizeof(int2));
-    FMM_CUDA(cudaMemsetAsync(&ctr->n_m2l, 0, sizeof(unsigned long long) * 5, s));  // list and frontier counts
-    FMM_CUDA(cudaMemsetAsync(&ctr->list_overflow, 0, sizeof(int), s));
-    FMM_CUDA(cudaMemsetAsync(&ctr->walk_resid, 0, sizeof(int), s));
+    // list and frontier counts, and the counters of the M2L grouping
+    FMM_CUDA(cudaMemsetAsync(&ctr->n_m2l, 0, sizeof(DevCounters) - offsetof(DevCounters, n_m2l), s));
     // group keys of the M2L entries, and the keys and targets that occur
     h.m2l_key.need(h.m2l_cap * sizeof(int));
-    FMM_CUDA(cudaMemsetAsync(occ, 0, (size_t)ks * sizeof(int), s));
+    FMM_CUDA(cudaMemsetAsync(occ, 0, (size_t)ks, s));
     FMM_CUDA(cudaMemsetAsync(gflag, 0, (size_t)C * sizeof(int), s));
     k_seed<<<grid_for(std::max(h.nsys, 32), 256), 256, 0, s>>>(h.frontier[0].as<int2>(), &ctr->frontier[0], images,
                                                                 h.nsys, h.prm.dim == 2 ? 2 : 3);
@@ -433,23 +436,29 @@ void build_lists(Handle &h) {
       h.launches++;
       FMM_LAUNCH();
     }
-    FMM_CUDA(cudaMemcpyAsync(&h.hc, ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-    FMM_CUDA(cudaStreamSynchronize(s));
-    if (h.hc.list_overflow) {
+    const bool group = m2l_groups_raw(h);
+    if (group) m2l_group_launch(h, (long)h.m2l_cap);
+    read_counters(h);
+    if (h.hc->list_overflow) {
       // a dropped frontier pair also hides its descendants' entries: grow
       // everything and walk again
       if (attempt >= 4) throw Error{EXAFMM_ERR_CAPACITY, "interaction list buffers kept overflowing"};
-      h.m2l_cap = std::max<size_t>(2 * h.m2l_cap, (size_t)(h.hc.n_m2l * 5 / 4 + 1024));
-      h.p2p_cap = std::max<size_t>(2 * h.p2p_cap, (size_t)(h.hc.n_p2p * 5 / 4 + 1024));
+      h.m2l_cap = std::max<size_t>(2 * h.m2l_cap, (size_t)(h.hc->n_m2l * 5 / 4 + 1024));
+      h.p2p_cap = std::max<size_t>(2 * h.p2p_cap, (size_t)(h.hc->n_p2p * 5 / 4 + 1024));
       h.frontier_cap *= 4;
+      h.op_P = -1;  // the dropped entries' keys may hold operator slots
       continue;
     }
-    if (h.hc.frontier[steps % 3] != 0)
+    if (group) {
+      m2l_group_commit(h);
+      h.g_grouped = true;
+    }
+    if (h.hc->frontier[steps % 3] != 0)
       throw Error{EXAFMM_ERR_STATE, "dual-tree walk did not finish in 2*depth+3 steps"};
     break;
   }
-  h.n_m2l = (int64_t)h.hc.n_m2l;
-  h.n_p2p = (int64_t)h.hc.n_p2p;
+  h.n_m2l = (int64_t)h.hc->n_m2l;
+  h.n_p2p = (int64_t)h.hc->n_p2p;
   // The grouped M2L reads the raw entries in any order, so the M2L lists
   // become per-target CSR in the reference's order only when something reads
   // that order: an export, the direct-form kernel, or residual entries.  The

@@ -34,7 +34,6 @@
 //   k_m2l_tc   the mixed form's contraction on tcgen05 (below).
 #include <map>
 #include <mutex>
-#include <unordered_map>
 #include <vector>
 
 #include "fmm.cuh"
@@ -83,8 +82,6 @@ int default_flush(int P) { return P <= 10 ? 2 : (P <= 12 ? 1 : 4); }
 // already in flight gets twice as long): a wait that runs out flags
 // EXAFMM_ERR_TIMEOUT instead of hanging the GPU.
 constexpr long TC_WAIT_NS = 2000000000L;
-// group keys read back with the counts (more take a second read)
-constexpr int OP_KEYS_HOST = 8192;
 
 // Group key of every M2L entry of the ordered CSR lists (expanded to pairs);
 // marks the keys that occur and the targets that have grouped entries.  (The
@@ -92,7 +89,7 @@ constexpr int OP_KEYS_HOST = 8192;
 // With `gscan` (mixed form, periodic): an image entry that has a ghost takes
 // the ghost's free-space key, and its source becomes the ghost's multipole
 // row, ncells + ghost index.
-__global__ void k_gkeys(long n, int2 *pairs, const double4 *xr, const int *level, int *ekey, int *occ,
+__global__ void k_gkeys(long n, int2 *pairs, const double4 *xr, const int *level, int *ekey, unsigned char *occ,
                         int *gflag, int *nres, double cycle, int depth, const int *gscan, int ncells) {
   const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
   int key = -1;
@@ -146,9 +143,72 @@ __global__ void k_csr_pairs(int ncells, const int *off, const u32 *ent, int2 *pa
   }
 }
 
-__global__ void k_key_of_gid(long nkeys, const int *occ, const int *gidx, int *key_of) {
-  const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < nkeys && occ[k]) key_of[gidx[k]] = (int)k;
+// Groups of the marked keys, in key order.  k_occ_words: the marks of 32 keys
+// as a mask, and every tile's number of marks.  k_occ_groups: the groups
+// before each mask (the earlier tiles' counts and a scan of the tile's), and
+// per group the slot of its operator -- from the cache table, or the next
+// free one, its key then listed in newkeys for k_gops (in any order: slots
+// only say where an operator is).
+__global__ void __launch_bounds__(1024) k_occ_words(GroupTables gt) {
+  __shared__ int ws[32];
+  const long w = (long)blockIdx.x * 1024 + threadIdx.x;
+  const uint4 *b = (const uint4 *)gt.occ + 2 * w;
+  const uint4 lo = b[0], hi = b[1];
+  auto nib = [](u32 x) { return (x * 0x10204080u) >> 28; };  // four 0/1 bytes to four bits
+  const u32 m = nib(lo.x) | nib(lo.y) << 4 | nib(lo.z) << 8 | nib(lo.w) << 12 | nib(hi.x) << 16 | nib(hi.y) << 20 |
+                nib(hi.z) << 24 | nib(hi.w) << 28;
+  gt.mask[w].x = m;
+  const int c = __reduce_add_sync(0xffffffffu, __popc(m));
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int t = __reduce_add_sync(0xffffffffu, ws[threadIdx.x]);
+    if (threadIdx.x == 0) gt.sums[blockIdx.x] = t;
+  }
+}
+
+__global__ void __launch_bounds__(1024) k_occ_groups(GroupTables gt, int *optab, int op_count, int *slot_of_gid,
+                                                     int *newkeys, long cap, int *ngroups, int *op_new) {
+  __shared__ int ws[32], s_pre;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long w = (long)blockIdx.x * 1024 + threadIdx.x;
+  int pre = 0;
+  for (int t = threadIdx.x; t < (int)blockIdx.x; t += 1024) pre += gt.sums[t];
+  pre = __reduce_add_sync(0xffffffffu, pre);
+  if (lane == 0) ws[warp] = pre;
+  __syncthreads();
+  if (warp == 0) {
+    const int t = __reduce_add_sync(0xffffffffu, ws[lane]);
+    if (lane == 0) s_pre = t;
+  }
+  __syncthreads();
+  u32 m = gt.mask[w].x;
+  const int c = __popc(m);
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) ws[warp] = incl;
+  __syncthreads();
+  int wpre = 0;
+  for (int k = 0; k < warp; k++) wpre += ws[k];
+  int gid = s_pre + wpre + incl - c;
+  gt.mask[w].y = (u32)gid;
+  for (; m; m &= m - 1, gid++) {
+    if (gid >= cap) break;
+    const int key = (int)(w * 32) + __ffs(m) - 1;
+    int slot = optab[key];
+    if (slot < 0) {
+      const int i = atomicAdd(op_new, 1);
+      newkeys[i] = key;
+      slot = op_count + i;
+      optab[key] = slot;
+    }
+    slot_of_gid[gid] = slot;
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 1023) *ngroups = s_pre + wpre + incl;
 }
 
 struct PlanDev {
@@ -214,10 +274,10 @@ __device__ double op_value(int row, int col, int P, int NT, int dl, const double
 }
 
 // One CTA per group: the realified, scaled operator in row-block layout.
-__global__ void k_gops(const int *keys, const int *slots, PlanDev pd, double *ops, KeyGeom kg) {
+__global__ void k_gops(const int *keys, int slot0, PlanDev pd, double *ops, KeyGeom kg) {
   extern __shared__ double2 Zsh[];  // NT irregular harmonics of v
   const int dl = group_harmonics(keys[blockIdx.x], pd.P, Zsh, kg);
-  double *W = ops + (size_t)slots[blockIdx.x] * pd.wsize;
+  double *W = ops + (size_t)(slot0 + blockIdx.x) * pd.wsize;
   for (int i = threadIdx.x; i < pd.wsize; i += blockDim.x) {
     int rb = 0;
     while (pd.woff[rb + 1] <= i) rb++;
@@ -379,12 +439,12 @@ struct TcFixed {
 
 // One CTA per group: the operator split into FP16 hi + lo parts, written as
 // the byte image the MMA reads from shared memory (hi image, then lo image).
-__global__ void k_gops16(const int *keys, const int *slots, int P, TcPlan pl, __half *ops16, KeyGeom kg) {
+__global__ void k_gops16(const int *keys, int slot0, int P, TcPlan pl, __half *ops16, KeyGeom kg) {
   extern __shared__ double2 Zsh[];
   const int NT = tri(P);
   const int dl = group_harmonics(keys[blockIdx.x], P, Zsh, kg);
   const int nh = pl.bimg / 2;  // halves per image
-  __half *Wh = ops16 + (size_t)slots[blockIdx.x] * 2 * nh;  // the whole image (hi and lo parts)
+  __half *Wh = ops16 + (size_t)(slot0 + blockIdx.x) * 2 * nh;  // the whole image (hi and lo parts)
   for (int e = threadIdx.x; e < nh; e += blockDim.x) {
     const int byte = 2 * e;
     // `byte` enumerates the hi values block by block, atom by atom; its hi
@@ -602,21 +662,21 @@ __global__ void k_tiles(int ntiles, int tile_n, int nflag, const u32 *sorted, in
 // order, groups in order within a tile), then write each entry's source into
 // its segment's slot.  A target has at most one entry per group, so every
 // (segment, slot) is written once.
-__global__ void k_gmark(long n, const int2 *pairs, const int *ekey, const int *gidx, const int *tslot, int tile_n,
+__global__ void k_gmark(long n, const int2 *pairs, const int *ekey, const uint2 *gmask, const int *tslot, int tile_n,
                         int ngroups, int *mark) {
   const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n || ekey[e] < 0) return;
   const int t = pairs[e].x & (int)IDX_MASK;
-  mark[(long)(tslot[t] / tile_n) * ngroups + gidx[ekey[e]]] = 1;
+  mark[(long)(tslot[t] / tile_n) * ngroups + group_id(gmask, ekey[e])] = 1;
 }
 
-__global__ void k_gfill(long n, const int2 *pairs, const int *ekey, const int *gidx, const int *tslot, int tile_n,
+__global__ void k_gfill(long n, const int2 *pairs, const int *ekey, const uint2 *gmask, const int *tslot, int tile_n,
                         int ngroups, const int *segid, int *tg_src) {
   const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n || ekey[e] < 0) return;
   const int2 pr = pairs[e];
   const int ts = tslot[pr.x & (int)IDX_MASK];
-  const int sg = segid[(long)(ts / tile_n) * ngroups + gidx[ekey[e]]];
+  const int sg = segid[(long)(ts / tile_n) * ngroups + group_id(gmask, ekey[e])];
   tg_src[(long)sg * tile_n + ts % tile_n] = pr.y;
 }
 
@@ -1471,6 +1531,83 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
   h.launches++;
 }
 
+bool m2l_groups_raw(const Handle &h) {
+  return h.prm.dim != 2 && !h.force_direct_m2l && m2l_grouped_available(h.prm.P) &&
+         !(h.prm.images > 0 && h.prm.precision == EXAFMM_MIXED && tc_available(h.prm.P));
+}
+
+// Queues, after the key and target marks: the group tables, the operator
+// slots, and the flagged targets' tile keys.  max_groups: an upper bound of
+// the groups.
+void m2l_group_launch(Handle &h, long max_groups) {
+  cudaStream_t s = h.stream;
+  const int P = h.prm.P, C = h.ncells;
+  const int layout = h.prm.precision == EXAFMM_MIXED && tc_available(P) ? 1 : 0;
+  const long ks = key_space(h.prm.images, h.depth), cap = std::min(ks, max_groups);
+  const double cyc = h.prm.images ? h.prm.cycle : 0.0;
+  // the cache holds operators of one order, layout and key space; image keys
+  // also depend on the period, the root radius and the depth
+  const bool geom_changed =
+      h.prm.images > 0 && (h.op_cycle != cyc || h.op_R0 != h.root_R0 || h.op_depth != h.depth);
+  if (h.op_P != P || h.op_layout != layout || h.op_ks != ks || geom_changed) {
+    h.g_optab.need((size_t)ks * sizeof(int));
+    FMM_CUDA(cudaMemsetAsync(h.g_optab.p, 0xff, (size_t)ks * sizeof(int), s));
+    h.op_count = 0;
+    h.op_layout = layout;
+    h.op_ks = ks;
+    h.op_cycle = cyc;
+    h.op_R0 = h.root_R0;
+    h.op_depth = h.depth;
+  }
+  h.op_P = -1;  // until m2l_group_commit() has built what the table now holds
+  const GroupTables gt = group_tables(h.g_occ.p, ks);
+  h.g_slot.need((size_t)cap * sizeof(int));
+  h.g_newkeys.need((size_t)cap * sizeof(int));
+  DevCounters *ctr = h.counters.as<DevCounters>();
+  const unsigned nt = (unsigned)(ks / OCC_TILE);
+  k_occ_words<<<nt, 1024, 0, s>>>(gt);
+  k_occ_groups<<<nt, 1024, 0, s>>>(gt, h.g_optab.as<int>(), h.op_count, h.g_slot.as<int>(), h.g_newkeys.as<int>(), cap,
+                                   &ctr->gcounts[2], &ctr->op_new);
+  h.g_tk.need((size_t)C * 2 * (sizeof(u64) + sizeof(u32)) + 64);
+  u64 *tk = h.g_tk.as<u64>();
+  k_tkeys<<<grid_for(C, TB), TB, 0, s>>>(C, h.g_cnt.as<int>(), h.c_level.as<int>(), h.c_parent.as<int>(),
+                                         h.c_child.as<int>(), tk, (u32 *)(tk + 2 * (size_t)C), ctr->gcounts);
+  h.launches += 3;
+  FMM_LAUNCH();
+}
+
+void m2l_group_commit(Handle &h) {
+  cudaStream_t s = h.stream;
+  const int P = h.prm.P, NT = tri(P), nnew = h.hc->op_new;
+  if (nnew > 0) {
+    const bool tcore = h.op_layout == 1;
+    PlanCache &pc = plan_cache(P);
+    const TcPlan tp = make_tc_plan(P, tc_kp(P), tc_pair_first(P));
+    const size_t op_bytes = tcore ? (size_t)2 * tp.bimg : (size_t)pc.host.wsize * sizeof(double);
+    const size_t nslots = (size_t)h.op_count + nnew;
+    if (nslots * op_bytes > h.g_ops.bytes) {  // grow, keeping the operators built so far
+      Buf grown;
+      grown.need(std::max(nslots, (size_t)64) * op_bytes * 2);
+      if (h.g_ops.p && h.op_count > 0)
+        FMM_CUDA(cudaMemcpyAsync(grown.p, h.g_ops.p, (size_t)h.op_count * op_bytes, cudaMemcpyDeviceToDevice, s));
+      FMM_CUDA(cudaStreamSynchronize(s));
+      h.g_ops.release();
+      h.g_ops = grown;
+    }
+    const KeyGeom kg{h.c_xr.as<double4>(), h.op_cycle, h.op_depth};
+    if (tcore)
+      k_gops16<<<nnew, 256, NT * sizeof(double2), s>>>(h.g_newkeys.as<int>(), h.op_count, P, tp, h.g_ops.as<__half>(),
+                                                        kg);
+    else
+      k_gops<<<nnew, 128, NT * sizeof(double2), s>>>(h.g_newkeys.as<int>(), h.op_count, plan_dev(pc),
+                                                      h.g_ops.as<double>(), kg);
+    h.launches++;
+    FMM_LAUNCH();
+    h.op_count += nnew;
+  }
+  h.op_P = P;
+}
+
 void m2l_grouped_pass(Handle &h) {
   cudaStream_t s = h.stream;
   const int P = h.prm.P, NT = tri(P), C = h.ncells;
@@ -1544,11 +1681,10 @@ void m2l_grouped_pass(Handle &h) {
   const int2 *pairs = h.m2l_raw.as<int2>();
   const int *ekey = h.m2l_key.as<int>();
   const long ks = key_space(h.prm.images, h.depth);
-  int *occ = h.g_occ.as<int>(), *gidx = occ + ks;  // sized by build_lists
+  const GroupTables gt = group_tables(h.g_occ.p, ks);  // sized by build_lists
   int *gflag = h.g_cnt.as<int>(), *tslot = gflag + C;
   DevCounters *ctr = h.counters.as<DevCounters>();
   int *counts = ctr->gcounts;
-  FMM_CUDA(cudaMemsetAsync(counts, 0, 4 * sizeof(int), s));
   // keys computed here: for the ordered lists, and for the mixed form's
   // periodic entries (ghost sources change their keys)
   const bool ghosts = tcore && h.prm.images > 0;
@@ -1564,7 +1700,9 @@ void m2l_grouped_pass(Handle &h) {
       FMM_CUDA(cudaMemcpyAsync(h.g_pairs.p, h.m2l_raw.p, nent * sizeof(int2), cudaMemcpyDeviceToDevice, s));
     pairs = h.g_pairs.as<int2>();
     h.g_ekey.need(nent * sizeof(int));
-    FMM_CUDA(cudaMemsetAsync(occ, 0, (size_t)ks * sizeof(int), s));
+    FMM_CUDA(cudaMemsetAsync(counts, 0, 4 * sizeof(int), s));
+    FMM_CUDA(cudaMemsetAsync(&ctr->op_new, 0, sizeof(int), s));
+    FMM_CUDA(cudaMemsetAsync(gt.occ, 0, (size_t)ks, s));
     FMM_CUDA(cudaMemsetAsync(gflag, 0, (size_t)C * sizeof(int), s));
     // ghosts: image entries with a tiny fractional offset use free-space
     // keys (mixed form only: the FP64 form keeps the reference's offsets)
@@ -1583,31 +1721,22 @@ void m2l_grouped_pass(Handle &h) {
       h.launches += 2;
     }
     k_gkeys<<<grid_for(nent, TB), TB, 0, s>>>(nent, h.g_pairs.as<int2>(), h.c_xr.as<double4>(), h.c_level.as<int>(),
-                                              h.g_ekey.as<int>(), occ, gflag, &counts[0], cyc, h.depth, gscan, C);
+                                              h.g_ekey.as<int>(), gt.occ, gflag, &counts[0], cyc, h.depth, gscan, C);
     ekey = h.g_ekey.as<int>();
     h.launches += 2;
   }
-  // dense group ids, the key of each, the flagged targets in tile order;
-  // then one read of the counts and of the keys (for the operator cache)
-  scan_exclusive_int(h, occ, gidx, ks, &counts[2]);
-  const long keys_cap = std::max<long>(OP_KEYS_HOST, std::min<long>(ks, nent));
-  h.g_keyof.need((size_t)keys_cap * sizeof(int));
-  k_key_of_gid<<<grid_for(ks, TB), TB, 0, s>>>(ks, occ, gidx, h.g_keyof.as<int>());
-  h.g_tk.need((size_t)C * 2 * (sizeof(u64) + sizeof(u32)) + 64);
-  u64 *tk = h.g_tk.as<u64>(), *tk2 = tk + C;
-  u32 *tv = (u32 *)(tk2 + C), *tv2 = tv + C;
-  k_tkeys<<<grid_for(C, TB), TB, 0, s>>>(C, gflag, h.c_level.as<int>(), h.c_parent.as<int>(), h.c_child.as<int>(),
-                                         tk, tv, counts);
-  if (!h.keys_host) FMM_CUDA(cudaMallocHost((void **)&h.keys_host, OP_KEYS_HOST * sizeof(int)));
-  FMM_CUDA(cudaMemcpyAsync(&h.hc, ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-  FMM_CUDA(cudaMemcpyAsync(h.keys_host, h.g_keyof.p, OP_KEYS_HOST * sizeof(int), cudaMemcpyDeviceToHost, s));
-  double4 root{};
-  FMM_CUDA(cudaMemcpyAsync(&root, h.c_xr.p, sizeof(double4), cudaMemcpyDeviceToHost, s));
-  FMM_CUDA(cudaStreamSynchronize(s));
-  const int nres = rekey ? h.hc.gcounts[0] : h.hc.walk_resid;
-  const int nflag = h.hc.gcounts[1], ngroups = h.hc.gcounts[2];
-  h.g_nghost = rekey ? h.hc.nghost : 0;
-  h.launches += 4;
+  // dense group ids, the operator slot of each, the flagged targets' tile
+  // keys: from the lists, or made here from the keys just computed
+  if (rekey) {
+    m2l_group_launch(h, nent);
+    read_counters(h);
+    m2l_group_commit(h);
+  } else if (!h.g_grouped) {
+    throw Error{EXAFMM_ERR_STATE, "grouped M2L without the lists' group tables"};
+  }
+  const int nres = rekey ? h.hc->gcounts[0] : h.hc->walk_resid;
+  const int nflag = h.hc->gcounts[1], ngroups = h.hc->gcounts[2];
+  h.g_nghost = rekey ? h.hc->nghost : 0;
   if (nres > 0 && !h.m2l_ordered) {  // residual entries are summed in list order: order, then start over
     order_m2l_lists(h);
     m2l_grouped_pass(h);
@@ -1615,73 +1744,10 @@ void m2l_grouped_pass(Handle &h) {
   }
   h.g_ngroups = ngroups;
   if (ngroups > 0) {
-    // operators: cached per handle by group key (they depend only on the key
-    // and P); only keys not seen before are built
-    const int layout = tcore ? 1 : 0;
-    // image keys also depend on the period, the root radius and the depth
-    const bool img_geom_changed = h.prm.images > 0 && (h.op_cycle != cyc || h.op_R0 != root.w || h.op_depth != h.depth);
-    if (h.op_P != P || h.op_layout != layout || img_geom_changed) {
-      h.op_slot.clear();
-      h.op_P = P;
-      h.op_layout = layout;
-    }
-    if (h.prm.images > 0) {
-      h.op_cycle = cyc;
-      h.op_R0 = root.w;
-      h.op_depth = h.depth;
-    }
-    const size_t op_bytes = tcore ? (size_t)2 * tp.bimg : (size_t)gp.wsize * sizeof(double);
-    std::vector<int> &key_of = h.op_host_keys;
-    key_of.assign(h.keys_host, h.keys_host + std::min(ngroups, OP_KEYS_HOST));
-    if (ngroups > OP_KEYS_HOST) {  // more keys than the first read carried
-      key_of.resize(ngroups);
-      FMM_CUDA(cudaMemcpy(key_of.data() + OP_KEYS_HOST, h.g_keyof.as<int>() + OP_KEYS_HOST,
-                          (size_t)(ngroups - OP_KEYS_HOST) * sizeof(int), cudaMemcpyDeviceToHost));
-    }
-    std::vector<int> &slot_of = h.op_host_slots, &new_keys = h.op_host_new_keys, &new_slots = h.op_host_new_slots;
-    slot_of.resize(ngroups);
-    new_keys.clear();
-    new_slots.clear();
-    for (int g = 0; g < ngroups; g++) {
-      auto it = h.op_slot.find(key_of[g]);
-      if (it == h.op_slot.end()) {
-        const int sl = (int)h.op_slot.size();
-        it = h.op_slot.emplace(key_of[g], sl).first;
-        new_keys.push_back(key_of[g]);
-        new_slots.push_back(sl);
-      }
-      slot_of[g] = it->second;
-    }
-    const size_t nslots = h.op_slot.size();
-    if (nslots * op_bytes > h.g_ops.bytes) {  // grow, keeping the operators built so far
-      Buf grown;
-      grown.need(std::max(nslots, (size_t)64) * op_bytes * 2);
-      if (h.g_ops.p && nslots > new_keys.size())
-        FMM_CUDA(cudaMemcpyAsync(grown.p, h.g_ops.p, (nslots - new_keys.size()) * op_bytes, cudaMemcpyDeviceToDevice,
-                                 s));
-      FMM_CUDA(cudaStreamSynchronize(s));
-      h.g_ops.release();
-      h.g_ops = grown;
-    }
-    h.g_slot.need((size_t)(ngroups + 2 * new_keys.size() + 2) * sizeof(int));
-    int *d_slot_of = h.g_slot.as<int>(), *d_new_keys = d_slot_of + ngroups,
-        *d_new_slots = d_new_keys + new_keys.size();
-    FMM_CUDA(cudaMemcpyAsync(d_slot_of, slot_of.data(), (size_t)ngroups * sizeof(int), cudaMemcpyHostToDevice, s));
-    if (!new_keys.empty()) {
-      FMM_CUDA(cudaMemcpyAsync(d_new_keys, new_keys.data(), new_keys.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-      FMM_CUDA(cudaMemcpyAsync(d_new_slots, new_slots.data(), new_slots.size() * sizeof(int), cudaMemcpyHostToDevice,
-                               s));
-      const KeyGeom kg{h.c_xr.as<double4>(), cyc, h.depth};
-      if (tcore)
-        k_gops16<<<(int)new_keys.size(), 256, NT * sizeof(double2), s>>>(d_new_keys, d_new_slots, P, tp,
-                                                                          h.g_ops.as<__half>(), kg);
-      else
-        k_gops<<<(int)new_keys.size(), 128, NT * sizeof(double2), s>>>(d_new_keys, d_new_slots, pd,
-                                                                        h.g_ops.as<double>(), kg);
-      h.launches++;
-    }
     // tiles of targets
     const int ntiles = (nflag + tile_n - 1) / tile_n;
+    u64 *tk = h.g_tk.as<u64>(), *tk2 = tk + C;
+    u32 *tv = (u32 *)(tk2 + C), *tv2 = tv + C;
     radix_sort_pairs(h, tk, tv, tk2, tv2, C, 0, 8);
     h.g_tile.need((size_t)ntiles * tile_n * sizeof(int) + 64);
     k_tiles<<<grid_for((long)ntiles * tile_n, TB), TB, 0, s>>>(ntiles, tile_n, nflag, tv, h.g_tile.as<int>(), tslot);
@@ -1690,22 +1756,21 @@ void m2l_grouped_pass(Handle &h) {
     h.g_seg.need((size_t)(nmark + 1) * sizeof(int) * 2);
     int *mark = h.g_seg.as<int>(), *segid = mark + nmark + 1;
     FMM_CUDA(cudaMemsetAsync(mark, 0, (size_t)nmark * sizeof(int), s));
-    k_gmark<<<grid_for(nent, TB), TB, 0, s>>>(nent, pairs, ekey, gidx, tslot, tile_n, ngroups, mark);
+    k_gmark<<<grid_for(nent, TB), TB, 0, s>>>(nent, pairs, ekey, gt.mask, tslot, tile_n, ngroups, mark);
     scan_exclusive_int(h, mark, segid, nmark, &counts[3]);
     // segment tables sized for every (tile, group) pair when that is small
     // (no read of the segment count), else read the count
     long nseg = nmark;
     if ((size_t)nmark * (tile_n + 1) * sizeof(int) > ((size_t)1 << 30)) {
-      FMM_CUDA(cudaMemcpyAsync(&h.hc, ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-      FMM_CUDA(cudaStreamSynchronize(s));
-      nseg = h.hc.gcounts[3];
+      read_counters(h);
+      nseg = h.hc->gcounts[3];
     }
     h.g_tg.need(((size_t)nseg * (tile_n + 1) + ntiles + 2) * sizeof(int));
     // tg_src first: its rows of tile_n slots stay 16-byte aligned
     int *tg_src = h.g_tg.as<int>(), *tg_gid = tg_src + (size_t)nseg * tile_n, *tg_off = tg_gid + nseg;
     k_fill_rows<<<148 * 4, TB, 0, s>>>(tg_src, &counts[3], tile_n);  // absent targets: -1
-    k_gfill<<<grid_for(nent, TB), TB, 0, s>>>(nent, pairs, ekey, gidx, tslot, tile_n, ngroups, segid, tg_src);
-    k_seg_gid<<<grid_for(nmark, TB), TB, 0, s>>>(nmark, ngroups, mark, segid, d_slot_of, tg_gid);
+    k_gfill<<<grid_for(nent, TB), TB, 0, s>>>(nent, pairs, ekey, gt.mask, tslot, tile_n, ngroups, segid, tg_src);
+    k_seg_gid<<<grid_for(nmark, TB), TB, 0, s>>>(nmark, ngroups, mark, segid, h.g_slot.as<int>(), tg_gid);
     k_tg_off<<<grid_for(ntiles + 1, TB), TB, 0, s>>>(ntiles, ngroups, segid, &counts[3], tg_off);
     h.g_ntiles = ntiles;
     h.g_nseg = nseg;  // an upper bound unless it was read

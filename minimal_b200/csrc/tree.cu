@@ -456,16 +456,15 @@ void build_tree(Handle &h) {
     h.launches++;
     FMM_LAUNCH();
     scan_exclusive_int(h, h.chain.as<int>(), h.prebase.as<int>(), n, &ctr->ncells);
-    FMM_CUDA(cudaMemcpyAsync(&h.hc, ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-    FMM_CUDA(cudaStreamSynchronize(s));
-    if (h.hc.overflow) {
+    read_counters(h);
+    if (h.hc->overflow) {
       if (D == max_levels)
         throw Error{EXAFMM_ERR_DEPTH, "more than ncrit bodies share a cell at the deepest level (" +
                                           std::to_string(max_levels) + "): coincident bodies?"};
       D = max_levels;
       continue;
     }
-    const long C = h.hc.ncells;
+    const long C = h.hc->ncells;
     h.ncells = (int)C;
     h.key_levels = D;
     // pre-order tables (reuse the idle sort buffers' siblings)
@@ -515,14 +514,15 @@ void build_tree(Handle &h) {
     k_compact_leaves<<<grid_for(C, TB), TB, 0, s>>>(is_leaf, leafpos, C, h.leaves.as<int>());
     h.launches++;
     FMM_LAUNCH();
-    FMM_CUDA(cudaMemcpyAsync(&h.hc, ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-    FMM_CUDA(cudaStreamSynchronize(s));
-    h.nleaves = h.hc.nleaves;
+    if (h.prm.images > 0)  // the root radius, for the M2L operators of image keys
+      FMM_CUDA(cudaMemcpyAsync(&h.root_R0, &g->R0, sizeof(double), cudaMemcpyDeviceToHost, s));
+    read_counters(h);
+    h.nleaves = h.hc->nleaves;
     h.depth = 0;
     h.level_base[0] = 0;
     for (int l = 0; l <= EXAFMM_MAX_LEVEL; l++) {
-      h.level_base[l + 1] = h.level_base[l] + h.hc.level_count[l];
-      if (h.hc.level_count[l]) h.depth = l;
+      h.level_base[l + 1] = h.level_base[l] + h.hc->level_count[l];
+      if (h.hc->level_count[l]) h.depth = l;
     }
     // 6. bodies of each leaf back to input order and gathered (the mixed
     // form's FP32 sources with them)
