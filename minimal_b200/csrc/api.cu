@@ -102,7 +102,7 @@ void need_3d(Handle &h, const char *what) {
 
 // Body records (8 doubles in 3D, 6 in 2D: X[dim], q, p, F[dim]) -> x, y, z, q
 // (z = 0 in 2D).
-__global__ void k_pack_in(const double *rec, long n, int len, double4 *in, int *bad) {
+__global__ void k_pack_in(const double *rec, long n, int len, double4 *in, volatile int *bad) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double *r = rec + len * i;
@@ -111,7 +111,7 @@ __global__ void k_pack_in(const double *rec, long n, int len, double4 *in, int *
   in[i] = v;
 }
 
-__global__ void k_check_finite(const double *q, long n, int *bad) {
+__global__ void k_check_finite(const double *q, long n, volatile int *bad) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && !isfinite(q[i])) *bad = 1;
 }
@@ -349,7 +349,9 @@ int exafmm_b200_create(const exafmm_params *params, exafmm_b200 **out) {
       FMM_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     FMM_CUDA(cudaMallocHost(&h.flags_host, 4 * sizeof(int)));
     FMM_CUDA(cudaMallocHost(&h.hc, sizeof(DevCounters)));
-    h.flags_host[0] = 0;
+    h.flags_host[0] = h.flags_host[1] = 0;
+    h.counters.need(sizeof(DevCounters));
+    FMM_CUDA(cudaMemsetAsync(h.counters.p, 0, sizeof(DevCounters), h.stream));
     h.ev_ok = true;
     for (int p = 0; p < PH_COUNT + 1; p++)
       for (int k = 0; k < 2; k++)
@@ -432,11 +434,9 @@ int exafmm_b200_set_bodies(exafmm_b200 *H, const double *rec, int64_t n, int whe
     FMM_CUDA(cudaSetDevice(h.prm.device));
     h.n = n;
     h.in.need(n * sizeof(double4));
-    h.counters.need(sizeof(DevCounters));
     const double *drec = rec;
     const int len = rec_len(h);
-    int *bad = &h.counters.as<DevCounters>()->overflow;
-    FMM_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), h.stream));
+    h.flags_host[1] = 0;
     // whole records cross the bus (a strided copy of only X and q, half the
     // bytes, measured slower: the copy engine moves 32-byte rows poorly)
     if (where == EXAFMM_HOST) {
@@ -444,13 +444,11 @@ int exafmm_b200_set_bodies(exafmm_b200 *H, const double *rec, int64_t n, int whe
       FMM_CUDA(cudaMemcpyAsync(h.stage.p, rec, n * len * sizeof(double), cudaMemcpyHostToDevice, h.stream));
       drec = h.stage.as<double>();
     }
-    k_pack_in<<<grid_for(n, 256), 256, 0, h.stream>>>(drec, n, len, h.in.as<double4>(), bad);
+    k_pack_in<<<grid_for(n, 256), 256, 0, h.stream>>>(drec, n, len, h.in.as<double4>(), h.flags_host + 1);
     h.launches++;
     FMM_LAUNCH();
-    int hb = 0;
-    FMM_CUDA(cudaMemcpyAsync(&hb, bad, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
     FMM_CUDA(cudaStreamSynchronize(h.stream));
-    if (hb) throw Error{EXAFMM_ERR_ARG, "non-finite body position or charge"};
+    if (h.flags_host[1]) throw Error{EXAFMM_ERR_ARG, "non-finite body position or charge"};
     h.have_tree = h.have_lists = h.have_up = h.have_horiz = h.have_down = false;
     h.nsys = 1;
     h.sys_off_host.clear();
@@ -534,15 +532,12 @@ int exafmm_b200_set_charges(exafmm_b200 *H, const double *q, int where) {
       FMM_CUDA(cudaMemcpyAsync(h.stage.p, q, h.n * sizeof(double), cudaMemcpyHostToDevice, h.stream));
       dq = h.stage.as<double>();
     }
-    int *bad = &h.counters.as<DevCounters>()->overflow;
-    FMM_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), h.stream));
-    k_check_finite<<<grid_for(h.n, 256), 256, 0, h.stream>>>(dq, h.n, bad);
+    h.flags_host[1] = 0;
+    k_check_finite<<<grid_for(h.n, 256), 256, 0, h.stream>>>(dq, h.n, h.flags_host + 1);
     h.launches++;
     FMM_LAUNCH();
-    int hb = 0;
-    FMM_CUDA(cudaMemcpyAsync(&hb, bad, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
     FMM_CUDA(cudaStreamSynchronize(h.stream));
-    if (hb) throw Error{EXAFMM_ERR_ARG, "non-finite charge"};  // nothing changed
+    if (h.flags_host[1]) throw Error{EXAFMM_ERR_ARG, "non-finite charge"};  // nothing changed
     k_set_charges<<<grid_for(h.n, 256), 256, 0, h.stream>>>(dq, h.n, h.in.as<double4>(), h.perm.as<int>(),
                                                            h.have_tree ? h.src.as<double4>() : nullptr);
     h.launches++;

@@ -79,12 +79,12 @@ struct DevCounters {
   int max_m2l_seg, max_p2p_seg;
   int gcounts[4];      // grouped M2L: residual entries, flagged targets, groups, segments
   unsigned long long gfill;
-  int tc_error;        // a bounded tensor-core wait ran out
   // largest |scaled multipole| over the possible M2L sources, as the bits of
   // a non-negative double (the FP16 split's power-of-two normalisation)
   unsigned long long m16_max;
   int nghost;  // ghost sources of image entries (mixed form, periodic)
   int op_new;  // group keys without a cached M2L operator
+  unsigned bounds_ticket;  // blocks of the bounds kernel that are done (0 between launches)
 };
 
 // Per-phase timing slots (CUDA events on the handle stream).
@@ -201,8 +201,9 @@ struct Handle {
   // phase state
   bool have_tree = false, have_lists = false, have_up = false, have_horiz = false, have_down = false;
 
-  // device error flags copied back on the stream (pinned), checked after
-  // each synchronisation: [0] a bounded tensor-core wait ran out
+  // error flags in pinned host memory, set by kernels and checked after each
+  // synchronisation: [0] a bounded tensor-core wait ran out, [1] a body or
+  // charge handed in is not finite
   int *flags_host = nullptr;
 
   cudaEvent_t ev[PH_COUNT + 1][2];
@@ -213,6 +214,8 @@ struct Handle {
 // ---- launchers (each .cu file) ----
 // scan.cu / sort.cu
 void scan_exclusive_int(Handle &h, const int *in, int *out, long n, int *total_dev);
+void scan_exclusive_pair(Handle &h, const int *in0, int *out0, int *total0, const int *in1, int *out1, int *total1,
+                         long n);
 void radix_sort_pairs(Handle &h, u64 *&k, u32 *&v, u64 *&k2, u32 *&v2, long n, int lo_bit, int hi_bit);
 // tree.cu
 void build_tree(Handle &h);

@@ -138,21 +138,29 @@ __device__ __forceinline__ void m2l_mark_key(int key, int t, unsigned char *occ,
   if (gflag[t] == 0) gflag[t] = 1;
 }
 
-// Group tables of a key space of ks keys (a multiple of OCC_TILE), one buffer:
-// the marks (a byte per key), then per 32 keys {marks as a mask, groups before
-// them}, then per tile the number of marked keys.
+// Group tables of a key space of ks keys (a multiple of OCC_TILE) and a tree
+// of C cells, one buffer: the marks of the keys (a byte each) and of the
+// targets, the P2P counts of the targets (all three zeroed together), then
+// per 32 keys {marks as a mask, groups before them}, then per tile the number
+// of marked keys.
 constexpr long OCC_TILE = 32768;
 static_assert(KEY_SPACE % OCC_TILE == 0 && IKEY_SPACE % OCC_TILE == 0, "whole tiles of group keys");
 struct GroupTables {
   unsigned char *occ;
+  int *gflag, *cnt;  // C targets; C + 1 counts
   uint2 *mask;
   int *sums;
 };
-inline size_t group_table_bytes(long ks) { return (size_t)ks + (size_t)ks / 32 * sizeof(uint2) + ks / OCC_TILE * sizeof(int); }
-inline GroupTables group_tables(void *p, long ks) {
+inline size_t group_cells(int C) { return ((size_t)C + 3) / 4 * 4; }  // the counts start 16-byte aligned
+inline size_t group_mark_bytes(long ks, int C) { return (size_t)ks + (group_cells(C) + C + 1) * sizeof(int); }
+inline size_t group_table_bytes(long ks, int C) {
+  return (group_mark_bytes(ks, C) + 15) / 16 * 16 + (size_t)ks / 32 * sizeof(uint2) + ks / OCC_TILE * sizeof(int);
+}
+inline GroupTables group_tables(void *p, long ks, int C) {
   unsigned char *b = (unsigned char *)p;
-  uint2 *m = (uint2 *)(b + ks);
-  return GroupTables{b, m, (int *)(m + ks / 32)};
+  int *f = (int *)(b + ks);
+  uint2 *m = (uint2 *)(b + (group_mark_bytes(ks, C) + 15) / 16 * 16);
+  return GroupTables{b, f, f + group_cells(C), m, (int *)(m + ks / 32)};
 }
 
 // Group id of a marked key.

@@ -55,14 +55,41 @@ __device__ __forceinline__ int radius_level_diff(double rb, double ra) {
 // ranges of CHUNK pairs; a thread's entries of one list are consecutive.
 // PERIODIC false: every pair is of image 13 (no shift), so the shift terms,
 // zero, are left out: x - 0 is x in every rounding.
+constexpr int CHUNK = TB * WALK_PAIRS;  // frontier pairs of one block iteration
+
+struct WalkArgs {
+  CellView cv;
+  int2 *front[2];                // frontiers of the even and odd steps
+  unsigned long long *nfront;    // their counts, three words in rotation
+  u64 fcap;
+  int2 *m2l, *p2p;
+  unsigned long long *nm2l, *np2p;
+  u64 mcap, pcap;
+  double theta, cycle;
+  int depth;
+  int *overflow, *m2l_key;
+  unsigned char *occ;
+  int *gflag, *nres;
+};
+
+// Step st: reads frontier st & 1 and count word st % 3, appends to the other
+// frontier and word (st + 1) % 3, and zeroes word (st + 2) % 3, which
+// nothing reads any more.
 template <int WP, bool PERIODIC>
-__global__ void __launch_bounds__(TB) k_walk(CellView cv, const int2 *fin, const unsigned long long *nin_p,
-                                            int2 *fout, unsigned long long *nout, unsigned long long *nnext,
-                                            u64 fcap, int2 *m2l, unsigned long long *nm2l, u64 mcap, int2 *p2p,
-                                            unsigned long long *np2p, u64 pcap, double theta, double cycle,
-                                            int depth, int *overflow, int *m2l_key, unsigned char *occ, int *gflag,
-                                            int *nres) {
-  constexpr int NW = TB / 32, CHUNK = TB * WP;
+__device__ __forceinline__ void walk_step(const WalkArgs &wa, int st) {
+  const CellView &cv = wa.cv;
+  const int2 *fin = wa.front[st & 1];
+  int2 *fout = wa.front[(st & 1) ^ 1], *m2l = wa.m2l, *p2p = wa.p2p;
+  const unsigned long long *nin_p = &wa.nfront[st % 3];
+  unsigned long long *nout = &wa.nfront[(st + 1) % 3], *nnext = &wa.nfront[(st + 2) % 3];
+  unsigned long long *nm2l = wa.nm2l, *np2p = wa.np2p;
+  const u64 fcap = wa.fcap, mcap = wa.mcap, pcap = wa.pcap;
+  const double theta = wa.theta, cycle = wa.cycle;
+  const int depth = wa.depth;
+  int *overflow = wa.overflow, *m2l_key = wa.m2l_key, *gflag = wa.gflag;
+  unsigned char *occ = wa.occ;
+  constexpr int NW = TB / 32;
+  static_assert(WP == WALK_PAIRS, "CHUNK follows WALK_PAIRS");
   static_assert(CHUNK < 4096, "per-block M2L and P2P counts are packed in 12-bit fields");
   __shared__ int s_tot[NW], s_totk[NW];    // every warp's packed list counts and frontier count
   __shared__ unsigned long long s_base[3];  // the block's M2L, P2P and frontier ranges
@@ -71,8 +98,7 @@ __global__ void __launch_bounds__(TB) k_walk(CellView cv, const int2 *fin, const
   int res = 0;
   // the producer counts appends past its capacity (to size the retry); only
   // the stored entries may be read
-  const u64 nin = min((u64)*nin_p, fcap);
-  // the counter the step after next appends to: nothing reads it any more
+  const u64 nin = min((u64)__ldcg(nin_p), fcap);
   if (blockIdx.x == 0 && threadIdx.x == 0) *nnext = 0;
   const u64 stride = (u64)gridDim.x * CHUNK;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -195,13 +221,17 @@ __global__ void __launch_bounds__(TB) k_walk(CellView cv, const int2 *fin, const
   }
   if (res) atomicAdd_block(&s_res, res);
   __syncthreads();
-  if (threadIdx.x == 0 && s_res) atomicAdd(nres, s_res);
+  if (threadIdx.x == 0 && s_res) atomicAdd(wa.nres, s_res);
+}
+
+template <int WP, bool PERIODIC>
+__global__ void __launch_bounds__(TB) k_walk(WalkArgs wa, int st) {
+  walk_step<WP, PERIODIC>(wa, st);
 }
 
 // Root pairs of the walk: (root, root) of every system of a batch (the roots
 // are the first nsys cells), or the 27 image pairs of a periodic system.
-__global__ void k_seed(int2 *f, unsigned long long *n, int images, int nsys, int dim) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void walk_seed(int t, int2 *f, unsigned long long *n, int images, int nsys, int dim) {
   if (images == 0) {
     if (t < nsys) f[t] = make_int2(t | (13 << IMG_SHIFT), t);
     if (t == 0) *n = (unsigned long long)nsys;
@@ -222,6 +252,23 @@ __global__ void k_seed(int2 *f, unsigned long long *n, int images, int nsys, int
   }
 }
 
+__global__ void k_seed(int2 *f, unsigned long long *n, int images, int nsys, int dim) {
+  walk_seed(blockIdx.x * blockDim.x + threadIdx.x, f, n, images, nsys, dim);
+}
+
+// The seeds and the first steps, whose frontiers (at most 8 times the step
+// before) fit one block iteration: one block in one launch, where each of
+// these steps was a launch of its own over all SMs (about 5 us).
+template <int WP, bool PERIODIC>
+__global__ void __launch_bounds__(TB) k_walk_head(WalkArgs wa, int nsteps, int images, int nsys, int dim) {
+  for (int t = threadIdx.x; t < max(nsys, 32); t += TB) walk_seed(t, wa.front[0], &wa.nfront[0], images, nsys, dim);
+  for (int st = 0; st < nsteps; st++) {
+    __threadfence();
+    __syncthreads();
+    walk_step<WP, PERIODIC>(wa, st);
+  }
+}
+
 // Entries of one target often arrive together (a split emits the children
 // of one cell side by side): lanes with the same target add once.
 __global__ void k_count_tgt(const int2 *e, const unsigned long long *n_p, u64 cap, int *cnt) {
@@ -233,7 +280,8 @@ __global__ void k_count_tgt(const int2 *e, const unsigned long long *n_p, u64 ca
   }
 }
 
-__global__ void k_bucket(const int2 *e, const unsigned long long *n_p, u64 cap, const int *off, int *fill,
+// Entries to their targets' ranges; left[t], the target's count, counts down.
+__global__ void k_bucket(const int2 *e, const unsigned long long *n_p, u64 cap, const int *off, int *left,
                          u32 *ent) {
   const u64 n = min((u64)*n_p, cap);
   const int lane = threadIdx.x & 31;
@@ -245,7 +293,7 @@ __global__ void k_bucket(const int2 *e, const unsigned long long *n_p, u64 cap, 
     const unsigned peers = __match_any_sync(act, t);
     const int leader = __ffs(peers) - 1;
     int base = 0;
-    if (lane == leader) base = atomicAdd(&fill[t], __popc(peers));
+    if (lane == leader) base = atomicSub(&left[t], __popc(peers)) - __popc(peers);
     base = __shfl_sync(act, base, leader);
     const int pos = off[t] + base + __popc(peers & ((1u << lane) - 1));
     ent[pos] = (u32)v.y | (img << IMG_SHIFT);
@@ -349,23 +397,19 @@ int walk_blocks(Handle &h, bool periodic) {
 
 }  // namespace
 
-// CSR by target from the raw (target, source) pairs.  With `order` the
-// entries of each target are put in the reference's recording order;
-// without it they stay in arrival order (not deterministic) until
-// order_m2l_lists() runs.
-static void bucket(Handle &h, const int2 *raw, unsigned long long *n_dev, int64_t n, Buf &off_b, Buf &ent_b,
+// CSR by target from the raw (target, source) pairs: at most n of them, their
+// number on the device; cnt: C + 1 zeros.  With `order` the entries of each
+// target are put in the reference's recording order; without it they stay
+// in arrival order (not deterministic).
+static void bucket(Handle &h, const int2 *raw, unsigned long long *n_dev, int64_t n, Buf &off_b, Buf &ent_b, int *cnt,
                    bool order) {
   cudaStream_t s = h.stream;
   const int C = h.ncells;
   off_b.need((size_t)(C + 1) * 4);
   ent_b.need((size_t)(n > 0 ? n : 1) * 4 * 2);
-  h.fill.need((size_t)(C + 1) * 4);
-  int *cnt = h.fill.as<int>();
-  FMM_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(C + 1) * 4, s));
-  const int g = 148 * 8;
+  const int g = (int)std::min<int64_t>(148 * 8, (n + TB - 1) / TB + 1);
   k_count_tgt<<<g, TB, 0, s>>>(raw, n_dev, (u64)n, cnt);
   scan_exclusive_int(h, cnt, off_b.as<int>(), C + 1, nullptr);
-  FMM_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(C + 1) * 4, s));
   u32 *tmp = ent_b.as<u32>() + (n > 0 ? n : 1);
   k_bucket<<<g, TB, 0, s>>>(raw, n_dev, (u64)n, off_b.as<int>(), cnt, order ? tmp : ent_b.as<u32>());
   h.launches += 2;
@@ -385,7 +429,10 @@ static void bucket(Handle &h, const int2 *raw, unsigned long long *n_dev, int64_
 // walk's raw entries when first needed.
 void order_m2l_lists(Handle &h) {
   if (h.m2l_ordered) return;
-  bucket(h, h.m2l_raw.as<int2>(), &h.counters.as<DevCounters>()->n_m2l, h.n_m2l, h.m2l_off, h.m2l_ent, true);
+  h.fill.need((size_t)(h.ncells + 1) * 4);
+  FMM_CUDA(cudaMemsetAsync(h.fill.p, 0, (size_t)(h.ncells + 1) * 4, h.stream));
+  bucket(h, h.m2l_raw.as<int2>(), &h.counters.as<DevCounters>()->n_m2l, h.n_m2l, h.m2l_off, h.m2l_ent,
+         h.fill.as<int>(), true);
   h.m2l_ordered = true;
 }
 
@@ -400,10 +447,9 @@ void build_lists(Handle &h) {
   h.p2p_cap = std::max<size_t>(h.p2p_cap, (size_t)h.nleaves * 90 + 1024);
   const int images = h.prm.images;
   const long ks = key_space(images, h.depth);
-  h.g_occ.need(group_table_bytes(ks));             // key marks and the tables made from them
-  h.g_cnt.need((size_t)C * sizeof(int) * 2 + 64);  // targets with grouped entries, then tile slots
-  unsigned char *occ = group_tables(h.g_occ.p, ks).occ;
-  int *gflag = h.g_cnt.as<int>();
+  h.g_occ.need(group_table_bytes(ks, C));      // marks and counts, and the tables made from them
+  h.g_cnt.need((size_t)C * sizeof(int) + 64);  // tile slots of the targets
+  const GroupTables gt = group_tables(h.g_occ.p, ks, C);
   h.g_grouped = false;
   for (int attempt = 0;; attempt++) {
     h.frontier[0].need(h.frontier_cap * sizeof(int2));
@@ -414,28 +460,42 @@ void build_lists(Handle &h) {
     FMM_CUDA(cudaMemsetAsync(&ctr->n_m2l, 0, sizeof(DevCounters) - offsetof(DevCounters, n_m2l), s));
     // group keys of the M2L entries, and the keys and targets that occur
     h.m2l_key.need(h.m2l_cap * sizeof(int));
-    FMM_CUDA(cudaMemsetAsync(occ, 0, (size_t)ks, s));
-    FMM_CUDA(cudaMemsetAsync(gflag, 0, (size_t)C * sizeof(int), s));
-    k_seed<<<grid_for(std::max(h.nsys, 32), 256), 256, 0, s>>>(h.frontier[0].as<int2>(), &ctr->frontier[0], images,
-                                                                h.nsys, h.prm.dim == 2 ? 2 : 3);
+    FMM_CUDA(cudaMemsetAsync(gt.occ, 0, group_mark_bytes(ks, C), s));
+    const int dim = h.prm.dim == 2 ? 2 : 3, steps = 2 * h.depth + 3;
+    const WalkArgs wa{CellView{h.c_xr.as<double4>(), h.c_child.as<int>(), h.c_nchild.as<int>()},
+                      {h.frontier[0].as<int2>(), h.frontier[1].as<int2>()}, &ctr->frontier[0], h.frontier_cap,
+                      h.m2l_raw.as<int2>(), h.p2p_raw.as<int2>(), &ctr->n_m2l, &ctr->n_p2p, h.m2l_cap, h.p2p_cap,
+                      h.prm.theta, images ? h.prm.cycle : 0.0, h.depth, &ctr->list_overflow, h.m2l_key.as<int>(),
+                      gt.occ, gt.gflag, &ctr->walk_resid};
+    // the steps whose frontier, at most `most` pairs, fits one block
+    // iteration run in one launch; later steps take as many blocks as their
+    // frontier can fill, up to one wave
+    long most = images != 0 ? (dim == 2 ? 9 : 27) : h.nsys;
+    int st = 0;
+    if (most <= CHUNK) {
+      for (; st < steps && most <= CHUNK; st++) most *= 8;
+      auto head = images != 0 ? k_walk_head<WALK_PAIRS, true> : k_walk_head<WALK_PAIRS, false>;
+      head<<<1, TB, 0, s>>>(wa, st, images, h.nsys, dim);
+    } else {
+      k_seed<<<grid_for(h.nsys, 256), 256, 0, s>>>(wa.front[0], wa.nfront, images, h.nsys, dim);
+    }
     h.launches++;
-    CellView cv{h.c_xr.as<double4>(), h.c_child.as<int>(), h.c_nchild.as<int>()};
-    const int steps = 2 * h.depth + 3;
-    const int walk_grid = walk_blocks(h, images != 0);
+    FMM_LAUNCH();
+    const long wave = walk_blocks(h, images != 0);
     auto walk = images != 0 ? k_walk<WALK_PAIRS, true> : k_walk<WALK_PAIRS, false>;
-    // frontier counters rotate over three words: step st reads word st % 3,
-    // appends to (st + 1) % 3 (zeroed by step st - 1, or above) and zeroes
-    // (st + 2) % 3
-    for (int st = 0; st < steps; st++) {
-      const int a = st & 1, b = a ^ 1;
-      walk<<<walk_grid, TB, 0, s>>>(cv, h.frontier[a].as<int2>(), &ctr->frontier[st % 3], h.frontier[b].as<int2>(),
-                                    &ctr->frontier[(st + 1) % 3], &ctr->frontier[(st + 2) % 3], h.frontier_cap,
-                                    h.m2l_raw.as<int2>(), &ctr->n_m2l, h.m2l_cap, h.p2p_raw.as<int2>(), &ctr->n_p2p,
-                                    h.p2p_cap, h.prm.theta, images ? h.prm.cycle : 0.0, h.depth, &ctr->list_overflow,
-                                    h.m2l_key.as<int>(), occ, gflag, &ctr->walk_resid);
+    for (; st < steps; st++) {
+      walk<<<(unsigned)std::min(wave, (most + CHUNK - 1) / CHUNK), TB, 0, s>>>(wa, st);
+      if (most < wave * CHUNK) most *= 8;
       h.launches++;
       FMM_LAUNCH();
     }
+    // the P2P lists and the M2L group tables, before the counts are read.
+    // The grouped M2L reads the raw entries in any order, so the M2L lists
+    // become per-target CSR in the reference's order only when something
+    // reads that order: an export, the direct-form kernel, or residual
+    // entries.  The P2P lists are ordered always: their order is the near
+    // field's summation order, which keeps results reproducible.
+    bucket(h, h.p2p_raw.as<int2>(), &ctr->n_p2p, (int64_t)h.p2p_cap, h.p2p_off, h.p2p_ent, gt.cnt, true);
     const bool group = m2l_groups_raw(h);
     if (group) m2l_group_launch(h, (long)h.m2l_cap);
     read_counters(h);
@@ -459,14 +519,8 @@ void build_lists(Handle &h) {
   }
   h.n_m2l = (int64_t)h.hc->n_m2l;
   h.n_p2p = (int64_t)h.hc->n_p2p;
-  // The grouped M2L reads the raw entries in any order, so the M2L lists
-  // become per-target CSR in the reference's order only when something reads
-  // that order: an export, the direct-form kernel, or residual entries.  The
-  // P2P lists are ordered always: their order is the near field's summation
-  // order, which keeps results reproducible.
   h.m2l_ordered = false;
   if (h.force_direct_m2l || h.prm.dim == 2) order_m2l_lists(h);
-  bucket(h, h.p2p_raw.as<int2>(), &ctr->n_p2p, h.n_p2p, h.p2p_off, h.p2p_ent, true);
 }
 
 // Lists in the reference's cell numbering (host arrays, CSR over ref index).

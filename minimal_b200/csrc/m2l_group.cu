@@ -680,11 +680,17 @@ __global__ void k_gfill(long n, const int2 *pairs, const int *ekey, const uint2 
   tg_src[(long)sg * tile_n + ts % tile_n] = pr.y;
 }
 
-// Every marked (tile, group): its segment's operator slot in the cache.
+// Every marked (tile, group): its segment's operator slot in the cache; and
+// the first segment of every tile (the exclusive scan at the tile's first
+// group), and the end.
 __global__ void k_seg_gid(long nmark, int ngroups, const int *mark, const int *segid, const int *slot_of_gid,
-                          int *tg_gid) {
+                          int *tg_gid, int ntiles, const int *nseg, int *tg_off) {
   const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < nmark && mark[r]) tg_gid[segid[r]] = slot_of_gid[(int)(r % ngroups)];
+  if (r == 0) tg_off[ntiles] = *nseg;
+  if (r >= nmark) return;
+  const int t = (int)(r / ngroups), g = (int)(r - (long)t * ngroups), sg = segid[r];
+  if (g == 0) tg_off[t] = sg;
+  if (mark[r]) tg_gid[sg] = slot_of_gid[g];
 }
 
 // The rows of the segments that exist (count on the device) set to -1.
@@ -692,16 +698,6 @@ __global__ void k_fill_rows(int *tg_src, const int *nseg, int tile_n) {
   const long n = (long)*nseg * tile_n;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) tg_src[i] = -1;
 }
-
-// First segment of every tile (the exclusive scan at the tile's first
-// group), and the end.
-__global__ void k_tg_off(int ntiles, int ngroups, const int *segid, const int *nseg, int *tg_off) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < ntiles) tg_off[t] = segid[(long)t * ngroups];
-  if (t == ntiles) tg_off[t] = *nseg;
-}
-
-
 
 __device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -1146,7 +1142,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
     }
     if (!ok) {
       *abort = 1;
-      if (lane == 0) atomicExch(err, 1);
+      if (lane == 0) *(volatile int *)err = 1;
     }
   } else if (warp < TC_LOAD_WARP + TC_LOAD_WARPS) {
     // ---- producers: warp pw copies target rows 32pw..32pw+31 of the tile
@@ -1218,7 +1214,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
     }
     if (!ok) {
       *abort = 1;
-      if (lane == 0) atomicExch(err, 1);
+      if (lane == 0) *(volatile int *)err = 1;
     }
     // drain this thread's copies; the operator's bulk copy completes by
     // itself (bounded wait, no abort: the copy must land before exit)
@@ -1314,7 +1310,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
       }
       if (!ok) {
         *abort = 1;
-        atomicExch(err, 1);
+        *(volatile int *)err = 1;
       }
       // drain: the MMAs already issued complete by themselves (no abort)
       if (last >= 0) tc::mbar_wait(&empty[lst], parity(last), 2 * wait_ns);
@@ -1460,7 +1456,6 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
   DevCounters *ctr = h.counters.as<DevCounters>();
   if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   if (tcore) {
-    FMM_CUDA(cudaMemsetAsync(&ctr->tc_error, 0, sizeof(int), s));
     // orders with a running sum in TMEM (6, 8, 10 and 12, compiled with their
     // plan, and the others up to 12) take balanced segment ranges, one CTA
     // per SM
@@ -1473,7 +1468,7 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
       kern<<<G, TC_THREADS, tc_smem(tp), s>>>(h.g_tile.as<int>(), tg_off, tg_gid, tg_src, h.g_ops.as<unsigned char>(),
                                               h.g_m16.as<__half>(), h.c_xr.as<double4>(), h.L.as<double2>(), P, KP16,
                                               tp, tc_stages(tp), tc_acc_layout(KP16), m2l_flush_interval(h),
-                                              &ctr->m16_max, &ctr->tc_error, TC_WAIT_NS, h.tc_stall_ns, ntiles, part);
+                                              &ctr->m16_max, h.flags_host, TC_WAIT_NS, h.tc_stall_ns, ntiles, part);
     };
     switch (P) {
       case 6: launch(k_m2l_tc<6>); break;
@@ -1488,7 +1483,6 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
       h.launches++;
     }
     h.tc_stall_ns = 0;  // the test hook stalls one launch
-    FMM_CUDA(cudaMemcpyAsync(h.flags_host, &ctr->tc_error, sizeof(int), cudaMemcpyDeviceToHost, s));
     h.g_used_tc = true;
   } else {
     // two pipeline stages where they fit in shared memory (P <= 12), else
@@ -1560,7 +1554,7 @@ void m2l_group_launch(Handle &h, long max_groups) {
     h.op_depth = h.depth;
   }
   h.op_P = -1;  // until m2l_group_commit() has built what the table now holds
-  const GroupTables gt = group_tables(h.g_occ.p, ks);
+  const GroupTables gt = group_tables(h.g_occ.p, ks, C);
   h.g_slot.need((size_t)cap * sizeof(int));
   h.g_newkeys.need((size_t)cap * sizeof(int));
   DevCounters *ctr = h.counters.as<DevCounters>();
@@ -1570,7 +1564,7 @@ void m2l_group_launch(Handle &h, long max_groups) {
                                    &ctr->gcounts[2], &ctr->op_new);
   h.g_tk.need((size_t)C * 2 * (sizeof(u64) + sizeof(u32)) + 64);
   u64 *tk = h.g_tk.as<u64>();
-  k_tkeys<<<grid_for(C, TB), TB, 0, s>>>(C, h.g_cnt.as<int>(), h.c_level.as<int>(), h.c_parent.as<int>(),
+  k_tkeys<<<grid_for(C, TB), TB, 0, s>>>(C, gt.gflag, h.c_level.as<int>(), h.c_parent.as<int>(),
                                          h.c_child.as<int>(), tk, (u32 *)(tk + 2 * (size_t)C), ctr->gcounts);
   h.launches += 3;
   FMM_LAUNCH();
@@ -1681,8 +1675,8 @@ void m2l_grouped_pass(Handle &h) {
   const int2 *pairs = h.m2l_raw.as<int2>();
   const int *ekey = h.m2l_key.as<int>();
   const long ks = key_space(h.prm.images, h.depth);
-  const GroupTables gt = group_tables(h.g_occ.p, ks);  // sized by build_lists
-  int *gflag = h.g_cnt.as<int>(), *tslot = gflag + C;
+  const GroupTables gt = group_tables(h.g_occ.p, ks, C);  // sized by build_lists
+  int *gflag = gt.gflag, *tslot = h.g_cnt.as<int>();
   DevCounters *ctr = h.counters.as<DevCounters>();
   int *counts = ctr->gcounts;
   // keys computed here: for the ordered lists, and for the mixed form's
@@ -1702,8 +1696,7 @@ void m2l_grouped_pass(Handle &h) {
     h.g_ekey.need(nent * sizeof(int));
     FMM_CUDA(cudaMemsetAsync(counts, 0, 4 * sizeof(int), s));
     FMM_CUDA(cudaMemsetAsync(&ctr->op_new, 0, sizeof(int), s));
-    FMM_CUDA(cudaMemsetAsync(gt.occ, 0, (size_t)ks, s));
-    FMM_CUDA(cudaMemsetAsync(gflag, 0, (size_t)C * sizeof(int), s));
+    FMM_CUDA(cudaMemsetAsync(gt.occ, 0, (size_t)ks + (size_t)C * sizeof(int), s));  // gflag follows occ
     // ghosts: image entries with a tiny fractional offset use free-space
     // keys (mixed form only: the FP64 form keeps the reference's offsets)
     const int *gscan = nullptr;
@@ -1770,8 +1763,8 @@ void m2l_grouped_pass(Handle &h) {
     int *tg_src = h.g_tg.as<int>(), *tg_gid = tg_src + (size_t)nseg * tile_n, *tg_off = tg_gid + nseg;
     k_fill_rows<<<148 * 4, TB, 0, s>>>(tg_src, &counts[3], tile_n);  // absent targets: -1
     k_gfill<<<grid_for(nent, TB), TB, 0, s>>>(nent, pairs, ekey, gt.mask, tslot, tile_n, ngroups, segid, tg_src);
-    k_seg_gid<<<grid_for(nmark, TB), TB, 0, s>>>(nmark, ngroups, mark, segid, h.g_slot.as<int>(), tg_gid);
-    k_tg_off<<<grid_for(ntiles + 1, TB), TB, 0, s>>>(ntiles, ngroups, segid, &counts[3], tg_off);
+    k_seg_gid<<<grid_for(nmark, TB), TB, 0, s>>>(nmark, ngroups, mark, segid, h.g_slot.as<int>(), tg_gid,
+                                                    ntiles, &counts[3], tg_off);
     h.g_ntiles = ntiles;
     h.g_nseg = nseg;  // an upper bound unless it was read
     ghost_rows();

@@ -3,6 +3,9 @@
 // pairs.  Both are plain three-kernel designs sized for B200 (1024-thread scan
 // tiles, 2048-key sort tiles with warp-match ranking); all traffic is
 // coalesced except the radix scatter, which writes runs per digit.
+#include <algorithm>
+#include <utility>
+
 #include "fmm.cuh"
 
 namespace fmm {
@@ -131,8 +134,16 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles2(const int *in, int
 // Exclusive scan of a short array (a few tiles) in one launch: block b
 // first sums all input before its tile (every block reads at most a few
 // hundred KB), then scans its tile as k_scan_tile does; the last block also
-// writes the total.  Input and output must not overlap.
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_small(const int *in, int *out, long n, int *total_dev) {
+// writes the total.  Input and output must not overlap.  blockIdx.y: one of
+// two arrays of the same length.
+struct ScanPair {
+  const int *in[2];
+  int *out[2], *total[2];
+};
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_small(ScanPair a, long n) {
+  const int *in = a.in[blockIdx.y];
+  int *out = a.out[blockIdx.y], *total_dev = a.total[blockIdx.y];
   __shared__ int warp_sum[SCAN_THREADS / 32];
   __shared__ int s_prefix;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -205,6 +216,12 @@ constexpr int RS_THREADS = 256;
 constexpr int RS_ITEMS = 8;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_BINS = 256;
+// Up to this many tiles (65,536 keys) a scatter block adds up the tiles'
+// counts itself and counts the next pass's digits as it writes, so a pass is
+// one launch instead of three: such sorts are launches and latency (20,000
+// keys, 3 passes: 9 launches of 2-9 us).  Above, the counts are too many for
+// every block to read.
+constexpr int RS_SMALL_TILES = 32;
 
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const u64 *keys, long n, int shift, u64 mask, int *hist,
                                                        int ntiles) {
@@ -219,6 +236,24 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const u64 *keys, long n,
   }
   __syncthreads();
   hist[(long)threadIdx.x * ntiles + blockIdx.x] = hs[threadIdx.x];
+}
+
+// The same for a short sort: counts in rows by tile; the tables of the later
+// passes are zeroed for the scatters that count them.
+__global__ void __launch_bounds__(RS_THREADS) k_rs_hist_small(const u64 *keys, long n, int shift, u64 mask, int *hist,
+                                                             int npass) {
+  __shared__ int hs[RS_BINS];
+  hs[threadIdx.x] = 0;
+  __syncthreads();
+  const long base = (long)blockIdx.x * RS_TILE;
+#pragma unroll
+  for (int k = 0; k < RS_ITEMS; k++) {
+    long i = base + k * RS_THREADS + threadIdx.x;
+    if (i < n) atomicAdd(&hs[(keys[i] >> shift) & mask], 1);
+  }
+  for (int p = 1; p < npass; p++) hist[((long)p * gridDim.x + blockIdx.x) * RS_BINS + threadIdx.x] = 0;
+  __syncthreads();
+  hist[(long)blockIdx.x * RS_BINS + threadIdx.x] = hs[threadIdx.x];
 }
 
 // Block d: exclusive scan of digit d's counts over the tiles, into
@@ -254,10 +289,13 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_digit_scan(const int *hist, i
 // each group of equal digits), the counts of the 8 warps are combined into
 // tile-local digit offsets, the items are sorted by digit inside the tile in
 // shared memory, and then written out in order: items of one digit are
-// contiguous in the output, so the stores coalesce.
+// contiguous in the output, so the stores coalesce.  SMALL: offs holds the
+// tiles' counts in rows (a short sort), and `next` the next pass's table, or
+// null.
+template <bool SMALL>
 __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const u64 *kin, const u32 *vin, u64 *kout, u32 *vout,
                                                           long n, int shift, u64 mask, const int *offs,
-                                                          const int *dtot, int ntiles) {
+                                                          const int *dtot, int ntiles, int *next, u64 next_mask) {
   constexpr int NW = RS_THREADS / 32, PER = RS_TILE / NW;  // 256 items per warp
   static_assert(RS_BINS == RS_THREADS, "one thread per digit scans the digit totals");
   __shared__ int wcnt[NW][RS_BINS + 1];                     // per-warp digit counts, then offsets
@@ -269,14 +307,24 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const u64 *kin, const
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   for (int k = t; k < NW * (RS_BINS + 1); k += RS_THREADS) (&wcnt[0][0])[k] = 0;
   {  // exclusive scan of the digit totals
-    const int c = dtot[t];
+    int c = 0, before = 0;  // of this digit: all keys, and those of earlier tiles
+    if (SMALL) {
+#pragma unroll 8
+      for (int q = 0; q < ntiles; q++) {
+        const int v = offs[q * RS_BINS + t];
+        c += v;
+        before += q < (int)blockIdx.x ? v : 0;
+      }
+    } else {
+      c = dtot[t];
+    }
     const int incl = warp_incl_scan(c);
     if (lane == 31) dsum[warp] = incl;
     __syncthreads();
     int wpre = 0;
 #pragma unroll
     for (int w = 0; w < NW; w++) wpre += w < warp ? dsum[w] : 0;
-    dbase[t] = wpre + incl - c;
+    dbase[t] = wpre + incl - c + before;
   }
   __syncthreads();
   const long tile0 = (long)blockIdx.x * RS_TILE;
@@ -349,9 +397,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const u64 *kin, const
   for (int j = t; j < valid; j += RS_THREADS) {
     const u64 k = sk[j];
     const int d = (int)((k >> shift) & mask);
-    const long o = (long)dbase[d] + offs[(long)d * ntiles + blockIdx.x] + (j - loff[d]);
+    const long o = (long)dbase[d] + (SMALL ? 0 : offs[(long)d * ntiles + blockIdx.x]) + (j - loff[d]);
     kout[o] = k;
     vout[o] = sv[j];
+    if (SMALL && next) atomicAdd(&next[(o / RS_TILE) * RS_BINS + ((k >> (shift + 8)) & next_mask)], 1);
   }
 }
 
@@ -361,7 +410,7 @@ void scan_exclusive_int(Handle &h, const int *in, int *out, long n, int *total_d
   if (n <= 0) return;
   const long nb = (n + SCAN_TILE - 1) / SCAN_TILE;
   if (nb <= SCAN_SMALL_TILES && ((uintptr_t)in & 15) == 0) {  // short: one launch
-    k_scan_small<<<(unsigned)nb, SCAN_THREADS, 0, h.stream>>>(in, out, n, total_dev);
+    k_scan_small<<<(unsigned)nb, SCAN_THREADS, 0, h.stream>>>(ScanPair{{in, in}, {out, out}, {total_dev, total_dev}}, n);
     h.launches++;
     FMM_LAUNCH();
     return;
@@ -385,28 +434,63 @@ void scan_exclusive_int(Handle &h, const int *in, int *out, long n, int *total_d
   scan_rec(h, in, out, n, total_dev, h.scan_tmp.as<int>());
 }
 
+// Two scans of the same length, in one launch where both are short.
+void scan_exclusive_pair(Handle &h, const int *in0, int *out0, int *total0, const int *in1, int *out1, int *total1,
+                         long n) {
+  const long nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+  if (n > 0 && nb <= SCAN_SMALL_TILES && (((uintptr_t)in0 | (uintptr_t)in1) & 15) == 0) {
+    k_scan_small<<<dim3((unsigned)nb, 2), SCAN_THREADS, 0, h.stream>>>(
+        ScanPair{{in0, in1}, {out0, out1}, {total0, total1}}, n);
+    h.launches++;
+    FMM_LAUNCH();
+    return;
+  }
+  scan_exclusive_int(h, in0, out0, n, total0);
+  scan_exclusive_int(h, in1, out1, n, total1);
+}
+
 // Sorts bits [lo_bit, hi_bit) of the keys, stable, 8 bits per pass.  On
 // return k/v point at the sorted data (the buffers may have been swapped).
 void radix_sort_pairs(Handle &h, u64 *&k, u32 *&v, u64 *&k2, u32 *&v2, long n, int lo_bit, int hi_bit) {
   if (n <= 1 || hi_bit <= lo_bit) return;
   const int ntiles = (int)((n + RS_TILE - 1) / RS_TILE);
+  auto mask_at = [&](int shift) { return (1ull << std::min(hi_bit - shift, 8)) - 1; };
+  if (ntiles <= RS_SMALL_TILES) {
+    const int npass = (hi_bit - lo_bit + 7) / 8;
+    const size_t table = (size_t)ntiles * RS_BINS;
+    h.hist.need(npass * table * sizeof(int));
+    int *hist = h.hist.as<int>();
+    k_rs_hist_small<<<ntiles, RS_THREADS, 0, h.stream>>>(k, n, lo_bit, mask_at(lo_bit), hist, npass);
+    for (int p = 0; p < npass; p++) {
+      const int shift = lo_bit + 8 * p;
+      const bool more = p + 1 < npass;
+      k_rs_scatter<true><<<ntiles, RS_THREADS, 0, h.stream>>>(k, v, k2, v2, n, shift, mask_at(shift), hist + p * table,
+                                                             nullptr, ntiles, more ? hist + (p + 1) * table : nullptr,
+                                                             more ? mask_at(shift + 8) : 0);
+      std::swap(k, k2);
+      std::swap(v, v2);
+    }
+    h.launches += npass + 1;
+    FMM_LAUNCH();
+    return;
+  }
   h.hist.need(((size_t)2 * RS_BINS * ntiles + RS_BINS) * sizeof(int));
   int *hist = h.hist.as<int>();
   int *offs = hist + (long)RS_BINS * ntiles;
   int *dtot = offs + (long)RS_BINS * ntiles;
   for (int shift = lo_bit; shift < hi_bit; shift += 8) {
-    const int bits = hi_bit - shift < 8 ? hi_bit - shift : 8;
-    const u64 mask = (1ull << bits) - 1;
+    const u64 mask = mask_at(shift);
     k_rs_hist<<<ntiles, RS_THREADS, 0, h.stream>>>(k, n, shift, mask, hist, ntiles);
     // per digit over the tiles; the scatter adds the scanned digit totals
     k_rs_digit_scan<<<RS_BINS, RS_THREADS, 0, h.stream>>>(hist, offs, dtot, ntiles);
     h.launches += 2;
     FMM_LAUNCH();
-    k_rs_scatter<<<ntiles, RS_THREADS, 0, h.stream>>>(k, v, k2, v2, n, shift, mask, offs, dtot, ntiles);
+    k_rs_scatter<false><<<ntiles, RS_THREADS, 0, h.stream>>>(k, v, k2, v2, n, shift, mask, offs, dtot, ntiles, nullptr,
+                                                            0);
     h.launches++;
     FMM_LAUNCH();
-    u64 *tk = k; k = k2; k2 = tk;
-    u32 *tv = v; v = v2; v2 = tv;
+    std::swap(k, k2);
+    std::swap(v, v2);
   }
 }
 

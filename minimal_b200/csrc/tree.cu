@@ -43,30 +43,6 @@ constexpr int TB = 256;
 __device__ __forceinline__ double dmin(double a, double b) { return fmin(a, b); }
 __device__ __forceinline__ double dmax(double a, double b) { return fmax(a, b); }
 
-__global__ void k_bounds_partial(const double4 *in, long n, double *part) {
-  double lo[3] = {in[0].x, in[0].y, in[0].z}, hi[3] = {lo[0], lo[1], lo[2]};
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const double4 b = in[i];
-    lo[0] = dmin(b.x, lo[0]); lo[1] = dmin(b.y, lo[1]); lo[2] = dmin(b.z, lo[2]);
-    hi[0] = dmax(b.x, hi[0]); hi[1] = dmax(b.y, hi[1]); hi[2] = dmax(b.z, hi[2]);
-  }
-  for (int o = 16; o > 0; o >>= 1)
-    for (int d = 0; d < 3; d++) {
-      lo[d] = dmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-      hi[d] = dmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-    }
-  __shared__ double s[TB / 32][6];
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0)
-    for (int d = 0; d < 3; d++) { s[w][d] = lo[d]; s[w][3 + d] = hi[d]; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < TB / 32; k++)
-      for (int d = 0; d < 3; d++) { s[0][d] = dmin(s[0][d], s[k][d]); s[0][3 + d] = dmax(s[0][3 + d], s[k][3 + d]); }
-    for (int d = 0; d < 6; d++) part[blockIdx.x * 6 + d] = s[0][d];
-  }
-}
-
 // Min/max of the block's threads into thread 0 (exact operations: the
 // reduction order cannot change the result).
 __device__ void block_minmax(double lo[3], double hi[3]) {
@@ -86,12 +62,40 @@ __device__ void block_minmax(double lo[3], double hi[3]) {
 }
 
 // getBounds (3d/build_tree.h:7-21): centre = (max+min)/2, R0 = largest
-// half-extent about that centre, times 1.00001.
-__global__ void k_bounds_final(const double *part, int nb, RootGeom *g) {
-  double lo[3] = {part[0], part[1], part[2]}, hi[3] = {part[3], part[4], part[5]};
-  for (int k = threadIdx.x; k < nb; k += blockDim.x)
-    for (int d = 0; d < 3; d++) { lo[d] = dmin(part[6 * k + d], lo[d]); hi[d] = dmax(part[6 * k + 3 + d], hi[d]); }
+// half-extent about that centre, times 1.00001.  The blocks' bounds go to
+// `part`; the last block to finish combines them, and zeroes the counters for
+// the build (one launch where the combination and the zeroing took two more).
+__global__ void __launch_bounds__(TB) k_bounds(const double4 *in, long n, double *part, RootGeom *g, DevCounters *ctr) {
+  double lo[3] = {in[0].x, in[0].y, in[0].z}, hi[3] = {lo[0], lo[1], lo[2]};
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    const double4 b = in[i];
+    lo[0] = dmin(b.x, lo[0]); lo[1] = dmin(b.y, lo[1]); lo[2] = dmin(b.z, lo[2]);
+    hi[0] = dmax(b.x, hi[0]); hi[1] = dmax(b.y, hi[1]); hi[2] = dmax(b.z, hi[2]);
+  }
   block_minmax(lo, hi);
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    for (int d = 0; d < 3; d++) {
+      part[blockIdx.x * 6 + d] = lo[d];
+      part[blockIdx.x * 6 + 3 + d] = hi[d];
+    }
+    __threadfence();
+    last = atomicAdd(&ctr->bounds_ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int d = 0; d < 3; d++) {
+    lo[d] = __ldcg(&part[d]);
+    hi[d] = __ldcg(&part[3 + d]);
+  }
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += TB)
+    for (int d = 0; d < 3; d++) {
+      lo[d] = dmin(__ldcg(&part[6 * k + d]), lo[d]);
+      hi[d] = dmax(__ldcg(&part[6 * k + 3 + d]), hi[d]);
+    }
+  block_minmax(lo, hi);
+  for (int k = threadIdx.x; k < (int)(sizeof(DevCounters) / sizeof(int)); k += TB) ((int *)ctr)[k] = 0;
   if (threadIdx.x != 0) return;
   double R0 = 0;
   for (int d = 0; d < 3; d++) {
@@ -351,17 +355,15 @@ __global__ void k_gather_cells(const u32 *pre_of_bfs, const int *bfs_of_pre, lon
 }
 
 // Reference cell number: 1 + (children allocated by parents earlier in
-// pre-order) + rank among siblings (3d/build_tree.h:69-84).
-__global__ void k_ref_index(BfsCells o, long c, const int *blockstart_pre, int *ref) {
+// pre-order) + rank among siblings (3d/build_tree.h:69-84); and the leaves in
+// BFS order.
+__global__ void k_ref_leaves(BfsCells o, long c, const int *blockstart_pre, int *ref, const int *is_leaf,
+                             const int *leafpos, int *leaves) {
   const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= c) return;
   const int par = o.parent[b];
   ref[b] = par < 0 ? 0 : 1 + blockstart_pre[o.pre[par]] + (int)(b - o.child[par]);
-}
-
-__global__ void k_compact_leaves(const int *is_leaf, const int *pos, long c, int *leaves) {
-  const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < c && is_leaf[b]) leaves[pos[b]] = (int)b;
+  if (is_leaf[b]) leaves[leafpos[b]] = (int)b;
 }
 
 // Bodies of one leaf back into input order (warp per leaf, rank sort).
@@ -393,12 +395,6 @@ __global__ void k_leaf_order(const int *leaves, int nleaves, const int *begin, c
 }
 
 
-__global__ void k_zero_counters(DevCounters *c) {
-  const int t = threadIdx.x;
-  int *w = (int *)c;
-  for (int k = t; k < (int)(sizeof(DevCounters) / sizeof(int)); k += blockDim.x) w[k] = 0;
-}
-
 }  // namespace
 
 void build_tree(Handle &h) {
@@ -419,9 +415,8 @@ void build_tree(Handle &h) {
   } else {
     const int nbp = (int)std::min<long>(4 * 148, (n + TB - 1) / TB);
     h.hist.need((size_t)nbp * 6 * sizeof(double));
-    k_bounds_partial<<<nbp, TB, 0, s>>>(h.in.as<double4>(), n, h.hist.as<double>());
-    k_bounds_final<<<1, TB, 0, s>>>(h.hist.as<double>(), nbp, g);
-    h.launches += 2;
+    k_bounds<<<nbp, TB, 0, s>>>(h.in.as<double4>(), n, h.hist.as<double>(), g, ctr);
+    h.launches++;
   }
   FMM_LAUNCH();
 
@@ -441,12 +436,14 @@ void build_tree(Handle &h) {
     D = std::min(std::max(D, 2), max_levels);
   }
   D = std::min(D, max_levels);
+  bool zeroed = nsys == 1;  // by k_bounds
   for (h.keys[0].need(n * 8), h.keys[1].need(n * 8), h.vals[0].need(n * 4), h.vals[1].need(n * 4);;) {
-    k_zero_counters<<<1, 256, 0, s>>>(ctr);
+    if (!zeroed) FMM_CUDA(cudaMemsetAsync(ctr, 0, sizeof(DevCounters), s));
+    zeroed = false;
     u64 *k = h.keys[0].as<u64>(), *k2 = h.keys[1].as<u64>();
     u32 *v = h.vals[0].as<u32>(), *v2 = h.vals[1].as<u32>();
     k_keys<<<grid_for(n, TB), TB, 0, s>>>(h.in.as<double4>(), n, g, sys_off, nsys, D, k, v);
-    h.launches += 2;
+    h.launches++;
     FMM_LAUNCH();
     radix_sort_pairs(h, k, v, k2, v2, n, 0, 3 * D + sys_bits);
     h.lfirst.need(n * 4);
@@ -468,15 +465,16 @@ void build_tree(Handle &h) {
     h.ncells = (int)C;
     h.key_levels = D;
     // pre-order tables (reuse the idle sort buffers' siblings)
-    h.pre_tmp.need(C * (6 * sizeof(int) + sizeof(double4)) + 256);
+    const long Cp = (C + 3) & ~3L;  // every table starts 16-byte aligned (vector loads in the scans)
+    h.pre_tmp.need(Cp * (6 * sizeof(int) + sizeof(double4)) + 256);
     PreTables t;
     t.xr = h.pre_tmp.as<double4>();
-    t.begin = (int *)(t.xr + C);
-    t.count = t.begin + C;
-    t.level = t.count + C;
-    t.parent = t.level + C;
-    t.nchild = t.parent + C;
-    int *owner = t.nchild + C;
+    t.begin = (int *)(t.xr + Cp);
+    t.count = t.begin + Cp;
+    t.level = t.count + Cp;
+    t.parent = t.level + Cp;
+    t.nchild = t.parent + Cp;
+    int *owner = t.nchild + Cp;
     FMM_CUDA(cudaMemsetAsync(t.nchild, 0, C * sizeof(int), s));
     k_cell_owner<<<grid_for(n, TB), TB, 0, s>>>(n, h.chain.as<int>(), h.prebase.as<int>(), owner);
     k_cells<<<grid_for(C, TB), TB, 0, s>>>(k, n, C, D, h.lfirst.as<int>(), owner, h.prebase.as<int>(), g, t, ctr);
@@ -484,7 +482,6 @@ void build_tree(Handle &h) {
     FMM_LAUNCH();
 
     // 5. BFS order = stable sort of pre-order cells by level
-    const long Cp = (C + 3) & ~3L;  // every table starts 16-byte aligned (vector loads in the scans)
     h.ctmp.need(Cp * (2 * sizeof(u64) + 2 * sizeof(u32) + 4 * sizeof(int)) + 256);
     u64 *lk = h.ctmp.as<u64>(), *lk2 = lk + Cp;
     u32 *lv = (u32 *)(lk2 + Cp), *lv2 = lv + Cp;
@@ -504,14 +501,11 @@ void build_tree(Handle &h) {
     k_gather_cells<<<grid_for(C, TB), TB, 0, s>>>(lv, bfs_of_pre, C, t, o, is_leaf);
     h.launches++;
     FMM_LAUNCH();
-    // reference numbering
-    scan_exclusive_int(h, t.nchild, blockstart, C, nullptr);
-    k_ref_index<<<grid_for(C, TB), TB, 0, s>>>(o, C, blockstart, h.c_ref.as<int>());
-    h.launches++;
-    // leaves
-    scan_exclusive_int(h, is_leaf, leafpos, C, &ctr->nleaves);
+    // reference numbering, and the leaves
     h.leaves.need(C * 4);
-    k_compact_leaves<<<grid_for(C, TB), TB, 0, s>>>(is_leaf, leafpos, C, h.leaves.as<int>());
+    scan_exclusive_pair(h, t.nchild, blockstart, nullptr, is_leaf, leafpos, &ctr->nleaves, C);
+    k_ref_leaves<<<grid_for(C, TB), TB, 0, s>>>(o, C, blockstart, h.c_ref.as<int>(), is_leaf, leafpos,
+                                                h.leaves.as<int>());
     h.launches++;
     FMM_LAUNCH();
     if (h.prm.images > 0)  // the root radius, for the M2L operators of image keys
