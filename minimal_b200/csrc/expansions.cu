@@ -9,6 +9,7 @@
 // harmonics they need depend only on level and octant and come from a
 // table built once per upward pass.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "fmm.cuh"
@@ -462,9 +463,23 @@ __global__ void __launch_bounds__(SH_T) k_l2l(int c0, const int *child, const in
 // range of the scaled values.  (In FP64 the per-octant M2M kernel above is
 // as fast as an octant-batched one: its eight children bring eight
 // different inputs; the mixed form uses the octant-batched k_m2m_ob32.)
-constexpr int OB_PAR = 2;    // parents per CTA
-constexpr int OB_T = 64;     // threads per parent (outputs)
+// A level of few parents is latency: a chain of up to P^2 terms per output
+// (P = 10, one parent: 28 us in FP64). There SL lanes share an output's terms
+// and add their sums by shuffles, in a CTA of one parent.
+constexpr int OB_PAR = 2;    // parents per CTA (levels of many parents, SL = 1)
+constexpr int OB_T = 64;     // outputs of a parent worked on at once
+constexpr int OB_SL = 4;     // lanes per output at levels of few parents
 constexpr int OB_MAXP = 16;
+
+// Sum of v over the SL adjacent lanes of an output.
+template <int SL, class V>
+__device__ __forceinline__ void slice_sum(V &v) {
+#pragma unroll
+  for (int o = 1; o < SL; o <<= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+}
 
 // degree of coefficient index ci
 __device__ __forceinline__ int deg_of(int ci) {
@@ -511,17 +526,19 @@ __device__ void stage_unit_variants(V *Yv, const double2 *ytab, int dir, int nt,
 // staged as scaled multipoles M(d) / rho^d (plain and conjugate copies, zero
 // for an absent child), the unit harmonics in four sign variants, products
 // in FP32 on these order-one values, the output rescaled by rho^j in FP64.
-__global__ void __launch_bounds__(OB_PAR * OB_T) k_m2m_ob32(int c0, int np, const int *child, const int *nchild,
+template <int PAR, int SL>
+__global__ void __launch_bounds__(PAR * OB_T * SL) k_m2m_ob32(int c0, int np, const int *child, const int *nchild,
                                                          const double4 *xr, const double2 *ytab, TermTable tab,
                                                          double2 *M, int P) {
   extern __shared__ __align__(16) unsigned char smraw[];
   float2 *sm2 = (float2 *)smraw;
   const int nt = tri(P);
   float2 *Yv = sm2;           // [4][8][nt] unit harmonics (parent - child)
-  float2 *A = Yv + 32 * nt;   // [OB_PAR][8][2][nt] scaled child multipoles, plain and conjugate
-  __shared__ int cho[OB_PAR][8];
-  const int slot = threadIdx.x / OB_T, tl = threadIdx.x % OB_T;
-  const int pi = blockIdx.x * OB_PAR + slot, c = c0 + pi;
+  float2 *A = Yv + 32 * nt;   // [PAR][8][2][nt] scaled child multipoles, plain and conjugate
+  __shared__ int cho[PAR][8];
+  constexpr int T = OB_T * SL;  // threads per parent
+  const int slot = threadIdx.x / T, tl = threadIdx.x % T;
+  const int pi = blockIdx.x * PAR + slot, c = c0 + pi;
   const bool has = pi < np && nchild[c] > 0;  // a leaf keeps its P2M multipole
   if (tl < 8) cho[slot][tl] = -1;
   __syncthreads();
@@ -532,7 +549,7 @@ __global__ void __launch_bounds__(OB_PAR * OB_T) k_m2m_ob32(int c0, int np, cons
   stage_unit_variants(Yv, ytab, 0, nt, 4);
   __syncthreads();
   const double inv = has ? 1.0 / (xr[c].w * 0.5) : 0.0;  // 1 / R_child
-  for (int e = tl; e < 8 * nt; e += OB_T) {
+  for (int e = tl; e < 8 * nt; e += T) {
     const int oct = e / nt, ci = e - oct * nt, q = cho[slot][oct];
     double2 v = make_double2(0, 0);
     if (has && q >= 0) {
@@ -547,14 +564,17 @@ __global__ void __launch_bounds__(OB_PAR * OB_T) k_m2m_ob32(int c0, int np, cons
   if (!has) return;
   const float2 *As = A + (size_t)slot * 8 * 2 * nt;
   const double rho = xr[c].w * 0.5;
-  for (int r = tl; r < nt; r += OB_T) {
+  const int sl = tl % SL;
+  for (int r0 = 0; r0 < nt; r0 += OB_T) {  // whole warps: the shuffles of slice_sum
+    const int r = min(r0 + tl / SL, nt - 1);
     const int o = tab.perm[r];
     const unsigned *t = tab.terms + tab.off[r];
     const int nterm = tab.off[r + 1] - tab.off[r];
     float2 acc[8];  // one chain per octant
 #pragma unroll
     for (int oct = 0; oct < 8; oct++) acc[oct] = make_float2(0.f, 0.f);
-    for (int qq = 0; qq < nterm; qq++) {
+#pragma unroll 2
+    for (int qq = sl; qq < nterm; qq += SL) {
       const unsigned e = t[qq];
       const int ia = (int)(e & 2047u), iy = (int)(e >> 11);
 #pragma unroll
@@ -566,6 +586,8 @@ __global__ void __launch_bounds__(OB_PAR * OB_T) k_m2m_ob32(int c0, int np, cons
       v.x += acc[oct].x;
       v.y += acc[oct].y;
     }
+    slice_sum<SL>(v);
+    if (sl != 0 || r0 + tl / SL >= nt) continue;
     for (int d = deg_of(o); d > 0; d--) v = make_double2(v.x * rho, v.y * rho);
     M[(long)c * nt + o] = v;
   }
@@ -573,8 +595,8 @@ __global__ void __launch_bounds__(OB_PAR * OB_T) k_m2m_ob32(int c0, int np, cons
 
 // F32 (mixed form): the products in FP32 on the scaled (order-one) values;
 // staging, the rescaling and the sums into L stay FP64.
-template <bool F32>
-__global__ void __launch_bounds__(OB_PAR * OB_T) k_l2l_ob(int c0, int np, const int *child, const int *nchild,
+template <bool F32, int PAR, int SL>
+__global__ void __launch_bounds__(PAR * OB_T * SL) k_l2l_ob(int c0, int np, const int *child, const int *nchild,
                                                        const double4 *xr, const double2 *ytab, TermTable tab,
                                                        double2 *L, int P) {
   typedef typename Cplx<F32>::V V;
@@ -582,10 +604,11 @@ __global__ void __launch_bounds__(OB_PAR * OB_T) k_l2l_ob(int c0, int np, const 
   V *sm2 = (V *)smraw;
   const int nt = tri(P);
   V *Yv = sm2;          // [2][8][nt] unit harmonics (child - parent)
-  V *A = Yv + 16 * nt;  // [OB_PAR][4][nt] scaled parent local: plain, conjugate, negated, both
-  __shared__ int cho[OB_PAR][8];
-  const int slot = threadIdx.x / OB_T, tl = threadIdx.x % OB_T;
-  const int pi = blockIdx.x * OB_PAR + slot, c = c0 + pi;
+  V *A = Yv + 16 * nt;  // [PAR][4][nt] scaled parent local: plain, conjugate, negated, both
+  __shared__ int cho[PAR][8];
+  constexpr int T = OB_T * SL;  // threads per parent
+  const int slot = threadIdx.x / T, tl = threadIdx.x % T;
+  const int pi = blockIdx.x * PAR + slot, c = c0 + pi;
   const bool has = pi < np && nchild[c] > 0;  // a leaf has no children to shift to
   if (tl < 8) cho[slot][tl] = -1;
   __syncthreads();
@@ -595,7 +618,7 @@ __global__ void __launch_bounds__(OB_PAR * OB_T) k_l2l_ob(int c0, int np, const 
   }
   stage_unit_variants(Yv, ytab, 1, nt, 2);
   const double rho = has ? xr[c].w * 0.5 : 0.0;  // R_child
-  for (int ci = tl; ci < nt; ci += OB_T) {
+  for (int ci = tl; ci < nt; ci += T) {
     double2 v = make_double2(0, 0);
     if (has) {
       v = L[(long)c * nt + ci];
@@ -618,24 +641,30 @@ __global__ void __launch_bounds__(OB_PAR * OB_T) k_l2l_ob(int c0, int np, const 
   int kids[8];
 #pragma unroll
   for (int oct = 0; oct < 8; oct++) kids[oct] = cho[slot][oct];
-  for (int r = tl; r < nt; r += OB_T) {
+  const int sl = tl % SL;
+  for (int r0 = 0; r0 < nt; r0 += OB_T) {  // whole warps: the shuffles of slice_sum
+    const int r = min(r0 + tl / SL, nt - 1);
     const int o = tab.perm[r];
     const unsigned *t = tab.terms + tab.off[r];
     const int nterm = tab.off[r + 1] - tab.off[r];
     V acc[8];
 #pragma unroll
     for (int oct = 0; oct < 8; oct++) acc[oct].x = acc[oct].y = 0;
-    for (int qq = 0; qq < nterm; qq++) {
+#pragma unroll 2
+    for (int qq = sl; qq < nterm; qq += SL) {
       const unsigned e = t[qq];
       const V a = As[e & 2047u];
       const int iy = (int)(e >> 11);
 #pragma unroll
       for (int oct = 0; oct < 8; oct++) cfma(acc[oct], a, Yv[iy + oct * nt]);
     }
+#pragma unroll
+    for (int oct = 0; oct < 8; oct++) slice_sum<SL>(acc[oct]);
+    if (r0 + tl / SL >= nt) continue;
     const int dj = deg_of(o);
 #pragma unroll
     for (int oct = 0; oct < 8; oct++) {
-      if (kids[oct] < 0) continue;
+      if (kids[oct] < 0 || oct % SL != sl) continue;  // the lanes share the octants
       double2 v = make_double2(acc[oct].x, acc[oct].y);
       for (int d = dj; d > 0; d--) v = make_double2(v.x * inv, v.y * inv);
       double2 &dst = L[(long)kids[oct] * nt + o];
@@ -736,9 +765,12 @@ void expansions_set_attributes() {
   EXAFMM_UNROLLED_ORDERS(EXAFMM_F32_ATTR)
 #undef EXAFMM_F32_ATTR
   cudaFuncSetAttribute(k_m2m, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_l2l_ob<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_m2m_ob32, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_l2l_ob<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_l2l_ob<false, OB_PAR, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_l2l_ob<false, 1, OB_SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_l2l_ob<true, OB_PAR, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_l2l_ob<true, 1, OB_SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_m2m_ob32<OB_PAR, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_m2m_ob32<1, OB_SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaFuncSetAttribute(k_l2l, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
@@ -812,6 +844,18 @@ void unit_tables(Handle &h, cudaStream_t s) {
   h.shift_P = P;
 }
 
+// The octant-batched kernels' shape for a level of np parents: few parents
+// (up to OB_FEW per SM) take one per CTA and OB_SL lanes per output.
+constexpr int OB_FEW = 2;
+template <class F>
+void ob_level(Handle &h, int np, F launch) {
+  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
+  if (np <= OB_FEW * h.nsm)
+    launch(std::integral_constant<int, 1>{}, std::integral_constant<int, OB_SL>{});
+  else
+    launch(std::integral_constant<int, OB_PAR>{}, std::integral_constant<int, 1>{});
+}
+
 void upward_pass(Handle &h, cudaStream_t s) {
   if (h.prm.dim == 2) return upward_pass_2d(h, s);
   const int P = h.prm.P, nt = tri(P);
@@ -853,9 +897,12 @@ void upward_pass(Handle &h, cudaStream_t s) {
     const int c0 = h.level_base[l], c1 = h.level_base[l + 1];
     if (c1 <= c0) continue;
     if (P <= OB_MAXP && h.prm.precision == EXAFMM_MIXED)
-      k_m2m_ob32<<<(c1 - c0 + OB_PAR - 1) / OB_PAR, OB_PAR * OB_T, (32 + OB_PAR * 16) * nt * sizeof(float2), s>>>(
-          c0, c1 - c0, h.c_child.as<int>(), h.c_nchild.as<int>(), h.c_xr.as<double4>(), h.shift_ops.as<double2>(),
-          table_view(h, P, 2), h.M.as<double2>(), P);
+      ob_level(h, c1 - c0, [&](auto par, auto sl) {
+        constexpr int PAR = decltype(par)::value, SL = decltype(sl)::value;
+        k_m2m_ob32<PAR, SL><<<(c1 - c0 + PAR - 1) / PAR, PAR * OB_T * SL, (32 + PAR * 16) * nt * sizeof(float2), s>>>(
+            c0, c1 - c0, h.c_child.as<int>(), h.c_nchild.as<int>(), h.c_xr.as<double4>(), h.shift_ops.as<double2>(),
+            table_view(h, P, 2), h.M.as<double2>(), P);
+      });
     else
       k_m2m<<<c1 - c0, SH_T, 24 * nt * sizeof(double2), s>>>(c0, h.c_child.as<int>(), h.c_nchild.as<int>(),
                                                             h.c_xr.as<double4>(), h.shift_ops.as<double2>(),
@@ -872,15 +919,18 @@ void downward_pass(Handle &h, cudaStream_t s, cudaEvent_t before_l2p) {
   for (int l = 0; l < h.depth; l++) {  // parents at level l push to their children
     const int c0 = h.level_base[l], c1 = h.level_base[l + 1];
     if (c1 <= c0) continue;
-    const dim3 grid((c1 - c0 + OB_PAR - 1) / OB_PAR), block(OB_PAR * OB_T);
-    if (P <= OB_MAXP && h.prm.precision == EXAFMM_MIXED)
-      k_l2l_ob<true><<<grid, block, (16 + OB_PAR * 4) * nt * sizeof(float2), s>>>(
-          c0, c1 - c0, h.c_child.as<int>(), h.c_nchild.as<int>(), h.c_xr.as<double4>(), h.shift_ops.as<double2>(),
-          table_view(h, P, 3), h.L.as<double2>(), P);
-    else if (P <= OB_MAXP)
-      k_l2l_ob<false><<<grid, block, (16 + OB_PAR * 4) * nt * sizeof(double2), s>>>(
-          c0, c1 - c0, h.c_child.as<int>(), h.c_nchild.as<int>(), h.c_xr.as<double4>(), h.shift_ops.as<double2>(),
-          table_view(h, P, 3), h.L.as<double2>(), P);
+    auto ob = [&](auto f32) {
+      ob_level(h, c1 - c0, [&](auto par, auto sl) {
+        constexpr bool F32 = decltype(f32)::value;
+        constexpr int PAR = decltype(par)::value, SL = decltype(sl)::value;
+        k_l2l_ob<F32, PAR, SL><<<(c1 - c0 + PAR - 1) / PAR, PAR * OB_T * SL,
+                                 (16 + PAR * 4) * nt * sizeof(typename Cplx<F32>::V), s>>>(
+            c0, c1 - c0, h.c_child.as<int>(), h.c_nchild.as<int>(), h.c_xr.as<double4>(), h.shift_ops.as<double2>(),
+            table_view(h, P, 3), h.L.as<double2>(), P);
+      });
+    };
+    if (P <= OB_MAXP && h.prm.precision == EXAFMM_MIXED) ob(std::true_type{});
+    else if (P <= OB_MAXP) ob(std::false_type{});
     else
       k_l2l<<<c1 - c0, SH_T, 9 * nt * sizeof(double2), s>>>(c0, h.c_child.as<int>(), h.c_nchild.as<int>(),
                                                            h.c_xr.as<double4>(), h.shift_ops.as<double2>(),
