@@ -200,10 +200,10 @@ void do_tree(Handle &h) {
   h.have_lists = h.have_up = h.have_horiz = h.have_down = false;
 }
 
-void do_lists(Handle &h) {
+void do_lists(Handle &h, const std::function<void()> &near_field = nullptr) {
   need_tree(h);
   Timer t(h, PH_LISTS);
-  build_lists(h);
+  build_lists(h, near_field);
   h.have_lists = true;
 }
 
@@ -267,14 +267,19 @@ void run_all(Handle &h, bool rebuild) {
     }
     FMM_CUDA(cudaEventRecord(h.up_ev, up));
     h.have_up = true;
-    if (rebuild) do_lists(h);
-    FMM_CUDA(cudaEventRecord(h.lists_ev, h.stream));
-    FMM_CUDA(cudaStreamWaitEvent(h.side, h.lists_ev, 0));
-    {
-      Timer t(h, PH_P2P, h.side);
-      p2p_pass(h, h.side);
-    }
-    FMM_CUDA(cudaEventRecord(h.join_ev, h.side));
+    auto near_field = [&] {
+      FMM_CUDA(cudaEventRecord(h.lists_ev, h.stream));
+      FMM_CUDA(cudaStreamWaitEvent(h.side, h.lists_ev, 0));
+      {
+        Timer t(h, PH_P2P, h.side);
+        p2p_pass(h, h.side);
+      }
+      FMM_CUDA(cudaEventRecord(h.join_ev, h.side));
+    };
+    // the near field starts as soon as its lists are made: it runs while the
+    // host waits for the lists' counts
+    if (rebuild) do_lists(h, near_field);
+    else near_field();
     FMM_CUDA(cudaStreamWaitEvent(h.stream, h.up_ev, 0));
     Timer t(h, PH_M2L);
     m2l_pass(h);

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -220,7 +221,10 @@ void radix_sort_pairs(Handle &h, u64 *&k, u32 *&v, u64 *&k2, u32 *&v2, long n, i
 // tree.cu
 void build_tree(Handle &h);
 // lists.cu
-void build_lists(Handle &h);
+// near_field (or empty): queues the near field on h.side; called once the P2P
+// lists are queued on h.stream, before the host waits for their counts (again
+// if the lists overflowed their buffers and are made again)
+void build_lists(Handle &h, const std::function<void()> &near_field);
 void export_lists(Handle &h, int *m2l_off, int *m2l_src, int *m2l_img, int *p2p_off, int *p2p_src, int *p2p_img);
 void order_m2l_lists(Handle &h);
 // expansions.cu

@@ -17,6 +17,7 @@
 // of one target in pre-order, because a target-side split never reorders
 // them).  The result equals getList's per-cell lists entry for entry.
 #include <cstddef>
+#include <functional>
 
 #include "group_key.cuh"
 
@@ -436,7 +437,7 @@ void order_m2l_lists(Handle &h) {
   h.m2l_ordered = true;
 }
 
-void build_lists(Handle &h) {
+void build_lists(Handle &h, const std::function<void()> &near_field) {
   cudaStream_t s = h.stream;
   h.g_plan.valid = false;  // new lists: the M2L grouping is redone
   DevCounters *ctr = h.counters.as<DevCounters>();
@@ -496,12 +497,14 @@ void build_lists(Handle &h) {
     // entries.  The P2P lists are ordered always: their order is the near
     // field's summation order, which keeps results reproducible.
     bucket(h, h.p2p_raw.as<int2>(), &ctr->n_p2p, (int64_t)h.p2p_cap, h.p2p_off, h.p2p_ent, gt.cnt, true);
+    if (near_field) near_field();
     const bool group = m2l_groups_raw(h);
     if (group) m2l_group_launch(h, (long)h.m2l_cap);
     read_counters(h);
     if (h.hc->list_overflow) {
       // a dropped frontier pair also hides its descendants' entries: grow
-      // everything and walk again
+      // everything and walk again, once a near field on these lists is over
+      if (near_field) FMM_CUDA(cudaStreamSynchronize(h.side));
       if (attempt >= 4) throw Error{EXAFMM_ERR_CAPACITY, "interaction list buffers kept overflowing"};
       h.m2l_cap = std::max<size_t>(2 * h.m2l_cap, (size_t)(h.hc->n_m2l * 5 / 4 + 1024));
       h.p2p_cap = std::max<size_t>(2 * h.p2p_cap, (size_t)(h.hc->n_p2p * 5 / 4 + 1024));

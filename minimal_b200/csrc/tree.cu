@@ -234,13 +234,19 @@ __device__ long run_ahead(const u64 *keys, long i, long n, int D, int l, u64 p, 
 // first-children), plus the depth overflow check.  A run that starts at i
 // holds more than ncrit bodies iff body i + ncrit shares its prefix, so the
 // chain length follows from one comparison of keys; the parent test counts
-// at most ncrit + 1 bodies on either side of i.
-__global__ void k_chain(const u64 *keys, long n, int D, int ncrit, int *lfirst, int *chain, DevCounters *ctr) {
+// at most ncrit + 1 bodies on either side of i.  A chain's cells lie on
+// consecutive levels and its last one is a leaf, so the cells per level and
+// the leaves are counted here too: one read of the counts tells the host all
+// that the launches up to the lists need.
+__global__ void __launch_bounds__(TB) k_chain(const u64 *keys, long n, int D, int ncrit, int *lfirst, int *chain,
+                                              DevCounters *ctr) {
+  __shared__ int lc[EXAFMM_MAX_LEVEL + 2];  // cells per level that start in this block
+  if (threadIdx.x < EXAFMM_MAX_LEVEL + 2) lc[threadIdx.x] = 0;
+  __syncthreads();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int lf = first_level(keys, i, D);
-  lfirst[i] = lf;
   int len = 0;
+  const int lf = i < n ? first_level(keys, i, D) : D + 1;
+  if (i < n) lfirst[i] = lf;
   if (lf <= D) {
     const u64 key = keys[i];
     bool parent_splits = true;  // a system's root is always a cell
@@ -261,7 +267,11 @@ __global__ void k_chain(const u64 *keys, long n, int D, int ncrit, int *lfirst, 
       len = last - lf + 1;
     }
   }
-  chain[i] = len;
+  if (i < n) chain[i] = len;
+  for (int k = 0; k < len; k++) atomicAdd_block(&lc[lf + k], 1);
+  const int leaves = __syncthreads_count(len > 0);
+  if (threadIdx.x == 0 && leaves) atomicAdd(&ctr->nleaves, leaves);
+  if (threadIdx.x < EXAFMM_MAX_LEVEL + 2 && lc[threadIdx.x]) atomicAdd(&ctr->level_count[threadIdx.x], lc[threadIdx.x]);
 }
 
 struct PreTables {
@@ -280,10 +290,7 @@ __global__ void k_cell_owner(long n, const int *chain, const int *prebase, int *
 // One thread per cell (pre-order rank p): the k-th cell of the chain that
 // starts at body i = owner[p] is at level lfirst[i] + k.
 __global__ void k_cells(const u64 *keys, long n, long C, int D, const int *lfirst, const int *owner,
-                        const int *prebase, const RootGeom *g, PreTables t, DevCounters *ctr) {
-  __shared__ int lc[EXAFMM_MAX_LEVEL + 2];  // cells per level made by this block
-  if (threadIdx.x < EXAFMM_MAX_LEVEL + 2) lc[threadIdx.x] = 0;
-  __syncthreads();
+                        const int *prebase, const RootGeom *g, PreTables t) {
   const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p < C) {
     const long i = owner[p];
@@ -313,11 +320,8 @@ __global__ void k_cells(const u64 *keys, long n, long C, int D, const int *lfirs
     t.level[p] = l;
     t.parent[p] = parent;
     t.xr[p] = make_double4(cx, cy, cz, r);
-    atomicAdd_block(&lc[l], 1);
     if (parent >= 0) atomicAdd(&t.nchild[parent], 1);
   }
-  __syncthreads();
-  if (threadIdx.x < EXAFMM_MAX_LEVEL + 2 && lc[threadIdx.x]) atomicAdd(&ctr->level_count[threadIdx.x], lc[threadIdx.x]);
 }
 
 __global__ void k_level_keys(const int *level, long c, u64 *k, u32 *v) {
@@ -453,6 +457,8 @@ void build_tree(Handle &h) {
     h.launches++;
     FMM_LAUNCH();
     scan_exclusive_int(h, h.chain.as<int>(), h.prebase.as<int>(), n, &ctr->ncells);
+    if (h.prm.images > 0)  // the root radius, for the M2L operators of image keys
+      FMM_CUDA(cudaMemcpyAsync(&h.root_R0, &g->R0, sizeof(double), cudaMemcpyDeviceToHost, s));
     read_counters(h);
     if (h.hc->overflow) {
       if (D == max_levels)
@@ -464,6 +470,13 @@ void build_tree(Handle &h) {
     const long C = h.hc->ncells;
     h.ncells = (int)C;
     h.key_levels = D;
+    h.nleaves = h.hc->nleaves;
+    h.depth = 0;
+    h.level_base[0] = 0;
+    for (int l = 0; l <= EXAFMM_MAX_LEVEL; l++) {
+      h.level_base[l + 1] = h.level_base[l] + h.hc->level_count[l];
+      if (h.hc->level_count[l]) h.depth = l;
+    }
     // pre-order tables (reuse the idle sort buffers' siblings)
     const long Cp = (C + 3) & ~3L;  // every table starts 16-byte aligned (vector loads in the scans)
     h.pre_tmp.need(Cp * (6 * sizeof(int) + sizeof(double4)) + 256);
@@ -477,7 +490,7 @@ void build_tree(Handle &h) {
     int *owner = t.nchild + Cp;
     FMM_CUDA(cudaMemsetAsync(t.nchild, 0, C * sizeof(int), s));
     k_cell_owner<<<grid_for(n, TB), TB, 0, s>>>(n, h.chain.as<int>(), h.prebase.as<int>(), owner);
-    k_cells<<<grid_for(C, TB), TB, 0, s>>>(k, n, C, D, h.lfirst.as<int>(), owner, h.prebase.as<int>(), g, t, ctr);
+    k_cells<<<grid_for(C, TB), TB, 0, s>>>(k, n, C, D, h.lfirst.as<int>(), owner, h.prebase.as<int>(), g, t);
     h.launches += 2;
     FMM_LAUNCH();
 
@@ -503,21 +516,11 @@ void build_tree(Handle &h) {
     FMM_LAUNCH();
     // reference numbering, and the leaves
     h.leaves.need(C * 4);
-    scan_exclusive_pair(h, t.nchild, blockstart, nullptr, is_leaf, leafpos, &ctr->nleaves, C);
+    scan_exclusive_pair(h, t.nchild, blockstart, nullptr, is_leaf, leafpos, nullptr, C);
     k_ref_leaves<<<grid_for(C, TB), TB, 0, s>>>(o, C, blockstart, h.c_ref.as<int>(), is_leaf, leafpos,
                                                 h.leaves.as<int>());
     h.launches++;
     FMM_LAUNCH();
-    if (h.prm.images > 0)  // the root radius, for the M2L operators of image keys
-      FMM_CUDA(cudaMemcpyAsync(&h.root_R0, &g->R0, sizeof(double), cudaMemcpyDeviceToHost, s));
-    read_counters(h);
-    h.nleaves = h.hc->nleaves;
-    h.depth = 0;
-    h.level_base[0] = 0;
-    for (int l = 0; l <= EXAFMM_MAX_LEVEL; l++) {
-      h.level_base[l + 1] = h.level_base[l] + h.hc->level_count[l];
-      if (h.hc->level_count[l]) h.depth = l;
-    }
     // 6. bodies of each leaf back to input order and gathered (the mixed
     // form's FP32 sources with them)
     h.perm.need(n * 4);
