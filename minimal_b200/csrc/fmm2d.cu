@@ -10,13 +10,12 @@
 // rules are the 2D ones (2d/traverse_lazy.h:27-44), and a 2dp system seeds
 // the nine in-plane images (2dp/traverse_lazy.h:124-141).  What is new here
 // is the arithmetic:
-//   P2M, L2P   warp per leaf, lane per body, z^n/n! generated as in the
-//              reference (powZ *= Z / n);
-//   M2M, L2L   per level, thread per (cell, coefficient);
-//   M2L        warp per target cell over its ordered M2L list, lane n owns
-//              L[n]: lane 0 the log term and 1/z^k series, lane 1 the 1/z^(k+1)
-//              series, lane n >= 2 the (n+k-1)!/z^(n+k) series
+//   P2M, L2P   a few lanes per leaf, the leaf's coefficients in registers;
+//   M2M, L2L   per level, a lane per child cell, coefficients in registers;
+//   M2L        warp per target cell over its ordered M2L list, lane per entry
 //              (2d/kernel.h:61-90; the 2dp image shift :63);
+// these for orders up to 16, as compile-time constants; above, warps per leaf,
+// threads per coefficient and a warp per M2L entry;
 //   P2P        warp per target leaf over its ordered P2P list, lane per
 //              target body, q log(1/R) and q dX / R^2 (2d/kernel.h:12-31);
 //   periodic   one warp: the 72 root M2Ls and the 8-copy M2M per image level
@@ -39,6 +38,16 @@ __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_doub
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 cmulr(double2 a, double r) { return make_double2(a.x * r, a.y * r); }
 
+// a += b c, a -= b c
+__device__ __forceinline__ void cadd_mul(double2 &a, double2 b, double2 c) {
+  a.x = fma(b.x, c.x, fma(-b.y, c.y, a.x));
+  a.y = fma(b.x, c.y, fma(b.y, c.x, a.y));
+}
+__device__ __forceinline__ void csub_mul(double2 &a, double2 b, double2 c) {
+  a.x = fma(-b.x, c.x, fma(b.y, c.y, a.x));
+  a.y = fma(-b.x, c.y, fma(-b.y, c.x, a.y));
+}
+
 // 1/z with Smith's scaling (no overflow for large or small |z|).
 __device__ __forceinline__ double2 crecip(double2 z) {
   if (fabs(z.x) >= fabs(z.y)) {
@@ -50,6 +59,20 @@ __device__ __forceinline__ double2 crecip(double2 z) {
 }
 
 __device__ __forceinline__ double2 clog2(double2 z) { return make_double2(log(hypot(z.x, z.y)), atan2(z.y, z.x)); }
+
+// 1/z and log z of one offset from |z|^2 where that is well inside the range
+// (one division, no hypot), else by crecip and clog2.
+__device__ __forceinline__ void crecip_log(double2 z, double2 &iz, double2 &lz) {
+  const double r2 = z.x * z.x + z.y * z.y;
+  if (r2 > 1e-280 && r2 < 1e280) {
+    const double inv = 1.0 / r2;
+    iz = make_double2(z.x * inv, -z.y * inv);
+    lz = make_double2(0.5 * log(r2), atan2(z.y, z.x));
+  } else {
+    iz = crecip(z);
+    lz = clog2(z);
+  }
+}
 
 // Image shift of a list entry: periodic1D of the 3D walk with z = 0.
 __device__ __forceinline__ void img_shift(u32 img, double cycle, double &sx, double &sy) {
@@ -216,8 +239,9 @@ __global__ void __launch_bounds__(W2 * 32) k2_m2l_lane(int ncells, const int *of
     double2 Mk[P];
 #pragma unroll
     for (int k = 0; k < P; k++) Mk[k] = M[(long)s * P + k];
-    const double2 iz = crecip(Z);
-    acc[0] = csub(acc[0], cmul(Mk[0], clog2(Z)));
+    double2 iz, lz;
+    crecip_log(Z, iz, lz);
+    csub_mul(acc[0], Mk[0], lz);
     double2 q = iz;  // q_1
 #pragma unroll
     for (int m = 1; m <= 2 * P - 2; m++) {
@@ -225,8 +249,8 @@ __global__ void __launch_bounds__(W2 * 32) k2_m2l_lane(int ncells, const int *of
       for (int n = 0; n < P; n++) {
         const int k = m - n;
         if (k < 0 || k >= P) continue;
-        const double2 term = cmul(Mk[k], q);
-        acc[n] = (n & 1) ? csub(acc[n], term) : cadd(acc[n], term);
+        if (n & 1) csub_mul(acc[n], Mk[k], q);
+        else cadd_mul(acc[n], Mk[k], q);
       }
       if (m < 2 * P - 2) q = cmulr(cmul(q, iz), (double)m);
     }
@@ -347,6 +371,152 @@ __global__ void __launch_bounds__(W2 * 32) k2_l2p(const int *leaves, int nleaves
   }
 }
 
+// ---- orders up to 16: the same operators with every coefficient in
+// registers (P a compile-time constant) and z^n/n! built with the reciprocals
+// 1/n as constants.  With a warp per leaf of about 4 bodies and a division
+// per term, the four took 650, 318, 316 and 355 us at 1M bodies, P = 10,
+// ncrit = 8, where they now take 28, 42, 82 and 77 us (their reads and writes, 60-130 MB
+// each, take 10-20 us; the rest is latency of short leaves and levels).
+template <int P>
+__device__ __forceinline__ double2 next_power(double2 pz, double2 Z, int n) {
+  return cmul(pz, cmulr(Z, 1.0 / n));  // n is a constant of the unrolled loop
+}
+
+// P2M: G lanes per leaf (a power of two), each summing every G-th body; the
+// lanes' sums are added in butterfly order.
+template <int P, int G>
+__global__ void __launch_bounds__(128) k2_p2m_r(const int *leaves, int nleaves, const int *begin, const int *count,
+                                                const double4 *xr, const double4 *src, double2 *M) {
+  const int t = blockIdx.x * 128 + threadIdx.x, w = min(t / G, nleaves - 1), g = t % G;
+  const int c = leaves[w], b0 = begin[c], nb = count[c];
+  const double4 C = xr[c];
+  double2 acc[P];
+#pragma unroll
+  for (int n = 0; n < P; n++) acc[n] = make_double2(0, 0);
+  for (int b = g; b < nb; b += G) {
+    const double4 B = src[b0 + b];
+    const double2 Z = make_double2(B.x - C.x, B.y - C.y);
+    double2 pz = make_double2(1, 0);
+    acc[0].x += B.w;
+#pragma unroll
+    for (int n = 1; n < P; n++) {
+      pz = next_power<P>(pz, Z, n);
+      acc[n].x = fma(pz.x, B.w, acc[n].x);
+      acc[n].y = fma(pz.y, B.w, acc[n].y);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < P; n++)
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      acc[n].x += __shfl_xor_sync(0xffffffffu, acc[n].x, o);
+      acc[n].y += __shfl_xor_sync(0xffffffffu, acc[n].y, o);
+    }
+  if (t / G >= nleaves) return;
+#pragma unroll
+  for (int n = 0; n < P; n++)
+    if (n % G == g) M[(long)c * P + n] = acc[n];
+}
+
+// M2M for the parents of one level: four lanes per parent, a lane per child
+// (a quadtree cell has at most four), added in butterfly order.
+template <int P>
+__global__ void __launch_bounds__(128) k2_m2m_r(int c0, int ncell, const int *child, const int *nchild,
+                                                const double4 *xr, double2 *M) {
+  const int t = blockIdx.x * 128 + threadIdx.x, q = t & 3;
+  const int c = c0 + min(t >> 2, ncell - 1), nc = nchild[c];
+  double2 acc[P];
+#pragma unroll
+  for (int n = 0; n < P; n++) acc[n] = make_double2(0, 0);
+  if (q < nc) {
+    const int j = child[c] + q;
+    const double4 X = xr[c], Y = xr[j];
+    const double2 Z = make_double2(Y.x - X.x, Y.y - X.y);
+    double2 Mc[P], pz = make_double2(1, 0);
+#pragma unroll
+    for (int n = 0; n < P; n++) acc[n] = Mc[n] = M[(long)j * P + n];
+#pragma unroll
+    for (int n = 1; n < P; n++) {
+      pz = next_power<P>(pz, Z, n);
+#pragma unroll
+      for (int k = n; k < P; k++) cadd_mul(acc[k], Mc[k - n], pz);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < P; n++)
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1) {
+      acc[n].x += __shfl_xor_sync(0xffffffffu, acc[n].x, o);
+      acc[n].y += __shfl_xor_sync(0xffffffffu, acc[n].y, o);
+    }
+  if ((t >> 2) >= ncell || nc == 0) return;  // a leaf keeps its P2M
+#pragma unroll
+  for (int n = 0; n < P; n++)
+    if ((n & 3) == q) M[(long)c * P + n] = acc[n];
+}
+
+// L2L into the cells [c0, c0 + ncell) of one level: a thread per cell.
+template <int P>
+__global__ void __launch_bounds__(128) k2_l2l_r(int c0, int ncell, const int *parent, const double4 *xr, double2 *L) {
+  const int t = blockIdx.x * 128 + threadIdx.x;
+  if (t >= ncell) return;
+  const int j = c0 + t, c = parent[j];
+  if (c < 0) return;
+  const double4 X = xr[c], Y = xr[j];
+  const double2 Z = make_double2(Y.x - X.x, Y.y - X.y);
+  double2 Lp[P], acc[P], pz = make_double2(1, 0);
+#pragma unroll
+  for (int n = 0; n < P; n++) {
+    Lp[n] = L[(long)c * P + n];
+    acc[n] = cadd(L[(long)j * P + n], Lp[n]);
+  }
+#pragma unroll
+  for (int k = 1; k < P; k++) {
+    pz = next_power<P>(pz, Z, k);
+#pragma unroll
+    for (int l = 0; l + k < P; l++) cadd_mul(acc[l], Lp[l + k], pz);
+  }
+#pragma unroll
+  for (int n = 0; n < P; n++) L[(long)j * P + n] = acc[n];
+}
+
+// L2P: G lanes per leaf, each taking every G-th body; Horner's scheme for the
+// potential and the force: sum L_n z^n/n! = L_0 + z/1 (L_1 + z/2 (L_2 + ...)).
+template <int P, int G>
+__global__ void __launch_bounds__(128) k2_l2p_r(const int *leaves, int nleaves, const int *begin, const int *count,
+                                                const double4 *xr, const double4 *src, const double2 *L,
+                                                double4 *out) {
+  const int t = blockIdx.x * 128 + threadIdx.x, w = t / G, g = t % G;
+  if (w >= nleaves) return;
+  const int c = leaves[w], b0 = begin[c], nb = count[c];
+  const double4 C = xr[c];
+  double2 Lc[P];
+#pragma unroll
+  for (int n = 0; n < P; n++) Lc[n] = L[(long)c * P + n];
+  for (int b = b0 + g; b < b0 + nb; b += G) {
+    const double4 B = src[b];
+    const double2 Z = make_double2(B.x - C.x, B.y - C.y);
+    double2 h = Lc[P - 1], f = Lc[P - 1];
+#pragma unroll
+    for (int n = P - 1; n > 0; n--) {
+      const double2 zn = cmulr(Z, 1.0 / n);
+      if (n < P - 1) {
+        double2 v = Lc[n];
+        cadd_mul(v, f, zn);
+        f = v;
+      }
+      double2 v = Lc[n - 1];
+      cadd_mul(v, h, zn);
+      h = v;
+    }
+    double4 o = out[b];
+    o.x += h.x;
+    o.y += f.x;
+    o.z -= f.y;
+    out[b] = o;
+  }
+}
+
 // P2P (2d/kernel.h:12-31; 2dp: the image shift of each list entry):
 // p += q log(1/r), F -= q (dx, dy) / r^2 over the target leaf's ordered near
 // list, each source leaf's sums added to the body as one term, as the
@@ -464,10 +634,53 @@ void flatten_tree_2d(Handle &h) {
   FMM_LAUNCH();
 }
 
+// f(P as a constant) for the orders with register kernels; false for others.
+template <class F>
+bool with_order(int P, F f) {
+  switch (P) {
+#define EXAFMM_2D_ORDER(p) \
+  case p:                  \
+    f(std::integral_constant<int, p>{}); \
+    return true;
+    EXAFMM_2D_ORDER(2) EXAFMM_2D_ORDER(3) EXAFMM_2D_ORDER(4) EXAFMM_2D_ORDER(5) EXAFMM_2D_ORDER(6)
+    EXAFMM_2D_ORDER(7) EXAFMM_2D_ORDER(8) EXAFMM_2D_ORDER(9) EXAFMM_2D_ORDER(10) EXAFMM_2D_ORDER(11)
+    EXAFMM_2D_ORDER(12) EXAFMM_2D_ORDER(13) EXAFMM_2D_ORDER(14) EXAFMM_2D_ORDER(15) EXAFMM_2D_ORDER(16)
+#undef EXAFMM_2D_ORDER
+  }
+  return false;
+}
+
+// Lanes per leaf of P2M and L2P: one while the leaves are short on average,
+// else eight.
+constexpr int LEAF_LANES = 8, LONG_LEAF = 12;
+bool long_leaves(const Handle &h) { return h.n > (int64_t)LONG_LEAF * h.nleaves; }
+
 void upward_pass_2d(Handle &h, cudaStream_t s) {
   const int P = h.prm.P;
   h.M.need((size_t)h.ncells * P * sizeof(double2));
   h.L.need((size_t)h.ncells * P * sizeof(double2));
+  const bool done = with_order(P, [&](auto pc) {
+    constexpr int PP = decltype(pc)::value;
+    auto p2m = [&](auto gc) {
+      constexpr int G = decltype(gc)::value;
+      k2_p2m_r<PP, G><<<grid_for((long)h.nleaves * G, 128), 128, 0, s>>>(
+          h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.c_xr.as<double4>(),
+          h.src.as<double4>(), h.M.as<double2>());
+    };
+    if (long_leaves(h)) p2m(std::integral_constant<int, LEAF_LANES>{});
+    else p2m(std::integral_constant<int, 1>{});
+    h.launches++;
+    for (int l = h.depth - 1; l >= 0; l--) {
+      const int c0 = h.level_base[l], c1 = h.level_base[l + 1];
+      if (c1 <= c0) continue;
+      k2_m2m_r<PP><<<grid_for((long)(c1 - c0) * 4, 128), 128, 0, s>>>(c0, c1 - c0, h.c_child.as<int>(),
+                                                                     h.c_nchild.as<int>(), h.c_xr.as<double4>(),
+                                                                     h.M.as<double2>());
+      h.launches++;
+    }
+    FMM_LAUNCH();
+  });
+  if (done) return;
   k2_p2m<<<grid_for(h.nleaves, W2), W2 * 32, W2 * P * sizeof(double2), s>>>(
       h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.c_xr.as<double4>(),
       h.src.as<double4>(), h.M.as<double2>(), P);
@@ -489,31 +702,14 @@ void m2l_pass_2d(Handle &h) {
   order_m2l_lists(h);
   const double cyc = h.prm.images ? h.prm.cycle : 0.0;
   const int g = grid_for(h.ncells, W2);
-  auto lane_form = [&](auto pc) {
+  const bool done = with_order(P, [&](auto pc) {
     constexpr int PP = decltype(pc)::value;
     k2_m2l_lane<PP><<<g, W2 * 32, 0, h.stream>>>(h.ncells, h.m2l_off.as<int>(), h.m2l_ent.as<u32>(),
                                                 h.c_xr.as<double4>(), h.M.as<double2>(), h.L.as<double2>(), cyc);
-  };
-  switch (P) {
-    case 2: lane_form(std::integral_constant<int, 2>{}); break;
-    case 3: lane_form(std::integral_constant<int, 3>{}); break;
-    case 4: lane_form(std::integral_constant<int, 4>{}); break;
-    case 5: lane_form(std::integral_constant<int, 5>{}); break;
-    case 6: lane_form(std::integral_constant<int, 6>{}); break;
-    case 7: lane_form(std::integral_constant<int, 7>{}); break;
-    case 8: lane_form(std::integral_constant<int, 8>{}); break;
-    case 9: lane_form(std::integral_constant<int, 9>{}); break;
-    case 10: lane_form(std::integral_constant<int, 10>{}); break;
-    case 11: lane_form(std::integral_constant<int, 11>{}); break;
-    case 12: lane_form(std::integral_constant<int, 12>{}); break;
-    case 13: lane_form(std::integral_constant<int, 13>{}); break;
-    case 14: lane_form(std::integral_constant<int, 14>{}); break;
-    case 15: lane_form(std::integral_constant<int, 15>{}); break;
-    case 16: lane_form(std::integral_constant<int, 16>{}); break;
-    default:  // larger orders: a warp per entry, a lane per coefficient
-      k2_m2l<<<g, W2 * 32, 0, h.stream>>>(h.ncells, h.m2l_off.as<int>(), h.m2l_ent.as<u32>(), h.c_xr.as<double4>(),
-                                          h.M.as<double2>(), h.L.as<double2>(), P, cyc);
-  }
+  });
+  if (!done)  // larger orders: a warp per entry, a lane per coefficient
+    k2_m2l<<<g, W2 * 32, 0, h.stream>>>(h.ncells, h.m2l_off.as<int>(), h.m2l_ent.as<u32>(), h.c_xr.as<double4>(),
+                                        h.M.as<double2>(), h.L.as<double2>(), P, cyc);
   h.launches++;
   FMM_LAUNCH();
 }
@@ -538,6 +734,28 @@ void p2p_pass_2d(Handle &h, cudaStream_t s) {
 
 void downward_pass_2d(Handle &h, cudaStream_t s, cudaEvent_t before_l2p) {
   const int P = h.prm.P;
+  const bool done = with_order(P, [&](auto pc) {
+    constexpr int PP = decltype(pc)::value;
+    for (int l = 1; l <= h.depth; l++) {
+      const int c0 = h.level_base[l], c1 = h.level_base[l + 1];
+      if (c1 <= c0) continue;
+      k2_l2l_r<PP><<<grid_for(c1 - c0, 128), 128, 0, s>>>(c0, c1 - c0, h.c_parent.as<int>(), h.c_xr.as<double4>(),
+                                                          h.L.as<double2>());
+      h.launches++;
+    }
+    if (before_l2p) FMM_CUDA(cudaStreamWaitEvent(s, before_l2p, 0));
+    auto l2p = [&](auto gc) {
+      constexpr int G = decltype(gc)::value;
+      k2_l2p_r<PP, G><<<grid_for((long)h.nleaves * G, 128), 128, 0, s>>>(
+          h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.c_xr.as<double4>(),
+          h.src.as<double4>(), h.L.as<double2>(), h.out.as<double4>());
+    };
+    if (long_leaves(h)) l2p(std::integral_constant<int, LEAF_LANES>{});
+    else l2p(std::integral_constant<int, 1>{});
+    h.launches++;
+    FMM_LAUNCH();
+  });
+  if (done) return;
   for (int l = 0; l < h.depth; l++) {
     const int c0 = h.level_base[l], c1 = h.level_base[l + 1];
     if (c1 <= c0) continue;
