@@ -519,66 +519,120 @@ __global__ void __launch_bounds__(128) k2_l2p_r(const int *leaves, int nleaves, 
 
 // P2P (2d/kernel.h:12-31; 2dp: the image shift of each list entry):
 // p += q log(1/r), F -= q (dx, dy) / r^2 over the target leaf's ordered near
-// list, each source leaf's sums added to the body as one term, as the
-// reference's per-pair calls do; writes out (the first writer).  A warp per
-// target leaf.  For leaves of up to 16
-// bodies the lanes are (target i, entry group g), G = floor(32 / nb) groups
-// taking the list entries round-robin, and the groups' sums are added in
-// group order at the end (deterministic); larger leaves take a lane per
-// target.  log(1/r) is formed as -log(r^2) / 2 and the force with one
-// reciprocal of r^2 (the reference's quantities, to rounding).
+// list; writes out (the first writer).  A warp per target leaf.  The bodies of
+// the list's leaves are staged S2 at a time in shared memory (PERIODIC: with
+// their image's shift, subtracted after the positions as the reference does:
+// whether two bodies a period apart coincide depends on it), and the lanes are (target i, part g): every lane takes every
+// G-th staged body, G = floor(32 / targets), so the lanes are busy whatever
+// the sizes of the source leaves (with the entries dealt to the parts, 884 us
+// at 1M bodies, ncrit = 8; now 650).  The parts' sums are added in part
+// order at the end (deterministic).  log(1/r) is -log(r^2) / 2; pairs at
+// distance zero count nothing.
+constexpr int S2 = 128;
+
+// 1/x for a normal x far from the ends of the range: the hardware's estimate
+// and one third-order Newton step.
+__device__ __forceinline__ double recip_normal(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+template <bool PERIODIC>
 __global__ void __launch_bounds__(W2 * 32) k2_p2p(const int *leaves, int nleaves, const int *begin, const int *count,
                                                   const int *off, const u32 *ent, const double4 *src, double4 *out,
                                                   double cycle) {
+  __shared__ double2 sxy[W2][S2];
+  __shared__ double sq[W2][S2];
+  __shared__ double2 ssh[W2][PERIODIC ? S2 : 1];
+  constexpr unsigned FULL = 0xffffffffu;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w = blockIdx.x * W2 + wid;
   if (w >= nleaves) return;  // warp-uniform
   const int c = leaves[w], b0 = begin[c], nb = count[c];
   const int e0 = off[c], e1 = off[c + 1];
-  const int G = nb <= 16 ? 32 / nb : 1;  // entry groups
-  const int span = nb <= 16 ? nb : 32;   // targets per pass
+  const int span = min(nb, 32), G = 32 / span;  // targets per pass, parts
   const int i = lane % span, g = lane / span;
-  const bool lane_ok = g < G;
   for (int tb = 0; tb < nb; tb += span) {
     const int t = tb + i;
-    const bool ok = lane_ok && t < nb;
+    const bool ok = g < G && t < nb;
     const double4 T = ok ? src[b0 + t] : make_double4(0, 0, 0, 0);
-    double p = 0, fx = 0, fy = 0;
-    if (lane_ok) {
-      for (int e = e0 + g; e < e1; e += G) {
-        const u32 en = ent[e];
+    double lp = 0, fx = 0, fy = 0;  // sums of q log r^2, q dx / r^2, q dy / r^2
+    for (int e = e0; e < e1; e += 32) {
+      // lane k: the k-th of up to 32 source leaves
+      int n = 0, base = 0;
+      double sx = 0, sy = 0;
+      if (e + lane < e1) {
+        const u32 en = ent[e + lane];
         const int s = (int)(en & IDX_MASK);
-        double sx, sy;
+        n = count[s];
+        base = begin[s];
         img_shift(en >> IMG_SHIFT, cycle, sx, sy);
-        double pp = 0, px = 0, py = 0;
-        for (int j = begin[s]; j < begin[s] + count[s]; j++) {
-          const double4 S = src[j];
-          const double dx = T.x - S.x - sx, dy = T.y - S.y - sy;
-          const double R2 = dx * dx + dy * dy;
-          if (R2 != 0) {
-            const double invR2 = 1 / R2;
-            pp -= 0.5 * S.w * log(R2);
-            px += dx * S.w * invR2;
-            py += dy * S.w * invR2;
+      }
+      int inc = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(FULL, inc, o);
+        if (lane >= o) inc += v;
+      }
+      const int total = __shfl_sync(FULL, inc, 31);
+      base -= inc - n;  // body of slot j of this leaf: base + j
+      for (int w0 = 0; w0 < total; w0 += S2) {
+        const int m = min(S2, total - w0);
+        __syncwarp();
+        for (int k = lane; k - lane < m; k += 32) {
+          const int j = w0 + k;
+          int lo = 0;  // the leaves that end at or before slot j
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1)
+            if (__shfl_sync(FULL, inc, lo + step - 1) <= j) lo += step;
+          const int bk = __shfl_sync(FULL, base, lo & 31);
+          double2 sh;
+          if (PERIODIC) sh = make_double2(__shfl_sync(FULL, sx, lo & 31), __shfl_sync(FULL, sy, lo & 31));
+          if (k < m) {
+            const double4 B = src[bk + j];
+            sxy[wid][k] = make_double2(B.x, B.y);
+            sq[wid][k] = B.w;
+            if (PERIODIC) ssh[wid][k] = sh;
           }
         }
-        p += pp;
-        fx -= px;
-        fy -= py;
+        __syncwarp();
+        if (ok) {
+#pragma unroll 2
+          for (int k = g; k < m; k += G) {
+            const double2 S = sxy[wid][k];
+            double q = sq[wid][k];
+            double dx = T.x - S.x, dy = T.y - S.y;
+            if (PERIODIC) {
+              dx -= ssh[wid][k].x;
+              dy -= ssh[wid][k].y;
+            }
+            double r2 = dx * dx + dy * dy;
+            if (r2 == 0) {
+              r2 = 1;
+              q = 0;
+            }
+            const double inv = r2 > 1e-280 && r2 < 1e280 ? recip_normal(r2) : 1.0 / r2;
+            const double qi = q * inv;
+            lp = fma(q, log(r2), lp);
+            fx = fma(dx, qi, fx);
+            fy = fma(dy, qi, fy);
+          }
+        }
       }
     }
-    // group 0 adds the other groups' sums in group order
+    // part 0 adds the other parts' sums in part order
     for (int gg = 1; gg < G; gg++) {
       const int from = (gg * span + i) & 31;
-      const double vp = __shfl_sync(0xffffffffu, p, from), vx = __shfl_sync(0xffffffffu, fx, from),
-                   vy = __shfl_sync(0xffffffffu, fy, from);
+      const double vp = __shfl_sync(FULL, lp, from), vx = __shfl_sync(FULL, fx, from), vy = __shfl_sync(FULL, fy, from);
       if (g == 0) {
-        p += vp;
+        lp += vp;
         fx += vx;
         fy += vy;
       }
     }
-    if (ok && g == 0) out[b0 + t] = make_double4(p, fx, fy, 0.0);
+    if (ok && g == 0) out[b0 + t] = make_double4(-0.5 * lp, -fx, -fy, 0.0);
   }
 }
 
@@ -724,7 +778,8 @@ void periodic_pass_2d(Handle &h) {
 
 void p2p_pass_2d(Handle &h, cudaStream_t s) {
   h.out.need((size_t)h.n * sizeof(double4));
-  k2_p2p<<<grid_for(h.nleaves, W2), W2 * 32, 0, s>>>(h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(),
+  auto kern = h.prm.images ? k2_p2p<true> : k2_p2p<false>;
+  kern<<<grid_for(h.nleaves, W2), W2 * 32, 0, s>>>(h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(),
                                                      h.c_count.as<int>(), h.p2p_off.as<int>(), h.p2p_ent.as<u32>(),
                                                      h.src.as<double4>(), h.out.as<double4>(),
                                                      h.prm.images ? h.prm.cycle : 0.0);
