@@ -236,6 +236,7 @@ void m2l_pass(Handle &h);
 // m2l_group.cu: group tables from the key and target marks of the lists.
 // m2l_group_launch() queues the kernels; once the counters have been read,
 // m2l_group_commit() builds the operators of the keys not seen before.
+bool m2l_keyed(const Handle &h);       // the M2L is the grouped one: the walk computes and marks keys
 bool m2l_groups_raw(const Handle &h);  // the walk's own marks are what the grouped M2L contracts
 void m2l_group_launch(Handle &h, long max_groups);
 void m2l_group_commit(Handle &h);

@@ -215,21 +215,22 @@ __global__ void __launch_bounds__(W2 * 32) k2_m2l(int ncells, const int *off, co
 // one reciprocal, one logarithm, the q_m by the recurrence
 // q_(m+1) = q_m m / z and P^2 complex products, summed along n + k = m --
 // with every coefficient in registers (P is a compile-time constant), while
-// the warp's lanes take the target's entries 32 at a time.  The lanes' sums
-// are then added in a fixed butterfly order (deterministic).  The operations
+// M2L_G lanes take a target's entries in turn.  The lanes' sums are then added
+// in a fixed butterfly order (deterministic).  Lists hold about 30 entries
+// (33 to 35 inside a uniform tree), so a warp per target had 60% of its lanes
+// busy (1M bodies, P = 10: 1100 us; 16, 8 and 4 lanes: 823, 689 and 654); trees
+// too small to fill the GPU with 4 lanes per target take 16.  The operations
 // are those of m2l_term in another order: the expansions agree with it, and
 // with the reference, to rounding.
-template <int P>
+template <int P, int M2L_G>
 __global__ void __launch_bounds__(W2 * 32) k2_m2l_lane(int ncells, const int *off, const u32 *ent, const double4 *xr,
                                                        const double2 *M, double2 *L, double cycle) {
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * W2 + wid;
-  if (t >= ncells) return;  // warp-uniform
+  const int g = threadIdx.x % M2L_G, tt = (blockIdx.x * W2 * 32 + threadIdx.x) / M2L_G, t = min(tt, ncells - 1);
   const double4 X = xr[t];
   double2 acc[P];
 #pragma unroll
   for (int n = 0; n < P; n++) acc[n] = make_double2(0, 0);
-  for (int e = off[t] + lane; e < off[t + 1]; e += 32) {
+  for (int e = off[t] + g; e < off[t + 1]; e += M2L_G) {
     const u32 en = ent[e];
     const int s = (int)(en & IDX_MASK);
     double sx, sy;
@@ -258,11 +259,11 @@ __global__ void __launch_bounds__(W2 * 32) k2_m2l_lane(int ncells, const int *of
 #pragma unroll
   for (int n = 0; n < P; n++) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = M2L_G / 2; o > 0; o >>= 1) {
       acc[n].x += __shfl_xor_sync(0xffffffffu, acc[n].x, o);
       acc[n].y += __shfl_xor_sync(0xffffffffu, acc[n].y, o);
     }
-    if (lane == (n & 31)) L[(long)t * P + n] = acc[n];
+    if (g == n % M2L_G && tt < ncells) L[(long)t * P + n] = acc[n];
   }
 }
 
@@ -750,6 +751,8 @@ void upward_pass_2d(Handle &h, cudaStream_t s) {
   }
 }
 
+constexpr int M2L_MANY = 20000;  // cells: about 16 warps per SM at 4 lanes per target
+
 void m2l_pass_2d(Handle &h) {
   const int P = h.prm.P;
   h.L.need((size_t)h.ncells * P * sizeof(double2));
@@ -758,8 +761,14 @@ void m2l_pass_2d(Handle &h) {
   const int g = grid_for(h.ncells, W2);
   const bool done = with_order(P, [&](auto pc) {
     constexpr int PP = decltype(pc)::value;
-    k2_m2l_lane<PP><<<g, W2 * 32, 0, h.stream>>>(h.ncells, h.m2l_off.as<int>(), h.m2l_ent.as<u32>(),
-                                                h.c_xr.as<double4>(), h.M.as<double2>(), h.L.as<double2>(), cyc);
+    auto lanes = [&](auto gc) {
+      constexpr int G = decltype(gc)::value;
+      k2_m2l_lane<PP, G><<<grid_for((long)h.ncells * G, W2 * 32), W2 * 32, 0, h.stream>>>(
+          h.ncells, h.m2l_off.as<int>(), h.m2l_ent.as<u32>(), h.c_xr.as<double4>(), h.M.as<double2>(),
+          h.L.as<double2>(), cyc);
+    };
+    if (h.ncells >= M2L_MANY) lanes(std::integral_constant<int, 4>{});
+    else lanes(std::integral_constant<int, 16>{});
   });
   if (!done)  // larger orders: a warp per entry, a lane per coefficient
     k2_m2l<<<g, W2 * 32, 0, h.stream>>>(h.ncells, h.m2l_off.as<int>(), h.m2l_ent.as<u32>(), h.c_xr.as<double4>(),

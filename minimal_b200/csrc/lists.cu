@@ -137,12 +137,15 @@ __device__ __forceinline__ void walk_step(const WalkArgs &wa, int st) {
       if (R2 > __dmul_rn(rs, rs)) {
         kind[r] = 0;
         // the group key of the grouped M2L (radii are R0 / 2^level exactly,
-        // so their exponents give the level difference)
-        const int dl = radius_level_diff(b.w, a.w);
-        if (img == 13) key[r] = m2l_group_key(a, b, dl);
-        else key[r] = m2l_image_key(a, b, dl, img, cv.xr[0].w, cycle, depth);
-        if (key[r] >= 0) m2l_mark_key(key[r], i, occ, gflag);
-        else res++;
+        // so their exponents give the level difference); without marks (2D,
+        // orders without a grouped M2L) nothing reads keys
+        if (occ) {
+          const int dl = radius_level_diff(b.w, a.w);
+          if (img == 13) key[r] = m2l_group_key(a, b, dl);
+          else key[r] = m2l_image_key(a, b, dl, img, cv.xr[0].w, cycle, depth);
+          if (key[r] >= 0) m2l_mark_key(key[r], i, occ, gflag);
+          else res++;
+        }
         nm++;
       } else if (ci == 0 && cj == 0) {
         kind[r] = 1;
@@ -198,7 +201,7 @@ __device__ __forceinline__ void walk_step(const WalkArgs &wa, int st) {
       if (kind[r] == 0) {
         if (sm < mcap) {
           m2l[sm] = pr[r];
-          m2l_key[sm] = key[r];
+          if (occ) m2l_key[sm] = key[r];
         } else {
           *overflow = 1;
         }
@@ -460,14 +463,19 @@ void build_lists(Handle &h, const std::function<void()> &near_field) {
     // list and frontier counts, and the counters of the M2L grouping
     FMM_CUDA(cudaMemsetAsync(&ctr->n_m2l, 0, sizeof(DevCounters) - offsetof(DevCounters, n_m2l), s));
     // group keys of the M2L entries, and the keys and targets that occur
-    h.m2l_key.need(h.m2l_cap * sizeof(int));
-    FMM_CUDA(cudaMemsetAsync(gt.occ, 0, group_mark_bytes(ks, C), s));
+    const bool keyed = m2l_keyed(h);
+    if (keyed) {
+      h.m2l_key.need(h.m2l_cap * sizeof(int));
+      FMM_CUDA(cudaMemsetAsync(gt.occ, 0, group_mark_bytes(ks, C), s));
+    } else {
+      FMM_CUDA(cudaMemsetAsync(gt.cnt, 0, (size_t)(C + 1) * sizeof(int), s));
+    }
     const int dim = h.prm.dim == 2 ? 2 : 3, steps = 2 * h.depth + 3;
     const WalkArgs wa{CellView{h.c_xr.as<double4>(), h.c_child.as<int>(), h.c_nchild.as<int>()},
                       {h.frontier[0].as<int2>(), h.frontier[1].as<int2>()}, &ctr->frontier[0], h.frontier_cap,
                       h.m2l_raw.as<int2>(), h.p2p_raw.as<int2>(), &ctr->n_m2l, &ctr->n_p2p, h.m2l_cap, h.p2p_cap,
                       h.prm.theta, images ? h.prm.cycle : 0.0, h.depth, &ctr->list_overflow, h.m2l_key.as<int>(),
-                      gt.occ, gt.gflag, &ctr->walk_resid};
+                      keyed ? gt.occ : nullptr, gt.gflag, &ctr->walk_resid};
     // the steps whose frontier, at most `most` pairs, fits one block
     // iteration run in one launch; later steps take as many blocks as their
     // frontier can fill, up to one wave

@@ -1525,8 +1525,12 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
   h.launches++;
 }
 
+bool m2l_keyed(const Handle &h) {
+  return h.prm.dim != 2 && !h.force_direct_m2l && m2l_grouped_available(h.prm.P);
+}
+
 bool m2l_groups_raw(const Handle &h) {
-  return h.prm.dim != 2 && !h.force_direct_m2l && m2l_grouped_available(h.prm.P) &&
+  return m2l_keyed(h) &&
          !(h.prm.images > 0 && h.prm.precision == EXAFMM_MIXED && tc_available(h.prm.P));
 }
 
