@@ -16,6 +16,7 @@
 
 #include "fmm.cuh"
 #include "pair64.cuh"
+#include "srcf.cuh"
 
 namespace fmm {
 
@@ -117,14 +118,16 @@ __global__ void __launch_bounds__(DT) k_direct(const double4 *tgt, long nt, cons
 // rounding), so the pair offset dx = (xi - ci) + (ci - cj) - (xj - cj) keeps
 // the bits that an FP32 copy of the absolute coordinates would lose.
 __global__ void k_make_srcf(const int *leaves, int nleaves, const int *begin, const int *count, const double4 *xr,
-                            const double4 *src, float4 *srcf, int *body_leaf) {
+                            const double4 *src, float4 *srcf, float4 *pairs, int *body_leaf) {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= nleaves) return;
   const int c = leaves[w];
   const double4 C = xr[c];
   for (int b = begin[c] + lane; b < begin[c] + count[c]; b += 32) {
     const double4 B = src[b];
-    srcf[b] = make_float4((float)(B.x - C.x), (float)(B.y - C.y), (float)(B.z - C.z), (float)B.w);
+    const float4 f = make_float4((float)(B.x - C.x), (float)(B.y - C.y), (float)(B.z - C.z), (float)B.w);
+    srcf[b] = f;
+    put_pair(pairs, begin[c], b - begin[c], count[c], f);
     body_leaf[b] = w;
   }
 }
@@ -207,9 +210,6 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-
-// A staged source that adds nothing: zero charge, far from every target.
-constexpr float NEAR_DUMMY = 1e15f;
 
 // One target (X, Y, Z = the coordinate in both lanes) against a staged
 // source pair (sx, sy from the first slot, sz, sq from the second); the same
@@ -335,7 +335,7 @@ constexpr int CT_TPT = 2;         // targets per thread (register blocking)
 constexpr int CT_BLOCK = 256;     // sources summed in FP32 before one compensated addition
 // 32-body blocks a warp loads before storing them (register-bound)
 template <bool F32>
-constexpr int ct_unroll() { return F32 ? 2 : 1; }
+constexpr int ct_unroll() { return 1; }
 
 template <bool F32>
 struct NearBody;
@@ -353,8 +353,8 @@ struct NearBody<true> {
 template <bool F32, int CAP>
 __global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, const int *begin, const int *count,
                                                 const int *off, const u32 *ent, const double4 *xr,
-                                                const typename NearBody<F32>::T *bodies, double4 *out,
-                                                double cycle) {
+                                                const typename NearBody<F32>::T *bodies, const float4 *pairs,
+                                                double4 *out, double cycle) {
   typedef typename NearBody<F32>::T BT;
   typedef typename NearBody<F32>::R RT;
   constexpr int CT_UNROLL = ct_unroll<F32>();
@@ -397,9 +397,12 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, 
 #pragma unroll
     for (int q = 0; q < 4; q++) sacc[u][q] = eacc[u][q] = 0;
   const int eb = off[c], ee = off[c + 1];
-  // slots [0, pre) of the first chunk: the target leaf itself, padded to an
-  // even count in the FP32 form (whose stage holds sources in pairs)
-  int pre = F32 ? tn + (tn & 1) : tn;
+  // staging slots: bodies (FP64), or pairs of a leaf's bodies (FP32: the last
+  // pair of an odd leaf holds a zero charge); slots [0, pre) of the first
+  // chunk: the target leaf itself
+  constexpr int SLOTS = F32 ? CAP / 2 : CAP;
+  auto slots_of = [](int bodies_n) { return F32 ? (bodies_n + 1) >> 1 : bodies_n; };
+  int pre = slots_of(tn);
   for (int e0i = eb; e0i < ee;) {
     // lane k: source leaf k of the chunk candidates
     const int cand = min(32, ee - e0i);
@@ -414,7 +417,7 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, 
       const int sc = (int)(en & IDX_MASK);
       img = (int)(en >> IMG_SHIFT);
       self = sc == c && img == 13;
-      n = self ? 0 : count[sc];
+      n = self ? 0 : slots_of(count[sc]);
       base = begin[sc];
       if constexpr (F32) {
         const double sx = (img % 3 - 1) * cycle, sy = ((img / 3) % 3 - 1) * cycle, sz = (img / 9 - 1) * cycle;
@@ -433,35 +436,32 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, 
     inc += pre;
     // the running sums grow, so the leaves that fit are a prefix (at least
     // one: no leaf exceeds the buffer less the target leaf)
-    const int nl = __popc(__ballot_sync(FULL, lane < cand && inc <= CAP));
+    const int nl = __popc(__ballot_sync(FULL, lane < cand && inc <= SLOTS));
     const int T = __shfl_sync(FULL, inc, nl - 1);
     const int start = inc - n;  // first staging slot of leaf `lane`
-    base -= start;              // body index = base + staging slot
+    base -= start;              // body (pair) index = base + staging slot
     const bool inchunk = lane < nl;
     // the size-0 self entry shares its start with the next leaf
     const unsigned zm = __ballot_sync(FULL, inchunk && self);
     const int zs = zm ? __shfl_sync(FULL, start, __ffs(zm) - 1) : -1;
     __syncthreads();  // the previous chunk's sweep is done with the buffer
     if constexpr (F32) {
-      for (int pp = tid; 2 * pp < pre; pp += CT) {  // the target leaf, in slots [0, tn), in pairs
-        float4 a = bodies[tb + 2 * pp], b = make_float4(NEAR_DUMMY, NEAR_DUMMY, NEAR_DUMMY, 0.f);
+      for (int j = tid; j < pre; j += CT) {
+        float4 a = pairs[2 * (tb + j)], b = pairs[2 * (tb + j) + 1];
         a.x *= scale;
         a.y *= scale;
         a.z *= scale;
-        if (2 * pp + 1 < tn) {
-          b = bodies[tb + 2 * pp + 1];
-          b.x *= scale;
-          b.y *= scale;
-          b.z *= scale;
-        }
-        stage[2 * pp] = make_float4(a.x, b.x, a.y, b.y);
-        stage[2 * pp + 1] = make_float4(a.z, b.z, a.w, b.w);
+        a.w *= scale;
+        b.x *= scale;
+        b.y *= scale;
+        stage[2 * j] = a;
+        stage[2 * j + 1] = b;
       }
     } else {
       for (int j = tid; j < pre; j += CT) stage[j] = bodies[tb + j];
     }
     for (int j0 = pre + wid * 32; j0 < T; j0 += CT * CT_UNROLL) {
-      BT v[CT_UNROLL];
+      BT v[CT_UNROLL], v2[F32 ? CT_UNROLL : 1];
       int kk[CT_UNROLL];
 #pragma unroll
       for (int u = 0; u < CT_UNROLL; u++) {
@@ -474,7 +474,14 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, 
         const int k = k0 + __popc(st & (FULL >> (31 - lane))) + (zs > jb && zs <= j);
         kk[u] = k;
         const int bk = __shfl_sync(FULL, base, k);
-        if (j < T) v[u] = bodies[bk + j];
+        if constexpr (F32) {
+          if (j < T) {
+            v[u] = pairs[2 * (bk + j)];
+            v2[u] = pairs[2 * (bk + j) + 1];
+          }
+        } else if (j < T) {
+          v[u] = bodies[bk + j];
+        }
       }
 #pragma unroll
       for (int u = 0; u < CT_UNROLL; u++) {
@@ -490,18 +497,11 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, 
           sy = -((im / 3) % 3 - 1) * cycle;
           sz = -(im / 9 - 1) * cycle;
         }
-        if constexpr (F32) {  // into the target frame, scaled (exact); stored in source pairs
-          float4 t = make_float4(NEAR_DUMMY, NEAR_DUMMY, NEAR_DUMMY, 0.f);
-          if (j < T) t = make_float4(fmaf(v[u].x, scale, -sx), fmaf(v[u].y, scale, -sy), fmaf(v[u].z, scale, -sz), v[u].w);
-          const float4 o = make_float4(__shfl_xor_sync(FULL, t.x, 1), __shfl_xor_sync(FULL, t.y, 1),
-                                       __shfl_xor_sync(FULL, t.z, 1), __shfl_xor_sync(FULL, t.w, 1));
+        if constexpr (F32) {  // into the target frame, scaled (exact)
           if (j < T) {
-            if ((j & 1) == 0) {  // the pair's first slot (its partner, or a dummy past the end)
-              stage[j] = make_float4(t.x, o.x, t.y, o.y);
-              if (j + 1 == T) stage[j + 1] = make_float4(t.z, NEAR_DUMMY, t.w, 0.f);
-            } else {
-              stage[j] = make_float4(o.z, t.z, o.w, t.w);
-            }
+            stage[2 * j] = make_float4(fmaf(v[u].x, scale, -sx), fmaf(v[u].y, scale, -sx), fmaf(v[u].z, scale, -sy),
+                                       fmaf(v[u].w, scale, -sy));
+            stage[2 * j + 1] = make_float4(fmaf(v2[u].x, scale, -sz), fmaf(v2[u].y, scale, -sz), v2[u].z, v2[u].w);
           }
         } else if (j < T) {
           BT t;
@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, 
               acc[u][q] = 0ull;
             }
         };
-        const int nps = pre / 2, npt = (T + 1) / 2;  // pairs of the target leaf, of the chunk
+        const int nps = pre, npt = T;  // pairs of the target leaf, of the chunk
         for (int pp = divG(g * nps), pe = divG((g + 1) * nps); pp < pe; pp++) step(pp, std::true_type{});
         const int rest = npt - nps, from = nps + divG(g * rest), to = nps + divG((g + 1) * rest);
         for (int c0 = from; c0 < to; c0 += CT_BLOCK / 2) {
@@ -633,10 +633,11 @@ __global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, 
 void make_srcf(Handle &h) {
   if (h.srcf_ready) return;
   h.srcf.need((size_t)h.n * sizeof(float4));
+  h.srcp.need((size_t)h.n * 2 * sizeof(float4));
   h.body_leaf.need((size_t)h.n * sizeof(int));
   k_make_srcf<<<grid_for((long)h.nleaves * 32, 256), 256, 0, h.stream>>>(
       h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.c_xr.as<double4>(),
-      h.src.as<double4>(), h.srcf.as<float4>(), h.body_leaf.as<int>());
+      h.src.as<double4>(), h.srcf.as<float4>(), h.srcp.as<float4>(), h.body_leaf.as<int>());
   h.launches++;
   FMM_LAUNCH();
   h.srcf_ready = true;
@@ -682,7 +683,7 @@ void p2p_pass(Handle &h, cudaStream_t s) {
     if (cta)
       launch_p2p_cta<true>(p2p_tile(h), h.nleaves, s, h.leaves.as<int>(), h.c_begin.as<int>(), h.c_count.as<int>(),
                            h.p2p_off.as<int>(), h.p2p_ent.as<u32>(), h.c_xr.as<double4>(), h.srcf.as<float4>(),
-                           h.out.as<double4>(), cyc);
+                           h.srcp.as<float4>(), h.out.as<double4>(), cyc);
     else
       k_p2p_f32<<<grid_for(h.nleaves, WARPS), WARPS * 32, 0, s>>>(
           h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.p2p_off.as<int>(),
@@ -694,7 +695,7 @@ void p2p_pass(Handle &h, cudaStream_t s) {
   if (cta)
     launch_p2p_cta<false>(p2p_tile(h), h.nleaves, s, h.leaves.as<int>(), h.c_begin.as<int>(), h.c_count.as<int>(),
                           h.p2p_off.as<int>(), h.p2p_ent.as<u32>(), h.c_xr.as<double4>(), h.src.as<double4>(),
-                          h.out.as<double4>(), cyc);
+                          (const float4 *)nullptr, h.out.as<double4>(), cyc);
   else
     k_p2p<<<grid_for(h.nleaves, WARPS), WARPS * 32, 0, s>>>(
         h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.p2p_off.as<int>(),

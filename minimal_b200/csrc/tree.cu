@@ -33,6 +33,7 @@
 #include <cmath>
 
 #include "fmm.cuh"
+#include "srcf.cuh"
 
 namespace fmm {
 
@@ -378,7 +379,7 @@ __global__ void k_ref_leaves(BfsCells o, long c, const int *blockstart_pre, int 
 // them: one pass over the bodies instead of three.
 __global__ void k_leaf_order(const int *leaves, int nleaves, const int *begin, const int *count, const double4 *xr,
                              const u32 *vals, const double4 *in, int *perm, double4 *src, float4 *srcf,
-                             int *body_leaf) {
+                             float4 *pairs, int *body_leaf) {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= nleaves) return;
   const int c = leaves[w], b0 = begin[c], nb = count[c];
@@ -392,7 +393,9 @@ __global__ void k_leaf_order(const int *leaves, int nleaves, const int *begin, c
     const double4 B = in[v];
     src[b] = B;
     if (srcf) {
-      srcf[b] = make_float4((float)(B.x - C.x), (float)(B.y - C.y), (float)(B.z - C.z), (float)B.w);
+      const float4 f = make_float4((float)(B.x - C.x), (float)(B.y - C.y), (float)(B.z - C.z), (float)B.w);
+      srcf[b] = f;
+      put_pair(pairs, b0, r, nb, f);
       body_leaf[b] = w;
     }
   }
@@ -528,11 +531,13 @@ void build_tree(Handle &h) {
     const bool srcf = h.prm.precision == EXAFMM_MIXED && h.prm.dim == 3;
     if (srcf) {
       h.srcf.need((size_t)n * sizeof(float4));
+      h.srcp.need((size_t)n * 2 * sizeof(float4));
       h.body_leaf.need((size_t)n * sizeof(int));
     }
     k_leaf_order<<<grid_for((long)h.nleaves * 32, TB), TB, 0, s>>>(
         h.leaves.as<int>(), h.nleaves, o.begin, o.count, o.xr, v, h.in.as<double4>(), h.perm.as<int>(),
-        h.src.as<double4>(), srcf ? h.srcf.as<float4>() : nullptr, srcf ? h.body_leaf.as<int>() : nullptr);
+        h.src.as<double4>(), srcf ? h.srcf.as<float4>() : nullptr, h.srcp.as<float4>(),
+        srcf ? h.body_leaf.as<int>() : nullptr);
     h.launches++;
     FMM_LAUNCH();
     h.srcf_ready = srcf;
