@@ -323,15 +323,28 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2p_f32(const int *leaves, int n
 // the zero-distance check; every group takes its share of both parts, so the
 // warps stay converged.  FP64 form: likewise the target leaf first, its pairs
 // with the zero-distance check (pair), the others without (pair_normal).
-constexpr int CT = 128;           // threads per CTA
-// bodies staged at once (the source tile): a template parameter, chosen at
-// run time among 1024, 1536 and 2048 (exafmm_b200_set_tile / the
-// autotuner); the defaults, FP32 1536 (7 CTAs per SM, register-bound) and
-// FP64 1024 (4 CTAs per SM), were tuned on B200 at 1M uniform bodies
+// Threads per CTA (CT) and bodies staged at once (CAP, the source tile) are
+// template parameters.  128 threads stage 1536 bodies (FP32; 7 CTAs per SM,
+// register-bound) or 1024 (FP64; 4 CTAs per SM), tuned at 1M uniform bodies,
+// or what exafmm_b200_set_tile / the autotuner chose among 1024, 1536 and
+// 2048.  Trees of many small leaves take 64 or 32 threads, staging 768 / 512
+// and 512 / 256 bodies: a CTA's fixed part (its chain of dependent loads, the
+// barriers, the sum over 128 / ceil(n / 2) parts) is then shared by more CTAs
+// per SM.  Measured near field, 32 / 64 / 128 threads, in us: 32,768 uniform
+// leaves of 4, 8, 14, 20, 24 and 32 bodies, mixed 134/197/396, 199/256/447,
+// 383/406/574, 715/668/795, 1020/902/988, 1938/1528/1496; FP64 184/260/545,
+// 357/412/705, 883/814/1084, 1754/1510/1704, 2491/2113/2245, 4831/3660/3603;
+// 1M Plummer bodies (the pairs lie in the larger leaves), average leaf 9, 14,
+// 19 and 29: mixed 887/1041/1661, 1207/1145/1464, 1554/1344/1497, -/2315/1909.
+// A leaf must fit two targets per thread (ncrit), and there must be enough
+// leaves to fill the GPU (512 of 39 bodies: 164/97/60; 5,266 of 9.5:
+// 95/82/95; 2,752 of 18: 287/168/103).
 template <bool F32>
 constexpr int ct_cap() { return F32 ? 1536 : 1024; }
+constexpr int CT_MAX = 128;
 constexpr int CT_MAXTGT = 256;    // target-leaf bodies: two per thread
 constexpr int CT_TPT = 2;         // targets per thread (register blocking)
+constexpr int CT32_LEAVES = 96, CT64_LEAVES = 32;  // leaves per SM from which 32, 64 threads are considered
 constexpr int CT_BLOCK = 256;     // sources summed in FP32 before one compensated addition
 // 32-body blocks a warp loads before storing them (register-bound)
 template <bool F32>
@@ -350,8 +363,8 @@ struct NearBody<true> {
   typedef float R;
 };
 
-template <bool F32, int CAP>
-__global__ void __launch_bounds__(CT, F32 ? 7 : 4) k_p2p_cta(const int *leaves, const int *begin, const int *count,
+template <bool F32, int CAP, int CT>
+__global__ void __launch_bounds__(CT, (F32 ? 7 : 4) * (CT_MAX / CT)) k_p2p_cta(const int *leaves, const int *begin, const int *count,
                                                 const int *off, const u32 *ent, const double4 *xr,
                                                 const typename NearBody<F32>::T *bodies, const float4 *pairs,
                                                 double4 *out, double cycle) {
@@ -643,23 +656,44 @@ void make_srcf(Handle &h) {
   h.srcf_ready = true;
 }
 
-// The near-field CTA kernel with source tile `cap` (1024, 1536 or 2048).
+// The near-field CTA kernel with `ct` threads, or with CT_MAX threads and
+// source tile `cap` (1024, 1536 or 2048).
+template <bool F32, class F>
+void with_p2p_shape(int ct, int cap, F f) {
+  auto shape = [&](auto capc, auto ctc) {
+    constexpr int CAP = decltype(capc)::value, CT = decltype(ctc)::value;
+    f(k_p2p_cta<F32, CAP, CT>, CT, CAP * sizeof(typename NearBody<F32>::T));
+  };
+  typedef std::integral_constant<int, CT_MAX> Full;
+  if (ct == 32) shape(std::integral_constant<int, F32 ? 512 : 256>{}, std::integral_constant<int, 32>{});
+  else if (ct == 64) shape(std::integral_constant<int, F32 ? 768 : 512>{}, std::integral_constant<int, 64>{});
+  else if (cap == 1024) shape(std::integral_constant<int, 1024>{}, Full{});
+  else if (cap == 2048) shape(std::integral_constant<int, 2048>{}, Full{});
+  else shape(std::integral_constant<int, 1536>{}, Full{});
+}
+
 template <bool F32, class... A>
-void launch_p2p_cta(int cap, int nleaves, cudaStream_t s, A... args) {
-  typedef typename NearBody<F32>::T BT;
-  switch (cap) {
-    case 1024: k_p2p_cta<F32, 1024><<<nleaves, CT, 1024 * sizeof(BT), s>>>(args...); break;
-    case 2048: k_p2p_cta<F32, 2048><<<nleaves, CT, 2048 * sizeof(BT), s>>>(args...); break;
-    default: k_p2p_cta<F32, 1536><<<nleaves, CT, 1536 * sizeof(BT), s>>>(args...);
-  }
+void launch_p2p_cta(int ct, int cap, int nleaves, cudaStream_t s, A... args) {
+  with_p2p_shape<F32>(ct, cap, [&](auto kern, int threads, size_t smem) { kern<<<nleaves, threads, smem, s>>>(args...); });
 }
 
 template <bool F32>
 void set_p2p_attributes() {
-  typedef typename NearBody<F32>::T BT;
-  cudaFuncSetAttribute(k_p2p_cta<F32, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 * (int)sizeof(BT));
-  cudaFuncSetAttribute(k_p2p_cta<F32, 1536>, cudaFuncAttributeMaxDynamicSharedMemorySize, 1536 * (int)sizeof(BT));
-  cudaFuncSetAttribute(k_p2p_cta<F32, 2048>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2048 * (int)sizeof(BT));
+  auto set = [](auto kern, int, size_t smem) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  };
+  for (int ct : {32, 64}) with_p2p_shape<F32>(ct, 0, set);
+  for (int cap : {1024, 1536, 2048}) with_p2p_shape<F32>(CT_MAX, cap, set);
+}
+
+// Threads per near-field CTA for the tree's leaves (see CT above).
+int p2p_threads(const Handle &h) {
+  if (h.tile_p2p_stage > 0) return CT_MAX;
+  const bool f32 = h.prm.precision == EXAFMM_MIXED;
+  const double avg = (double)h.n / std::max(h.nleaves, 1);  // bodies per leaf
+  if (avg <= (f32 ? 12 : 9) && h.prm.ncrit <= 64 && h.nleaves >= CT32_LEAVES * h.nsm) return 32;
+  if (avg <= (f32 ? 24 : 22) && h.prm.ncrit <= 128 && h.nleaves >= CT64_LEAVES * h.nsm) return 64;
+  return CT_MAX;
 }
 
 void p2p_set_attributes() {
@@ -676,12 +710,13 @@ void p2p_pass(Handle &h, cudaStream_t s) {
   if (h.prm.dim == 2) return p2p_pass_2d(h, s);
   h.out.need((size_t)h.n * sizeof(double4));
   const double cyc = h.prm.images ? h.prm.cycle : 0.0;
+  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   const bool cta = h.prm.ncrit <= CT_MAXTGT;  // every leaf fits two targets per thread and the buffer
   if (h.prm.precision == EXAFMM_MIXED) {
     if (s != h.stream && !h.srcf_ready) throw Error{EXAFMM_ERR_STATE, "near field on a side stream before its sources"};
     make_srcf(h);
     if (cta)
-      launch_p2p_cta<true>(p2p_tile(h), h.nleaves, s, h.leaves.as<int>(), h.c_begin.as<int>(), h.c_count.as<int>(),
+      launch_p2p_cta<true>(p2p_threads(h), p2p_tile(h), h.nleaves, s, h.leaves.as<int>(), h.c_begin.as<int>(), h.c_count.as<int>(),
                            h.p2p_off.as<int>(), h.p2p_ent.as<u32>(), h.c_xr.as<double4>(), h.srcf.as<float4>(),
                            h.srcp.as<float4>(), h.out.as<double4>(), cyc);
     else
@@ -693,7 +728,7 @@ void p2p_pass(Handle &h, cudaStream_t s) {
     return;
   }
   if (cta)
-    launch_p2p_cta<false>(p2p_tile(h), h.nleaves, s, h.leaves.as<int>(), h.c_begin.as<int>(), h.c_count.as<int>(),
+    launch_p2p_cta<false>(p2p_threads(h), p2p_tile(h), h.nleaves, s, h.leaves.as<int>(), h.c_begin.as<int>(), h.c_count.as<int>(),
                           h.p2p_off.as<int>(), h.p2p_ent.as<u32>(), h.c_xr.as<double4>(), h.src.as<double4>(),
                           (const float4 *)nullptr, h.out.as<double4>(), cyc);
   else
