@@ -94,9 +94,6 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2m(const int *leaves, int nleav
 // the FP32 copy the near field uses), same lock-step generator in float;
 // expansions stay FP64 in memory.
 __constant__ float c_recip_f[2 * EXAFMM_MAX_P + 4];
-#ifndef P2M_TRANSPOSE
-#define P2M_TRANSPOSE 1
-#endif
 #ifndef L2P_F32_MIN_BLOCKS
 #define L2P_F32_MIN_BLOCKS 6  // 128-thread blocks per SM: up to 80 registers a thread
 #endif
@@ -167,14 +164,13 @@ __device__ __forceinline__ void regular_all_f(int Prt, const SphF &g, float2 e1,
 // in units of 2^e, where the radius lies in [1, 2).
 __device__ __forceinline__ int leaf_exponent(double R) { return R > 0 ? max(-100, min(100, ilogb(R))) : 0; }
 
-// P2M in FP32: lane per body, each coefficient reduced over the warp by a
-// float butterfly, chunks of 32 bodies summed in FP64.
-template <int PT>
+// P2M in FP32 for orders without column lanes: lane per body, each
+// coefficient reduced over the warp by a float butterfly, chunks of 32 bodies
+// summed in FP64.
 __global__ void __launch_bounds__(WARPS * 32) k_p2m_f32(const int *leaves, int nleaves, const int *begin,
                                                         const int *count, const double4 *xr, const float4 *srcf,
-                                                        double2 *M, int Prt) {
+                                                        double2 *M, int P) {
   extern __shared__ double2 sh[];
-  const int P = PT > 0 ? PT : Prt;
   const int nt = tri(P);
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w = blockIdx.x * WARPS + wid;
@@ -190,7 +186,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2m_f32(const int *leaves, int n
     const bool ok = t + lane < nb;
     const float4 B = ok ? srcf[b0 + t + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
     const SphF g = sph_of_f(B.x * sc, B.y * sc, B.z * sc);
-    regular_all_f<PT, false>(P, g, make_float2(g.e.x, -g.e.y), [&](int n, int m, float2 Y, float2) {
+    regular_all_f<0, false>(P, g, make_float2(g.e.x, -g.e.y), [&](int n, int m, float2 Y, float2) {
       float x = B.w * Y.x, y = B.w * Y.y;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -210,75 +206,158 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2m_f32(const int *leaves, int n
   }
 }
 
-// P2M in FP32 for a compile-time order: each lane writes its body's q Y
-// terms to shared memory 32 terms at a time, then lane k sums term k of the
-// batch over the 32 bodies (rows padded to 33 entries: conflict-free), and
-// the sums are added in FP64.  The batch buffer (8 KB per warp) keeps
-// enough warps resident to hide the recurrence's latency.
-constexpr int P2M_ROW = 33;
-constexpr size_t p2m_t_smem(int nt) { return WARPS * (nt * sizeof(double2) + 32 * P2M_ROW * sizeof(float2) + 32 * sizeof(int)); }
+// ---- P2M and (FP64) L2P from the Cartesian recurrences of the regular
+// harmonics, orders up to COLS_MAXP as compile-time constants.  In the
+// normalisation of harmonics.cuh, Y_n^m = T_n^m (x + iy)^m / (2^m m!) with
+//   T_m^m = 1,  T_{n+1}^m = -((2n+1) z T_n^m + r^2 T_{n-1}^m) / ((n-m+1)(n+m+1)),
+//   dY_n^m/dz = -Y_{n-1}^m,  (d/dx + i d/dy) Y_n^m = -Y_{n-1}^{m+1},
+//   (d/dx - i d/dy) Y_n^m = Y_{n-1}^{m-1}  (m >= 1)
+// (the regular solid harmonics and their derivatives, e.g. Hobson, The Theory
+// of Spherical and Ellipsoidal Harmonics): no radius, angle, square root or
+// division, and polynomials also at a leaf's centre and on its axis.
+constexpr int COLS_MAXP = 16;
+#define EXAFMM_COLS_ORDERS(X) X(1) EXAFMM_UNROLLED_ORDERS(X)
 
-template <int PT>
-__global__ void __launch_bounds__(WARPS * 32) k_p2m_f32t(const int *leaves, int nleaves, const int *begin,
-                                                         const int *count, const double4 *xr, const float4 *srcf,
-                                                         double2 *M) {
-  constexpr int NT = PT * (PT + 1) / 2, ROW = P2M_ROW;
-  extern __shared__ double2 sh[];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w = blockIdx.x * WARPS + wid;
-  if (w >= nleaves) return;
-  double2 *acc = sh + wid * NT;
-  float2 *buf = (float2 *)(sh + WARPS * NT) + wid * 32 * ROW;
-  int *rowidx = (int *)((float2 *)(sh + WARPS * NT) + WARPS * 32 * ROW) + wid * 32;
-  for (int k = lane; k < NT; k += 32) acc[k] = make_double2(0, 0);
-  const int c = leaves[w];
-  const int ex = leaf_exponent(xr[c].w);
-  const float sc = exp2f((float)-ex);  // coordinates in units where the leaf radius is in [1, 2)
-  const int b0 = begin[c], nb = count[c];
-  for (int t = 0; t < nb; t += 32) {
-    const bool ok = t + lane < nb;
-    const float4 B = ok ? srcf[b0 + t + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const SphF g = sph_of_f(B.x * sc, B.y * sc, B.z * sc);
-    int gen = 0;  // terms generated so far (a constant at every unrolled step)
-    __syncwarp();
-    regular_all_f<PT, false>(PT, g, make_float2(g.e.x, -g.e.y), [&](int n, int m, float2 Y, float2) {
-      const int slot = gen & 31;
-      buf[slot * ROW + lane] = make_float2(B.w * Y.x, B.w * Y.y);
-      if (lane == 0) rowidx[slot] = tri(n) + m;
-      gen++;
-      if ((gen & 31) == 0 || gen == NT) {  // sum the batch over the bodies
-        __syncwarp();
-        if (lane <= ((gen - 1) & 31)) {
-          float sx = 0.f, sy = 0.f;
-#pragma unroll 8
-          for (int b = 0; b < 32; b++) {
-            const float2 v = buf[lane * ROW + b];
-            sx += v.x;
-            sy += v.y;
-          }
-          double2 &a = acc[rowidx[lane]];
-          a.x += (double)sx;
-          a.y += (double)sy;
-        }
-        __syncwarp();
-      }
-    });
+// complex value type of a compute precision
+template <bool F32>
+struct Cplx {
+  typedef double2 V;
+  typedef double R;
+};
+template <>
+struct Cplx<true> {
+  typedef float2 V;
+  typedef float R;
+};
+
+template <bool F32>
+struct P2mBody {
+  typedef double4 T;
+  typedef double R;
+};
+template <>
+struct P2mBody<true> {
+  typedef float4 T;
+  typedef float R;
+};
+
+// P2M: M[n][m] += q Y_n^m(x, -y, z).  H = ceil(P / 2) lanes per leaf (32 / H
+// leaves per warp); lane j sums the columns m = j and m = P - 1 - j over the
+// leaf's bodies, P + 1 coefficients in registers (the middle column of an odd
+// P alone), so every lane does the same work and nothing is exchanged.  With
+// a lane per body and a sum over the warp per coefficient it took, at 1M
+// uniform bodies and P = 10, 344 us in FP64 and 90 us in the mixed form; now
+// 103 and 65.  F32: the bodies' leaf-relative FP32 copy in units of the leaf
+// radius rounded to a power of two, FP32 sums over 32 bodies at a time, those
+// sums added in FP64.
+template <int P, bool F32>
+__global__ void __launch_bounds__(128) k_p2m_cols(const int *leaves, int nleaves, const int *begin, const int *count,
+                                                  const double4 *xr, const typename P2mBody<F32>::T *src, double2 *M) {
+  typedef typename P2mBody<F32>::T BT;
+  typedef typename P2mBody<F32>::R R;
+  constexpr int H = (P + 1) / 2, LPW = 32 / H, NT = P * (P + 1) / 2;
+  // a and b of T_{n+1} = a z T_n + b r^2 T_{n-1}, by step and lane (FP64:
+  // volatile, read at every step -- held in registers they cost a third of the
+  // warps, 119 against 103 us; FP32 is faster with them, 65 against 73)
+  typedef typename std::conditional<F32, R, volatile R>::type CR;
+  __shared__ CR ca[P + 1][H], cb[P + 1][H];
+  for (int e = threadIdx.x; e < (P + 1) * H; e += 128) {
+    const int k = e / H, j = e % H, m = k < P - j ? j : P - 1 - j, n = k < P - j ? j + k : m + k - (P - j);
+    const double d = -1.0 / ((double)(n - m + 1) * (n + m + 1));
+    ca[k][j] = (R)((2 * n + 1) * d);
+    cb[k][j] = (R)d;
   }
-  __syncwarp();
-  for (int k = lane; k < NT; k += 32) {  // back to the input units: M_n = M~_n R_s^n (exact)
-    const int n = order_of(k);
-    M[(long)c * NT + k] = make_double2(scalbn(acc[k].x, ex * n), scalbn(acc[k].y, ex * n));
+  __syncthreads();
+  const int lane = threadIdx.x & 31, sub = lane / H, j = lane % H;
+  const int w = (blockIdx.x * 4 + (threadIdx.x >> 5)) * LPW + sub;
+  if (sub >= LPW || w >= nleaves) return;
+  const int m1 = j, m2 = P - 1 - j, n1 = P - m1;  // steps [0, n1): column m1, then m2
+  const int c = leaves[w], b0 = begin[c], nb = count[c];
+  const double4 C = xr[c];
+  const int ex = F32 ? leaf_exponent(C.w) : 0;
+  const R sc = F32 ? (R)exp2f((float)-ex) : (R)1;
+  double2 acc[F32 ? P + 1 : 1];
+  if constexpr (F32)
+#pragma unroll
+    for (int k = 0; k <= P; k++) acc[k] = make_double2(0, 0);
+  BT next = src[b0];
+  R sx[P + 1], sy[P + 1];  // F32: sums of this chunk
+  const int chunk = F32 ? 32 : nb;
+  for (int t = 0; t < nb; t += chunk) {
+#pragma unroll
+    for (int k = 0; k <= P; k++) sx[k] = sy[k] = 0;
+    const int te = min(nb, t + chunk);
+    for (int b = t; b < te; b++) {
+      const BT B = next;
+      if (b + 1 < nb) next = src[b0 + b + 1];
+      R x, y, z;
+      if constexpr (F32) {
+        x = B.x * sc;
+        y = B.y * sc;
+        z = B.z * sc;
+      } else {
+        x = B.x - C.x;
+        y = B.y - C.y;
+        z = B.z - C.z;
+      }
+      const R r2 = x * x + y * y + z * z;
+      // q (x - iy)^m / (2^m m!) for the two columns
+      R px = B.w, py = 0, w1x = px, w1y = 0, w2x = px, w2y = 0;
+#pragma unroll
+      for (int k = 1; k < P; k++) {
+        const R ux = x * (R)(0.5 / k), uy = -y * (R)(0.5 / k), qx = px * ux - py * uy;
+        py = px * uy + py * ux;
+        px = qx;
+        if (k == m1) {
+          w1x = px;
+          w1y = py;
+        }
+        if (k == m2) {
+          w2x = px;
+          w2y = py;
+        }
+      }
+      if (m1 == m2) w2x = w2y = 0;
+      R T = 1, Tp = 0, wx = w1x, wy = w1y;
+#pragma unroll
+      for (int k = 0; k <= P; k++) {
+        sx[k] = fma(T, wx, sx[k]);
+        sy[k] = fma(T, wy, sy[k]);
+        const R Tn = fma(ca[k][j], z * T, cb[k][j] * (r2 * Tp));
+        Tp = T;
+        T = Tn;
+        if (k + 1 == n1) {  // the second column starts
+          T = 1;
+          Tp = 0;
+          wx = w2x;
+          wy = w2y;
+        }
+      }
+    }
+    if constexpr (F32)
+#pragma unroll
+      for (int k = 0; k <= P; k++) {
+        acc[k].x += (double)sx[k];
+        acc[k].y += (double)sy[k];
+      }
+  }
+#pragma unroll
+  for (int k = 0; k <= P; k++) {
+    const bool first = k < n1;
+    if (!first && m1 == m2) continue;
+    const int m = first ? m1 : m2, n = first ? m1 + k : m2 + k - n1;
+    // back to the input units: M_n = M~_n R_s^n (exact)
+    double2 &dst = M[(long)c * NT + tri(n) + m];
+    if constexpr (F32) dst = make_double2(scalbn(acc[k].x, ex * n), scalbn(acc[k].y, ex * n));
+    else dst = make_double2(sx[k], sy[k]);
   }
 }
 
-// L2P in FP32, in two parts.  k_l2p_prep (before the wait for the near
+// L2P of the mixed form, its first part (before the wait for the near
 // field): per leaf, the local expansion in the leaf's units, L~_n = L_n R^n
-// with R the leaf radius rounded down to a power of two (exact), as FP32,
-// and the scale 1/R for the coordinates -- so the FP32 terms stay in range
-// at any domain size.  k_l2p_f32: a thread per body over all bodies (tree
-// order, every lane busy whatever the leaf sizes), its leaf's expansion
-// read through L1 (the lanes of a warp share one or two leaves); p and F
-// added to the FP64 results.
+// with R the leaf radius rounded down to a power of two (exact), as FP32, and
+// the scale 1/R for the coordinates -- so the FP32 terms stay in range at any
+// domain size.
 __global__ void k_l2p_prep(const int *leaves, int nleaves, const double4 *xr, const double2 *L, int nt, float2 *Lf,
                            float *lsc) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -290,11 +369,94 @@ __global__ void k_l2p_prep(const int *leaves, int nleaves, const double4 *xr, co
   if (k == 0) lsc[w] = exp2f((float)-ex);
 }
 
-template <int PT>
+// L2P: a thread per body over all bodies (tree order, every lane busy whatever
+// the leaf sizes), its leaf's expansion read through L1 (the lanes of a warp
+// share one or two leaves).  With S0, Sz, Sm, Sp the sums over n of T_n^m
+// times L_n^m, L_{n+1}^m, L_{n+1}^{m-1} and L_{n+1}^{m+1}, column m adds, with
+// u = (x + iy)^m / (2^m m!) and w_m = 1 (m = 0) or 2,  w_m Re(S0 u) to p,
+// Re((Sp - Sm) u), -Im((Sp + Sm) u) and -w_m Re(Sz u) to its gradient; p and F
+// are added to the FP64 results.  1M uniform bodies, P = 10: FP64 286 us (a
+// warp per leaf, spherical derivatives) -> 66; mixed 70 -> 37.
+// F32: in the leaf's units, from what k_l2p_prep made before the wait for the
+// near field.
+template <int P, bool F32>
+__global__ void __launch_bounds__(128) k_l2p_body(long nbodies, const int *leaves, const int *body_leaf,
+                                                  const double4 *xr, const typename P2mBody<F32>::T *src,
+                                                  const typename Cplx<F32>::V *L, const float *lsc, double4 *out) {
+  typedef typename P2mBody<F32>::R R;
+  typedef typename Cplx<F32>::V V;
+  constexpr int NT = P * (P + 1) / 2;
+  const long b = (long)blockIdx.x * 128 + threadIdx.x;
+  if (b >= nbodies) return;
+  const int w = body_leaf[b];
+  const auto B = src[b];
+  R x, y, z, sc = 1;
+  const V *Lc;
+  if constexpr (F32) {
+    sc = lsc[w];
+    x = B.x * sc;
+    y = B.y * sc;
+    z = B.z * sc;
+    Lc = L + (long)w * NT;
+  } else {
+    const int c = leaves[w];
+    const double4 C = xr[c];
+    x = B.x - C.x;
+    y = B.y - C.y;
+    z = B.z - C.z;
+    Lc = L + (long)c * NT;
+  }
+  const R r2 = x * x + y * y + z * z;
+  R p = 0, fx = 0, fy = 0, fz = 0, ux = 1, uy = 0;
+  V zero;
+  zero.x = zero.y = 0;
+#pragma unroll
+  for (int m = 0; m < P; m++) {
+    V S0 = zero, Sz = zero, Sm = zero, Sp = zero, l = __ldg(Lc + tri(m) + m);
+    R T = 1, Tp = 0;
+#pragma unroll
+    for (int n = m; n < P; n++) {
+      S0.x = fma(T, l.x, S0.x);
+      S0.y = fma(T, l.y, S0.y);
+      if (n + 1 < P) {
+        const V lp = __ldg(Lc + tri(n + 1) + m + 1);
+        l = __ldg(Lc + tri(n + 1) + m);  // L_{n+1}^m: S0's of the next step
+        Sz.x = fma(T, l.x, Sz.x);
+        Sz.y = fma(T, l.y, Sz.y);
+        Sp.x = fma(T, lp.x, Sp.x);
+        Sp.y = fma(T, lp.y, Sp.y);
+        if (m > 0) {
+          const V lm = __ldg(Lc + tri(n + 1) + m - 1);
+          Sm.x = fma(T, lm.x, Sm.x);
+          if (m > 1) Sm.y = fma(T, lm.y, Sm.y);  // of an m = 0 coefficient only the real part counts
+        }
+        const double d = -1.0 / ((double)(n - m + 1) * (n + m + 1));
+        const R Tn = fma((R)((2 * n + 1) * d), z * T, (R)d * (r2 * Tp));
+        Tp = T;
+        T = Tn;
+      }
+    }
+    const R wm = m == 0 ? 1 : 2;
+    p += wm * (S0.x * ux - S0.y * uy);
+    fz -= wm * (Sz.x * ux - Sz.y * uy);
+    fx += (Sp.x - Sm.x) * ux - (Sp.y - Sm.y) * uy;
+    fy -= (Sp.x + Sm.x) * uy + (Sp.y + Sm.y) * ux;
+    const R vx = x * (R)(0.5 / (m + 1)), vy = y * (R)(0.5 / (m + 1)), nx = ux * vx - uy * vy;
+    uy = ux * vy + uy * vx;
+    ux = nx;
+  }
+  double4 d = out[b];  // F32: the gradient back to the input units
+  d.x += p;
+  d.y += fx * sc;
+  d.z += fy * sc;
+  d.w += fz * sc;
+  out[b] = d;
+}
+
+// The same for orders above COLS_MAXP.
 __global__ void __launch_bounds__(128, L2P_F32_MIN_BLOCKS) k_l2p_f32(long nbodies, const int *body_leaf,
                                                                    const float4 *srcf, const float2 *Lf,
-                                                                   const float *lsc, double4 *out, int Prt) {
-  const int P = PT > 0 ? PT : Prt;
+                                                                   const float *lsc, double4 *out, int P) {
   const int nt = tri(P);
   const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nbodies) return;
@@ -304,7 +466,7 @@ __global__ void __launch_bounds__(128, L2P_F32_MIN_BLOCKS) k_l2p_f32(long nbodie
   const float4 B = srcf[b];
   const SphF g = sph_of_f(B.x * sc, B.y * sc, B.z * sc);
   float pot = 0.f, s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  regular_all_f<PT, true>(P, g, g.e, [&](int n, int m, float2 Y, float2 dY) {
+  regular_all_f<0, true>(P, g, g.e, [&](int n, int m, float2 Y, float2 dY) {
     const float2 l = __ldg(Lw + tri(n) + m);
     const float w2 = m == 0 ? 1.f : 2.f;
     const float re = l.x * Y.x - l.y * Y.y;
@@ -494,18 +656,6 @@ __device__ __forceinline__ void cfma(V &acc, const V a, const V y) {
   acc.x = fma(a.x, y.x, fma(-a.y, y.y, acc.x));
   acc.y = fma(a.x, y.y, fma(a.y, y.x, acc.y));
 }
-
-// complex value type of a compute precision
-template <bool F32>
-struct Cplx {
-  typedef double2 V;
-  typedef double R;
-};
-template <>
-struct Cplx<true> {
-  typedef float2 V;
-  typedef float R;
-};
 
 // Unit harmonic variants into shared memory: Yv[v][oct][idx], v bit 0
 // conjugate, bit 1 negate (nv = 2 or 4 variants).
@@ -758,12 +908,7 @@ void expansions_set_attributes() {
   FMM_CUDA(cudaMemcpyToSymbol(c_recip_f, rf, sizeof(rf)));
   cudaFuncSetAttribute(k_p2m, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaFuncSetAttribute(k_l2p, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-#define EXAFMM_F32_ATTR(p)                                                                     \
-  cudaFuncSetAttribute(k_p2m_f32<p>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
-  cudaFuncSetAttribute(k_p2m_f32t<p>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  cudaFuncSetAttribute(k_p2m_f32<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  EXAFMM_UNROLLED_ORDERS(EXAFMM_F32_ATTR)
-#undef EXAFMM_F32_ATTR
+  cudaFuncSetAttribute(k_p2m_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaFuncSetAttribute(k_m2m, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaFuncSetAttribute(k_l2l_ob<false, OB_PAR, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaFuncSetAttribute(k_l2l_ob<false, 1, OB_SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -861,34 +1006,37 @@ void upward_pass(Handle &h, cudaStream_t s) {
   const int P = h.prm.P, nt = tri(P);
   h.M.need((size_t)h.ncells * nt * sizeof(double2));
   h.L.need((size_t)h.ncells * nt * sizeof(double2));
-  if (h.prm.precision == EXAFMM_MIXED) {
+  const bool mixed = h.prm.precision == EXAFMM_MIXED;
+  if (mixed) {
     if (s != h.stream && !h.srcf_ready) throw Error{EXAFMM_ERR_STATE, "upward pass on a side stream before its sources"};
     make_srcf(h);
-    const dim3 grid(grid_for(h.nleaves, WARPS)), block(WARPS * 32);
-    const size_t sm = WARPS * nt * sizeof(double2);
-    auto args = [&](auto kernel) {
-      kernel<<<grid, block, sm, s>>>(h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(),
-                                     h.c_xr.as<double4>(), h.srcf.as<float4>(), h.M.as<double2>(), P);
-    };
-    const size_t smt = p2m_t_smem(nt);
-    auto argst = [&](auto kernel) {
-      kernel<<<grid, block, smt, s>>>(h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(),
-                                      h.c_xr.as<double4>(), h.srcf.as<float4>(), h.M.as<double2>());
-    };
-    switch (P) {
+  }
+  auto cols = [&](auto pc) {
+    constexpr int PP = decltype(pc)::value, LPW = 32 / ((PP + 1) / 2);
+    const unsigned g = grid_for(h.nleaves, 4 * LPW);
+    if (mixed)
+      k_p2m_cols<PP, true><<<g, 128, 0, s>>>(h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(),
+                                             h.c_xr.as<double4>(), h.srcf.as<float4>(), h.M.as<double2>());
+    else
+      k_p2m_cols<PP, false><<<g, 128, 0, s>>>(h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(),
+                                              h.c_xr.as<double4>(), h.src.as<double4>(), h.M.as<double2>());
+  };
+  switch (P) {
 #define EXAFMM_P2M_CASE(p) \
   case p:                  \
-    if (P2M_TRANSPOSE) argst(k_p2m_f32t<p>); else args(k_p2m_f32<p>); \
+    cols(std::integral_constant<int, p>{}); \
     break;
-      EXAFMM_UNROLLED_ORDERS(EXAFMM_P2M_CASE)
+    EXAFMM_COLS_ORDERS(EXAFMM_P2M_CASE)
 #undef EXAFMM_P2M_CASE
-      default:
-        args(k_p2m_f32<0>);
-    }
-  } else {
-    k_p2m<<<grid_for(h.nleaves, WARPS), WARPS * 32, WARPS * nt * sizeof(double2), s>>>(
-        h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.c_xr.as<double4>(),
-        h.src.as<double4>(), h.M.as<double2>(), P);
+    default:
+      if (mixed)
+        k_p2m_f32<<<grid_for(h.nleaves, WARPS), WARPS * 32, WARPS * nt * sizeof(double2), s>>>(
+            h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.c_xr.as<double4>(),
+            h.srcf.as<float4>(), h.M.as<double2>(), P);
+      else
+        k_p2m<<<grid_for(h.nleaves, WARPS), WARPS * 32, WARPS * nt * sizeof(double2), s>>>(
+            h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.c_xr.as<double4>(),
+            h.src.as<double4>(), h.M.as<double2>(), P);
   }
   h.launches++;
   FMM_LAUNCH();
@@ -953,25 +1101,33 @@ void downward_pass(Handle &h, cudaStream_t s, cudaEvent_t before_l2p) {
     h.launches++;
   }
   if (before_l2p) FMM_CUDA(cudaStreamWaitEvent(s, before_l2p, 0));
-  if (h.prm.precision == EXAFMM_MIXED) {
-    auto args = [&](auto kernel) {
-      kernel<<<grid_for(h.n, 128), 128, 0, s>>>((long)h.n, h.body_leaf.as<int>(), h.srcf.as<float4>(), Lf, lsc,
-                                                h.out.as<double4>(), P);
-    };
-    switch (P) {
+  const bool mixed = h.prm.precision == EXAFMM_MIXED;
+  auto body = [&](auto pc) {
+    constexpr int PP = decltype(pc)::value;
+    const unsigned g = grid_for(h.n, 128);
+    if (mixed)
+      k_l2p_body<PP, true><<<g, 128, 0, s>>>((long)h.n, h.leaves.as<int>(), h.body_leaf.as<int>(),
+                                             h.c_xr.as<double4>(), h.srcf.as<float4>(), Lf, lsc, h.out.as<double4>());
+    else
+      k_l2p_body<PP, false><<<g, 128, 0, s>>>((long)h.n, h.leaves.as<int>(), h.body_leaf.as<int>(),
+                                              h.c_xr.as<double4>(), h.src.as<double4>(), h.L.as<double2>(), nullptr,
+                                              h.out.as<double4>());
+  };
+  switch (P) {
 #define EXAFMM_L2P_CASE(p) \
   case p:                  \
-    args(k_l2p_f32<p>);    \
+    body(std::integral_constant<int, p>{}); \
     break;
-      EXAFMM_UNROLLED_ORDERS(EXAFMM_L2P_CASE)
+    EXAFMM_COLS_ORDERS(EXAFMM_L2P_CASE)
 #undef EXAFMM_L2P_CASE
-      default:
-        args(k_l2p_f32<0>);
-    }
-  } else {
-    k_l2p<<<grid_for(h.nleaves, WARPS), WARPS * 32, WARPS * nt * sizeof(double2), s>>>(
-        h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.c_xr.as<double4>(),
-        h.src.as<double4>(), h.L.as<double2>(), h.out.as<double4>(), P);
+    default:
+      if (mixed)
+        k_l2p_f32<<<grid_for(h.n, 128), 128, 0, s>>>((long)h.n, h.body_leaf.as<int>(), h.srcf.as<float4>(), Lf, lsc,
+                                                     h.out.as<double4>(), P);
+      else
+        k_l2p<<<grid_for(h.nleaves, WARPS), WARPS * 32, WARPS * nt * sizeof(double2), s>>>(
+            h.leaves.as<int>(), h.nleaves, h.c_begin.as<int>(), h.c_count.as<int>(), h.c_xr.as<double4>(),
+            h.src.as<double4>(), h.L.as<double2>(), h.out.as<double4>(), P);
   }
   h.launches++;
   FMM_LAUNCH();

@@ -373,10 +373,10 @@ __global__ void k_ref_leaves(BfsCells o, long c, const int *blockstart_pre, int 
 
 // Bodies of one leaf back into input order (warp per leaf, rank sort).
 // Bodies of each leaf back to input order (a body's slot is the rank of its
-// input index among the leaf's), gathered into src.  With srcf (3D mixed
-// form) also the FP32 copy of each body as an offset from its leaf centre
-// (FP64 subtraction, one rounding) and the body's leaf, as k_make_srcf makes
-// them: one pass over the bodies instead of three.
+// input index among the leaf's), gathered into src, and (3D) the body's leaf.
+// With srcf (3D mixed form) also the FP32 copy of each body as an offset from
+// its leaf centre (FP64 subtraction, one rounding), alone and in pairs, as
+// k_make_srcf makes them: one pass over the bodies instead of three.
 __global__ void k_leaf_order(const int *leaves, int nleaves, const int *begin, const int *count, const double4 *xr,
                              const u32 *vals, const double4 *in, int *perm, double4 *src, float4 *srcf,
                              float4 *pairs, int *body_leaf) {
@@ -396,8 +396,8 @@ __global__ void k_leaf_order(const int *leaves, int nleaves, const int *begin, c
       const float4 f = make_float4((float)(B.x - C.x), (float)(B.y - C.y), (float)(B.z - C.z), (float)B.w);
       srcf[b] = f;
       put_pair(pairs, b0, r, nb, f);
-      body_leaf[b] = w;
     }
+    if (body_leaf) body_leaf[b] = w;
   }
 }
 
@@ -528,16 +528,16 @@ void build_tree(Handle &h) {
     // form's FP32 sources with them)
     h.perm.need(n * 4);
     h.src.need(n * sizeof(double4));
-    const bool srcf = h.prm.precision == EXAFMM_MIXED && h.prm.dim == 3;
+    const bool srcf = h.prm.precision == EXAFMM_MIXED && h.prm.dim != 2;
     if (srcf) {
       h.srcf.need((size_t)n * sizeof(float4));
       h.srcp.need((size_t)n * 2 * sizeof(float4));
-      h.body_leaf.need((size_t)n * sizeof(int));
     }
+    if (h.prm.dim != 2) h.body_leaf.need((size_t)n * sizeof(int));
     k_leaf_order<<<grid_for((long)h.nleaves * 32, TB), TB, 0, s>>>(
         h.leaves.as<int>(), h.nleaves, o.begin, o.count, o.xr, v, h.in.as<double4>(), h.perm.as<int>(),
         h.src.as<double4>(), srcf ? h.srcf.as<float4>() : nullptr, h.srcp.as<float4>(),
-        srcf ? h.body_leaf.as<int>() : nullptr);
+        h.prm.dim != 2 ? h.body_leaf.as<int>() : nullptr);
     h.launches++;
     FMM_LAUNCH();
     h.srcf_ready = srcf;
