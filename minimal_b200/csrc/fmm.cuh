@@ -131,6 +131,7 @@ struct Handle {
   int ncells = 0, nleaves = 0, depth = 0;
   int level_base[EXAFMM_MAX_LEVEL + 3] = {0};
   Buf c_begin, c_count, c_child, c_nchild, c_parent, c_level, c_xr, c_pre, c_ref, c_leaf_of_body;
+  Buf c_face;  // which faces of the root a cell's parent touches (k_cells)
   Buf leaves;  // BFS indices of leaves
   Buf pre_tmp; // preorder tables
   Buf ctmp;    // cell-count scratch (level sort, index maps)

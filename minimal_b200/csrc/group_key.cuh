@@ -132,27 +132,32 @@ __device__ __forceinline__ int m2l_ghost_key(const double4 &X, const double4 &Y,
 
 // Marks a key and a target as present.  A few hundred keys (and every
 // target) take millions of entries: store only what this SM has not seen
-// set, so the L1-cached reads keep the stores off a few hot L2 lines.
-__device__ __forceinline__ void m2l_mark_key(int key, int t, unsigned char *occ, int *gflag) {
+// set, so the L1-cached reads keep the stores off a few hot L2 lines.  The
+// target's entries from finer sources (dl < 0, few) are counted: the number
+// tells targets at a change of refinement from others (k_tkeys).
+__device__ __forceinline__ void m2l_mark_key(int key, int t, int dl, unsigned char *occ, int *gflag, int *gfine) {
   if (occ[key] == 0) occ[key] = 1;
   if (gflag[t] == 0) gflag[t] = 1;
+  if (dl < 0) atomicAdd(&gfine[t], 1);
 }
 
 // Group tables of a key space of ks keys (a multiple of OCC_TILE) and a tree
 // of C cells, one buffer: the marks of the keys (a byte each) and of the
-// targets, the P2P counts of the targets (all three zeroed together), then
+// targets, the targets' entries from finer sources, the P2P counts of the
+// targets (these four zeroed together), then
 // per 32 keys {marks as a mask, groups before them}, then per tile the number
 // of marked keys.
 constexpr long OCC_TILE = 32768;
 static_assert(KEY_SPACE % OCC_TILE == 0 && IKEY_SPACE % OCC_TILE == 0, "whole tiles of group keys");
 struct GroupTables {
   unsigned char *occ;
-  int *gflag, *cnt;  // C targets; C + 1 counts
+  int *gflag, *gfine, *cnt;  // C, C and C + 1 ints
   uint2 *mask;
   int *sums;
 };
 inline size_t group_cells(int C) { return ((size_t)C + 3) / 4 * 4; }  // the counts start 16-byte aligned
-inline size_t group_mark_bytes(long ks, int C) { return (size_t)ks + (group_cells(C) + C + 1) * sizeof(int); }
+inline size_t group_key_bytes(long ks, int C) { return (size_t)ks + 2 * group_cells(C) * sizeof(int); }  // without cnt
+inline size_t group_mark_bytes(long ks, int C) { return group_key_bytes(ks, C) + (size_t)(C + 1) * sizeof(int); }
 inline size_t group_table_bytes(long ks, int C) {
   return (group_mark_bytes(ks, C) + 15) / 16 * 16 + (size_t)ks / 32 * sizeof(uint2) + ks / OCC_TILE * sizeof(int);
 }
@@ -160,7 +165,7 @@ inline GroupTables group_tables(void *p, long ks, int C) {
   unsigned char *b = (unsigned char *)p;
   int *f = (int *)(b + ks);
   uint2 *m = (uint2 *)(b + (group_mark_bytes(ks, C) + 15) / 16 * 16);
-  return GroupTables{b, f, f + group_cells(C), m, (int *)(m + ks / 32)};
+  return GroupTables{b, f, f + group_cells(C), f + 2 * group_cells(C), m, (int *)(m + ks / 32)};
 }
 
 // Group id of a marked key.

@@ -70,7 +70,7 @@ struct WalkArgs {
   int depth;
   int *overflow, *m2l_key;
   unsigned char *occ;
-  int *gflag, *nres;
+  int *gflag, *gfine, *nres;
 };
 
 // Step st: reads frontier st & 1 and count word st % 3, appends to the other
@@ -143,7 +143,7 @@ __device__ __forceinline__ void walk_step(const WalkArgs &wa, int st) {
           const int dl = radius_level_diff(b.w, a.w);
           if (img == 13) key[r] = m2l_group_key(a, b, dl);
           else key[r] = m2l_image_key(a, b, dl, img, cv.xr[0].w, cycle, depth);
-          if (key[r] >= 0) m2l_mark_key(key[r], i, occ, gflag);
+          if (key[r] >= 0) m2l_mark_key(key[r], i, dl, occ, gflag, wa.gfine);
           else res++;
         }
         nm++;
@@ -475,7 +475,7 @@ void build_lists(Handle &h, const std::function<void()> &near_field) {
                       {h.frontier[0].as<int2>(), h.frontier[1].as<int2>()}, &ctr->frontier[0], h.frontier_cap,
                       h.m2l_raw.as<int2>(), h.p2p_raw.as<int2>(), &ctr->n_m2l, &ctr->n_p2p, h.m2l_cap, h.p2p_cap,
                       h.prm.theta, images ? h.prm.cycle : 0.0, h.depth, &ctr->list_overflow, h.m2l_key.as<int>(),
-                      keyed ? gt.occ : nullptr, gt.gflag, &ctr->walk_resid};
+                      keyed ? gt.occ : nullptr, gt.gflag, gt.gfine, &ctr->walk_resid};
     // the steps whose frontier, at most `most` pairs, fits one block
     // iteration run in one launch; later steps take as many blocks as their
     // frontier can fill, up to one wave

@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(TB) k_chain(const u64 *keys, long n, int D, in
 }
 
 struct PreTables {
-  int *begin, *count, *level, *parent, *nchild;
+  int *begin, *count, *level, *parent, *nchild, *face;
   double4 *xr;
 };
 
@@ -337,8 +337,13 @@ __global__ void k_cells(const u64 *keys, long n, long C, int D, const int *lfirs
     const RootGeom *gs = g + (long)(key >> (3 * D));  // the body's system
     double cx = gs->X0[0], cy = gs->X0[1], cz = gs->X0[2];
     double r = gs->R0;  // R0 / 2^l, halved exactly level by level
+    int any = 0, all = l > 1 ? 7 : 0;  // octant bits on the way to the parent
     for (int q = 0; q < l; q++) {  // centre of the level-l cell holding body i
       const int o = (int)((key >> (3 * (D - 1 - q))) & 7);
+      if (q < l - 1) {
+        any |= o;
+        all &= o;
+      }
       r = __dmul_rn(r, 0.5);
       cx = __dadd_rn(cx, (o & 1) ? r : -r);
       cy = __dadd_rn(cy, (o & 2) ? r : -r);
@@ -358,6 +363,11 @@ __global__ void k_cells(const u64 *keys, long n, long C, int D, const int *lfirs
     t.level[p] = l;
     t.parent[p] = parent;
     t.xr[p] = make_double4(cx, cy, cz, r);
+    // per axis 0, 1 or 2: the parent lies at the root's low face, inside, at
+    // its high face
+    int face = 0;
+    for (int d = 2; d >= 0; d--) face = 3 * face + ((any >> d & 1) ? 1 + (all >> d & 1) : 0);
+    t.face[p] = face;
     if (parent >= 0) atomicAdd(&t.nchild[parent], 1);
   }
 }
@@ -375,7 +385,7 @@ __global__ void k_invert(const u32 *pre_of_bfs, long c, int *bfs_of_pre) {
 }
 
 struct BfsCells {
-  int *begin, *count, *child, *nchild, *parent, *level, *pre;
+  int *begin, *count, *child, *nchild, *parent, *level, *pre, *face;
   double4 *xr;
 };
 
@@ -387,6 +397,7 @@ __global__ void k_gather_cells(const u32 *pre_of_bfs, const int *bfs_of_pre, lon
   o.begin[b] = t.begin[p];
   o.count[b] = t.count[p];
   o.level[b] = t.level[p];
+  o.face[b] = t.face[p];
   o.xr[b] = t.xr[p];
   o.parent[b] = t.parent[p] >= 0 ? bfs_of_pre[t.parent[p]] : -1;
   const int nc = t.nchild[p];
@@ -532,7 +543,7 @@ void build_tree(Handle &h) {
     }
     // pre-order tables (reuse the idle sort buffers' siblings)
     const long Cp = (C + 3) & ~3L;  // every table starts 16-byte aligned (vector loads in the scans)
-    h.pre_tmp.need(Cp * (6 * sizeof(int) + sizeof(double4)) + 256);
+    h.pre_tmp.need(Cp * (7 * sizeof(int) + sizeof(double4)) + 256);
     PreTables t;
     t.xr = h.pre_tmp.as<double4>();
     t.begin = (int *)(t.xr + Cp);
@@ -540,7 +551,8 @@ void build_tree(Handle &h) {
     t.level = t.count + Cp;
     t.parent = t.level + Cp;
     t.nchild = t.parent + Cp;
-    int *owner = t.nchild + Cp;
+    t.face = t.nchild + Cp;
+    int *owner = t.face + Cp;
     FMM_CUDA(cudaMemsetAsync(t.nchild, 0, C * sizeof(int), s));
     k_cell_owner<<<grid_for(n, TB), TB, 0, s>>>(n, h.chain.as<int>(), h.prebase.as<int>(), owner);
     k_cells<<<grid_for(C, TB), TB, 0, s>>>(k, n, C, D, h.lfirst.as<int>(), owner, h.prebase.as<int>(), g, t);
@@ -561,9 +573,10 @@ void build_tree(Handle &h) {
     h.launches++;
     h.c_begin.need(C * 4); h.c_count.need(C * 4); h.c_child.need(C * 4); h.c_nchild.need(C * 4);
     h.c_parent.need(C * 4); h.c_level.need(C * 4); h.c_pre.need(C * 4); h.c_ref.need(C * 4);
+    h.c_face.need(C * 4);
     h.c_xr.need(C * sizeof(double4));
     BfsCells o{h.c_begin.as<int>(), h.c_count.as<int>(), h.c_child.as<int>(), h.c_nchild.as<int>(),
-               h.c_parent.as<int>(), h.c_level.as<int>(), h.c_pre.as<int>(), h.c_xr.as<double4>()};
+               h.c_parent.as<int>(), h.c_level.as<int>(), h.c_pre.as<int>(), h.c_face.as<int>(), h.c_xr.as<double4>()};
     k_gather_cells<<<grid_for(C, TB), TB, 0, s>>>(lv, bfs_of_pre, C, t, o, is_leaf);
     h.launches++;
     FMM_LAUNCH();
