@@ -63,6 +63,7 @@ constexpr int TC_LOAD_WARP = 4; // first of the producer warps
 constexpr int TC_LOAD_WARPS = 4;
 constexpr int TC_MMA_WARP = TC_LOAD_WARP + TC_LOAD_WARPS;  // MMA issuer, TMEM owner
 constexpr int TC_THREADS = 32 * (TC_MMA_WARP + 1);
+constexpr int TC_IDX = 4;         // groups whose indices a producer loads at once
 constexpr int TC_MAX_STAGES = 4;  // pipeline stages (groups in flight), as many as shared memory holds
 // Groups accumulated in FP32 in tensor memory before the partial sum is
 // folded into the compensated running sum.  The tensor core's FP32
@@ -1058,7 +1059,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
   const TcAcc ta = FIX ? TcFixed<PT>::acc : ta_;
   extern __shared__ __align__(1024) unsigned char smraw[];
   unsigned char *base = smraw + ((1024u - (tc::smem_u32(smraw) & 1023u)) & 1023u);  // swizzle atoms: 1024-aligned
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t abytes = (uint32_t)pl.abytes, bimg = (uint32_t)pl.bimg;
   const uint32_t stage_bytes = 2 * abytes + 2 * bimg;  // A hi, A lo, B hi, B lo
   uint64_t *full = (uint64_t *)(base + (size_t)nstage * stage_bytes);  // [stage] multipoles landed (producer warps)
@@ -1090,7 +1091,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  const uint32_t tmem = *tslot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
   // this CTA's segments [g0, g1) and the first tile they touch
   int g0, g1, tfirst;
   if (BAL) {
@@ -1156,70 +1157,108 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
     }
   } else if (warp < TC_LOAD_WARP + TC_LOAD_WARPS) {
     // ---- producers: warp pw copies target rows 32pw..32pw+31 of the tile
-    // with cp.async into the swizzled layout.  Lane l takes rows
-    // 32pw + (l >> 1) and 32pw + 16 + (l >> 1), and of each source row (the
-    // multipole's hi then lo halves, 4 KP contiguous bytes in global memory)
-    // the 16-byte chunks of parity l & 1: the two lanes of a pair copy the
-    // two halves of every 32-byte sector in the same instruction, so each
-    // sector is requested from L2 once (one lane per row requested every
-    // sector twice, and the L1-to-L2 request path was the kernel's limit).
-    // Absent targets are zero-filled.  Producer thread 0 also starts the
-    // operator's bulk copy.  Each thread's copies arrive on the stage's
-    // barrier by themselves (cp.async.mbarrier.arrive), so the producers run
-    // up to `nstage` groups ahead of the MMAs.  The next group's source rows
-    // and operator slot are loaded one group ahead.
-    const int pw = warp - TC_LOAD_WARP, par = lane & 1;
-    const int ra = 32 * pw + (lane >> 1), rb = ra + 16;
-    const int half = KP / 8;  // 16-byte chunks of one half (hi or lo) of a source row; even
-    auto src_of = [&](int k) {
-      const int *row = tg_src + (long)(g0 + k) * TC_TILE;
-      return k < n ? make_int2(row[ra], row[rb]) : make_int2(-1, -1);
+    // with cp.async into the swizzled layout.  A source row (the multipole's
+    // hi then lo halves) is C = KP / 4 chunks of 16 contiguous bytes; the
+    // lanes take consecutive chunks of consecutive rows, so an instruction
+    // reads one to three rows' contiguous pieces (with two lanes per row it
+    // asked for sixteen rows' single sectors: at 1M uniform bodies, P = 10,
+    // the kernel took 477 us against 425).  C is a multiple of four: every
+    // C / 4 instructions the pattern starts again eight rows further down,
+    // where the swizzle is the same.  Absent targets are zero-filled.
+    // Producer thread 0 also starts the operator's bulk copy.  Each thread's
+    // copies arrive on the stage's barrier by themselves
+    // (cp.async.mbarrier.arrive), so the producers run up to `nstage` groups
+    // ahead of the MMAs.  Source rows (lane l: row 32pw + l) and operator
+    // slots are loaded TC_IDX groups at a time, a whole batch ahead: the
+    // indices come from L2 or DRAM, and one group ahead their latency was the
+    // producers' time per group at low orders (256 systems, P = 6: 1247 us
+    // against 930; 1M bodies, P = 10: 417 against 380).
+    const int pw = warp - TC_LOAD_WARP;
+    const int half = KP / 8, C = 2 * half;  // 16-byte chunks of one half (hi or lo), of a source row
+    // byte offset of chunk c of row r (r < 8) in the stage
+    auto place = [&](int r, int c) {
+      const int hl = c >= half, cc = c - hl * half;
+      return (uint32_t)hl * abytes + (uint32_t)(cc >> 3) * (TC_TILE * 128) + (uint32_t)r * 128 +
+             (((uint32_t)(cc & 7) ^ (uint32_t)r) << 4);
     };
+    constexpr int NI = FIX ? TcFixed<PT>::KP / 16 : 1;
+    uint32_t so[NI];
+    int sr[NI], sc[NI];
+    if (FIX)
+#pragma unroll
+      for (int i = 0; i < NI; i++) {
+        const int id = 32 * i + lane;
+        sr[i] = id / C;
+        sc[i] = id % C;
+        so[i] = place(sr[i], sc[i]);
+      }
     const bool bulk = pw == 0 && lane == 0;  // the thread that starts the operator's bulk copy
-    auto gid_of = [&](int k) { return bulk && k < n ? tg_gid[g0 + k] : 0; };
-    auto issue = [&](int st, int2 s2, int gid) {
+    auto load_idx = [&](int k, int *s, int *g) {
+#pragma unroll
+      for (int j = 0; j < TC_IDX; j++) {
+        s[j] = k + j < n ? tg_src[(long)(g0 + k + j) * TC_TILE + 32 * pw + lane] : -1;
+        g[j] = bulk && k + j < n ? tg_gid[g0 + k + j] : 0;
+      }
+    };
+    auto issue = [&](int st, int srow, int gid) {
       unsigned char *S = base + (size_t)st * stage_bytes;
       if (bulk) {
         tc::mbar_arrive_expect_tx(&bful[st], 2 * bimg);
         tc::bulk_g2s(S + 2 * abytes, ops + (size_t)gid * 2 * bimg, 2 * bimg, &bful[st]);
       }
-      // chunk c = c0 + par with c0 even: half is even, so c0 alone decides
-      // the half (hl) and the atom, and the lane's parity only sets bit 4 of
-      // the in-row offset (folded into the row's swizzle q)
+      unsigned char *R = S + 32 * pw * 128;
+      if (FIX) {
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const int r = j ? rb : ra, s = j ? s2.y : s2.x;
-        const __half *src = M16 + (size_t)(s < 0 ? 0 : s) * 2 * KP + par * 8;
-        const uint32_t nb = s >= 0 ? 16u : 0u, q = ((uint32_t)par << 4) ^ ((uint32_t)(r & 7) << 4);
-        unsigned char *R = S + r * 128;
+        for (int r8 = 0; r8 < 32; r8 += 8)
 #pragma unroll
-        for (int c0 = 0; c0 < 2 * half; c0 += 2) {
-          const int hl = c0 >= half, cc0 = c0 - hl * half;
-          const uint32_t off = hl * abytes + (cc0 >> 3) * (TC_TILE * 128) + ((((uint32_t)cc0 & 7) << 4) ^ q);
-          tc::cp_async16(R + off, src + c0 * 8, nb);
+          for (int i = 0; i < NI; i++) {
+            const int s = __shfl_sync(0xffffffffu, srow, r8 + sr[i]);
+            tc::cp_async16(R + r8 * 128 + so[i], M16 + (size_t)(s < 0 ? 0 : s) * 2 * KP + sc[i] * 8, s >= 0 ? 16u : 0u);
+          }
+      } else {
+        int r = lane / C, c = lane % C;
+        for (int i = 0; i < C; i++) {
+          const int s = __shfl_sync(0xffffffffu, srow, r);
+          tc::cp_async16(R + (r & ~7) * 128 + place(r & 7, c), M16 + (size_t)(s < 0 ? 0 : s) * 2 * KP + c * 8,
+                         s >= 0 ? 16u : 0u);
+          r += 32 / C;
+          c += 32 % C;
+          if (c >= C) {
+            c -= C;
+            r++;
+          }
         }
       }
       tc::cp_async_commit();
     };
     bool ok = true;
     int last = -1, lst = 0;
-    int2 s_next = src_of(0);
-    int gid_next = gid_of(0);
+    int s_cur[TC_IDX], g_cur[TC_IDX], s_next[TC_IDX], g_next[TC_IDX];
+    load_idx(0, s_cur, g_cur);
     // stage st of round rnd = k / nstage (counters, no divisions)
-    for (int k = 0, st = 0, rnd = 0; k < n; k++) {
-      if (rnd > 0) {  // the stage is free once the MMAs of group k - nstage are done
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(&empty[st], (uint32_t)(rnd - 1) & 1u, wait_ns, abort));
-        if (!ok) break;
+    for (int k0 = 0, st = 0, rnd = 0; ok && k0 < n; k0 += TC_IDX) {
+      load_idx(k0 + TC_IDX, s_next, g_next);
+#pragma unroll
+      for (int j = 0; j < TC_IDX; j++) {
+        const int k = k0 + j;
+        if (k >= n) break;
+        if (rnd > 0) {  // the stage is free once the MMAs of group k - nstage are done
+          ok = __all_sync(0xffffffffu, tc::mbar_wait(&empty[st], (uint32_t)(rnd - 1) & 1u, wait_ns, abort));
+          if (!ok) break;
+        }
+        issue(st, s_cur[j], g_cur[j]);
+        tc::cp_async_arrive(&full[st]);  // arrives when this thread's copies have landed
+        last = k;
+        lst = st;
+        if (++st == nstage) {
+          st = 0;
+          rnd++;
+        }
       }
-      issue(st, s_next, gid_next);
-      tc::cp_async_arrive(&full[st]);  // arrives when this thread's copies have landed
-      last = k;
-      lst = st;
-      s_next = src_of(k + 1);
-      gid_next = gid_of(k + 1);
-      if (++st == nstage) {
-        st = 0;
-        rnd++;
+#pragma unroll
+      for (int j = 0; j < TC_IDX; j++) {
+        s_cur[j] = s_next[j];
+        g_cur[j] = g_next[j];
       }
     }
     if (!ok) {
@@ -1231,50 +1270,63 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
     tc::cp_async_wait_all();
     if (pw == 0 && lane == 0 && last >= 0) tc::mbar_wait(&bful[lst], parity(last), 2 * wait_ns);
   } else if (warp == TC_MMA_WARP) {
-    // ---- MMA issuer (one thread): per group and output block, K steps of
-    // hi*hi + hi*lo + lo*hi into the window's accumulator
-    if (lane == 0) {
-      int rows[4], ksteps[4];
-      uint32_t boff[4], idesc[4], idesc2[4];
+    // ---- MMA issuer: per group and output block, K steps of hi*hi + hi*lo +
+    // lo*hi into the window's accumulator.  The whole warp waits and counts,
+    // so that the descriptors are uniform, and one elected lane issues: with
+    // a single thread running the loop, an MMA took it about 70 clocks to
+    // issue against the 48 that the tensor core needs, and each of the up to
+    // three waits another 130 (1M uniform bodies, P = 10: 422 us against 375
+    // now; 256 systems, P = 6: 1194 against 924).
+    int rows[4], ksteps[4];
+    uint32_t boff[4], idesc[4], idesc2[4];
 #pragma unroll
-      for (int b = 0; b < 4; b++) {
-        rows[b] = b < pl.nb ? pl.rows[b] : 0;
-        ksteps[b] = b < pl.nb ? pl.ksteps[b] : 0;
-        boff[b] = b < pl.nb ? (uint32_t)pl.boff[b] : 0u;
-        idesc[b] = tc::idesc_f16_f32(TC_TILE, rows[b] > 0 ? rows[b] : 16);
-        idesc2[b] = tc::idesc_f16_f32(TC_TILE, rows[b] > 0 ? 2 * rows[b] : 16);  // paired: hi and lo rows
+    for (int b = 0; b < 4; b++) {
+      rows[b] = b < pl.nb ? pl.rows[b] : 0;
+      ksteps[b] = b < pl.nb ? pl.ksteps[b] : 0;
+      boff[b] = b < pl.nb ? (uint32_t)pl.boff[b] : 0u;
+      idesc[b] = tc::idesc_f16_f32(TC_TILE, rows[b] > 0 ? rows[b] : 16);
+      idesc2[b] = tc::idesc_f16_f32(TC_TILE, rows[b] > 0 ? 2 * rows[b] : 16);  // paired: hi and lo rows
+    }
+    // test hook: a wait on a barrier that nothing arrives at, as if the
+    // tensor core's inputs never came; it runs out after stall_ns
+    bool ok = stall_ns <= 0 || __all_sync(0xffffffffu, tc::mbar_wait(stall, 0u, stall_ns, abort));
+    int last = -1, lst = 0;
+    // end of the current tile's segments in the range (a window closes
+    // there too)
+    int tcur = tfirst, tend = BAL ? min(g1, tg_off[tfirst + 1]) : g1;
+    // stage st of round rnd = k / nstage; the window has kf groups so far
+    // and uses accumulator a for the u-th time (counters, no divisions)
+    for (int k = 0, st = 0, rnd = 0, kf = 0, a = 0, u = 0; ok && k < n; k++) {
+      if (BAL && g0 + k >= tend) {  // next tile (skipping tiles without segments)
+        do tcur++;
+        while (tg_off[tcur + 1] <= g0 + k);
+        tend = min(g1, tg_off[tcur + 1]);
       }
-      // test hook: a wait on a barrier that nothing arrives at, as if the
-      // tensor core's inputs never came; it runs out after stall_ns
-      bool ok = stall_ns <= 0 || tc::mbar_wait(stall, 0u, stall_ns, abort);
-      int last = -1, lst = 0;
-      // end of the current tile's segments in the range (a window closes
-      // there too)
-      int tcur = tfirst, tend = BAL ? min(g1, tg_off[tfirst + 1]) : g1;
-      // stage st of round rnd = k / nstage; the window has kf groups so far
-      // and uses accumulator a for the u-th time (counters, no divisions)
-      for (int k = 0, st = 0, rnd = 0, kf = 0, a = 0, u = 0; ok && k < n; k++) {
-        if (BAL && g0 + k >= tend) {  // next tile (skipping tiles without segments)
-          do tcur++;
-          while (tg_off[tcur + 1] <= g0 + k);
-          tend = min(g1, tg_off[tcur + 1]);
-        }
-        const bool close = kf == flush_every - 1 || g0 + k + 1 == tend;
-        const uint32_t ph = (uint32_t)rnd & 1u;
-        ok = tc::mbar_wait(&full[st], ph, wait_ns, abort) && tc::mbar_wait(&bful[st], ph, wait_ns, abort);
-        // a new window reuses accumulator a once the epilogue has folded
-        // its previous use
-        if (ok && kf == 0 && u > 0) ok = tc::mbar_wait(&acce[a], (uint32_t)(u - 1) & 1u, wait_ns, abort);
-        if (!ok) break;
-        tc::fence_after();
-        const uint32_t sA = tc::smem_u32(base + (size_t)st * stage_bytes), sB = sA + 2 * abytes;
-        const uint64_t dA = tc::smem_desc_sw128(sA), dB = tc::smem_desc_sw128(sB), dB32 = tc::smem_desc_sw32(sB);
-        const uint64_t lo_a = abytes >> 4;  // descriptor start fields count 16 bytes
-        const bool fresh = kf == 0;
-        const uint32_t acc = tmem + (uint32_t)a * ta.stride;
-        // per K step: hi*hi, then hi*lo with the same A, then lo*hi (issuing
-        // the small products first lowered the truncation bias by a third
-        // but cost 15% of the M2L time: consecutive MMAs on one A are faster)
+      const bool close = kf == flush_every - 1 || g0 + k + 1 == tend;
+      const uint32_t ph = (uint32_t)rnd & 1u;
+      // the stage's multipoles and operator, and for a new window its
+      // accumulator folded since its last use: asked for together, so that
+      // three waits that are over cost the latency of one
+      const bool reuse = kf == 0 && u > 0;
+      const uint32_t pa = (uint32_t)(u - 1) & 1u;
+      const bool f = tc::mbar_try_wait(&full[st], ph), o = tc::mbar_try_wait(&bful[st], ph);
+      const bool e = !reuse || tc::mbar_try_wait(&acce[a], pa);
+      ok = f && o && e;
+      if (!__all_sync(0xffffffffu, ok))
+        ok = __all_sync(0xffffffffu,
+                        tc::mbar_wait(&full[st], ph, wait_ns, abort) && tc::mbar_wait(&bful[st], ph, wait_ns, abort) &&
+                            (!reuse || tc::mbar_wait(&acce[a], pa, wait_ns, abort)));
+      if (!ok) break;
+      tc::fence_after();
+      const uint32_t sA = tc::smem_u32(base + (size_t)st * stage_bytes), sB = sA + 2 * abytes;
+      const uint64_t dA = tc::smem_desc_sw128(sA), dB = tc::smem_desc_sw128(sB), dB32 = tc::smem_desc_sw32(sB);
+      const uint64_t lo_a = abytes >> 4;  // descriptor start fields count 16 bytes
+      const bool fresh = kf == 0;
+      const uint32_t acc = tmem + (uint32_t)a * ta.stride;
+      // per K step: hi*hi, then hi*lo with the same A, then lo*hi (issuing
+      // the small products first lowered the truncation bias by a third
+      // but cost 15% of the M2L time: consecutive MMAs on one A are faster)
+      if (tc::elect_one()) {
 #pragma unroll
         for (int b = 0; b < 4; b++) {
           if (b >= pl.nb) break;
@@ -1302,29 +1354,30 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
         }
         tc::commit(&empty[st]);
         if (close) tc::commit(&accf[a]);
-        last = k;
-        lst = st;
-        if (++st == nstage) {
-          st = 0;
-          rnd++;
-        }
-        if (close) {
-          kf = 0;
-          if (++a == ta.nacc) {
-            a = 0;
-            u++;
-          }
-        } else {
-          kf++;
-        }
       }
-      if (!ok) {
-        *abort = 1;
-        *(volatile int *)err = 1;
+      __syncwarp();
+      last = k;
+      lst = st;
+      if (++st == nstage) {
+        st = 0;
+        rnd++;
       }
-      // drain: the MMAs already issued complete by themselves (no abort)
-      if (last >= 0) tc::mbar_wait(&empty[lst], parity(last), 2 * wait_ns);
+      if (close) {
+        kf = 0;
+        if (++a == ta.nacc) {
+          a = 0;
+          u++;
+        }
+      } else {
+        kf++;
+      }
     }
+    if (!ok) {
+      *abort = 1;
+      if (lane == 0) *(volatile int *)err = 1;
+    }
+    // drain: the MMAs already issued complete by themselves (no abort)
+    if (last >= 0) tc::mbar_wait(&empty[lst], parity(last), 2 * wait_ns);
     __syncwarp();
   }
   tc::fence_before();
