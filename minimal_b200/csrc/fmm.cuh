@@ -160,12 +160,13 @@ struct Handle {
   int m2l_units_P = -1;
 
   // grouped M2L (m2l_group.cu)
-  Buf g_mt, g_ekey, g_occ, g_cnt, g_newkeys, g_ops, g_tk, g_tile, g_seg, g_tg, g_m16, g_slot, g_pairs;
+  Buf g_mt, g_ekey, g_occ, g_cnt, g_ops, g_tk, g_tile, g_seg, g_tg, g_m16, g_pairs;
   Buf g_gmark;      // ghost slots: marks, their scan, the slot of every ghost
   int g_nghost = 0;  // ghost multipole rows after the cells' in g_m16
   // operator cache: g_optab[group key] is the operator's slot in g_ops (-1:
   // not built), op_count slots built for order op_P, layout op_layout (0:
-  // FP64 row blocks, 1: tensor-core FP16 images) and key space op_ks
+  // FP64 row blocks, 1: tensor-core FP16 images) and key space op_ks; after
+  // the table, the evaluation's group slots and new keys (op_ks ints each)
   Buf g_optab;
   int op_P = -1, op_layout = -1, op_count = 0;
   long op_ks = 0;

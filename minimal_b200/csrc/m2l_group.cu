@@ -1597,6 +1597,12 @@ bool m2l_groups_raw(const Handle &h) {
          !(h.prm.images > 0 && h.prm.precision == EXAFMM_MIXED && tc_available(h.prm.P));
 }
 
+// g_optab holds three arrays of the key space (one allocation: each costs a
+// new handle's first evaluation about 0.3 ms): the operator table, the
+// operator slot of each group, the keys whose operators are to be built.
+int *group_slots(const Handle &h) { return h.g_optab.as<int>() + h.op_ks; }
+int *new_keys(const Handle &h) { return h.g_optab.as<int>() + 2 * h.op_ks; }
+
 // Queues, after the key and target marks: the group tables, the operator
 // slots, and the flagged targets' tile keys.  max_groups: an upper bound of
 // the groups.
@@ -1610,8 +1616,10 @@ void m2l_group_launch(Handle &h, long max_groups) {
   // also depend on the period, the root radius and the depth
   const bool geom_changed =
       h.prm.images > 0 && (h.op_cycle != cyc || h.op_R0 != h.root_R0 || h.op_depth != h.depth);
-  if (h.op_P != P || h.op_layout != layout || h.op_ks != ks || geom_changed) {
-    h.g_optab.need((size_t)ks * sizeof(int));
+  const bool stale = h.op_P != P || h.op_layout != layout || h.op_ks != ks || geom_changed;
+  h.op_P = -1;  // until m2l_group_commit() has built what the table now holds
+  if (stale) {
+    h.g_optab.need((size_t)3 * ks * sizeof(int));  // the table, the groups' slots, the new keys
     FMM_CUDA(cudaMemsetAsync(h.g_optab.p, 0xff, (size_t)ks * sizeof(int), s));
     h.op_count = 0;
     h.op_layout = layout;
@@ -1620,14 +1628,11 @@ void m2l_group_launch(Handle &h, long max_groups) {
     h.op_R0 = h.root_R0;
     h.op_depth = h.depth;
   }
-  h.op_P = -1;  // until m2l_group_commit() has built what the table now holds
   const GroupTables gt = group_tables(h.g_occ.p, ks, C);
-  h.g_slot.need((size_t)cap * sizeof(int));
-  h.g_newkeys.need((size_t)cap * sizeof(int));
   DevCounters *ctr = h.counters.as<DevCounters>();
   const unsigned nt = (unsigned)(ks / OCC_TILE);
   k_occ_words<<<nt, 1024, 0, s>>>(gt);
-  k_occ_groups<<<nt, 1024, 0, s>>>(gt, h.g_optab.as<int>(), h.op_count, h.g_slot.as<int>(), h.g_newkeys.as<int>(), cap,
+  k_occ_groups<<<nt, 1024, 0, s>>>(gt, h.g_optab.as<int>(), h.op_count, group_slots(h), new_keys(h), cap,
                                    &ctr->gcounts[2], &ctr->op_new);
   h.g_tk.need((size_t)C * 2 * (sizeof(u64) + sizeof(u32)) + 64);
   u64 *tk = h.g_tk.as<u64>();
@@ -1657,10 +1662,10 @@ void m2l_group_commit(Handle &h) {
     }
     const KeyGeom kg{h.c_xr.as<double4>(), h.op_cycle, h.op_depth};
     if (tcore)
-      k_gops16<<<nnew, 256, NT * sizeof(double2), s>>>(h.g_newkeys.as<int>(), h.op_count, P, tp, h.g_ops.as<__half>(),
+      k_gops16<<<nnew, 256, NT * sizeof(double2), s>>>(new_keys(h), h.op_count, P, tp, h.g_ops.as<__half>(),
                                                         kg);
     else
-      k_gops<<<nnew, 128, NT * sizeof(double2), s>>>(h.g_newkeys.as<int>(), h.op_count, plan_dev(pc),
+      k_gops<<<nnew, 128, NT * sizeof(double2), s>>>(new_keys(h), h.op_count, plan_dev(pc),
                                                       h.g_ops.as<double>(), kg);
     h.launches++;
     FMM_LAUNCH();
@@ -1830,7 +1835,7 @@ void m2l_grouped_pass(Handle &h) {
     int *tg_src = h.g_tg.as<int>(), *tg_gid = tg_src + (size_t)nseg * tile_n, *tg_off = tg_gid + nseg;
     k_fill_rows<<<148 * 4, TB, 0, s>>>(tg_src, &counts[3], tile_n);  // absent targets: -1
     k_gfill<<<grid_for(nent, TB), TB, 0, s>>>(nent, pairs, ekey, gt.mask, tslot, tile_n, ngroups, segid, tg_src);
-    k_seg_gid<<<grid_for(nmark, TB), TB, 0, s>>>(nmark, ngroups, mark, segid, h.g_slot.as<int>(), tg_gid,
+    k_seg_gid<<<grid_for(nmark, TB), TB, 0, s>>>(nmark, ngroups, mark, segid, group_slots(h), tg_gid,
                                                     ntiles, &counts[3], tg_off);
     h.g_ntiles = ntiles;
     h.g_nseg = nseg;  // an upper bound unless it was read
