@@ -32,7 +32,7 @@ namespace fmm {
 
 namespace {
 
-constexpr int PT = 256;  // threads of the periodic CTA
+constexpr int PT = 256;  // threads of the harmonic sums' CTA
 
 // The harmonic sums of the far images, per sublevel l (period cycle * 3^l):
 // H[2l] the irregular harmonics summed over the 702 M2L offsets, H[2l + 1]
@@ -108,31 +108,56 @@ __global__ void __launch_bounds__(PT) k_periodic_harm(int P, int images, double 
 }
 
 // Per evaluation: the root's multipole through the sublevels with the kept
-// harmonic sums -- L_root += M2L(Mp, H[2l]), Mp += M2M(Mp, H[2l + 1]).
-__global__ void __launch_bounds__(PT) k_periodic(const double2 *M, double2 *L, int P, int images, const double2 *H) {
-  extern __shared__ double2 sp[];  // Mp[nt], Mn[nt]
+// harmonic sums -- L_root += M2L(Mp, H[2l]), Mp += M2M(Mp, H[2l + 1]).  One
+// CTA, a chain of images - 1 levels, so latency is all: PS lanes share an
+// output, each taking every PS-th input degree (a lane's chain is about 20
+// products instead of 100 at P = 10), the level's two translations run side
+// by side, and the harmonic sums and the running L are in shared memory
+// (P = 10, three images: 34.9 -> 11.2 us).
+constexpr int PPT = 512, PS = 8;
+
+__global__ void __launch_bounds__(PPT) k_periodic(const double2 *M, double2 *L, int P, int images, const double2 *H) {
+  extern __shared__ double2 sp[];  // Mp[nt], Mn[nt], Lr[nt], H1[nt], H2[nt]
   const int nt = tri(P);
-  double2 *Mp = sp, *Mn = Mp + nt;
-  const int tid = threadIdx.x;
-  for (int o = tid; o < nt; o += PT) Mp[o] = M[o];  // the root is cell 0
-  __syncthreads();
-  for (int level = 0; level < images - 1; level++) {
-    const double2 *H1 = H + (size_t)(2 * level) * nt, *H2 = H1 + nt;
-    for (int o = tid; o < nt; o += PT) {
-      const int j = order_of(o), k = o - tri(j);
-      const double2 v = m2l_coeff(j, k, P, Mp, H1);
-      L[o].x += v.x;
-      L[o].y += v.y;
-    }
-    for (int o = tid; o < nt; o += PT) {
-      const int j = order_of(o), k = o - tri(j);
-      const double2 v = m2m_coeff(j, k, Mp, H2);
-      Mn[o] = make_double2(Mp[o].x + v.x, Mp[o].y + v.y);
-    }
-    __syncthreads();
-    for (int o = tid; o < nt; o += PT) Mp[o] = Mn[o];
-    __syncthreads();
+  double2 *Mp = sp, *Mn = Mp + nt, *Lr = Mn + nt, *H1 = Lr + nt, *H2 = H1 + nt;
+  const int tid = threadIdx.x, sl = tid & (PS - 1);
+  const unsigned grp = 0xffu << (tid & 24);  // the PS lanes of an output
+  for (int o = tid; o < nt; o += PPT) {
+    Mp[o] = M[o];  // the root is cell 0
+    Lr[o] = L[o];
   }
+  for (int level = 0; level < images - 1; level++) {
+    for (int o = tid; o < 2 * nt; o += PPT) H1[o] = H[(size_t)(2 * level) * nt + o];
+    __syncthreads();
+    for (int g = tid / PS; g < 2 * nt; g += PPT / PS) {
+      const bool up = g >= nt;  // outputs of the M2M after those of the M2L
+      const int o = up ? g - nt : g, j = order_of(o), k = o - tri(j);
+      double2 v = make_double2(0, 0);
+      if (up) {
+        for (int n = sl; n <= j; n += PS)
+          m2m_terms_of(j, k, n, [&](int ia, bool ca, int nn, int oo, int f) {
+            const double2 a = cmul(ca ? cconj(Mp[ia]) : Mp[ia], ylook(H2, nn, oo));
+            v.x += a.x * (double)f;
+            v.y += a.y * (double)f;
+          });
+      } else {
+        for (int n = sl; n <= P - 1 - j; n += PS) m2l_add(j, k, n, Mp, H1, v.x, v.y);
+      }
+#pragma unroll
+      for (int s = PS / 2; s > 0; s >>= 1) {
+        v.x += __shfl_xor_sync(grp, v.x, s);
+        v.y += __shfl_xor_sync(grp, v.y, s);
+      }
+      if (sl == 0) {
+        if (up) Mn[o] = make_double2(Mp[o].x + v.x, Mp[o].y + v.y);
+        else Lr[o] = make_double2(Lr[o].x + v.x, Lr[o].y + v.y);
+      }
+    }
+    __syncthreads();
+    for (int o = tid; o < nt; o += PPT) Mp[o] = Mn[o];
+  }
+  __syncthreads();
+  for (int o = tid; o < nt; o += PPT) L[o] = Lr[o];
 }
 
 int periodic_threads(int P) {
@@ -583,7 +608,7 @@ void periodic_pass(Handle &h) {
     k_root_monopole<<<1, 32, 0, h.stream>>>(h.per_part.as<double>(), nblk, h.M.as<double2>());
     h.launches += 2;
   }
-  k_periodic<<<1, PT, (size_t)2 * nt * sizeof(double2), h.stream>>>(h.M.as<double2>(), h.L.as<double2>(), P, images,
+  k_periodic<<<1, PPT, (size_t)5 * nt * sizeof(double2), h.stream>>>(h.M.as<double2>(), h.L.as<double2>(), P, images,
                                                                     h.per_harm.as<double2>());
   h.launches++;
   FMM_LAUNCH();

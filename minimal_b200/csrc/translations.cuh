@@ -29,17 +29,20 @@ __host__ __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : 
 __host__ __device__ __forceinline__ int imax(int a, int b) { return a > b ? a : b; }
 __host__ __device__ __forceinline__ int sgn_hd(int n) { return (n & 1) ? -1 : 1; }
 
-// The terms of one M2M output (j,k), in the reference's order: each is
-// emit(ia, conjugate input?, n, o, sign) for  sign * A[ia]' * Y(n, o), with
-// A the child's multipole and Y(n, o) the offset harmonic (ylook).
+// The terms of one M2M output (j,k) with harmonics of degree n (n <= j), and
+// all of them in the reference's order: each is emit(ia, conjugate input?, n,
+// o, sign) for  sign * A[ia]' * Y(n, o), with A the child's multipole and
+// Y(n, o) the offset harmonic (ylook).
+template <class E>
+__host__ __device__ inline void m2m_terms_of(int j, int k, int n, E emit) {
+  const int lo = imax(-n, -j + k + n), hi = imin(k - 1, n);
+  for (int m = lo; m <= hi; m++) emit(tri(j - n) + k - m, false, n, -m, (m >= 0 ? 1 : sgn_hd(m)) * sgn_hd(n));
+  const int hi2 = imin(n, j + k - n);
+  for (int m = k; m <= hi2; m++) emit(tri(j - n) - k + m, true, n, -m, sgn_hd(k + n + m));
+}
 template <class E>
 __host__ __device__ inline void m2m_terms(int j, int k, E emit) {
-  for (int n = 0; n <= j; n++) {
-    const int lo = imax(-n, -j + k + n), hi = imin(k - 1, n);
-    for (int m = lo; m <= hi; m++) emit(tri(j - n) + k - m, false, n, -m, (m >= 0 ? 1 : sgn_hd(m)) * sgn_hd(n));
-    const int hi2 = imin(n, j + k - n);
-    for (int m = k; m <= hi2; m++) emit(tri(j - n) - k + m, true, n, -m, sgn_hd(k + n + m));
-  }
+  for (int n = 0; n <= j; n++) m2m_terms_of(j, k, n, emit);
 }
 
 // The terms of one L2L output (j,k): A = the parent's local expansion.
@@ -105,20 +108,22 @@ __device__ __forceinline__ double2 apply_terms(const unsigned *t, int nterms, co
 // M2L output (j,k) (3d/kernel.h:233-260) from the source multipole A and the
 // irregular harmonics Z of the offset target - source; only degrees j+n < P
 // contribute, as in the reference (its harmonics table is zero beyond).
+// m2l_add: the inputs of order n alone, added to (sx, sy).
+__device__ inline void m2l_add(int j, int k, int n, const double2 *A, const double2 *Z, double &sx, double &sy) {
+  const int d = j + n;
+  for (int m = -n; m <= n; m++) {
+    const double2 a = m >= 0 ? A[tri(n) + m] : cconj(A[tri(n) - m]);
+    const int om = m - k;
+    const double2 z = om >= 0 ? Z[tri(d) + om] : cconj(Z[tri(d) - om]);
+    const int e2 = m < 0 ? 0 : (m <= k ? m : k);
+    const double f = ((j + e2) & 1) ? -1.0 : 1.0;
+    sx += f * (a.x * z.x - a.y * z.y);
+    sy += f * (a.x * z.y + a.y * z.x);
+  }
+}
 __device__ inline double2 m2l_coeff(int j, int k, int P, const double2 *A, const double2 *Z) {
   double sx = 0, sy = 0;
-  for (int n = 0; n <= P - 1 - j; n++) {
-    const int d = j + n;
-    for (int m = -n; m <= n; m++) {
-      const double2 a = m >= 0 ? A[tri(n) + m] : cconj(A[tri(n) - m]);
-      const int om = m - k;
-      const double2 z = om >= 0 ? Z[tri(d) + om] : cconj(Z[tri(d) - om]);
-      const int e2 = m < 0 ? 0 : (m <= k ? m : k);
-      const double f = ((j + e2) & 1) ? -1.0 : 1.0;
-      sx += f * (a.x * z.x - a.y * z.y);
-      sy += f * (a.x * z.y + a.y * z.x);
-    }
-  }
+  for (int n = 0; n <= P - 1 - j; n++) m2l_add(j, k, n, A, Z, sx, sy);
   return make_double2(sx, sy);
 }
 
