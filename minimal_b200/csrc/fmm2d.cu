@@ -12,12 +12,13 @@
 // is the arithmetic:
 //   P2M, L2P   a few lanes per leaf, the leaf's coefficients in registers;
 //   M2M, L2L   per level, a lane per child cell, coefficients in registers;
-//   M2L        warp per target cell over its ordered M2L list, lane per entry
-//              (2d/kernel.h:61-90; the 2dp image shift :63);
+//   M2L        4 lanes per target cell (16 in small trees) over its ordered
+//              M2L list, lane per entry (2d/kernel.h:61-90; the 2dp image
+//              shift :63);
 // these for orders up to 16, as compile-time constants; above, warps per leaf,
 // threads per coefficient and a warp per M2L entry;
-//   P2P        warp per target leaf over its ordered P2P list, lane per
-//              target body, q log(1/R) and q dX / R^2 (2d/kernel.h:12-31);
+//   P2P        warp per target leaf over its ordered P2P list, the sources
+//              staged, q log(1/R) and q dX / R^2 (2d/kernel.h:12-31);
 //   periodic   one warp: the 72 root M2Ls and the 8-copy M2M per image level
 //              (2dp/traverse_eager.h:46-93).
 #include <type_traits>

@@ -25,12 +25,14 @@
 //              (k_tkeys) and cut into tiles (32 targets for DMMA, 128 for tcgen05); the
 //              (tile, group) pairs that hold entries are marked, scanned into
 //              segment ids and filled with the source cell of every tile slot;
-//   k_gemm64   one CTA (8 warps) per tile: for each group of the tile, the
-//              operator and the 32 gathered scaled multipoles are copied into
-//              shared memory with cp.async (two stages: the next group's
-//              copies run under this group's contraction), accumulated with
-//              FP64 DMMA (mma.m8n8k4) in registers; then the warps' pieces
-//              are reduced, unscaled and stored in L;
+//   k_gemm64   CTAs of 8 warps, each on an equal range of the (tile, group)
+//              segments (or a tile each): per segment the operator and the
+//              32 gathered scaled multipoles are copied into shared memory
+//              with cp.async (two stages: the next group's copies run under
+//              this group's contraction) and accumulated with FP64 DMMA
+//              (mma.m8n8k4) in registers; at a tile's end the warps' pieces
+//              are reduced, unscaled and stored in L (or as parts of a tile
+//              cut by a range boundary, which k_m2l_join adds);
 //   k_m2l_tc   the mixed form's contraction on tcgen05 (below).
 #include <map>
 #include <mutex>
@@ -878,18 +880,18 @@ __global__ void __launch_bounds__(GP_WARPS * 32, MAXP == GP_MAXP_SMALL ? 2 : 1)
   }
 }
 
-// Mixed form on the tensor core: one CTA per tile of 128 targets, warp
-// specialised.  For every group of the tile the operator (B: N = output rows
+// Mixed form on the tensor core: tiles of 128 targets, a CTA per SM on an
+// equal range of their groups (or a tile each above P = 12), warp specialised.  For every group of the tile the operator (B: N = output rows
 // in blocks of 64, K-truncated per block) and the 128 gathered scaled
 // multipoles (A: 128 targets x KP inputs), both as FP16 hi + lo parts in the
 // 128-byte swizzled K-major layout, are staged in shared memory, and one
-// thread issues the three products hi*hi + hi*lo + lo*hi per K step of 16
+// elected lane issues the three products hi*hi + hi*lo + lo*hi per K step of 16
 // (tcgen05.mma kind::f16), accumulating in FP32 in tensor memory.
 //   producer warps: per group, wait for its stage to be free, then one bulk
 //     copy (operator) and 16-byte cp.async copies of the gathered multipole
 //     rows land on the stage's barriers; two stages;
 //   MMA warp: waits for the stage, issues the MMAs, commits the stage back;
-//     two TMEM accumulators alternate every `flush_every` groups;
+//     the TMEM accumulators take turns every `flush_every` groups;
 //   epilogue warps: fold each finished accumulator into a double-FP32
 //     running sum in TMEM (or into L when TMEM has no room) while the tensor
 //     core fills the other, so no FP32 sum runs over more than `flush_every`
