@@ -382,9 +382,10 @@ constexpr size_t tc_smem(const TcPlan &t) { return tc_stages(t) * tc_stage_bytes
 // nacc accumulators of KP columns `stride` apart, used in turn, one per
 // window (the tensor core fills one while the epilogue folds another; with
 // one, the tensor core waits for each fold).  fold = 1: the double-FP32
-// running sum at columns [hi, hi + KP) and [lo, lo + KP); fold = 2: an FP32
-// running sum at [hi, hi + KP) (round-to-nearest adds); fold = 0: windows are
-// added to L in global memory.  ncols is the allocation (a power of two).
+// running sum at columns [hi, hi + KP) and [lo, lo + KP); fold = 3: a paired
+// plan's FP32 running sum at [hi, hi + KP) (round-to-nearest adds); fold = 0:
+// windows are added to L in global memory.  ncols is the allocation (a power
+// of two).
 struct TcAcc {
   int nacc, fold;
   uint32_t stride, hi, lo, ncols;
@@ -408,14 +409,14 @@ constexpr TcAcc tc_acc_layout(int KP) {
   return TcAcc{2, 0, hc, 0, 0, 2 * hc};
 }
 
-// Orders compiled with their plan: three accumulators, so that a fold has
-// two windows' time before the tensor core needs its accumulator again --
-// with the double-FP32 running sum where five fit (KP <= 64), else (KP <=
-// 128) with an FP32 running sum.  The window sums carry the tensor core's
-// truncating FP32 accumulation, which the short window bounds; the running
-// sum's round-to-nearest adds are unbiased, ~sqrt(windows) * 2^-24 relative
-// (about 6e-7 over the ~95 windows of a tile at P = 10, far below the
-// expansion's error).  Otherwise the layout above.
+// Orders compiled with their plan: three accumulators and the double-FP32
+// running sum where five fit (KP <= 64), so that a fold has two windows' time
+// before the tensor core needs its accumulator again; with a paired block (P
+// = 8 and 10) two and an FP32 running sum.  The window sums carry the tensor
+// core's truncating FP32 accumulation, which the short window bounds; the
+// running sum's round-to-nearest adds are unbiased, ~sqrt(windows) * 2^-24
+// relative (about 6e-7 over the ~95 windows of a tile at P = 10, far below
+// the expansion's error).  Otherwise the layout above.
 constexpr TcAcc tc_acc_fixed(int KP, const TcPlan &t) {
   if (t.pair[0]) {  // two accumulators of the paired width (64-column steps) and an FP32 running sum
     const uint32_t st = ((uint32_t)t.accw + 63u) / 64u * 64u;
@@ -423,15 +424,17 @@ constexpr TcAcc tc_acc_fixed(int KP, const TcPlan &t) {
   }
   const uint32_t hc = tc_half_cols(KP);
   if (5 * hc <= 512) return TcAcc{3, 1, hc, 3 * hc, 4 * hc, 5 * hc <= 256 ? 256u : 512u};
-  if (4 * hc <= 512) return TcAcc{3, 2, hc, 3 * hc, 0, 512};
   return tc_acc_layout(KP);
 }
 
-// The orders compiled with their plan as constants (6, 8, 10 and 12, the
-// switch in contract()): the MMA issue loop and the producers' copy loop
-// unroll with immediate offsets, so the issuing thread and the producers
-// spend fewer instructions per segment.  Other orders take the plan at run
+// The orders compiled with their plan as constants (4 to 12, the switch in
+// with_tc_order()): the MMA issue loop and the producers' copy loop unroll with
+// immediate offsets, so the issuing warp and the producers spend fewer
+// instructions per segment (600,000 uniform bodies, an evaluation with the
+// plan at run time against this: 1.62 -> 1.51 ms at
+// P = 4, 1.78 -> 1.65 at 7, 2.00 -> 1.83 at 9, 2.79 -> 2.40 at 11).  Other orders take the plan at run
 // time.
+constexpr int TC_FIXED_MIN = 4, TC_FIXED_MAX = 12;
 template <int PT>
 struct TcFixed {
   static constexpr int KP = tc_kp(PT);
@@ -924,21 +927,8 @@ __device__ __forceinline__ void tc_fold(uint32_t acc, uint32_t hi, uint32_t lo, 
   tc::wait_st();
 }
 
-// tc_fold with an FP32 running sum (round-to-nearest adds, no error term).
-__device__ __forceinline__ void tc_fold32(uint32_t acc, uint32_t hi, int cb, int ce) {
-  for (int c0 = cb; c0 < ce; c0 += 16) {
-    uint32_t a[16], h[16];
-    tc::ld_32x32b_x16_async(acc + (uint32_t)c0, a);
-    tc::ld_32x32b_x16_async(hi + (uint32_t)c0, h);
-    tc::wait_ld();
-#pragma unroll
-    for (int k = 0; k < 16; k++) h[k] = __float_as_uint(__uint_as_float(h[k]) + __uint_as_float(a[k]));
-    tc::st_32x32b_x16(hi + (uint32_t)c0, h);
-  }
-  tc::wait_st();
-}
-
-// tc_fold32 for a plan with paired blocks: output column c of block b is
+// tc_fold for a plan with paired blocks, with an FP32 running sum (round-to-
+// nearest adds, no error term): output column c of block b is
 // the sum of accumulator columns dcol[b] + w and, paired, dcol[b] + rows[b]
 // + w (w = c - 64 b).
 __device__ __forceinline__ void tc_fold_paired(uint32_t acc, uint32_t sum, const TcPlan &pl, int KP) {
@@ -1134,7 +1124,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
         tc::fence_after();
         const uint32_t acc = lanes + (uint32_t)a * ta.stride;
         if (fold == 1) tc_fold(acc, sum_hi, sum_lo, 0, KP);
-        else if (fold == 2) tc_fold32(acc, sum_hi, 0, KP);
         else if (fold == 3) tc_fold_paired(acc, sum_hi, pl, KP);
         else tc_flush_global(acc, t, inv, us, 0, KP, NT, L);
         tc::fence_before();
@@ -1497,14 +1486,33 @@ bool m2l_grouped_available(int P) {
   return pc.host.P == P && gemm64_smem(pc.host) <= 200 * 1024;
 }
 
+// f(the kernel of order P)
+template <class F>
+void with_tc_order(int P, F f) {
+  switch (P) {
+    case 4: return f(k_m2l_tc<4>);
+    case 5: return f(k_m2l_tc<5>);
+    case 6: return f(k_m2l_tc<6>);
+    case 7: return f(k_m2l_tc<7>);
+    case 8: return f(k_m2l_tc<8>);
+    case 9: return f(k_m2l_tc<9>);
+    case 10: return f(k_m2l_tc<10>);
+    case 11: return f(k_m2l_tc<11>);
+    case 12: return f(k_m2l_tc<12>);
+    default: return f(k_m2l_tc<0>);
+  }
+}
+
 void m2l_grouped_set_attributes() {
   cudaFuncSetAttribute(k_gemm64<GP_MAXP_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
   cudaFuncSetAttribute(k_gemm64<GP_MAXP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
-  cudaFuncSetAttribute(k_m2l_tc<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
-  cudaFuncSetAttribute(k_m2l_tc<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
-  cudaFuncSetAttribute(k_m2l_tc<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
-  cudaFuncSetAttribute(k_m2l_tc<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
-  cudaFuncSetAttribute(k_m2l_tc<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
+  with_tc_order(0, [](auto kern) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
+  });
+  for (int P = TC_FIXED_MIN; P <= TC_FIXED_MAX; P++)
+    with_tc_order(P, [](auto kern) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
+    });
 }
 
 // Grouped M2L of the whole tree: L stored for every cell (zero where no
@@ -1521,10 +1529,9 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
   DevCounters *ctr = h.counters.as<DevCounters>();
   if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   if (tcore) {
-    // orders with a running sum in TMEM (6, 8, 10 and 12, compiled with their
-    // plan, and the others up to 12) take balanced segment ranges, one CTA
-    // per SM
-    const bool fixed = P == 6 || P == 8 || P == 10 || P == 12;
+    // orders with a running sum in TMEM (up to 12) take balanced segment
+    // ranges, one CTA per SM
+    const bool fixed = P >= TC_FIXED_MIN && P <= TC_FIXED_MAX;
     const bool bal = (fixed ? tc_acc_fixed(KP16, tp) : tc_acc_layout(KP16)).fold != 0;
     const int G = bal ? h.nsm : ntiles, NT = tri(P);
     if (bal) h.g_part.need((size_t)G * 2 * TC_TILE * NT * sizeof(double2));
@@ -1535,13 +1542,7 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
                                               tp, tc_stages(tp), tc_acc_layout(KP16), m2l_flush_interval(h),
                                               &ctr->m16_max, h.flags_host, TC_WAIT_NS, h.tc_stall_ns, ntiles, part);
     };
-    switch (P) {
-      case 6: launch(k_m2l_tc<6>); break;
-      case 8: launch(k_m2l_tc<8>); break;
-      case 10: launch(k_m2l_tc<10>); break;
-      case 12: launch(k_m2l_tc<12>); break;
-      default: launch(k_m2l_tc<0>);
-    }
+    with_tc_order(P, launch);
     if (bal) {
       k_m2l_join<<<join_grid(ntiles, h.nsm, TC_TILE * NT), JOIN_T, 0, s>>>(h.g_tile.as<int>(), tg_off, ntiles, G, part,
                                                                           NT, TC_TILE, h.L.as<double2>());

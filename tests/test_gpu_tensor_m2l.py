@@ -1,6 +1,6 @@
 """The tensor-core M2L's operand copies at every order: a multipole row is
 KP / 4 chunks of 16 bytes (KP from 16 to 192) that a warp's lanes take in
-sequence across rows, with the pattern compiled in (orders 6, 8, 10, 12) or
+sequence across rows, with the pattern compiled in (orders 4 to 12) or
 counted; ranges of fewer groups than a batch of indices, and of no multiple
 of it.  Against the oracle within 1e-5 (split-FP16 products and FP32 pairs
 carry about 2^-22, the cancellation of neutral charges a factor of ten or so
