@@ -1308,6 +1308,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
                         tc::mbar_wait(&full[st], ph, wait_ns, abort) && tc::mbar_wait(&bful[st], ph, wait_ns, abort) &&
                             (!reuse || tc::mbar_wait(&acce[a], pa, wait_ns, abort)));
       if (!ok) break;
+      // the producers' cp.async wrote the rows through the generic proxy, the
+      // tensor core reads them through the async proxy: the barrier orders
+      // the two only with this proxy fence between the wait and the MMAs
+      tc::fence_async_smem();
       tc::fence_after();
       const uint32_t sA = tc::smem_u32(base + (size_t)st * stage_bytes), sB = sA + 2 * abytes;
       const uint64_t dA = tc::smem_desc_sw128(sA), dB = tc::smem_desc_sw128(sB), dB32 = tc::smem_desc_sw32(sB);
