@@ -531,16 +531,18 @@ __device__ __forceinline__ int m16_exponent(unsigned long long bits) {
 }
 
 // Largest |real or imaginary part| of the scaled multipoles M_n / R^n over
-// the cells that can be M2L sources (every level but the roots'), into
-// *mx as double bits (non-negative doubles order like their bit patterns).
-__global__ void k_m16_max(int ncells, int P, const double4 *xr, const int *level, const double2 *M,
+// the cells that can be M2L sources, into *mx as double bits (non-negative
+// doubles order like their bit patterns): levels from `lowest` on -- 1 without
+// images, where a root meets only its own cells, 0 with them, where the root's
+// image is a source of the cells on the box's far side.
+__global__ void k_m16_max(int ncells, int P, const double4 *xr, const int *level, int lowest, const double2 *M,
                           unsigned long long *mx) {
   const int NT = tri(P);
   double v = 0.0;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < (long)ncells * NT;
        i += (long)gridDim.x * blockDim.x) {
     const int c = (int)(i / NT), ci = (int)(i - (long)c * NT);
-    if (level[c] == 0) continue;
+    if (level[c] < lowest) continue;
     const double2 m = M[i];
     const double s = mscale_factor(ci, xr[c].w);
     v = fmax(v, fmax(fabs(m.x), fabs(m.y)) * s);
@@ -1703,7 +1705,7 @@ void m2l_grouped_pass(Handle &h) {
     u64 *m16_max = &h.counters.as<DevCounters>()->m16_max;
     FMM_CUDA(cudaMemsetAsync(m16_max, 0, sizeof(u64), s));
     k_m16_max<<<std::min<long>(grid_for((long)C * NT, TB), 148 * 8), TB, 0, s>>>(
-        C, P, h.c_xr.as<double4>(), h.c_level.as<int>(), h.M.as<double2>(), m16_max);
+        C, P, h.c_xr.as<double4>(), h.c_level.as<int>(), h.prm.images > 0 ? 0 : 1, h.M.as<double2>(), m16_max);
     k_mscale16<<<grid_for((long)C * (KP16 / 2), TB), TB, 0, s>>>(C, P, KP16, h.c_xr.as<double4>(),
                                                                  h.M.as<double2>(), m16_max, h.g_m16.as<__half2>());
     h.launches++;
