@@ -172,6 +172,7 @@ struct Handle {
   long op_ks = 0;
   double op_cycle = 0, op_R0 = 0;  // image-key operators: the geometry they were built for
   int op_depth = -1;
+  double op_theta = 0;  // tensor-core operators: the acceptance test their scaling is for (TcScale)
   bool g_grouped = false;  // the group tables belong to the current lists
   int g_ntiles = 0, g_ngroups = 0, g_nseg = 0;
   bool g_used_tc = false;

@@ -445,7 +445,7 @@ struct TcFixed {
 
 // One CTA per group: the operator split into FP16 hi + lo parts, written as
 // the byte image the MMA reads from shared memory (hi image, then lo image).
-__global__ void k_gops16(const int *keys, int slot0, int P, TcPlan pl, __half *ops16, KeyGeom kg) {
+__global__ void k_gops16(const int *keys, int slot0, int P, TcPlan pl, __half *ops16, KeyGeom kg, TcScale sc) {
   extern __shared__ double2 Zsh[];
   const int NT = tri(P);
   const int dl = group_harmonics(keys[blockIdx.x], P, Zsh, kg);
@@ -477,7 +477,9 @@ __global__ void k_gops16(const int *keys, int slot0, int P, TcPlan pl, __half *o
       k = a * 64 + ((chunk ^ (rb & 7)) << 3) + q;
       ph = pl.boff[b] + a * pl.astride[b] + r2;
     }
-    const double w = k < 16 * pl.ksteps[b] ? op_value(64 * b + rb, k, P, NT, dl, Zsh) : 0.0;
+    const int row = 64 * b + rb;
+    double w = k < 16 * pl.ksteps[b] ? op_value(row, k, P, NT, dl, Zsh) : 0.0;
+    if (sc.any && row < 2 * NT && k < 2 * NT) w /= sc.in[order_of(k >> 1)] * sc.out[order_of(row >> 1)];
     const __half hi = __double2half(w);
     Wh[ph / 2] = hi;
     Wh[(ph + pl.lodelta[b]) / 2] = __double2half(w - (double)__half2float(hi));
@@ -506,8 +508,9 @@ __global__ void k_mscale(int ncells, int P, int KP, const double4 *xr, const dou
   Mt[i] = mscaled(c, k, tri(P), xr, M);
 }
 
-// Degree n of coefficient index ci (tri(n) <= ci < tri(n + 1)) and 1 / R^n.
-__device__ __forceinline__ double mscale_factor(int ci, double R) {
+// Scale of coefficient index ci, of degree n (tri(n) <= ci < tri(n + 1)):
+// 2^in[n] / R^n.
+__device__ __forceinline__ double mscale_factor(int ci, double R, const TcScale &sc) {
   int n = (int)((sqrtf(8.0f * ci + 1.0f) - 1.0f) * 0.5f);
   while (tri(n) > ci) n--;
   while (tri(n + 1) <= ci) n++;
@@ -515,7 +518,7 @@ __device__ __forceinline__ double mscale_factor(int ci, double R) {
   double s = 1, b = inv;  // inv^n
   for (int e = n; e; e >>= 1, b *= b)
     if (e & 1) s *= b;
-  return s;
+  return s * sc.in[n];
 }
 
 // Power-of-two exponent E of the FP16 split: the largest scaled multipole
@@ -530,13 +533,13 @@ __device__ __forceinline__ int m16_exponent(unsigned long long bits) {
   return e < -500 ? -500 : (e > 500 ? 500 : e);
 }
 
-// Largest |real or imaginary part| of the scaled multipoles M_n / R^n over
+// Largest |real or imaginary part| of the scaled multipoles over
 // the cells that can be M2L sources, into *mx as double bits (non-negative
 // doubles order like their bit patterns): levels from `lowest` on -- 1 without
 // images, where a root meets only its own cells, 0 with them, where the root's
 // image is a source of the cells on the box's far side.
 __global__ void k_m16_max(int ncells, int P, const double4 *xr, const int *level, int lowest, const double2 *M,
-                          unsigned long long *mx) {
+                          unsigned long long *mx, TcScale sc) {
   const int NT = tri(P);
   double v = 0.0;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < (long)ncells * NT;
@@ -544,7 +547,7 @@ __global__ void k_m16_max(int ncells, int P, const double4 *xr, const int *level
     const int c = (int)(i / NT), ci = (int)(i - (long)c * NT);
     if (level[c] < lowest) continue;
     const double2 m = M[i];
-    const double s = mscale_factor(ci, xr[c].w);
+    const double s = mscale_factor(ci, xr[c].w, sc);
     v = fmax(v, fmax(fabs(m.x), fabs(m.y)) * s);
   }
   for (int o = 16; o; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -562,7 +565,7 @@ __global__ void k_m16_max(int ncells, int P, const double4 *xr, const int *level
 // directly; one thread per coefficient (n, m) writes its real and imaginary
 // parts.
 __global__ void k_mscale16(int ncells, int P, int KP, const double4 *xr, const double2 *M,
-                           const unsigned long long *mx, __half2 *M16) {
+                           const unsigned long long *mx, __half2 *M16, TcScale sc) {
   const int half_kp = KP / 2;
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long)ncells * half_kp) return;
@@ -570,7 +573,7 @@ __global__ void k_mscale16(int ncells, int P, int KP, const double4 *xr, const d
   const int ci = (int)(i - c * half_kp), NT = tri(P);
   double2 v = make_double2(0, 0);
   if (ci < NT) {
-    const double s = scalbn(mscale_factor(ci, xr[c].w), m16_exponent(*mx));
+    const double s = scalbn(mscale_factor(ci, xr[c].w, sc), m16_exponent(*mx));
     const double2 m = M[c * NT + ci];
     v = make_double2(m.x * s, m.y * s);
   }
@@ -607,7 +610,7 @@ constexpr int GH_WARPS = 8;
 __global__ void __launch_bounds__(GH_WARPS * 32) k_ghost16(int nghost, const int *gslots, const double4 *xr,
                                                            const double2 *M, const double2 *Yh, int nlev, int P,
                                                            int KP, const unsigned long long *mx, int ncells,
-                                                           __half2 *M16) {
+                                                           __half2 *M16, TcScale scale) {
   extern __shared__ double2 gsh[];  // per warp: the source multipole
   const int NT = tri(P), wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = blockIdx.x * GH_WARPS + wp;
@@ -629,7 +632,7 @@ __global__ void __launch_bounds__(GH_WARPS * 32) k_ghost16(int nghost, const int
     if (ci < NT) {
       const int j = order_of(ci), k = ci - tri(j);
       const double2 mm = m2m_coeff(j, k, Msh, Ysh);
-      const double sc = mscale_factor(ci, Y.w) * E;
+      const double sc = mscale_factor(ci, Y.w, scale) * E;
       v = make_double2(mm.x * sc, mm.y * sc);
     }
     const __half hx = __double2half(v.x), hy = __double2half(v.y);
@@ -1423,6 +1426,18 @@ __global__ void __launch_bounds__(JOIN_T) k_m2l_join(const int *tile_tgt, const 
   }
 }
 
+// Local expansions made from scaled operators: the outputs of degree j times
+// 2^out[j] (rows without a grouped entry are zero).
+__global__ void k_l_unscale(long n, int NT, TcScale sc, double2 *L) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double f = sc.out[order_of((int)(i % NT))];
+  if (f != 1.0) {
+    const double2 l = L[i];
+    L[i] = make_double2(l.x * f, l.y * f);
+  }
+}
+
 // k_m2l_join's grid: about two CTAs per SM in all, at most one per JOIN_T
 // elements of a tile.
 dim3 join_grid(int ntiles, int nsm, int elems) {
@@ -1480,7 +1495,13 @@ size_t gemm64_smem(const GroupPlan &g, int nstage = 1) {
 
 bool tc_available(int P) {
   const int KP = tc_kp(P);
-  return KP <= 256 && tc_smem(make_tc_plan(P, KP, tc_pair_first(P))) <= TC_SMEM_MAX;
+  return KP <= 256 && P <= TC_MAX_P && tc_smem(make_tc_plan(P, KP, tc_pair_first(P))) <= TC_SMEM_MAX;
+}
+
+// The scaling of the handle's tensor-core operators.  Different cells of one
+// tree are at least sqrt(3) finer radii apart (a cell inside a coarser one).
+TcScale tc_scale(const Handle &h) {
+  return make_tc_scale(h.prm.P, h.prm.theta, -KEY_DL, KEY_DL - 1, h.prm.images > 0 ? 0.0 : 1.7);
 }
 
 }  // namespace
@@ -1527,7 +1548,8 @@ void m2l_grouped_set_attributes() {
 // 128 targets (orders whose operator does not fit fall back to DMMA).
 // The contraction over the grouping held in the handle (tiles, segment
 // tables, operator slots) with this evaluation's scaled multipoles.
-void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan &gp, const PlanDev &pd) {
+void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan &gp, const PlanDev &pd,
+              const TcScale &sc) {
   cudaStream_t s = h.stream;
   const int P = h.prm.P, ntiles = h.g_ntiles, tile_n = tcore ? TC_TILE : GP_TILE;
   const long nseg = h.g_nseg;
@@ -1552,6 +1574,11 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
     if (bal) {
       k_m2l_join<<<join_grid(ntiles, h.nsm, TC_TILE * NT), JOIN_T, 0, s>>>(h.g_tile.as<int>(), tg_off, ntiles, G, part,
                                                                           NT, TC_TILE, h.L.as<double2>());
+      h.launches++;
+    }
+    if (sc.any) {
+      const long n = (long)h.ncells * NT;
+      k_l_unscale<<<grid_for(n, TB), TB, 0, s>>>(n, NT, sc, h.L.as<double2>());
       h.launches++;
     }
     h.tc_stall_ns = 0;  // the test hook stalls one launch
@@ -1625,7 +1652,8 @@ void m2l_group_launch(Handle &h, long max_groups) {
   // also depend on the period, the root radius and the depth
   const bool geom_changed =
       h.prm.images > 0 && (h.op_cycle != cyc || h.op_R0 != h.root_R0 || h.op_depth != h.depth);
-  const bool stale = h.op_P != P || h.op_layout != layout || h.op_ks != ks || geom_changed;
+  const bool stale = h.op_P != P || h.op_layout != layout || h.op_ks != ks || geom_changed ||
+                     (layout == 1 && h.op_theta != h.prm.theta);
   h.op_P = -1;  // until m2l_group_commit() has built what the table now holds
   if (stale) {
     h.g_optab.need((size_t)3 * ks * sizeof(int));  // the table, the groups' slots, the new keys
@@ -1636,6 +1664,7 @@ void m2l_group_launch(Handle &h, long max_groups) {
     h.op_cycle = cyc;
     h.op_R0 = h.root_R0;
     h.op_depth = h.depth;
+    h.op_theta = h.prm.theta;
   }
   const GroupTables gt = group_tables(h.g_occ.p, ks, C);
   DevCounters *ctr = h.counters.as<DevCounters>();
@@ -1672,7 +1701,7 @@ void m2l_group_commit(Handle &h) {
     const KeyGeom kg{h.c_xr.as<double4>(), h.op_cycle, h.op_depth};
     if (tcore)
       k_gops16<<<nnew, 256, NT * sizeof(double2), s>>>(new_keys(h), h.op_count, P, tp, h.g_ops.as<__half>(),
-                                                        kg);
+                                                        kg, tc_scale(h));
     else
       k_gops<<<nnew, 128, NT * sizeof(double2), s>>>(new_keys(h), h.op_count, plan_dev(pc),
                                                       h.g_ops.as<double>(), kg);
@@ -1693,6 +1722,7 @@ void m2l_grouped_pass(Handle &h) {
   const int KP16 = tc_kp(P);
   const TcPlan tp = make_tc_plan(P, KP16, tc_pair_first(P));
   const int tile_n = tcore ? TC_TILE : GP_TILE;
+  const TcScale sc = tcore ? tc_scale(h) : TcScale{};
   const long nent = h.n_m2l;
   h.L.need((size_t)C * NT * sizeof(double2));
   FMM_CUDA(cudaMemsetAsync(h.L.p, 0, (size_t)C * NT * sizeof(double2), s));
@@ -1705,9 +1735,9 @@ void m2l_grouped_pass(Handle &h) {
     u64 *m16_max = &h.counters.as<DevCounters>()->m16_max;
     FMM_CUDA(cudaMemsetAsync(m16_max, 0, sizeof(u64), s));
     k_m16_max<<<std::min<long>(grid_for((long)C * NT, TB), 148 * 8), TB, 0, s>>>(
-        C, P, h.c_xr.as<double4>(), h.c_level.as<int>(), h.prm.images > 0 ? 0 : 1, h.M.as<double2>(), m16_max);
+        C, P, h.c_xr.as<double4>(), h.c_level.as<int>(), h.prm.images > 0 ? 0 : 1, h.M.as<double2>(), m16_max, sc);
     k_mscale16<<<grid_for((long)C * (KP16 / 2), TB), TB, 0, s>>>(C, P, KP16, h.c_xr.as<double4>(),
-                                                                 h.M.as<double2>(), m16_max, h.g_m16.as<__half2>());
+                                                                 h.M.as<double2>(), m16_max, h.g_m16.as<__half2>(), sc);
     h.launches++;
   } else {
     h.g_mt.need((size_t)C * gp.KP * sizeof(double));
@@ -1725,7 +1755,7 @@ void m2l_grouped_pass(Handle &h) {
       k_mscale16<<<grid_for((long)C * (KP16 / 2), TB), TB, 0, s>>>(C, P, KP16, h.c_xr.as<double4>(),
                                                                    h.M.as<double2>(),
                                                                    &h.counters.as<DevCounters>()->m16_max,
-                                                                   h.g_m16.as<__half2>());
+                                                                   h.g_m16.as<__half2>(), sc);
       h.launches++;
     }
     const long nsl = (long)C * GHOST_SLOTS;
@@ -1736,14 +1766,14 @@ void m2l_grouped_pass(Handle &h) {
     k_ghost_harm<<<26 * nlev, 32, 0, s>>>(nlev, h.c_xr.as<double4>(), P, cyc, h.g_gharm.as<double2>());
     k_ghost16<<<(h.g_nghost + GH_WARPS - 1) / GH_WARPS, GH_WARPS * 32, GH_WARPS * NT * sizeof(double2), s>>>(
         h.g_nghost, h.g_gmark.as<int>() + 2 * nsl, h.c_xr.as<double4>(), h.M.as<double2>(), h.g_gharm.as<double2>(),
-        nlev, P, KP16, &h.counters.as<DevCounters>()->m16_max, C, h.g_m16.as<__half2>());
+        nlev, P, KP16, &h.counters.as<DevCounters>()->m16_max, C, h.g_m16.as<__half2>(), sc);
     h.launches += 2;
     FMM_LAUNCH();
   };
   // same lists, P and form as the last grouping: contract directly
   if (h.g_plan.valid && h.g_plan.P == P && h.g_plan.tcore == tcore && h.g_plan.ordered == h.m2l_ordered) {
     ghost_rows();
-    if (h.g_ngroups > 0) contract(h, tcore, tp, KP16, gp, pd);
+    if (h.g_ngroups > 0) contract(h, tcore, tp, KP16, gp, pd, sc);
     h.launches++;
     FMM_LAUNCH();
     if (h.g_plan.nres > 0) m2l_residual(h, h.m2l_ordered ? h.g_ekey.as<int>() : h.m2l_key.as<int>());
@@ -1849,7 +1879,7 @@ void m2l_grouped_pass(Handle &h) {
     h.g_ntiles = ntiles;
     h.g_nseg = nseg;  // an upper bound unless it was read
     ghost_rows();
-    contract(h, tcore, tp, KP16, gp, pd);
+    contract(h, tcore, tp, KP16, gp, pd, sc);
     h.launches += 10;
     FMM_LAUNCH();
   }

@@ -17,6 +17,8 @@
 // it: fewer accumulator registers, so two CTAs share an SM.
 #pragma once
 #include <algorithm>
+#include <cmath>
+#include <cstdlib>
 #include <vector>
 
 namespace fmm {
@@ -98,6 +100,65 @@ inline GroupPlan make_group_plan(int P) {
     return g;
   }
   return GroupPlan{};
+}
+
+// Powers of two that keep the FP16 operators of the tensor-core form inside
+// FP16's range (65504).  An operator entry of output degree j and input degree
+// n (d = j + n) is at most
+//   c (2d-1)!! S^n T^(j+1) / |v|^(d+1),   c = 1 for n = 0, else 2,
+// with S, T the radii of source and target and |v| their distance in units of
+// the finer radius, and the acceptance test gives |v| > (S + T) / theta.  At
+// large orders that exceeds the range: at theta = 0.5 from P = 11 on between
+// cells four levels apart (1.5e5; 1.5e6 at P = 12), at 0.4 from P = 12.  The
+// inputs of degree n are therefore multiplied by 2^in[n], the operators by
+// 2^-(in[n] + out[j]) and the outputs of degree j by 2^out[j], exactly.  Where
+// the bound stays below 2^15 every exponent is 0 (P <= 10 at theta <= 0.5).
+// Pairs of one level need the same for every n + j = d and get exponents that
+// grow with the degree; a finer or coarser source needs them at the highest
+// n or j alone, so the low degrees, which carry the result, keep theirs.
+constexpr int TC_MAX_P = 16;
+struct TcScale {
+  double in[TC_MAX_P], out[TC_MAX_P];  // 2^in, 2^out
+  bool any;                            // some factor is not 1
+};
+
+// dl_lo, dl_hi: the level differences (target - source) that have group keys.
+// near: a lower bound of |v| between different cells, whatever theta (0: none,
+// for the shifted images of a periodic system).  Beyond theta = 4 or so, where
+// nothing converges, exponents are cut at 400.
+inline TcScale make_tc_scale(int P, double theta, int dl_lo, int dl_hi, double near) {
+  int in[TC_MAX_P] = {0}, out[TC_MAX_P] = {0};
+  P = std::min(P, TC_MAX_P);
+  double lf[TC_MAX_P];  // log2((2d-1)!!)
+  lf[0] = 0;
+  for (int d = 1; d < TC_MAX_P; d++) lf[d] = lf[d - 1] + std::log2(2.0 * d - 1);
+  // log2 of the smallest |v| of a level difference
+  auto dist = [&](int dl) { return std::log2(std::max((1 + std::ldexp(1.0, std::abs(dl))) / theta, near)); };
+  // bits by which the entries' bound exceeds 2^15
+  auto over = [&](int n, int j, int dl, double lv) {
+    const double b = lf[n + j] + (n > 0) + (dl >= 0 ? dl * n : -dl * (j + 1)) - (n + j + 1) * lv;
+    return std::max(0, (int)std::ceil(std::min(b - 15, 400.0)));
+  };
+  double slope = 0, lv = dist(0);
+  for (int d = 1; d < P; d++) slope = std::max(slope, (double)over(d, 0, 0, lv) / d);
+  for (int n = 0; n < P; n++) in[n] = out[n] = (int)std::ceil(slope * n);
+  for (int dl = 1; dl <= dl_hi; dl++) {
+    lv = dist(dl);
+    for (int n = 0; n < P; n++)
+      for (int j = 0; j < P - n; j++) in[n] = std::max(in[n], over(n, j, dl, lv) - out[j]);
+  }
+  for (int dl = -1; dl >= dl_lo; dl--) {
+    lv = dist(dl);
+    for (int j = 0; j < P; j++)
+      for (int n = 0; n < P - j; n++) out[j] = std::max(out[j], over(n, j, dl, lv) - in[n]);
+  }
+  TcScale s{};
+  for (int n = 0; n < TC_MAX_P; n++) {
+    s.in[n] = std::ldexp(1.0, in[n]);
+    s.out[n] = std::ldexp(1.0, out[n]);
+    s.any = s.any || in[n] != 0 || out[n] != 0;
+  }
+  return s;
 }
 
 }  // namespace fmm
