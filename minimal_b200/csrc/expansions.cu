@@ -1004,8 +1004,8 @@ void ob_level(Handle &h, int np, F launch) {
 void upward_pass(Handle &h, cudaStream_t s) {
   if (h.prm.dim == 2) return upward_pass_2d(h, s);
   const int P = h.prm.P, nt = tri(P);
-  h.M.need((size_t)h.ncells * nt * sizeof(double2));
-  h.L.need((size_t)h.ncells * nt * sizeof(double2));
+  const size_t expansions = (size_t)h.ncells * nt * sizeof(double2);
+  h.exp_mem.need({{&h.M, expansions}, {&h.L, expansions}});
   const bool mixed = h.prm.precision == EXAFMM_MIXED;
   if (mixed) {
     if (s != h.stream && !h.srcf_ready) throw Error{EXAFMM_ERR_STATE, "upward pass on a side stream before its sources"};

@@ -4,7 +4,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <functional>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -36,28 +38,77 @@ struct Error {
                                               __FILE__ + ":" + std::to_string(__LINE__)};                  \
   } while (0)
 
-// A device allocation that grows on demand and is kept between evaluations.
+// A device allocation that grows on demand and is kept between evaluations,
+// or a piece of a Slab.
 struct Buf {
   void *p = nullptr;
   size_t bytes = 0;
+  bool piece = false;  // p belongs to a Slab
   template <class T>
   T *as() const { return (T *)p; }
   void need(size_t b) {
     if (b <= bytes) return;
-    if (p) cudaFree(p);
-    p = nullptr;
-    bytes = 0;
-    size_t nb = b + b / 4 + 256;
+    release();
+    allocate(b + b / 4 + 256);
+  }
+  void allocate(size_t nb) {  // exactly nb bytes, into an empty Buf
     if (cudaMalloc(&p, nb) != cudaSuccess) {
       cudaGetLastError();
+      p = nullptr;
       throw Error{EXAFMM_ERR_NOMEM, "cudaMalloc of " + std::to_string(nb) + " bytes failed"};
     }
     bytes = nb;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p && !piece) cudaFree(p);
     p = nullptr;
     bytes = 0;
+    piece = false;
+  }
+};
+
+// One allocation for buffers of one life, which grow together: an allocation
+// that the CUDA allocator cannot serve from memory it has mapped costs 0.35 ms
+// (tens of ms on a busy host), and the first evaluation of a handle made ten.
+struct Slab {
+  Buf mem;
+  struct Part {
+    Buf *buf;
+    size_t bytes;
+  };
+  // Every part with room for its bytes; where one has not, all of them are
+  // allocated anew and lose their contents (true).
+  bool need(std::initializer_list<Part> parts) {
+    bool fits = true;
+    size_t total = 0;
+    for (const Part &q : parts) {
+      fits = fits && q.bytes <= q.buf->bytes;
+      total += room(q);
+    }
+    if (fits) return false;
+    size_t size[32];
+    int k = 0;
+    for (const Part &q : parts) size[k++] = room(q);
+    for (const Part &q : parts) q.buf->release();
+    mem.release();
+    mem.allocate(total);
+    char *at = (char *)mem.p;
+    k = 0;
+    for (const Part &q : parts) {
+      q.buf->p = at;
+      q.buf->bytes = size[k];
+      q.buf->piece = true;
+      at += size[k++];
+    }
+    return true;
+  }
+
+ private:
+  // a part that is large enough keeps its size, another gets a quarter more
+  // than it asks for; whole multiples of 256 bytes
+  static size_t room(const Part &q) {
+    const size_t b = q.bytes <= q.buf->bytes ? q.buf->bytes : q.bytes + q.bytes / 4;
+    return (b + 255) / 256 * 256;
   }
 };
 
@@ -112,6 +163,7 @@ struct Handle {
   Buf sys_off;                        // long long [nsys + 1] (device)
   std::vector<int64_t> sys_off_host;
   Buf in;      // double4 (x,y,z,q), caller order
+  Slab body_mem;  // the arrays by body that a tree build makes: sort buffers, src, out and the like
   Buf src;     // double4 (x,y,z,q), tree order
   Buf out;     // double4 (p,Fx,Fy,Fz), tree order
   Buf perm;    // int, tree position -> input index
@@ -130,6 +182,7 @@ struct Handle {
   // tree (BFS order: by level, then first body)
   int ncells = 0, nleaves = 0, depth = 0;
   int level_base[EXAFMM_MAX_LEVEL + 3] = {0};
+  Slab cell_mem;  // the tables by cell (c_*, leaves, pre_tmp, ctmp)
   Buf c_begin, c_count, c_child, c_nchild, c_parent, c_level, c_xr, c_pre, c_ref, c_leaf_of_body;
   Buf c_face;  // which faces of the root a cell's parent touches (k_cells)
   Buf leaves;  // BFS indices of leaves
@@ -141,6 +194,9 @@ struct Handle {
   double root_R0 = 0;  // radius of the root cell (one system)
 
   // lists (CSR by target, BFS indices)
+  // what a list build makes, the raw and ordered lists and the group tables,
+  // and the operator table
+  Slab list_mem;
   Buf frontier[2];
   size_t frontier_cap = 0;
   Buf m2l_raw, p2p_raw;  // emitted (tgt, src|img) pairs
@@ -151,7 +207,8 @@ struct Handle {
   bool m2l_ordered = false;  // m2l_off/m2l_ent built: per-target CSR in the reference's recording order
 
   // expansions
-  Buf M, L;   // double2 [ncells][nterm]
+  Slab exp_mem;  // M and L
+  Buf M, L;      // double2 [ncells][nterm]
   Buf shift_ops;   // M2M / L2L harmonics of the unit child offsets (expansions.cu)
   Buf shift_terms; // M2M / L2L term tables (expansions.cu)
   size_t shift_at[4] = {0, 0, 0, 0};  // offsets of the four term tables
@@ -165,9 +222,10 @@ struct Handle {
   int g_nghost = 0;  // ghost multipole rows after the cells' in g_m16
   // operator cache: g_optab[group key] is the operator's slot in g_ops (-1:
   // not built), op_count slots built for order op_P, layout op_layout (0:
-  // FP64 row blocks, 1: tensor-core FP16 images) and key space op_ks; after
-  // the table, the evaluation's group slots and new keys (op_ks ints each)
+  // FP64 row blocks, 1: tensor-core FP16 images) and key space op_ks
   Buf g_optab;
+  Buf g_new;         // operator slot of each group of the lists, then the keys whose operators are to be built
+  long g_groups = 0;  // room for groups in each
   int op_P = -1, op_layout = -1, op_count = 0;
   long op_ks = 0;
   double op_cycle = 0, op_R0 = 0;  // image-key operators: the geometry they were built for

@@ -713,8 +713,8 @@ bool long_leaves(const Handle &h) { return h.n > (int64_t)LONG_LEAF * h.nleaves;
 
 void upward_pass_2d(Handle &h, cudaStream_t s) {
   const int P = h.prm.P;
-  h.M.need((size_t)h.ncells * P * sizeof(double2));
-  h.L.need((size_t)h.ncells * P * sizeof(double2));
+  const size_t expansions = (size_t)h.ncells * P * sizeof(double2);
+  h.exp_mem.need({{&h.M, expansions}, {&h.L, expansions}});
   const bool done = with_order(P, [&](auto pc) {
     constexpr int PP = decltype(pc)::value;
     auto p2m = [&](auto gc) {

@@ -451,21 +451,28 @@ void build_lists(Handle &h, const std::function<void()> &near_field) {
   h.p2p_cap = std::max<size_t>(h.p2p_cap, (size_t)h.nleaves * 90 + 1024);
   const int images = h.prm.images;
   const long ks = key_space(images, h.depth);
-  h.g_occ.need(group_table_bytes(ks, C));      // marks and counts, and the tables made from them
-  h.g_cnt.need((size_t)C * sizeof(int) + 64);  // tile slots of the targets
-  const GroupTables gt = group_tables(h.g_occ.p, ks, C);
+  const bool keyed = m2l_keyed(h);
   h.g_grouped = false;
   for (int attempt = 0;; attempt++) {
-    h.frontier[0].need(h.frontier_cap * sizeof(int2));
-    h.frontier[1].need(h.frontier_cap * sizeof(int2));
-    h.m2l_raw.need(h.m2l_cap * sizeof(int2));
-    h.p2p_raw.need(h.p2p_cap * sizeof(int2));
+    if (keyed) h.g_groups = std::min<long>(ks, (long)h.m2l_cap);  // no more groups than entries
+    if (h.list_mem.need({{&h.frontier[0], h.frontier_cap * sizeof(int2)},
+                         {&h.frontier[1], h.frontier_cap * sizeof(int2)},
+                         {&h.m2l_raw, h.m2l_cap * sizeof(int2)},
+                         {&h.p2p_raw, h.p2p_cap * sizeof(int2)},
+                         {&h.p2p_off, (size_t)(C + 1) * sizeof(int)},
+                         {&h.p2p_ent, h.p2p_cap * 2 * sizeof(u32)},
+                         {&h.g_occ, group_table_bytes(ks, C)},      // marks and counts, and the tables made from them
+                         {&h.g_cnt, (size_t)C * sizeof(int) + 64},  // tile slots of the targets
+                         {&h.m2l_key, keyed ? h.m2l_cap * sizeof(int) : 0},
+                         {&h.g_tk, keyed ? (size_t)C * 2 * (sizeof(u64) + sizeof(u32)) + 64 : 0},
+                         {&h.g_new, keyed ? 2 * (size_t)h.g_groups * sizeof(int) : 0},
+                         {&h.g_optab, keyed ? (size_t)ks * sizeof(int) : 0}}))
+      h.op_P = -1;  // the operator table has moved
+    const GroupTables gt = group_tables(h.g_occ.p, ks, C);
     // list and frontier counts, and the counters of the M2L grouping
     FMM_CUDA(cudaMemsetAsync(&ctr->n_m2l, 0, sizeof(DevCounters) - offsetof(DevCounters, n_m2l), s));
     // group keys of the M2L entries, and the keys and targets that occur
-    const bool keyed = m2l_keyed(h);
     if (keyed) {
-      h.m2l_key.need(h.m2l_cap * sizeof(int));
       FMM_CUDA(cudaMemsetAsync(gt.occ, 0, group_mark_bytes(ks, C), s));
     } else {
       FMM_CUDA(cudaMemsetAsync(gt.cnt, 0, (size_t)(C + 1) * sizeof(int), s));

@@ -738,6 +738,13 @@ __device__ __forceinline__ int tile_at(const int *tg_off, int ntiles, int s) {
   return lo;
 }
 
+// Where CTA c of G writes its part of a tile cut by its range's boundary: the
+// tile it starts in (`first`), or the one it ends in, of which it is the only
+// such CTA.  In tiles of slots: G + min(G, ntiles).
+__host__ __device__ __forceinline__ int part_slot(int c, int G, bool first, int tile, int ntiles) {
+  return first ? c : G + (ntiles < G ? tile : c);
+}
+
 // First segment of CTA c of G when nseg segments are cut into equal ranges.
 __device__ __forceinline__ int range_start(int nseg, int c, int G) { return (int)((long long)nseg * c / G); }
 
@@ -870,7 +877,7 @@ __global__ void __launch_bounds__(GP_WARPS * 32, MAXP == GP_MAXP_SMALL ? 2 : 1)
   }
   // unscale (L = L~ / R_t^(j+1)) and store, or write the part
   const bool whole = tg_off[tile] >= r0 && tg_off[tile + 1] <= r1;
-  double2 *slot = whole ? nullptr : part + (size_t)(2 * blockIdx.x + (tile == tfirst ? 0 : 1)) * GP_TILE * pd.NT;
+  double2 *slot = whole ? nullptr : part + (size_t)part_slot(blockIdx.x, gridDim.x, tile == tfirst, tile, ntiles) * GP_TILE * pd.NT;
   for (int i = tid; i < GP_TILE * pd.NT; i += blockDim.x) {
     const int col = i / pd.NT, o = i - col * pd.NT;
     const int t = tile_tgt[tile * GP_TILE + col];
@@ -1038,8 +1045,8 @@ __device__ __forceinline__ void tc_flush_global(uint32_t acc, int t, double inv,
 // tiles than SMs, each a serial chain of a few hundred segments (20,000
 // bodies at P = 6: 5 tiles), so there too the ranges are what fills the GPU.
 // A CTA stores the tiles that lie wholly in its range; of a tile cut by a
-// range boundary it writes its partial sums to `part` (slot 0: its first
-// tile, 1: its last), which k_m2l_join adds in CTA order (deterministic).
+// range boundary it writes its partial sums to `part` (part_slot), which
+// k_m2l_join adds in CTA order (deterministic).
 // Orders whose running sum is L in global memory (P > 12): one CTA per tile.
 template <int PT>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, const int *tg_off, const int *tg_gid,
@@ -1143,7 +1150,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const int *tile_tgt, c
       if (tg_off[tt] >= g0 && tg_off[tt + 1] <= g1) {
         tc_store(sum_hi, sum_lo, fold == 1, t, inv, us, 0, KP, NT, L);
       } else {  // a part of a tile cut by a range boundary
-        double2 *slot = part + (size_t)(2 * blockIdx.x + (tt == tfirst ? 0 : 1)) * TC_TILE * NT;
+        double2 *slot = part + (size_t)part_slot(blockIdx.x, gridDim.x, tt == tfirst, tt, ntiles) * TC_TILE * NT;
         tc_store(sum_hi, sum_lo, fold == 1, t >= 0 ? tid : -1, inv, us, 0, KP, NT, slot);
       }
     }
@@ -1407,18 +1414,17 @@ __global__ void __launch_bounds__(JOIN_T) k_m2l_join(const int *tile_tgt, const 
   };
   const int c0 = cta_of(a), c1 = cta_of(b - 1);
   if (c0 == c1) return;  // the tile lies in one range: stored by its CTA
-  // the tile is the first tile (slot 0) of every CTA after c0, whose ranges
-  // start inside it; for c0 it is the last (slot 1) unless c0's range
-  // starts at the tile
-  const int slot0 = range_start(nseg, c0, G) < a ? 1 : 0;
+  // the tile is the first of every CTA after c0, whose ranges start inside
+  // it; for c0 it is the last unless c0's range starts at the tile
+  const int slot0 = part_slot(c0, grid, range_start(nseg, c0, G) >= a, t, ntiles);
   const size_t len = (size_t)tile_n * NT;
   for (int e = blockIdx.y * JOIN_T + threadIdx.x; e < (int)len; e += gridDim.y * JOIN_T) {
     const int row = e / NT, o = e - row * NT, tgt = tile_tgt[t * tile_n + row];
     if (tgt < 0) continue;
-    double2 sum = part[(size_t)(2 * c0 + slot0) * len + e];
+    double2 sum = part[(size_t)slot0 * len + e];
 #pragma unroll 4
     for (int c = c0 + 1; c <= c1; c++) {
-      const double2 v = part[(size_t)(2 * c) * len + e];
+      const double2 v = part[(size_t)c * len + e];
       sum.x += v.x;
       sum.y += v.y;
     }
@@ -1556,13 +1562,15 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
   int *tg_src = h.g_tg.as<int>(), *tg_gid = tg_src + (size_t)nseg * tile_n, *tg_off = tg_gid + nseg;
   DevCounters *ctr = h.counters.as<DevCounters>();
   if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
+  // as many CTAs as can have a range (range_ctas; nseg is an upper bound)
+  auto ranges = [&](int most) { return (int)std::max(1L, std::min((long)most, nseg / SEG_MIN)); };
   if (tcore) {
     // orders with a running sum in TMEM (up to 12) take balanced segment
     // ranges, one CTA per SM
     const bool fixed = P >= TC_FIXED_MIN && P <= TC_FIXED_MAX;
     const bool bal = (fixed ? tc_acc_fixed(KP16, tp) : tc_acc_layout(KP16)).fold != 0;
-    const int G = bal ? h.nsm : ntiles, NT = tri(P);
-    if (bal) h.g_part.need((size_t)G * 2 * TC_TILE * NT * sizeof(double2));
+    const int G = bal ? ranges(h.nsm) : ntiles, NT = tri(P);
+    if (bal) h.g_part.need((size_t)(G + std::min(G, ntiles)) * TC_TILE * NT * sizeof(double2));
     double2 *part = bal ? h.g_part.as<double2>() : nullptr;
     auto launch = [&](auto kern) {
       kern<<<G, TC_THREADS, tc_smem(tp), s>>>(h.g_tile.as<int>(), tg_off, tg_gid, tg_src, h.g_ops.as<unsigned char>(),
@@ -1608,8 +1616,8 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
     const int NT = tri(P);
     double2 *part = nullptr;
     if (bal) {
-      G = slots;
-      h.g_part.need((size_t)G * 2 * GP_TILE * NT * sizeof(double2));
+      G = ranges(slots);
+      h.g_part.need((size_t)(G + std::min(G, ntiles)) * GP_TILE * NT * sizeof(double2));
       part = h.g_part.as<double2>();
     }
     kern<<<G, GP_WARPS * 32, smem, s>>>(h.g_tile.as<int>(), tg_off, tg_gid, tg_src, h.g_ops.as<double>(),
@@ -1633,11 +1641,9 @@ bool m2l_groups_raw(const Handle &h) {
          !(h.prm.images > 0 && h.prm.precision == EXAFMM_MIXED && tc_available(h.prm.P));
 }
 
-// g_optab holds three arrays of the key space (one allocation: each costs a
-// new handle's first evaluation about 0.3 ms): the operator table, the
-// operator slot of each group, the keys whose operators are to be built.
-int *group_slots(const Handle &h) { return h.g_optab.as<int>() + h.op_ks; }
-int *new_keys(const Handle &h) { return h.g_optab.as<int>() + 2 * h.op_ks; }
+// The operator slot of each group, and the keys whose operators are to be built.
+int *group_slots(const Handle &h) { return h.g_new.as<int>(); }
+int *new_keys(const Handle &h) { return h.g_new.as<int>() + h.g_groups; }
 
 // Queues, after the key and target marks: the group tables, the operator
 // slots, and the flagged targets' tile keys.  max_groups: an upper bound of
@@ -1646,7 +1652,7 @@ void m2l_group_launch(Handle &h, long max_groups) {
   cudaStream_t s = h.stream;
   const int P = h.prm.P, C = h.ncells;
   const int layout = h.prm.precision == EXAFMM_MIXED && tc_available(P) ? 1 : 0;
-  const long ks = key_space(h.prm.images, h.depth), cap = std::min(ks, max_groups);
+  const long ks = key_space(h.prm.images, h.depth), cap = std::min(h.g_groups, max_groups);
   const double cyc = h.prm.images ? h.prm.cycle : 0.0;
   // the cache holds operators of one order, layout and key space; image keys
   // also depend on the period, the root radius and the depth
@@ -1656,7 +1662,6 @@ void m2l_group_launch(Handle &h, long max_groups) {
                      (layout == 1 && h.op_theta != h.prm.theta);
   h.op_P = -1;  // until m2l_group_commit() has built what the table now holds
   if (stale) {
-    h.g_optab.need((size_t)3 * ks * sizeof(int));  // the table, the groups' slots, the new keys
     FMM_CUDA(cudaMemsetAsync(h.g_optab.p, 0xff, (size_t)ks * sizeof(int), s));
     h.op_count = 0;
     h.op_layout = layout;
@@ -1672,7 +1677,6 @@ void m2l_group_launch(Handle &h, long max_groups) {
   k_occ_words<<<nt, 1024, 0, s>>>(gt);
   k_occ_groups<<<nt, 1024, 0, s>>>(gt, h.g_optab.as<int>(), h.op_count, group_slots(h), new_keys(h), cap,
                                    &ctr->gcounts[2], &ctr->op_new);
-  h.g_tk.need((size_t)C * 2 * (sizeof(u64) + sizeof(u32)) + 64);
   u64 *tk = h.g_tk.as<u64>();
   k_tkeys<<<grid_for(C, TB), TB, 0, s>>>(C, gt.gflag, gt.gfine, h.c_level.as<int>(), h.c_parent.as<int>(),
                                          h.c_child.as<int>(), h.c_face.as<int>(), tk, (u32 *)(tk + 2 * (size_t)C), ctr->gcounts);
@@ -1691,7 +1695,7 @@ void m2l_group_commit(Handle &h) {
     const size_t nslots = (size_t)h.op_count + nnew;
     if (nslots * op_bytes > h.g_ops.bytes) {  // grow, keeping the operators built so far
       Buf grown;
-      grown.need(std::max(nslots, (size_t)64) * op_bytes * 2);
+      grown.allocate(std::max(nslots, (size_t)64) * op_bytes * 2);
       if (h.g_ops.p && h.op_count > 0)
         FMM_CUDA(cudaMemcpyAsync(grown.p, h.g_ops.p, (size_t)h.op_count * op_bytes, cudaMemcpyDeviceToDevice, s));
       FMM_CUDA(cudaStreamSynchronize(s));

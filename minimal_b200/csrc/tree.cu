@@ -505,7 +505,14 @@ void build_tree(Handle &h) {
   }
   D = std::min(D, max_levels);
   bool zeroed = nsys == 1;  // by k_bounds
-  for (h.keys[0].need(n * 8), h.keys[1].need(n * 8), h.vals[0].need(n * 4), h.vals[1].need(n * 4);;) {
+  const bool srcf = h.prm.precision == EXAFMM_MIXED && h.prm.dim != 2;
+  const size_t nb = (size_t)n;
+  h.body_mem.need({{&h.keys[0], nb * 8}, {&h.keys[1], nb * 8}, {&h.vals[0], nb * 4}, {&h.vals[1], nb * 4},
+                   {&h.lfirst, nb * 4}, {&h.chain, nb * 4}, {&h.prebase, (nb + 1) * 4}, {&h.perm, nb * 4},
+                   {&h.src, nb * sizeof(double4)}, {&h.out, nb * sizeof(double4)},
+                   {&h.srcf, srcf ? nb * sizeof(float4) : 0}, {&h.srcp, srcf ? 2 * nb * sizeof(float4) : 0},
+                   {&h.body_leaf, h.prm.dim != 2 ? nb * sizeof(int) : 0}});
+  for (;;) {
     if (!zeroed) FMM_CUDA(cudaMemsetAsync(ctr, 0, sizeof(DevCounters), s));
     zeroed = false;
     u64 *k = h.keys[0].as<u64>(), *k2 = h.keys[1].as<u64>();
@@ -514,9 +521,6 @@ void build_tree(Handle &h) {
     h.launches++;
     FMM_LAUNCH();
     radix_sort_pairs(h, k, v, k2, v2, n, 0, 3 * D + sys_bits);
-    h.lfirst.need(n * 4);
-    h.chain.need(n * 4);
-    h.prebase.need((n + 1) * 4);
     k_chain<<<grid_for(n, TB), TB, 0, s>>>(k, n, D, h.prm.ncrit, h.lfirst.as<int>(), h.chain.as<int>(), ctr);
     h.launches++;
     FMM_LAUNCH();
@@ -543,7 +547,12 @@ void build_tree(Handle &h) {
     }
     // pre-order tables (reuse the idle sort buffers' siblings)
     const long Cp = (C + 3) & ~3L;  // every table starts 16-byte aligned (vector loads in the scans)
-    h.pre_tmp.need(Cp * (7 * sizeof(int) + sizeof(double4)) + 256);
+    const size_t cb = (size_t)C * sizeof(int);
+    h.cell_mem.need({{&h.pre_tmp, Cp * (7 * sizeof(int) + sizeof(double4)) + 256},
+                     {&h.ctmp, Cp * (2 * sizeof(u64) + 2 * sizeof(u32) + 4 * sizeof(int)) + 256},
+                     {&h.c_begin, cb}, {&h.c_count, cb}, {&h.c_child, cb}, {&h.c_nchild, cb}, {&h.c_parent, cb},
+                     {&h.c_level, cb}, {&h.c_pre, cb}, {&h.c_ref, cb}, {&h.c_face, cb}, {&h.leaves, cb},
+                     {&h.c_xr, (size_t)C * sizeof(double4)}});
     PreTables t;
     t.xr = h.pre_tmp.as<double4>();
     t.begin = (int *)(t.xr + Cp);
@@ -560,7 +569,6 @@ void build_tree(Handle &h) {
     FMM_LAUNCH();
 
     // 5. BFS order = stable sort of pre-order cells by level
-    h.ctmp.need(Cp * (2 * sizeof(u64) + 2 * sizeof(u32) + 4 * sizeof(int)) + 256);
     u64 *lk = h.ctmp.as<u64>(), *lk2 = lk + Cp;
     u32 *lv = (u32 *)(lk2 + Cp), *lv2 = lv + Cp;
     int *bfs_of_pre = (int *)(lv2 + Cp), *is_leaf = bfs_of_pre + Cp, *blockstart = is_leaf + Cp,
@@ -571,17 +579,12 @@ void build_tree(Handle &h) {
     radix_sort_pairs(h, lk, lv, lk2, lv2, C, 0, 5);
     k_invert<<<grid_for(C, TB), TB, 0, s>>>(lv, C, bfs_of_pre);
     h.launches++;
-    h.c_begin.need(C * 4); h.c_count.need(C * 4); h.c_child.need(C * 4); h.c_nchild.need(C * 4);
-    h.c_parent.need(C * 4); h.c_level.need(C * 4); h.c_pre.need(C * 4); h.c_ref.need(C * 4);
-    h.c_face.need(C * 4);
-    h.c_xr.need(C * sizeof(double4));
     BfsCells o{h.c_begin.as<int>(), h.c_count.as<int>(), h.c_child.as<int>(), h.c_nchild.as<int>(),
                h.c_parent.as<int>(), h.c_level.as<int>(), h.c_pre.as<int>(), h.c_face.as<int>(), h.c_xr.as<double4>()};
     k_gather_cells<<<grid_for(C, TB), TB, 0, s>>>(lv, bfs_of_pre, C, t, o, is_leaf);
     h.launches++;
     FMM_LAUNCH();
     // reference numbering, and the leaves
-    h.leaves.need(C * 4);
     scan_exclusive_pair(h, t.nchild, blockstart, nullptr, is_leaf, leafpos, nullptr, C);
     k_ref_leaves<<<grid_for(C, TB), TB, 0, s>>>(o, C, blockstart, h.c_ref.as<int>(), is_leaf, leafpos,
                                                 h.leaves.as<int>());
@@ -589,14 +592,6 @@ void build_tree(Handle &h) {
     FMM_LAUNCH();
     // 6. bodies of each leaf back to input order and gathered (the mixed
     // form's FP32 sources with them)
-    h.perm.need(n * 4);
-    h.src.need(n * sizeof(double4));
-    const bool srcf = h.prm.precision == EXAFMM_MIXED && h.prm.dim != 2;
-    if (srcf) {
-      h.srcf.need((size_t)n * sizeof(float4));
-      h.srcp.need((size_t)n * 2 * sizeof(float4));
-    }
-    if (h.prm.dim != 2) h.body_leaf.need((size_t)n * sizeof(int));
     k_leaf_order<<<grid_for((long)h.nleaves * 32, TB), TB, 0, s>>>(
         h.leaves.as<int>(), h.nleaves, o.begin, o.count, o.xr, v, h.in.as<double4>(), h.perm.as<int>(),
         h.src.as<double4>(), srcf ? h.srcf.as<float4>() : nullptr, h.srcp.as<float4>(),

@@ -1,0 +1,61 @@
+"""What a new handle's first evaluation takes from the GPU, for small systems:
+the tables of the grouped M2L are sized by what the lists can hold, not by
+several times the key space.  The operators of some 300 groups at P = 10 (40
+MB) and the parts of a contraction split over all SMs (21 MB) are the largest
+pieces of the free-space case, the table of a periodic key space (9 million
+keys, 4 bytes each and a quarter more) of the other: 100 MB holds either."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,P,images", [(10000, 10, 0), (2000, 4, 1)])
+def test_memory_of_a_small_handle(n, P, images):
+    import torch
+
+    from minimal_b200 import FMM
+
+    r = np.random.default_rng(n)
+    xq = np.concatenate([(r.random((n, 3)) * 2 - 1) * np.pi, r.random((n, 1)) - 0.5], 1)
+
+    def handle():
+        f = FMM(P=P, ncrit=64, theta=0.4, images=images, cycle=2 * np.pi)
+        f.set_bodies(xq)
+        f.evaluate()
+        return f
+
+    handle().close()  # the kernels are loaded
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    f = handle()
+    held = before - torch.cuda.mem_get_info()[0]
+    assert 0 < held < 100e6, held
+    f.close()
+    assert torch.cuda.mem_get_info()[0] >= before  # given back
+
+
+def test_growth_keeps_results():
+    """A handle taken through systems of other sizes, forms and dimensions of
+    its buffers gives each the bits that a new handle gives."""
+    from minimal_b200 import FMM
+
+    r = np.random.default_rng(3)
+    f = FMM(P=6, ncrit=32, theta=0.4)
+    for n, P, ncrit, precision in ((700, 6, 32, "fp64"), (9001, 6, 32, "mixed"), (9001, 9, 16, "fp64"),
+                                   (300, 4, 64, "mixed"), (20011, 9, 8, "mixed"), (20011, 9, 8, "fp64")):
+        xq = np.concatenate([r.random((n, 3)), r.random((n, 1)) - 0.5], 1)
+        xq = xq.astype(np.float32).astype(np.float64)
+        kw = dict(P=P, ncrit=ncrit, theta=0.4, precision=precision)
+        f.set_params(**kw)
+        f.set_bodies(xq)
+        f.evaluate()
+        g = FMM(**kw)
+        g.set_bodies(xq)
+        g.evaluate()
+        assert np.array_equal(f.bodies(), g.bodies())
+        q = r.random(n)
+        for h in (f, g):
+            h.set_charges(q)
+            h.reevaluate()
+        assert np.array_equal(f.bodies(), g.bodies())
