@@ -266,7 +266,7 @@ struct Handle {
 
   // error flags in pinned host memory, set by kernels and checked after each
   // synchronisation: [0] a bounded tensor-core wait ran out, [1] a body or
-  // charge handed in is not finite
+  // charge handed in is not finite; after the counters' host copy
   int *flags_host = nullptr;
 
   cudaEvent_t ev[PH_COUNT + 1][2];

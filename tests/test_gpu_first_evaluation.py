@@ -59,3 +59,28 @@ def test_growth_keeps_results():
             h.set_charges(q)
             h.reevaluate()
         assert np.array_equal(f.bodies(), g.bodies())
+
+def test_create_asks_for_little():
+    """A handle beside others costs its streams, events and counters: less
+    than one query of all device properties, a few ms, which it used to make."""
+    import ctypes
+    import time
+
+    import torch
+
+    from minimal_b200 import FMM
+
+    torch.cuda.init()
+    props, buf = ctypes.CDLL("libcudart.so.12").cudaGetDeviceProperties_v2, ctypes.create_string_buffer(1 << 14)
+
+    def best(call):
+        t = []
+        for _ in range(20):
+            a = time.perf_counter()
+            call()
+            t.append(time.perf_counter() - a)
+        return min(t)
+
+    keep = []
+    assert props(buf, 0) == 0
+    assert best(lambda: keep.append(FMM())) < best(lambda: props(buf, 0))
