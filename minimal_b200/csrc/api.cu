@@ -412,7 +412,7 @@ int exafmm_b200_destroy(exafmm_b200 *H) {
   if (h.side) cudaStreamSynchronize(h.side);
   if (h.aux) cudaStreamSynchronize(h.aux);
   if (h.aux_lo) cudaStreamSynchronize(h.aux_lo);
-  Buf *bufs[] = {&h.in, &h.src, &h.out, &h.perm, &h.srcf, &h.srcp, &h.keys[0], &h.keys[1], &h.vals[0], &h.vals[1],
+  Buf *bufs[] = {&h.sys_off, &h.in, &h.src, &h.out, &h.perm, &h.srcf, &h.srcp, &h.keys[0], &h.keys[1], &h.vals[0], &h.vals[1],
                  &h.lfirst, &h.chain, &h.prebase, &h.scan_tmp, &h.hist, &h.c_begin, &h.c_count, &h.c_child,
                  &h.c_nchild, &h.c_parent, &h.c_level, &h.c_xr, &h.c_pre, &h.c_ref, &h.c_leaf_of_body, &h.c_face,
                  &h.leaves, &h.pre_tmp, &h.ctmp, &h.geom, &h.counters, &h.frontier[0], &h.frontier[1],
