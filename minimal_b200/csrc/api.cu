@@ -162,6 +162,22 @@ __global__ void __launch_bounds__(256) k_unpack_out16(const double2 *src, const 
   rec[e] = v;
 }
 
+// Workspace of one call, until its end: the staging buffer where the call
+// needs no more than that holds or the handle's own bodies fill, else an
+// allocation of its own (a handle of few bodies asked about many targets keeps
+// nothing of their size).
+struct CallSpace {
+  Buf own;
+  void *p;
+  CallSpace(Handle &h, size_t bytes) {
+    Buf &b = bytes <= std::max(h.stage.bytes, (size_t)h.n * rec_len(h) * sizeof(double)) ? h.stage : own;
+    b.need(bytes);
+    p = b.p;
+  }
+  CallSpace(const CallSpace &) = delete;
+  ~CallSpace() { own.release(); }
+};
+
 __global__ void k_direct_prep(const double *rec, long n, int len, double4 *xq, double4 *pf) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -746,9 +762,9 @@ int exafmm_b200_direct(exafmm_b200 *H, double *targets, int64_t nt, int where) {
     const size_t bytes = (size_t)nt * len * sizeof(double);
     // records, then positions and results as double4 (aligned for them)
     const size_t at = (bytes + 31) / 32 * 32;
-    h.stage.need(at + 2 * nt * sizeof(double4));
-    double *rec = h.stage.as<double>();
-    double4 *xq = (double4 *)((char *)h.stage.p + at), *pf = xq + nt;
+    CallSpace space(h, at + 2 * nt * sizeof(double4));
+    double *rec = (double *)space.p;
+    double4 *xq = (double4 *)((char *)space.p + at), *pf = xq + nt;
     FMM_CUDA(cudaMemcpyAsync(rec, targets, bytes, where == EXAFMM_HOST ? cudaMemcpyHostToDevice
                                                                         : cudaMemcpyDeviceToDevice, h.stream));
     k_direct_prep<<<grid_for(nt, 256), 256, 0, h.stream>>>(rec, nt, len, xq, pf);
@@ -793,11 +809,10 @@ int exafmm_b200_ewald_parts(exafmm_b200 *H, int parts, int ksize, double alpha, 
     if (ksize < 1 || ksize > 64 || !(alpha > 0) || !(sigma > 0) || !(cutoff > 0))
       throw Error{EXAFMM_ERR_ARG, "ewald: ksize in [1, 64] and positive alpha, sigma, cutoff required"};
     if (!(h.prm.cycle > 0)) throw Error{EXAFMM_ERR_STATE, "ewald() needs a periodic handle (cycle > 0)"};
-    Buf &rec = h.stage;
-    rec.need(nt * 64);
+    CallSpace rec(h, nt * 64);
     FMM_CUDA(cudaMemcpyAsync(rec.p, targets, nt * 64, where == EXAFMM_HOST ? cudaMemcpyHostToDevice
                                                                           : cudaMemcpyDeviceToDevice, h.stream));
-    ewald(h, parts, ksize, alpha, sigma, cutoff, h.prm.cycle, rec.as<double>(), nt);
+    ewald(h, parts, ksize, alpha, sigma, cutoff, h.prm.cycle, (double *)rec.p, nt);
     FMM_CUDA(cudaMemcpyAsync(targets, rec.p, nt * 64, where == EXAFMM_HOST ? cudaMemcpyDeviceToHost
                                                                           : cudaMemcpyDeviceToDevice, h.stream));
     FMM_CUDA(cudaStreamSynchronize(h.stream));

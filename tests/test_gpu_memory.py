@@ -38,3 +38,22 @@ def test_batch_handles_give_all_back():
     for _ in range(10):
         handle()
     assert free() >= before - (4 << 20)
+
+
+@pytest.mark.parametrize("call", ["direct", "ewald"])
+def test_large_target_sets_are_not_kept(call):
+    """A call with many more targets than the handle has bodies works in
+    memory of its own (128 and 64 bytes per target: 128 and 64 MB here); one
+    with fewer stays in the handle's staging buffer, of the bodies' size."""
+    from minimal_b200 import FMM
+
+    f = FMM(P=4, ncrit=64, theta=0.5, cycle=2 * np.pi)
+    f.set_bodies(bodies(1000, 2))
+    f.evaluate()
+    targets = bodies(1000000, 3)
+    few = getattr(f, call)(targets[:64])
+    getattr(f, call)(targets[:200000])
+    before = free()
+    many = getattr(f, call)(targets)
+    assert free() >= before - (4 << 20)
+    assert np.allclose(many[:64, 4:], few[:, 4:], rtol=1e-11, atol=1e-11 * np.abs(few[:, 4:]).max())
