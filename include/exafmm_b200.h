@@ -267,10 +267,12 @@ EXAFMM_API int exafmm_b200_fma_peak(exafmm_b200 *h, int precision, double *tflop
  * fold work (the default: 2 for P <= 10, 1 for P = 11 and 12, 4 above).  Values 1-64; 0 restores
  * the default.  EXAFMM_TILE_P2P_STAGE: bodies of source leaves the near-field
  * kernel stages in shared memory per chunk (the source tile), 1024, 1536 or
- * 2048 (default: 1536 mixed, 1024 FP64, and less for trees of many small
- * leaves, whose leaves take fewer threads); a speed choice: the sums change only
- * by rounding (the chunks group the sources differently).  get_tile returns the value in effect.  exafmm_b200_autotune()
- * chooses the source tile after the leaf size. */
+ * 2048 (default: 1536 mixed, 1024 FP64, and 256 to 768 for trees of many small
+ * leaves, whose leaves take fewer threads; a tile set here takes 128 threads
+ * whatever the leaves); a speed choice: the sums change only by rounding (the
+ * chunks group the sources differently).  get_tile returns the value in effect
+ * for the tree now built.  exafmm_b200_autotune() chooses the source tile, or
+ * the default, after the leaf size. */
 enum { EXAFMM_TILE_M2L_FLUSH = 0, EXAFMM_TILE_P2P_STAGE = 1 };
 EXAFMM_API int exafmm_b200_set_tile(exafmm_b200 *h, int which, int value);
 EXAFMM_API int exafmm_b200_get_tile(exafmm_b200 *h, int which, int *value);

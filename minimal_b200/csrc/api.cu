@@ -387,6 +387,7 @@ int exafmm_b200_create(const exafmm_params *params, exafmm_b200 **out) {
     Handle &h = H->h;
     h.prm = *params;
     h.nterm = params->dim == 2 ? params->P : nterm_of(params->P);
+    FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, params->device));
     int least = 0, greatest = 0;
     FMM_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     FMM_CUDA(cudaStreamCreateWithPriority(&h.stream, cudaStreamNonBlocking, greatest));
@@ -617,6 +618,7 @@ int exafmm_b200_autotune(exafmm_b200 *H, const int *candidates, int ncand, int r
     };
     int best = -1;
     double tbest = 0;
+    h.tile_p2p_stage = 0;  // the default, whose threads per leaf follow the leaves, for the sweep and as a candidate
     for (int k = 0; k < ncand; k++) {
       h.prm.ncrit = candidates[k];
       h.key_levels = 0;  // the key depth follows ncrit
@@ -633,8 +635,7 @@ int exafmm_b200_autotune(exafmm_b200 *H, const int *candidates, int ncand, int r
     // then the near-field source tile at that leaf size (a speed choice:
     // the sums change only by rounding)
     if (best <= 256) {
-      const int saved = h.tile_p2p_stage;
-      int best_tile = saved;
+      int best_tile = 0;
       for (int tile : {1024, 1536, 2048}) {
         h.tile_p2p_stage = tile;
         run();

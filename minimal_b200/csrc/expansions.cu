@@ -994,7 +994,6 @@ void unit_tables(Handle &h, cudaStream_t s) {
 constexpr int OB_FEW = 2;
 template <class F>
 void ob_level(Handle &h, int np, F launch) {
-  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   if (np <= OB_FEW * h.nsm)
     launch(std::integral_constant<int, 1>{}, std::integral_constant<int, OB_SL>{});
   else

@@ -248,7 +248,7 @@ struct Handle {
   Buf per_part;  // partial charge sums (the mixed form's root monopole)
   Buf g_gharm;  // harmonics of the ghost shifts, per (image, finer level)
   Buf g_part;   // tensor-core M2L: partial local expansions of tiles split between CTAs
-  int nsm = 0;  // streaming multiprocessors of the device (0: not read yet)
+  int nsm = 0;  // streaming multiprocessors of the device
   int per_P = 0, per_images = 0;
   // Ewald: wave list and DFT units of ew_ksize, amplitudes, partial sums
   Buf ew_waves, ew_units, ew_amp, ew_part;

@@ -392,7 +392,6 @@ __global__ void __launch_bounds__(SEG_WARPS * 32) k_order_segments32(const int *
 
 // Blocks of one wave of the walk: as many as are resident on the GPU at once.
 int walk_blocks(Handle &h, bool periodic) {
-  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   int occ = 1;
   FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &occ, periodic ? k_walk<WALK_PAIRS, true> : k_walk<WALK_PAIRS, false>, TB, 0));

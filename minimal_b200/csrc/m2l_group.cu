@@ -1561,7 +1561,6 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
   const long nseg = h.g_nseg;
   int *tg_src = h.g_tg.as<int>(), *tg_gid = tg_src + (size_t)nseg * tile_n, *tg_off = tg_gid + nseg;
   DevCounters *ctr = h.counters.as<DevCounters>();
-  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   // as many CTAs as can have a range (range_ctas; nseg is an upper bound)
   auto ranges = [&](int most) { return (int)std::max(1L, std::min((long)most, nseg / SEG_MIN)); };
   if (tcore) {

@@ -656,6 +656,10 @@ void make_srcf(Handle &h) {
   h.srcf_ready = true;
 }
 
+// Bodies staged at once by the kernels of 32 and 64 threads.
+template <bool F32>
+constexpr int small_cap(int ct) { return ct == 32 ? (F32 ? 512 : 256) : (F32 ? 768 : 512); }
+
 // The near-field CTA kernel with `ct` threads, or with CT_MAX threads and
 // source tile `cap` (1024, 1536 or 2048).
 template <bool F32, class F>
@@ -665,8 +669,8 @@ void with_p2p_shape(int ct, int cap, F f) {
     f(k_p2p_cta<F32, CAP, CT>, CT, CAP * sizeof(typename NearBody<F32>::T));
   };
   typedef std::integral_constant<int, CT_MAX> Full;
-  if (ct == 32) shape(std::integral_constant<int, F32 ? 512 : 256>{}, std::integral_constant<int, 32>{});
-  else if (ct == 64) shape(std::integral_constant<int, F32 ? 768 : 512>{}, std::integral_constant<int, 64>{});
+  if (ct == 32) shape(std::integral_constant<int, small_cap<F32>(32)>{}, std::integral_constant<int, 32>{});
+  else if (ct == 64) shape(std::integral_constant<int, small_cap<F32>(64)>{}, std::integral_constant<int, 64>{});
   else if (cap == 1024) shape(std::integral_constant<int, 1024>{}, Full{});
   else if (cap == 2048) shape(std::integral_constant<int, 2048>{}, Full{});
   else shape(std::integral_constant<int, 1536>{}, Full{});
@@ -701,16 +705,19 @@ void p2p_set_attributes() {
   set_p2p_attributes<true>();
 }
 
+// Bodies of source leaves staged at once for the tree's leaves.
 int p2p_tile(const Handle &h) {
   if (h.tile_p2p_stage > 0) return h.tile_p2p_stage;
-  return h.prm.precision == EXAFMM_MIXED ? ct_cap<true>() : ct_cap<false>();
+  const bool f32 = h.prm.precision == EXAFMM_MIXED;
+  const int ct = h.have_tree ? p2p_threads(h) : CT_MAX;
+  if (ct < CT_MAX) return f32 ? small_cap<true>(ct) : small_cap<false>(ct);
+  return f32 ? ct_cap<true>() : ct_cap<false>();
 }
 
 void p2p_pass(Handle &h, cudaStream_t s) {
   if (h.prm.dim == 2) return p2p_pass_2d(h, s);
   h.out.need((size_t)h.n * sizeof(double4));
   const double cyc = h.prm.images ? h.prm.cycle : 0.0;
-  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   const bool cta = h.prm.ncrit <= CT_MAXTGT;  // every leaf fits two targets per thread and the buffer
   if (h.prm.precision == EXAFMM_MIXED) {
     if (s != h.stream && !h.srcf_ready) throw Error{EXAFMM_ERR_STATE, "near field on a side stream before its sources"};
@@ -742,7 +749,6 @@ void p2p_pass(Handle &h, cudaStream_t s) {
 void direct_sum(Handle &h, double4 *targets, double4 *out, long nt) {
   // as many source chunks as give whole waves of resident blocks (four, so
   // that a block is short against the whole), tiles of DT sources each
-  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   int occ = 1;
   FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_direct, DT, 0));
   const long gx = grid_for(nt, DT), want = std::max<long>(1, 4L * h.nsm * std::max(occ, 1) / gx);

@@ -671,7 +671,6 @@ static void ewald_plan(Handle &h, int ksize) {
 void ewald(Handle &h, int parts, int ksize, double alpha, double sigma, double cutoff, double cycle, double *rec_dev,
            long nt) {
   ewald_plan(h, ksize);
-  if (h.nsm == 0) FMM_CUDA(cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, h.prm.device));
   const int nw = h.ew_nw;
   const int4 *waves = h.ew_waves.as<int4>();
   h.ew_amp.need(nw * sizeof(double2));
