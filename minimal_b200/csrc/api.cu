@@ -431,10 +431,10 @@ int exafmm_b200_destroy(exafmm_b200 *H) {
   if (h.aux_lo) cudaStreamSynchronize(h.aux_lo);
   Buf *bufs[] = {&h.sys_off, &h.in, &h.src, &h.out, &h.perm, &h.srcf, &h.srcp, &h.keys[0], &h.keys[1], &h.vals[0], &h.vals[1],
                  &h.lfirst, &h.chain, &h.prebase, &h.scan_tmp, &h.hist, &h.c_begin, &h.c_count, &h.c_child,
-                 &h.c_nchild, &h.c_parent, &h.c_level, &h.c_xr, &h.c_pre, &h.c_ref, &h.c_leaf_of_body, &h.c_face,
+                 &h.c_nchild, &h.c_parent, &h.c_level, &h.c_xr, &h.c_pre, &h.c_ref, &h.c_face,
                  &h.leaves, &h.pre_tmp, &h.ctmp, &h.geom, &h.counters, &h.frontier[0], &h.frontier[1],
                  &h.m2l_raw, &h.m2l_key, &h.p2p_raw, &h.m2l_off, &h.m2l_ent, &h.p2p_off, &h.p2p_ent, &h.fill, &h.M, &h.L,
-                 &h.m2l_units, &h.stage, &h.g_mt, &h.g_ekey, &h.g_occ, &h.g_cnt, &h.g_optab, &h.g_new, &h.g_ops,
+                 &h.stage, &h.g_mt, &h.g_ekey, &h.g_occ, &h.g_cnt, &h.g_optab, &h.g_new, &h.g_ops,
                  &h.g_tk, &h.g_tile, &h.g_seg, &h.g_tg, &h.g_m16, &h.g_pairs, &h.shift_ops, &h.shift_terms,
                  &h.op_scratch, &h.g_gmark, &h.per_harm, &h.g_gharm, &h.per_part,
                  &h.g_part, &h.body_leaf, &h.l2p_f, &h.ew_waves, &h.ew_units, &h.ew_amp, &h.ew_part};

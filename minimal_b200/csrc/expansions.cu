@@ -4,10 +4,12 @@
 // the level-synchronous launches respect: a cell's children are complete
 // before its M2M, and its parent's local is final before its L2L).
 //
-// Mapping: P2M and L2P take one warp per leaf and one lane per body.  M2M
-// and L2L take one thread per (cell, output coefficient (j,k)); the offset
-// harmonics they need depend only on level and octant and come from a
-// table built once per upward pass.
+// Mapping, up to order 16: P2M takes ceil(P / 2) lanes per leaf (two columns
+// of coefficients each), L2P a thread per body; above, both take a warp per
+// leaf and a lane per body (L2P of the mixed form a thread per body).  M2M and
+// L2L take one to four threads per (cell, output coefficient (j,k)); the
+// offset harmonics they need depend only on level and octant and come from a
+// table built once per order.
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -89,16 +91,13 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2m(const int *leaves, int nleav
   for (int k = lane; k < nt; k += 32) M[(long)c * nt + k] = acc[k];
 }
 
-// M2M (3d/kernel.h:204-231), one warp per parent at one level.
-// ---- mixed form: P2M and L2P in FP32 (bodies relative to their leaf centre,
-// the FP32 copy the near field uses), same lock-step generator in float;
-// expansions stay FP64 in memory.
+// ---- mixed form above order 16: P2M and L2P in FP32 (bodies relative to
+// their leaf centre), same lock-step generator in float; expansions stay FP64
+// in memory.
 __constant__ float c_recip_f[2 * EXAFMM_MAX_P + 4];
 #ifndef L2P_F32_MIN_BLOCKS
 #define L2P_F32_MIN_BLOCKS 6  // 128-thread blocks per SM: up to 80 registers a thread
 #endif
-// orders with unrolled FP32 P2M / L2P kernels (others take the runtime-order ones)
-#define EXAFMM_UNROLLED_ORDERS(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 
 struct SphF {
   float r, c, s, inv_s;
@@ -127,12 +126,9 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// PT > 0: the order as a compile-time constant -- the loops unroll and the
-// integer factors and reciprocals become immediates; PT = 0: runtime order Prt.
-template <int PT, bool WITH_DY, class F>
-__device__ __forceinline__ void regular_all_f(int Prt, const SphF &g, float2 e1, F f) {
-  const int P = PT > 0 ? PT : Prt;
-  auto rcp = [](int k) { return PT > 0 ? 1.0f / (float)k : c_recip_f[k]; };
+template <bool WITH_DY, class F>
+__device__ __forceinline__ void regular_all_f(int P, const SphF &g, float2 e1, F f) {
+  auto rcp = [](int k) { return c_recip_f[k]; };
   float2 em = make_float2(1.f, 0.f);
   float pmm = 1.f, odd = 1.f, cm = 1.f;
 #pragma unroll
@@ -186,7 +182,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2m_f32(const int *leaves, int n
     const bool ok = t + lane < nb;
     const float4 B = ok ? srcf[b0 + t + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
     const SphF g = sph_of_f(B.x * sc, B.y * sc, B.z * sc);
-    regular_all_f<0, false>(P, g, make_float2(g.e.x, -g.e.y), [&](int n, int m, float2 Y, float2) {
+    regular_all_f<false>(P, g, make_float2(g.e.x, -g.e.y), [&](int n, int m, float2 Y, float2) {
       float x = B.w * Y.x, y = B.w * Y.y;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -206,7 +202,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2m_f32(const int *leaves, int n
   }
 }
 
-// ---- P2M and (FP64) L2P from the Cartesian recurrences of the regular
+// ---- P2M and L2P from the Cartesian recurrences of the regular
 // harmonics, orders up to COLS_MAXP as compile-time constants.  In the
 // normalisation of harmonics.cuh, Y_n^m = T_n^m (x + iy)^m / (2^m m!) with
 //   T_m^m = 1,  T_{n+1}^m = -((2n+1) z T_n^m + r^2 T_{n-1}^m) / ((n-m+1)(n+m+1)),
@@ -216,7 +212,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_p2m_f32(const int *leaves, int n
 // of Spherical and Ellipsoidal Harmonics): no radius, angle, square root or
 // division, and polynomials also at a leaf's centre and on its axis.
 constexpr int COLS_MAXP = 16;
-#define EXAFMM_COLS_ORDERS(X) X(1) EXAFMM_UNROLLED_ORDERS(X)
+#define EXAFMM_COLS_ORDERS(X) \
+  X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 
 // complex value type of a compute precision
 template <bool F32>
@@ -466,7 +463,7 @@ __global__ void __launch_bounds__(128, L2P_F32_MIN_BLOCKS) k_l2p_f32(long nbodie
   const float4 B = srcf[b];
   const SphF g = sph_of_f(B.x * sc, B.y * sc, B.z * sc);
   float pot = 0.f, s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  regular_all_f<0, true>(P, g, g.e, [&](int n, int m, float2 Y, float2 dY) {
+  regular_all_f<true>(P, g, g.e, [&](int n, int m, float2 Y, float2 dY) {
     const float2 l = __ldg(Lw + tri(n) + m);
     const float w2 = m == 0 ? 1.f : 2.f;
     const float re = l.x * Y.x - l.y * Y.y;

@@ -183,7 +183,7 @@ struct Handle {
   int ncells = 0, nleaves = 0, depth = 0;
   int level_base[EXAFMM_MAX_LEVEL + 3] = {0};
   Slab cell_mem;  // the tables by cell (c_*, leaves, pre_tmp, ctmp)
-  Buf c_begin, c_count, c_child, c_nchild, c_parent, c_level, c_xr, c_pre, c_ref, c_leaf_of_body;
+  Buf c_begin, c_count, c_child, c_nchild, c_parent, c_level, c_xr, c_pre, c_ref;
   Buf c_face;  // which faces of the root a cell's parent touches (k_cells)
   Buf leaves;  // BFS indices of leaves
   Buf pre_tmp; // preorder tables
@@ -213,8 +213,6 @@ struct Handle {
   Buf shift_terms; // M2M / L2L term tables (expansions.cu)
   size_t shift_at[4] = {0, 0, 0, 0};  // offsets of the four term tables
   int shift_P = -1;
-  Buf m2l_units;  // balanced contraction table for the M2L kernel (per P)
-  int m2l_units_P = -1;
 
   // grouped M2L (m2l_group.cu)
   Buf g_mt, g_ekey, g_occ, g_cnt, g_ops, g_tk, g_tile, g_seg, g_tg, g_m16, g_pairs;
@@ -233,7 +231,6 @@ struct Handle {
   double op_theta = 0;  // tensor-core operators: the acceptance test their scaling is for (TcScale)
   bool g_grouped = false;  // the group tables belong to the current lists
   int g_ntiles = 0, g_ngroups = 0, g_nseg = 0;
-  bool g_used_tc = false;
   // the grouping of the last grouped M2L (tiles, segments, operator slots),
   // valid for the same lists, P and form: a reevaluation contracts directly
   struct {
@@ -275,7 +272,7 @@ struct Handle {
 };
 
 // ---- launchers (each .cu file) ----
-// scan.cu / sort.cu
+// sort.cu
 void scan_exclusive_int(Handle &h, const int *in, int *out, long n, int *total_dev);
 void scan_exclusive_pair(Handle &h, const int *in0, int *out0, int *total0, const int *in1, int *out1, int *total1,
                          long n);

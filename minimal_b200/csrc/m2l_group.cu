@@ -1589,7 +1589,6 @@ void contract(Handle &h, bool tcore, const TcPlan &tp, int KP16, const GroupPlan
       h.launches++;
     }
     h.tc_stall_ns = 0;  // the test hook stalls one launch
-    h.g_used_tc = true;
   } else {
     // two pipeline stages where they fit in shared memory (P <= 12), else
     // one.  P <= 11: equal segment ranges over as many CTAs as fit on the GPU
@@ -1729,7 +1728,6 @@ void m2l_grouped_pass(Handle &h) {
   const long nent = h.n_m2l;
   h.L.need((size_t)C * NT * sizeof(double2));
   FMM_CUDA(cudaMemsetAsync(h.L.p, 0, (size_t)C * NT * sizeof(double2), s));
-  h.g_used_tc = false;
   if (nent == 0) return;
 
   // scaled multipoles: FP64 (DMMA) or FP16 hi/lo (tensor core)

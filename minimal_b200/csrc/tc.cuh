@@ -81,7 +81,8 @@ __device__ __forceinline__ void dealloc(uint32_t taddr, uint32_t ncols) {
 
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Generic-proxy shared-memory writes become visible to the tensor core.
+// Orders generic-proxy accesses to shared memory that this thread has observed
+// (a barrier's) before its later MMAs' reads, which go through the async proxy.
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
@@ -154,8 +155,6 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// all but the most recently committed group complete
-__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 // 32 lanes x 32 bit, 16 consecutive columns per thread.
 __device__ __forceinline__ void ld_32x32b_x16(uint32_t taddr, float *v) {

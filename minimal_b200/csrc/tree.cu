@@ -74,8 +74,9 @@ __device__ __forceinline__ void set_root(RootGeom *g, const double lo[3], const 
   g->R0 = __dmul_rn(R0, 1.00001);
 }
 
-// Bounds of one system.  The blocks' bounds go to `part`; the last block to finish combines them, and zeroes the counters for
-// the build (one launch where the combination and the zeroing took two more).
+// Bounds of one system.  The blocks' bounds go to `part`; the last block to
+// finish combines them and zeroes the counters for the build (one launch where
+// the combination and the zeroing took two more).
 __global__ void __launch_bounds__(TB) k_bounds(const double4 *in, long n, double *part, RootGeom *g, DevCounters *ctr) {
   double lo[3] = {in[0].x, in[0].y, in[0].z}, hi[3] = {lo[0], lo[1], lo[2]};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
@@ -419,9 +420,8 @@ __global__ void k_ref_leaves(BfsCells o, long c, const int *blockstart_pre, int 
   if (is_leaf[b]) leaves[leafpos[b]] = (int)b;
 }
 
-// Bodies of one leaf back into input order (warp per leaf, rank sort).
-// Bodies of each leaf back to input order (a body's slot is the rank of its
-// input index among the leaf's), gathered into src, and (3D) the body's leaf.
+// Bodies of each leaf back to input order (a warp per leaf; a body's slot is
+// the rank of its input index among the leaf's), gathered into src, and (3D) the body's leaf.
 // With srcf (3D mixed form) also the FP32 copy of each body as an offset from
 // its leaf centre (FP64 subtraction, one rounding), alone and in pairs, as
 // k_make_srcf makes them: one pass over the bodies instead of three.
