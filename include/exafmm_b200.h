@@ -233,8 +233,8 @@ EXAFMM_API int exafmm_b200_set_batch(exafmm_b200 *h, const double *bodies8, cons
  * batch) for each candidate leaf size ncrit (NULL = 32, 48, 64, 96, 128,
  * 192, 256), `repeats` timed runs each after one warm-up, keeps the fastest
  * in the handle's parameters, then at that leaf size times the near-field
- * source tiles (EXAFMM_TILE_P2P_STAGE 1024, 1536, 2048) and keeps the
- * fastest, and leaves the results of the chosen setting in the handle.  ncrit
+ * source tiles (EXAFMM_TILE_P2P_STAGE: the default, which the sweep ran,
+ * 1024, 1536, 2048) and keeps the fastest, and leaves the results of the chosen setting in the handle.  ncrit
  * shapes the tree, so results after tuning are those of the chosen ncrit,
  * not of the reference's; the plain drop-in configuration keeps ncrit = 64. */
 EXAFMM_API int exafmm_b200_autotune(exafmm_b200 *h, const int *ncrit_candidates, int ncand, int repeats,
