@@ -354,13 +354,16 @@ __global__ void __launch_bounds__(128) k_p2m_cols(const int *leaves, int nleaves
 // field): per leaf, the local expansion in the leaf's units, L~_n = L_n R^n
 // with R the leaf radius rounded down to a power of two (exact), as FP32, and
 // the scale 1/R for the coordinates -- so the FP32 terms stay in range at any
-// domain size.
-__global__ void k_l2p_prep(const int *leaves, int nleaves, const double4 *xr, const double2 *L, int nt, float2 *Lf,
-                           float *lsc) {
+// domain size.  A leaf of radius 0 (one body, or bodies in one place, alone in
+// the system) takes `lone` for its radius: the period, the distance of its
+// sources.
+__global__ void k_l2p_prep(const int *leaves, int nleaves, const double4 *xr, const double2 *L, int nt, double lone,
+                           float2 *Lf, float *lsc) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long)nleaves * nt) return;
   const int w = (int)(i / nt), k = (int)(i - (long)w * nt), c = leaves[w];
-  const int ex = leaf_exponent(xr[c].w), n = order_of(k);
+  const double R = xr[c].w;
+  const int ex = leaf_exponent(R > 0 ? R : lone), n = order_of(k);
   const double2 l = L[(long)c * nt + k];
   Lf[i] = make_float2((float)scalbn(l.x, ex * n), (float)scalbn(l.y, ex * n));
   if (k == 0) lsc[w] = exp2f((float)-ex);
@@ -1093,7 +1096,7 @@ void downward_pass(Handle &h, cudaStream_t s, cudaEvent_t before_l2p) {
     Lf = h.l2p_f.as<float2>();
     lsc = (float *)(Lf + nlf);
     k_l2p_prep<<<grid_for((long)nlf, 256), 256, 0, s>>>(h.leaves.as<int>(), h.nleaves, h.c_xr.as<double4>(),
-                                                         h.L.as<double2>(), nt, Lf, lsc);
+                                                         h.L.as<double2>(), nt, h.prm.images ? h.prm.cycle : 0.0, Lf, lsc);
     h.launches++;
   }
   if (before_l2p) FMM_CUDA(cudaStreamWaitEvent(s, before_l2p, 0));

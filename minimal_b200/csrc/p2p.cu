@@ -387,8 +387,11 @@ __global__ void __launch_bounds__(CT, (F32 ? 7 : 4) * (CT_MAX / CT)) k_p2p_cta(c
   };
   const bool act = g < G;
   const double4 CA = xr[c];
-  const int sexp = CA.w > 0 ? max(-100, min(100, ilogb(CA.w))) : 0;
-  const float scale = F32 ? exp2f((float)-sexp) : 1.0f;  // FP32: R * scale in [1, 2)
+  // FP32: R * scale in [1, 2), or the period's, the distance of the sources of
+  // a leaf of radius 0 (one body, or bodies in one place, alone in the system)
+  const double unit = CA.w > 0 ? CA.w : cycle;
+  const int sexp = unit > 0 ? max(-100, min(100, ilogb(unit))) : 0;
+  const float scale = F32 ? exp2f((float)-sexp) : 1.0f;
   BT A[CT_TPT];
 #pragma unroll
   for (int u = 0; u < CT_TPT; u++) {
